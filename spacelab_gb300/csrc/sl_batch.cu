@@ -208,45 +208,21 @@ __device__ void make_view(System& v, const Batch& b, int inst, int off, int n)
 }
 
 template <bool WRITE>
-__device__ double exact_tile_pass(const System& s, ABlock* blocks)
+__device__ double exact_tile_pass(const System& s, TileScratch* scratch)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    ABlock& ab = blocks[warp];
+    TileScratch& ws = scratch[warp];
     const int n = s.n;
-    const double Ha = s.mat.Ha;
-    const long long h_min_bits = __double_as_longlong(s.mat.h_min);  // h_min > 0
     double pe = 0;
     for (long long t = warp; t < s.ntiles; t += nwarps) {
         int X, Y;
         tile_coords(t, X, Y);
-        {
-            const int i = min(X * kBlock + lane, n - 1);  // padding rows repeat the last sphere (never paired)
-            ab.x[lane] = s.pos.c[0][i]; ab.y[lane] = s.pos.c[1][i]; ab.z[lane] = s.pos.c[2][i];
-            ab.R[lane] = s.R[i]; ab.twoR[lane] = s.twoR[i]; ab.fourR[lane] = s.fourR[i];
-            ab.cR3[lane] = s.cR3[i]; ab.m[lane] = s.m[i]; ab.rm[lane] = s.rm[i];
-        }
+        load_a(s, ws.ab, lane, min(X * kBlock + lane, n - 1));  // padding rows repeat the last sphere (never paired)
         __syncwarp();
         const int B = Y * kBlock + lane;
-        const bool bvalid = B < n;
-        const int Bc = min(B, n - 1);
-        const double bx = s.pos.c[0][Bc], by = s.pos.c[1][Bc], bz = s.pos.c[2][Bc];
-        const double Rb = s.R[Bc], twoRb = s.twoR[Bc], mb = s.m[Bc];
-        const unsigned long long rmb = s.rm[Bc];
-        const double R0 = ab.R[0];
-        const bool uni = __all_sync(0xffffffffu, ab.R[lane] == R0 && Rb == R0);
-        const double twoR0 = ab.twoR[0], sum0 = R0 + R0, c40 = ab.fourR[0] * R0;
-        const double P0 = ab.cR3[0] * R0 * R0 * R0;
-        const int a_end = min(kBlock, n - X * kBlock);
-        uint32_t rowbits = 0, colbits = 0;
-        double* rowA = s.pairbuf + (size_t)(X * kBlock) * s.npad + B;  // + a*npad: term for A
-        double* rowB = s.pairbuf + (size_t)B * s.npad + X * kBlock;    // + a: term for B
-        const TileUniform tu{R0, twoR0, sum0, c40, P0};
-        if (uni)
-            tile_pairs<WRITE, true>(s, ab, X, Y, lane, a_end, bx, by, bz, Rb, twoRb, mb, rmb, bvalid, tu, h_min_bits,
-                                    Ha, rowA, rowB, pe, rowbits, colbits);
-        else
-            tile_pairs<WRITE, false>(s, ab, X, Y, lane, a_end, bx, by, bz, Rb, twoRb, mb, rmb, bvalid, tu, h_min_bits,
-                                     Ha, rowA, rowB, pe, rowbits, colbits);
+        uint32_t rowbits, colbits;
+        tile_pairs<WRITE>(s, ws, X, Y, lane, 0, min(kBlock, n - X * kBlock), min(B, n - 1), B < n, pe, rowbits,
+                          colbits);
         if (X == Y) {
             s.cmask[(size_t)(X * kBlock + lane) * s.nb + X] = rowbits | colbits;
         } else {
@@ -292,7 +268,8 @@ __global__ void __launch_bounds__(32 * kExactTileWarps) batch_exact_tiles_kernel
                                                                                 int first_step, int nsteps, int skip,
                                                                                 int do_init)
 {
-    __shared__ ABlock blocks[kExactTileWarps];
+    extern __shared__ __align__(16) unsigned char tile_raw[];
+    TileScratch* scratch = reinterpret_cast<TileScratch*>(tile_raw);  // one per warp
     __shared__ System sv;
     __shared__ double sh[8][32];
     __shared__ int s_next;
@@ -311,7 +288,7 @@ __global__ void __launch_bounds__(32 * kExactTileWarps) batch_exact_tiles_kernel
         if (do_init) {
             drift(b, off, n, 0.0);
             __syncthreads();
-            const double pe = exact_tile_pass<true>(sv, blocks);
+            const double pe = exact_tile_pass<true>(sv, scratch);
             __syncthreads();
             exact_row_sums(sv);
             __syncthreads();
@@ -325,9 +302,9 @@ __global__ void __launch_bounds__(32 * kExactTileWarps) batch_exact_tiles_kernel
             __syncthreads();
             double pe = 0;
             if (write)
-                pe = exact_tile_pass<true>(sv, blocks);
+                pe = exact_tile_pass<true>(sv, scratch);
             else
-                exact_tile_pass<false>(sv, blocks);
+                exact_tile_pass<false>(sv, scratch);
             __syncthreads();
             exact_row_sums(sv);
             __syncthreads();
@@ -366,11 +343,24 @@ void launch_batch_derive(const Batch& b, cudaStream_t st)
     batch_derive_kernel<<<(b.total + 255) / 256, 256, 0, st>>>(b);
 }
 
+// Dynamic shared memory of the pair-tile pass (above the 48 KB that need no
+// opt-in at eight warps); the attribute belongs to the current device's
+// context, and setting it is a host-side table update.
+static size_t exact_tiles_smem(int threads)
+{
+    cudaFuncSetAttribute(batch_exact_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kExactTileWarps * (int)sizeof(TileScratch));
+    return (size_t)(threads / 32) * sizeof(TileScratch);
+}
+
 void launch_batch_exact(const Batch& b, int tile, int threads, int blocks, int first_step, int nsteps, int skip,
                         int do_init, cudaStream_t st)
 {
     switch (tile) {
-        case 0: batch_exact_tiles_kernel<<<blocks, threads, 0, st>>>(b, first_step, nsteps, skip, do_init); break;
+        case 0:
+            batch_exact_tiles_kernel<<<blocks, threads, exact_tiles_smem(threads), st>>>(b, first_step, nsteps, skip,
+                                                                                        do_init);
+            break;
         case 32: batch_exact_kernel<32><<<blocks, threads, 0, st>>>(b, first_step, nsteps, skip, do_init); break;
         case 64: batch_exact_kernel<64><<<blocks, threads, 0, st>>>(b, first_step, nsteps, skip, do_init); break;
         default: batch_exact_kernel<128><<<blocks, threads, 0, st>>>(b, first_step, nsteps, skip, do_init); break;
@@ -382,7 +372,10 @@ int batch_max_blocks_per_sm(int tile, int threads, bool mixed)
     if (mixed) return batch_mixed_max_blocks_per_sm(tile, threads);
     int nb = 0;
     switch (tile) {
-        case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_exact_tiles_kernel, threads, 0); break;
+        case 0:
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_exact_tiles_kernel, threads,
+                                                          exact_tiles_smem(threads));
+            break;
         case 32: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_exact_kernel<32>, threads, 0); break;
         case 64: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_exact_kernel<64>, threads, 0); break;
         default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_exact_kernel<128>, threads, 0); break;

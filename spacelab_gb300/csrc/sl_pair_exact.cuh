@@ -32,20 +32,6 @@ __device__ __forceinline__ double vdw_coef_fix(double h, double Ra, double Rb, d
     return cR3a * Rb * Rb * Rb * div_by_fixed<true>(h + Ra + Rb, den, recip_newton(den));
 }
 
-// vdw_coef_fix for a pair of equal radii R (Ra == Rb bit for bit), with the
-// pair-independent products hoisted: c4 = fourR * R and
-// P = ((cR3 * R) * R) * R.  Every remaining operation is the general
-// form's, in its order, so the result is the same bits.
-__device__ __forceinline__ double vdw_coef_uniform(double h, double R, double twoR, double c4, double P)
-{
-    const double h2 = h * h;
-    const double t = twoR * h;      // twoRa * h == twoRb * h
-    const double S = h2 + t + t;
-    const double T = S + c4;
-    const double den = S * S * T * T;
-    return P * div_by_fixed<true>(h + R + R, den, recip_newton(den));
-}
-
 // U_vdw of ColliderSingleCore.cpp:195-202 / :231-238.
 __device__ __forceinline__ double vdw_energy(double Ha, double h, double Ra, double Rb, double twoRa)
 {

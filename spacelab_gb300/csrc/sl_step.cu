@@ -77,8 +77,9 @@ __device__ __forceinline__ long long col_offset(int nb, int c) { return (long lo
 
 __device__ __forceinline__ void col_tile_coords(int nb, long long u, int& X, int& Y)
 {
-    const double b = 2.0 * nb + 1.0;
-    int c = (int)((b - sqrt(b * b - 8.0 * (double)u)) * 0.5);
+    // FP32 estimate (the FP64 pipe is what the kernel is short of), corrected exactly below
+    const float b = 2.0f * nb + 1.0f;
+    int c = (int)((b - sqrtf(fmaxf(b * b - 8.0f * (float)u, 0.0f))) * 0.5f);
     c = max(0, min(c, nb - 1));
     while (c + 1 < nb && col_offset(nb, c + 1) <= u) ++c;
     while (c > 0 && col_offset(nb, c) > u) --c;
@@ -90,14 +91,11 @@ template <bool WRITE>
 __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
                                                           int phase)
 {
-    __shared__ ABlock sA[4];
-    __shared__ double sB[4][kBStageDoubles];
+    __shared__ TileScratch scratch[4];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    ABlock& ab = sA[wib];
+    TileScratch& ws = scratch[wib];
     const long long nwarps = (long long)gridDim.x * 4;
-    const double Ha = s.mat.Ha;
-    const long long h_min_bits = __double_as_longlong(s.mat.h_min);  // h_min > 0
 
     // A first round of tiles in warp order; then whichever warp is free takes
     // the next tile from the launch's counter (zeroed by the drift kernel),
@@ -109,35 +107,12 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
         int X, Y;
         col_tile_coords(s.nb, u, X, Y);
         const long long t = (long long)X * (X + 1) / 2 + Y;  // this tile's PE slot
-        {
-            const int i = X * kBlock + lane;  // < npad always
-            ab.x[lane] = s.pos.c[0][i]; ab.y[lane] = s.pos.c[1][i]; ab.z[lane] = s.pos.c[2][i];
-            ab.R[lane] = s.R[i]; ab.twoR[lane] = s.twoR[i]; ab.fourR[lane] = s.fourR[i];
-            ab.cR3[lane] = s.cR3[i]; ab.m[lane] = s.m[i]; ab.rm[lane] = s.rm[i];
-        }
+        load_a(s, ws.ab, lane, X * kBlock + lane);  // < npad always
         __syncwarp();
         const int B = Y * kBlock + lane;
-        const bool bvalid = B < s.n;
-        const double bx = s.pos.c[0][B], by = s.pos.c[1][B], bz = s.pos.c[2][B];
-        const double Rb = s.R[B], twoRb = s.twoR[B], mb = s.m[B];
-        const unsigned long long rmb = s.rm[B];
-        const double R0 = ab.R[0];
-        const bool uni = __all_sync(0xffffffffu, ab.R[lane] == R0 && Rb == R0);
-        const double twoR0 = ab.twoR[0], sum0 = R0 + R0, c40 = ab.fourR[0] * R0;
-        const double P0 = ab.cR3[0] * R0 * R0 * R0;
-        const int a_end = min(kBlock, s.n - X * kBlock);
         double pe = 0;
-        uint32_t rowbits = 0, colbits = 0;
-        double* rowA = s.pairbuf + (size_t)(X * kBlock) * s.npad + B;  // + a*npad: term for A
-        double* rowB = s.pairbuf + (size_t)B * s.npad + X * kBlock;    // + a: term for B
-
-        const TileUniform tu{R0, twoR0, sum0, c40, P0};
-        if (uni)
-            tile_pairs<WRITE, true>(s, ab, X, Y, lane, a_end, bx, by, bz, Rb, twoRb, mb, rmb, bvalid, tu, h_min_bits,
-                                    Ha, rowA, rowB, pe, rowbits, colbits, sB[wib]);
-        else
-            tile_pairs<WRITE, false>(s, ab, X, Y, lane, a_end, bx, by, bz, Rb, twoRb, mb, rmb, bvalid, tu, h_min_bits,
-                                     Ha, rowA, rowB, pe, rowbits, colbits, sB[wib]);
+        uint32_t rowbits, colbits;
+        tile_pairs<WRITE>(s, ws, X, Y, lane, 0, min(kBlock, s.n - X * kBlock), B, B < s.n, pe, rowbits, colbits);
         // Contact bits: row A = 32X + lane gets block Y's bits, row B gets
         // block X's bits; on the diagonal both describe row 32X + lane.
         if (X == Y) {

@@ -3,10 +3,27 @@
 // orientation A > B), shared by the single-system pair kernel (sl_step.cu)
 // and the batched exact solver's pair-tile pass (sl_batch.cu).  Must be
 // compiled with --fmad=false (the exact arithmetic contract).
+//
+// Two passes per tile.  The sweep walks the A block and evaluates every pair
+// by the branch-free integer path (sl_pair_fast.cuh).  Pairs in contact, and
+// pairs whose rounding that path leaves open (about 4%), are marked; after
+// the sweep their (A, B) are packed into a list and evaluated 32 at a time by
+// the general path, one pair per lane.  A contact costs ~10,000 cycles of
+// dependent FP64 divisions and square roots: inside the sweep each row with
+// one held the whole warp for that long, which set the time of small systems
+// (N=96: 117 us for six tiles).
+//
+// What bounds it (N=5000, GB300, ncu): with every add and product on the FP64
+// pipe that pipe was the limit; now no unit is -- FP64 62% of its nominal
+// cycles (14 operations of a warp's 32 pairs), ALU 54%, the integer
+// multiplier (fmaheavy) 58%, issue 53%, at 16 warps per SM.  Pair kernel per
+// step: 0.775 ms with quotients rounded by exact remainders, 0.632 ms with
+// the unpacked path's divisions alone, 0.478 ms with its products too.
 #pragma once
 #include "sl_device.cuh"
 #include "sl_fp64_exact.cuh"
 #include "sl_pair_exact.cuh"
+#include "sl_pair_fast.cuh"
 #include "sl_vdw_energy.cuh"
 
 namespace sl {
@@ -17,13 +34,6 @@ struct ABlock {
     unsigned long long rm[kBlock];
 };
 
-// Equal radii across a tile (monodisperse clusters): the sum of radii and
-// the vdW coefficient's radius products are the same for every pair of the
-// tile and are formed once (vdw_coef_uniform).
-struct TileUniform {
-    double R0, twoR0, sum0, c40, P0;
-};
-
 // Per-warp shared staging of sphere B's terms (lane = B) for four
 // consecutive partners: [component][lane][4 + 1 padding] doubles, so that a
 // lane's 8-byte accesses at a 40-byte stride fall in distinct banks per
@@ -32,116 +42,244 @@ constexpr int kBStageRow = 5;
 constexpr int kBStagePlane = kBlock * kBStageRow;
 constexpr int kBStageDoubles = 3 * kBStagePlane;
 
-// The pairs of one tile (X, Y) for lane = sphere B: terms to pairbuf and
-// torqbuf, contact bits to rowbits/colbits, PE (write steps) to pe.
-// bstage (kBStageDoubles per warp, or NULL): off the diagonal, sphere B's
-// terms -- which go to B's own row of pairbuf, a different row per lane --
-// are gathered four at a time and written as whole 32-byte sectors (two
-// 16-byte stores per component) instead of one 8-byte store per term from
-// 32 rows at once; partners past the last sphere are written as +0.0, the
-// value those entries hold anyway.  On the diagonal tile, and with NULL,
-// every term is stored as it is computed.
-template <bool WRITE, bool UNI>
-__device__ __forceinline__ void tile_pairs(const System& s, const ABlock& ab, int X, int Y, int lane, int a_end,
-                                           double bx, double by, double bz, double Rb, double twoRb, double mb,
-                                           unsigned long long rmb, bool bvalid, const TileUniform& tu,
-                                           long long h_min_bits, double Ha, double* rowA, double* rowB,
-                                           double& pe, uint32_t& rowbits, uint32_t& colbits,
-                                           double* bstage = nullptr)
+// One warp's shared memory.  The list of marked pairs (at most 32 x 32
+// entries of 16 bits) takes the B staging's place after the sweep.
+struct TileScratch {
+    ABlock ab;
+    double bstage[kBStageDoubles];
+    uint32_t rowc[kBlock], colc[kBlock];  // contact bits found by the general path
+};
+static_assert(sizeof(double) * kBStageDoubles >= kBlock * kBlock * sizeof(uint16_t), "list fits in the staging");
+
+// One pair by the general path: rounds every quotient and root by its exact
+// remainder (sl_fp64_exact.cuh), with the hardware operations behind it, for
+// any operands; contact or not.
+template <bool WRITE>
+__device__ __forceinline__ bool general_pair(const System& s, const ABlock& ab, int X, int a, int B, double& pe)
 {
     const size_t plane = (size_t)s.npad * s.npad;
+    const int A = X * kBlock + a;
+    const double Ra = ab.R[a], Rb = s.R[B], twoRb = s.twoR[B], mb = s.m[B];
+    const double sumRaRb = Ra + Rb;                                                   // :104
+    const double rx = s.pos.c[0][B] - ab.x[a], ry = s.pos.c[1][B] - ab.y[a], rz = s.pos.c[2][B] - ab.z[a];  // :105
+    const double d2 = rx * rx + ry * ry + rz * rz;
+    int p;
+    unsigned long long F;
+    const unsigned long long Yr = rsqrt_fix(d2, p, F);            // ~1/sqrt(d2), integer pipe
+    const double dist = sqrt_fix(d2, F, Yr, p);                   // :107, RN(sqrt)
+    const double overlap = sumRaRb - dist;                        // :110
+    // the comparisons of the step are made on the bit patterns (integer
+    // pipe): for doubles of one sign the integer order is the FP order; NaN
+    // is excluded explicitly
+    const long long ob = __double_as_longlong(overlap);
+    const bool contact = ob > 0 && ob <= 0x7ff0000000000000ll;    // overlap > 0
+    double fx, fy, fz;
+    if (contact) {
+        const ContactIn in = gather_contact(s, A, B);
+        const ContactOut o = contact_pair_exact<WRITE>(in, s.mat, rx, ry, rz, dist, overlap, Ra, Rb, ab.twoR[a],
+                                                       twoRb, ab.fourR[a], ab.cR3[a]);
+        fx = o.fx; fy = o.fy; fz = o.fz;
+        const double im_a = s.inv_moi[A], mo_a = s.moi[A];
+        const double im_b = s.inv_moi[B], mo_b = s.moi[B];
+        double* ta = s.torqbuf + (size_t)A * s.npad + B;   // :187
+        double* tb = s.torqbuf + (size_t)B * s.npad + A;   // :188
+        ta[0] = div_by_recip(o.tax, mo_a, im_a);
+        ta[plane] = div_by_recip(o.tay, mo_a, im_a);
+        ta[2 * plane] = div_by_recip(o.taz, mo_a, im_a);
+        tb[0] = div_by_recip(o.tbx, mo_b, im_b);
+        tb[plane] = div_by_recip(o.tby, mo_b, im_b);
+        tb[2 * plane] = div_by_recip(o.tbz, mo_b, im_b);
+        if (WRITE) pe += o.pe;
+    } else {
+        long long hb = ob & 0x7fffffffffffffffll;                  // :211-215 |overlap|
+        const long long h_min_bits = __double_as_longlong(s.mat.h_min);
+        if (hb < h_min_bits) hb = h_min_bits;                      // h < h_min (NaN stays NaN)
+        const double h = __longlong_as_double(hb);
+        const double coef = vdw_coef_fix(h, Ra, Rb, ab.twoR[a], twoRb, ab.fourR[a], ab.cR3[a]);
+        fx = coef * div_by_rsqrt(rx, dist, Yr, p);                    // :221-227
+        fy = coef * div_by_rsqrt(ry, dist, Yr, p);
+        fz = coef * div_by_rsqrt(rz, dist, Yr, p);
+        if (WRITE) pe += vdw_energy_far_df(s.mat.Ha, h, Ra, Rb, ab.twoR[a]);          // :239
+    }
+    // :249-250 -- acc[A] += F/m[A]; acc[B] -= F/m[B] (stored negated)
+    const double ma = ab.m[a];
+    const unsigned long long rma = ab.rm[a], rmb = s.rm[B];
+    double* pa = s.pairbuf + (size_t)A * s.npad + B;
+    double* pb = s.pairbuf + (size_t)B * s.npad + A;
+    __stcs(pa, div_by_fixed<false>(fx, ma, rma));
+    __stcs(pa + plane, div_by_fixed<false>(fy, ma, rma));
+    __stcs(pa + 2 * plane, div_by_fixed<false>(fz, ma, rma));
+    __stcs(pb, div_by_fixed<false, true>(fx, mb, rmb));
+    __stcs(pb + plane, div_by_fixed<false, true>(fy, mb, rmb));
+    __stcs(pb + 2 * plane, div_by_fixed<false, true>(fz, mb, rmb));
+    return contact;
+}
+
+// The marked pairs of a tile (lane's bit a = pair (32X + a, 32Y + lane)),
+// packed and evaluated one per lane; rowbits/colbits get the contacts.  Out
+// of line: the sweep's registers are dead here.
+template <bool WRITE>
+__device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, int X, int Y, uint32_t marked)
+{
+    const int lane = threadIdx.x & 31;
+    double pe = 0;
+    uint16_t* list = reinterpret_cast<uint16_t*>(ws.bstage);
+    ws.rowc[lane] = 0;
+    ws.colc[lane] = 0;
+    const int cnt = __popc(marked);
+    int at = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, at, 31);
+    at -= cnt;
+    __syncwarp();  // the staging's last reads are done
+    for (uint32_t w = marked; w; w &= w - 1) list[at++] = (uint16_t)(((__ffs(w) - 1) << 5) | lane);
+    __syncwarp();
+    for (int e = lane; e < total; e += 32) {
+        const int a = list[e] >> 5, b = list[e] & 31;
+        if (general_pair<WRITE>(s, ws.ab, X, a, Y * kBlock + b, pe)) {
+            atomicOr(&ws.rowc[a], 1u << b);
+            atomicOr(&ws.colc[b], 1u << a);
+        }
+    }
+    __syncwarp();
+    return pe;
+}
+
+// The tile (X, Y) for lane = sphere B = 32Y + lane, partners A = 32X + a for
+// a in [a0, a1) (a0 a multiple of 4): terms to pairbuf and torqbuf, contact
+// bits to rowbits (row A = 32X + lane) and colbits (row B), PE (write steps)
+// to pe.  ws.ab must hold the A block.
+//
+// Off the diagonal, sphere B's terms -- which go to B's own row of pairbuf, a
+// different row per lane -- are gathered four at a time in ws.bstage and
+// written as whole 32-byte sectors (two 16-byte stores per component) instead
+// of one 8-byte store per term from 32 rows at once; partners past the last
+// sphere are written as +0.0, the value those entries hold anyway.  The
+// diagonal tile stores every term as it is computed, because its B-side and
+// A-side terms share rows.
+//
+// UNI: all 64 spheres have one radius and one mass (monodisperse clusters).
+// The radius products are formed once, and sphere B's term is the negation
+// of sphere A's (RN(-x) = -RN(x)).  Every remaining operation is the general
+// form's, in its order.
+template <bool WRITE, bool UNI>
+__device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
+                                            double bx, double by, double bz, const pf::Sphere& sb,
+                                            const pf::Uniform& un, bool bvalid, double& pe, uint32_t& marked)
+{
+    const ABlock& ab = ws.ab;
+    const size_t plane = (size_t)s.npad * s.npad;
     const int B = Y * kBlock + lane;
-    const bool staged = bstage != nullptr && X != Y;
-    double* my_stage = staged ? bstage + lane * kBStageRow : nullptr;
-    for (int a = 0; a < a_end; ++a) {
+    const long long h_min_bits = __double_as_longlong(s.mat.h_min);
+    const bool staged = X != Y;
+    double* my_stage = ws.bstage + lane * kBStageRow;
+    double* rowA = s.pairbuf + (size_t)(X * kBlock) * s.npad + B;  // + a*npad: term for A
+    double* rowB = s.pairbuf + (size_t)B * s.npad + X * kBlock;    // + a: term for B
+    for (int a = a0; a < a1; ++a) {
         const bool valid = bvalid && (X != Y || lane < a);
-        bool contact = false;
+        pf::Sphere sa;
+        if (UNI) {
+            sa = sb;
+        } else {
+            sa.R = ab.R[a];
+            sa.sR = pf::unpack(sa.R);
+            sa.cR3 = ab.cR3[a];
+            sa.rm = ab.rm[a];
+            sa.em = pf::unpack(ab.m[a]).e;
+        }
+        const pf::Pair pr = pf::pair_terms<UNI>(bx - ab.x[a], by - ab.y[a], bz - ab.z[a], sa, sb, un, h_min_bits);
+        // contact (overlap > 0), or a result this path does not settle: the
+        // general path writes these entries after the sweep
+        const bool mark = valid && (__double_as_longlong(pr.overlap) > 0 || !pr.fl.sure());
+        if (mark) marked |= 1u << a;
+        if (WRITE) {
+            if (valid && !mark) pe += vdw_energy_far_df(s.mat.Ha, pr.h, sa.R, sb.R, 2 * sa.R);  // :239
+        }
         if (valid) {
-            const int A = X * kBlock + a;
-            const double Ra = ab.R[a];
-            const double sumRaRb = UNI ? tu.sum0 : Ra + Rb;              // :104
-            const double rx = bx - ab.x[a], ry = by - ab.y[a], rz = bz - ab.z[a];  // :105
-            const double d2 = rx * rx + ry * ry + rz * rz;
-            int p;
-            unsigned long long F;
-            const unsigned long long Yr = rsqrt_fix(d2, p, F);            // ~1/sqrt(d2), integer pipe
-            const double dist = sqrt_fix(d2, F, Yr, p);                   // :107, RN(sqrt)
-            const double overlap = sumRaRb - dist;                        // :110
-            // the comparisons of the step are made on the bit patterns
-            // (integer pipe): for doubles of one sign the integer order
-            // is the FP order; NaN is excluded explicitly
-            const long long ob = __double_as_longlong(overlap);
-            double fx, fy, fz;
-            if (ob > 0 && ob <= 0x7ff0000000000000ll) {                    // overlap > 0
-                contact = true;
-                const ContactIn in = gather_contact(s, A, B);
-                const ContactOut o = contact_pair_exact<WRITE>(in, s.mat, rx, ry, rz, dist, overlap, Ra, Rb,
-                                                               ab.twoR[a], twoRb, ab.fourR[a], ab.cR3[a]);
-                fx = o.fx; fy = o.fy; fz = o.fz;
-                const double im_a = s.inv_moi[A], mo_a = s.moi[A];
-                const double im_b = s.inv_moi[B], mo_b = s.moi[B];
-                double* ta = s.torqbuf + (size_t)A * s.npad + B;   // :187
-                double* tb = s.torqbuf + (size_t)B * s.npad + A;   // :188
-                ta[0] = div_by_recip(o.tax, mo_a, im_a);
-                ta[plane] = div_by_recip(o.tay, mo_a, im_a);
-                ta[2 * plane] = div_by_recip(o.taz, mo_a, im_a);
-                tb[0] = div_by_recip(o.tbx, mo_b, im_b);
-                tb[plane] = div_by_recip(o.tby, mo_b, im_b);
-                tb[2 * plane] = div_by_recip(o.tbz, mo_b, im_b);
-                if (WRITE) pe += o.pe;
-            } else {
-                long long hb = ob & 0x7fffffffffffffffll;                  // :211-215 |overlap|
-                if (hb < h_min_bits) hb = h_min_bits;                      // h < h_min (NaN stays NaN)
-                const double h = __longlong_as_double(hb);
-                const double coef = UNI ? vdw_coef_uniform(h, tu.R0, tu.twoR0, tu.c40, tu.P0)
-                                        : vdw_coef_fix(h, Ra, Rb, ab.twoR[a], twoRb, ab.fourR[a], ab.cR3[a]);
-                fx = coef * div_by_rsqrt(rx, dist, Yr, p);                    // :221-227
-                fy = coef * div_by_rsqrt(ry, dist, Yr, p);
-                fz = coef * div_by_rsqrt(rz, dist, Yr, p);
-                if (WRITE) pe += vdw_energy_far_df(Ha, h, Ra, Rb, ab.twoR[a]);             // :239
-            }
-            // :249-250 -- acc[A] += F/m[A]; acc[B] -= F/m[B] (stored negated)
-            const double ma = ab.m[a];
-            const unsigned long long rma = ab.rm[a];
             double* pa = rowA + (size_t)a * s.npad;
-            __stcs(pa, div_by_fixed<false>(fx, ma, rma));
-            __stcs(pa + plane, div_by_fixed<false>(fy, ma, rma));
-            __stcs(pa + 2 * plane, div_by_fixed<false>(fz, ma, rma));
-            // -(F/m[B]), the sign set in the integer result
-            const double tbx = div_by_fixed<false, true>(fx, mb, rmb);
-            const double tby = div_by_fixed<false, true>(fy, mb, rmb);
-            const double tbz = div_by_fixed<false, true>(fz, mb, rmb);
+            __stcs(pa, pr.ta[0]);
+            __stcs(pa + plane, pr.ta[1]);
+            __stcs(pa + 2 * plane, pr.ta[2]);
             if (staged) {
                 double* st = my_stage + (a & 3);
-                st[0] = tbx;
-                st[kBStagePlane] = tby;
-                st[2 * kBStagePlane] = tbz;
+                st[0] = pr.tb[0];
+                st[kBStagePlane] = pr.tb[1];
+                st[2 * kBStagePlane] = pr.tb[2];
             } else {
                 double* pb = rowB + a;
-                __stcs(pb, tbx);
-                __stcs(pb + plane, tby);
-                __stcs(pb + 2 * plane, tbz);
+                __stcs(pb, pr.tb[0]);
+                __stcs(pb + plane, pr.tb[1]);
+                __stcs(pb + 2 * plane, pr.tb[2]);
             }
         }
-        const uint32_t bal = __ballot_sync(0xffffffffu, contact);
-        if (lane == a) rowbits = bal;
-        if (contact) colbits |= 1u << a;
-        if (staged && bvalid && ((a & 3) == 3 || a == a_end - 1)) {
-            // row B, partners a0 .. a0+3: a 32-byte aligned sector (npad and
+        if (staged && bvalid && ((a & 3) == 3 || a == a1 - 1)) {
+            // row B, partners q0 .. q0+3: a 32-byte aligned sector (npad and
             // 32X are multiples of 4, the buffer is 256-byte aligned)
-            const int a0 = a & ~3;
+            const int q0 = a & ~3;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const double* st = my_stage + c * kBStagePlane;
                 const double v0 = st[0];
-                const double v1 = a0 + 1 < a_end ? st[1] : 0.0;
-                const double v2 = a0 + 2 < a_end ? st[2] : 0.0;
-                const double v3 = a0 + 3 < a_end ? st[3] : 0.0;
-                double2* dst = reinterpret_cast<double2*>(rowB + c * plane + a0);
+                const double v1 = q0 + 1 < a1 ? st[1] : 0.0;
+                const double v2 = q0 + 2 < a1 ? st[2] : 0.0;
+                const double v3 = q0 + 3 < a1 ? st[3] : 0.0;
+                double2* dst = reinterpret_cast<double2*>(rowB + c * plane + q0);
                 __stcs(dst, make_double2(v0, v1));
                 __stcs(dst + 1, make_double2(v2, v3));
             }
         }
+    }
+}
+
+// Loads sphere i into lane's place of the A block.
+__device__ __forceinline__ void load_a(const System& s, ABlock& ab, int lane, int i)
+{
+    ab.x[lane] = s.pos.c[0][i]; ab.y[lane] = s.pos.c[1][i]; ab.z[lane] = s.pos.c[2][i];
+    ab.R[lane] = s.R[i]; ab.twoR[lane] = s.twoR[i]; ab.fourR[lane] = s.fourR[i];
+    ab.cR3[lane] = s.cR3[i]; ab.m[lane] = s.m[i]; ab.rm[lane] = s.rm[i];
+}
+
+// Partners a0 .. a1 - 1 of the tile (X, Y), the A block loaded: the sweep, or
+// where a constant leaves the integer path's range (no cohesion: cR3 = 0;
+// masses far from 1) the general path for every pair, then the marked pairs.
+template <bool WRITE>
+__device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
+                                           int iB, bool bvalid, double& pe, uint32_t& rowbits, uint32_t& colbits)
+{
+    const ABlock& ab = ws.ab;
+    const double bx = s.pos.c[0][iB], by = s.pos.c[1][iB], bz = s.pos.c[2][iB];
+    const double Rb = s.R[iB], mb = s.m[iB];
+    const pf::Sphere sb{Rb, pf::unpack(Rb), s.cR3[iB], s.rm[iB], pf::unpack(mb).e};
+    const bool areal = X * kBlock + lane < s.n;  // padding takes no part in a pair
+    const pf::Sphere sa{ab.R[lane], pf::unpack(ab.R[lane]), ab.cR3[lane], 0, pf::unpack(ab.m[lane]).e};
+    const bool sane = __all_sync(0xffffffffu, (!areal || (pf::in_range(sa) && pf::in_range_cR3(sa.cR3))) &&
+                                                  (!bvalid || pf::in_range(sb)));
+    // equality on the bit patterns (R, m > 0)
+    const auto same = [](double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); };
+    const double R0 = ab.R[0], m0 = ab.m[0];
+    const bool uni = __all_sync(0xffffffffu, (!areal || (same(sa.R, R0) && same(ab.m[lane], m0))) &&
+                                                 (!bvalid || (same(Rb, R0) && same(mb, m0))));
+    uint32_t marked = 0;
+    if (!sane) {
+        const uint32_t all = (a1 >= 32 ? ~0u : (1u << a1) - 1u) & ~((1u << a0) - 1u);
+        marked = bvalid ? (X != Y ? all : all & ~((2u << lane) - 1u)) : 0u;
+    } else if (uni) {
+        const pf::Uniform un{R0 + R0, ab.fourR[0] * R0, pf::unpack(ab.cR3[0] * R0 * R0 * R0)};
+        sweep_pairs<WRITE, true>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked);
+    } else {
+        const pf::Uniform un{0.0, 0.0, {0, 0}};
+        sweep_pairs<WRITE, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked);
+    }
+    rowbits = colbits = 0;
+    if (__any_sync(0xffffffffu, marked != 0u)) {
+        pe += general_pairs<WRITE>(s, ws, X, Y, marked);
+        rowbits = ws.rowc[lane];
+        colbits = ws.colc[lane];
+        __syncwarp();
     }
 }
 
