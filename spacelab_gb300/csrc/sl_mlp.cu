@@ -339,6 +339,237 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
 }
 
+// ----------------------------------------------- the whole forward pass --
+// The network's outputs for n rows in one launch.  A CTA takes 128 rows at a
+// time through every layer: the bf16 activations stay in shared memory (64
+// KB: up to 256 columns in 64-column chunks, the 128-byte-swizzled K-major
+// layout the MMA reads), the accumulator in 256 columns of tensor memory, and
+// the weights stream from L2 in 128 x 64 tiles (16 KB) through a ring of
+// three.  Six warps: four for the epilogues (a thread is a row: TMEM lane ->
+// bias, GELU, bf16 -> the next layer's operand), one issues the MMAs, one the
+// copies.  114,944 bytes of shared memory and 256 of the 512 TMEM columns let
+// two CTAs share an SM, so that one's MMAs and copies run under the other's
+// epilogue, which is what bounds the pass: 1024 erff per row, ~40
+// instructions each.  Rows are read and results written where the caller has
+// them.  The products are accumulated K chunk by K chunk as the
+// layer-by-layer kernel does, so the outputs are the same bits.
+//
+// Measured (GB300, 8-256x4-4, host arrays in and out): 1,000,000 rows 272 ->
+// 1.72 ms, 1000 rows 289 -> 67 us, 1 row 132 -> 68 us, against a batch of
+// 1024 rows at a time through six launches and three blocking copies, with
+// the epilogue's stores one row per lane (55 of a layer's 58 us).
+constexpr int kFwRows = 128, kFwMaxWidth = 256, kFwMaxLayers = 8, kFwStages = 3, kFwTileN = 128;
+constexpr int kFwXBytes = kFwRows * kFwMaxWidth * 2, kFwWBytes = kFwTileN * kTcK * 2;
+constexpr int kFwThreads = 192, kFwEpilogue = 128;
+constexpr int kFwSmem = kFwXBytes + kFwStages * kFwWBytes + 256;  // + barriers, TMEM address, failure flag
+
+struct FwNet {
+    CUtensorMap w[kFwMaxLayers];            // weights [dout][din], boxes of 64 x 128
+    const float* bias[kFwMaxLayers];
+    int din[kFwMaxLayers], dout[kFwMaxLayers];
+    int layers, n_in, n_out;
+};
+
+// Waits like mbar_wait, and gives up at once when another thread of the CTA has.
+__device__ __forceinline__ bool fw_wait(uint64_t* bar, uint32_t parity, volatile int* failed)
+{
+    if (sl::tma::mbar_test(bar, parity)) return true;
+    const long long t0 = clock64();
+    while (!sl::tma::mbar_test(bar, parity))
+        if (*failed || clock64() - t0 > sl::tma::kWaitCycles) {
+            *failed = 1;
+            return false;
+        }
+    return true;
+}
+
+__device__ __forceinline__ uint32_t bf16x2(float a, float b)
+{
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);  // a in the low half
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// byte of row r's 16-byte group g (8 columns) of the activations
+__device__ __forceinline__ int fw_x_offset(int r, int g) { return (g >> 3) * (kFwRows * 128) + r * 128 + (((g & 7) ^ (r & 7)) << 4); }
+
+__global__ void __launch_bounds__(kFwThreads, 2) mlp_forward_kernel(const __grid_constant__ FwNet net,
+                                                                    const float* __restrict__ x, float* y, int n,
+                                                                    int* err)
+{
+    extern __shared__ __align__(1024) unsigned char fw_raw[];
+    unsigned char* sx = fw_raw;
+    unsigned char* sw = fw_raw + kFwXBytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(sw + kFwStages * kFwWBytes);
+    uint64_t* empty = full + kFwStages;
+    uint64_t* acc_done = empty + kFwStages;   // a layer's MMAs have completed
+    uint64_t* x_ready = acc_done + 1;         // a layer's operand is in shared memory
+    uint64_t* drain = x_ready + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+    volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ntiles = (n + kFwRows - 1) / kFwRows;
+    // whole 16-byte groups of the caller's rows
+    const bool vec_in = net.n_in % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    const bool vec_out = net.n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
+
+    if (tid == 0) {
+        for (int k = 0; k < kFwStages; ++k) {
+            sl::tma::mbar_init(&full[k], 1);
+            sl::tma::mbar_init(&empty[k], 1);
+        }
+        sl::tma::mbar_init(acc_done, 1);
+        sl::tma::mbar_init(x_ready, kFwEpilogue);
+        sl::tma::mbar_init(drain, 1);
+        *failed = 0;
+        sl::tma::fence_barrier_init();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                     ::"r"(sl::tma::smem_addr(tmem_slot)), "r"(kFwMaxWidth)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp < 4) {  // ------------------------------------------- epilogues
+        const int r = warp * 32 + lane;
+        uint32_t phase = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+            const int row = t * kFwRows + r;
+            {  // the row's features, zero up to whole K chunks
+                const float* xr = x + (size_t)row * net.n_in;
+                const int groups = (net.din[0] + kTcK - 1) / kTcK * 8;
+                for (int g = 0; g < groups; ++g) {
+                    float f[8];
+                    if (vec_in && row < n && g * 8 + 8 <= net.n_in) {
+                        const float4 lo = *reinterpret_cast<const float4*>(xr + g * 8);
+                        const float4 hi = *reinterpret_cast<const float4*>(xr + g * 8 + 4);
+                        f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w;
+                        f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) f[k] = row < n && g * 8 + k < net.n_in ? xr[g * 8 + k] : 0.0f;
+                    }
+                    *reinterpret_cast<uint4*>(sx + fw_x_offset(r, g)) =
+                        make_uint4(bf16x2(f[0], f[1]), bf16x2(f[2], f[3]), bf16x2(f[4], f[5]), bf16x2(f[6], f[7]));
+                }
+            }
+            sl::tma::fence_proxy_async();
+            sl::tma::mbar_arrive(x_ready);
+            for (int l = 0; l < net.layers; ++l) {
+                ok = fw_wait(acc_done, phase, failed);
+                phase ^= 1u;
+                if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+                tc_fence_after();
+                const float* bias = net.bias[l];
+                const int N = net.dout[l];
+                const bool last = l == net.layers - 1;
+#pragma unroll 1
+                for (int cg = 0; cg < N / 32; ++cg) {
+                    float v[32];
+                    tc_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cg * 32), v);
+                    if (last) {
+                        float* yr = y + (size_t)row * net.n_out + cg * 32;
+                        const int cols = row < n ? net.n_out - cg * 32 : 0;
+#pragma unroll
+                        for (int i = 0; i < 32; i += 4) {
+                            const float4 b = __ldg(reinterpret_cast<const float4*>(bias + cg * 32 + i));
+                            const float4 o = make_float4(v[i] + b.x, v[i + 1] + b.y, v[i + 2] + b.z, v[i + 3] + b.w);
+                            if (vec_out && i < cols) {
+                                *reinterpret_cast<float4*>(yr + i) = o;
+                            } else {
+                                if (i < cols) yr[i] = o.x;
+                                if (i + 1 < cols) yr[i + 1] = o.y;
+                                if (i + 2 < cols) yr[i + 2] = o.z;
+                                if (i + 3 < cols) yr[i + 3] = o.w;
+                            }
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const float4 b0 = __ldg(reinterpret_cast<const float4*>(bias + cg * 32 + g * 8));
+                        const float4 b1 = __ldg(reinterpret_cast<const float4*>(bias + cg * 32 + g * 8 + 4));
+                        const float* z = v + g * 8;
+                        *reinterpret_cast<uint4*>(sx + fw_x_offset(r, cg * 4 + g)) =
+                            make_uint4(bf16x2(gelu(z[0] + b0.x), gelu(z[1] + b0.y)),
+                                       bf16x2(gelu(z[2] + b0.z), gelu(z[3] + b0.w)),
+                                       bf16x2(gelu(z[4] + b1.x), gelu(z[5] + b1.y)),
+                                       bf16x2(gelu(z[6] + b1.z), gelu(z[7] + b1.w)));
+                    }
+                }
+                if (!last) {
+                    for (int g = N / 8; g < (N + kTcK - 1) / kTcK * 8; ++g)
+                        *reinterpret_cast<uint4*>(sx + fw_x_offset(r, g)) = make_uint4(0, 0, 0, 0);
+                    tc_fence_before();
+                    sl::tma::fence_proxy_async();
+                    sl::tma::mbar_arrive(x_ready);
+                } else {
+                    tc_fence_before();  // the next tile's x_ready arrival follows these loads
+                }
+            }
+        }
+    } else if (warp == 4 && lane == 0) {  // ----------------------------- MMAs
+        int q = 0;
+        uint32_t xphase = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
+            for (int l = 0; l < net.layers && ok; ++l) {
+                ok = fw_wait(x_ready, xphase, failed);
+                xphase ^= 1u;
+                if (!ok) break;
+                tc_fence_after();
+                const int K = net.din[l], N = net.dout[l];
+                for (int kc = 0; kc * kTcK < K && ok; ++kc) {
+                    const uint32_t a0 = sl::tma::smem_addr(sx + kc * (kFwRows * 128));
+                    const int steps = min(kTcK, K - kc * kTcK) / 16;
+                    for (int n0 = 0; n0 < N; n0 += kFwTileN, ++q) {
+                        const int st = q % kFwStages;
+                        ok = fw_wait(&full[st], (uint32_t)(q / kFwStages) & 1u, failed);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t b0 = sl::tma::smem_addr(sw + st * kFwWBytes);
+                        const uint32_t idesc = tc_idesc_bf16(kTcM, min(kFwTileN, N - n0));
+                        for (int k = 0; k < steps; ++k)
+                            tc_mma(tmem + (uint32_t)n0, tc_desc_sw128(a0 + 32 * k), tc_desc_sw128(b0 + 32 * k), idesc,
+                                   (kc | k) != 0);
+                        tc_commit(&empty[st]);
+                    }
+                }
+                if (ok) tc_commit(acc_done);
+            }
+        // every MMA issued has completed before the tensor memory is freed
+        tc_commit(drain);
+        if (!sl::tma::mbar_wait(drain, 0)) *failed = 1;
+    } else if (warp == 5 && lane == 0) {  // ---------------------------- copies
+        int q = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x)
+            for (int l = 0; l < net.layers && ok; ++l)
+                for (int k0 = 0; k0 < net.din[l] && ok; k0 += kTcK)
+                    for (int n0 = 0; n0 < net.dout[l]; n0 += kFwTileN, ++q) {
+                        const int st = q % kFwStages;
+                        if (q >= kFwStages) ok = fw_wait(&empty[st], (uint32_t)(q / kFwStages - 1) & 1u, failed);
+                        if (!ok) break;
+                        sl::tma::mbar_arrive_expect_tx(&full[st], kFwWBytes);
+                        sl::tma::load_2d(sw + st * kFwWBytes, &net.w[l], k0, n0, &full[st]);
+                    }
+        // and every copy has landed before the shared memory is given back
+        for (int p = max(0, q - kFwStages); p < q; ++p)
+            if (!sl::tma::mbar_wait(&full[p % kFwStages], (uint32_t)(p / kFwStages) & 1u)) *failed = 1;
+    }
+    __syncwarp();
+    __syncthreads();
+    if (tid == 0 && *failed) atomicExch(err, 1);
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kFwMaxWidth)
+                     : "memory");
+}
+
 // out[c][r] = in[r][c]
 __global__ void transpose_kernel(const bf16* __restrict__ in, int rows, int cols, int ldi, bf16* out, int ldo)
 {
@@ -453,6 +684,10 @@ struct sl_mlp {
     int step = 0;
     int* d_err = nullptr;         // set by a tcgen05 GEMM whose bounded wait ran out
     bool tc_setup_failed = false; // a GEMM's tensor maps or launch attributes could not be set up
+    bool fused = false;           // `net` is set up: the whole forward pass in one launch
+    FwNet net{};
+    int num_sms = 0;
+    bool host_direct = false;     // the GPU reads and writes pageable host memory (cudaDevAttrPageableMemoryAccess)
     void* arena = nullptr;
 };
 
@@ -567,6 +802,46 @@ void forward(sl_mlp* h, int M, cudaStream_t st)
     }
 }
 
+// The one-launch forward pass: networks of up to kFwMaxLayers linear layers of
+// up to kFwMaxWidth padded columns (what fits in shared memory and TMEM).
+bool setup_forward(sl_mlp* h)
+{
+    if (h->nl > kFwMaxLayers) return false;
+    FwNet& f = h->net;
+    f.layers = h->nl; f.n_in = h->n_in; f.n_out = h->n_out;
+    for (int l = 0; l < h->nl; ++l) {
+        if (h->din[l] > kFwMaxWidth || h->dout[l] > kFwMaxWidth) return false;
+        f.din[l] = h->din[l];
+        f.dout[l] = h->dout[l];
+        f.bias[l] = h->P + h->b_off[l];
+        if (!make_tc_map(&f.w[l], h->Pb + h->w_off[l], h->dout[l], h->din[l], h->din[l], kFwTileN)) return false;
+    }
+    return true;
+}
+
+// y = network(x) for n rows; x and y where the GPU can reach them
+bool forward_fused(sl_mlp* h, const float* x, float* y, int n, cudaStream_t st)
+{
+    // set on every call: the attribute belongs to the current device's context
+    if (cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwSmem) != cudaSuccess)
+        return false;
+    const int tiles = (n + kFwRows - 1) / kFwRows;
+    mlp_forward_kernel<<<std::min(tiles, 2 * h->num_sms), kFwThreads, kFwSmem, st>>>(h->net, x, y, n, h->d_err);
+    return true;
+}
+
+// A caller's host array as the GPU can use it in place, or NULL
+void* device_view(const sl_mlp* h, const void* p)
+{
+    if (h->host_direct) return const_cast<void*>(p);
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged ? a.devicePointer : nullptr;
+}
+
 // backward for M rows with targets yin; fills G
 void backward(sl_mlp* h, int M, cudaStream_t st)
 {
@@ -664,6 +939,11 @@ int sl_mlp_create(int n_in, int hidden, int hidden_layers, int n_out, int max_ba
         sl_mlp_destroy(h);
         return sl_record_error(SL_ERR_CUDA, "MLP initialisation failed");
     }
+    int dev = 0, pageable = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, dev);
+    h->host_direct = cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess && pageable;
+    h->fused = setup_forward(h);
     *out = h;
     return SL_OK;
 }
@@ -773,6 +1053,26 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
 {
     if (!h || !x || !y || n < 1) return sl_record_error(SL_ERR_ARG, "bad arguments");
     const int B = h->max_batch, L = h->nl, ldo = h->dout[L - 1];
+    if (h->fused) {
+        float* vx = static_cast<float*>(device_view(h, x));
+        float* vy = static_cast<float*>(device_view(h, y));
+        // what the GPU cannot reach goes through the batch's staging, a batch at a time
+        const int step = vx && vy ? n : B;
+        for (int s0 = 0; s0 < n; s0 += step) {
+            const int M = std::min(step, n - s0);
+            const float* px = vx ? vx + (size_t)s0 * h->n_in : h->xin;
+            float* py = vy ? vy + (size_t)s0 * h->n_out : h->yin;
+            if (!vx)
+                cudaMemcpyAsync(h->xin, x + (size_t)s0 * h->n_in, (size_t)M * h->n_in * 4, cudaMemcpyHostToDevice,
+                                nullptr);
+            if (!forward_fused(h, px, py, M, nullptr)) h->tc_setup_failed = true;
+            if (!vy)
+                cudaMemcpyAsync(y + (size_t)s0 * h->n_out, h->yin, (size_t)M * h->n_out * 4, cudaMemcpyDeviceToHost,
+                                nullptr);
+        }
+        if (cudaStreamSynchronize(nullptr) != cudaSuccess) return sl_record_error(SL_ERR_CUDA, "prediction failed");
+        return mlp_status(h, "sl_mlp_predict");
+    }
     std::vector<float> zb((size_t)B * ldo);
     for (int s0 = 0; s0 < n; s0 += B) {
         const int M = std::min(B, n - s0);
