@@ -3,17 +3,19 @@
 // accumulation, trained and evaluated on the GPU by this file's kernels
 // (include/spacelab_mlp.h).
 //
-// Every matrix product is one kernel, gemm_nt_tc: C[M][N] = A[M][K] . B[N][K]^T
-// with A and B bf16 row-major (K contiguous) on the fifth-generation tensor
-// cores: TMA copies of 128-byte-swizzled K chunks into shared memory,
-// tcgen05.mma (M = 128, N <= 128, K = 16, bf16 x bf16 -> f32) into a tensor
-// memory accumulator, tcgen05.ld back to registers for the epilogue, which
-// adds the bias and writes the FP32 pre-activation and/or the BF16
-// activation (GELU or identity).
-//   forward   Z_l = X_l W_l^T + b_l,  X_{l+1} = bf16(GELU(Z_l))
-//   backward  dW_l = dZ_l^T X_l   (A = dZ^T, B = X^T: transposed copies)
-//             dX_l = dZ_l W_l     (B = W^T: a transposed copy of W)
-//             dZ_{l-1} = bf16(dX_l * GELU'(Z_{l-1}))
+// Every training product is one kernel, gemm_nt_tc: C[M][N] = A[M][K] .
+// B[N][K]^T with A and B bf16 row-major (K contiguous) on the
+// fifth-generation tensor cores: TMA copies of 128-byte-swizzled K chunks into
+// shared memory, tcgen05.mma (bf16 x bf16 -> f32) into a tensor memory
+// accumulator, tcgen05.ld back to registers for the epilogue.
+//   forward   Z_l = X_l W_l^T + b_l,  X_{l+1} = bf16(GELU(Z_l)) and X_{l+1}^T
+//   backward  dW_l = dZ_l^T X_l, db_l = the column sums of dZ_l, and
+//             dX_l = dZ_l W_l, dZ_{l-1} = bf16(dX_l * GELU'(Z_{l-1})) and its
+//             transpose: one launch per layer
+// The operands with the batch as their K dimension are the transposed copies
+// that the epilogues write; W^T is kept beside the bf16 weights by Adam.
+// Training runs a step as one CUDA graph over an epoch's rows packed on the
+// device.  Prediction takes all layers in one launch (mlp_forward_kernel).
 // Widths are padded to multiples of 32 with zero weights that stay zero
 // (their gradients are zero).  FP32 master weights are updated with Adam;
 // bf16 copies feed the GEMMs.  An mma.sync m16n8k16 kernel (gemm_nt_kernel)
@@ -143,30 +145,36 @@ __global__ void __launch_bounds__(128) gemm_nt_kernel(const bf16* __restrict__ A
 }
 
 // ------------------------------------------------------------- tcgen05 --
-// C[M][N] = A[M][K] . B[N][K]^T on the fifth-generation tensor cores.  One
-// CTA (4 warps) per 128-row block of C and BN columns; its accumulator is
-// BN f32 columns x 128 lanes of tensor memory (TMEM).  K is taken in chunks
-// of 64 elements (128 bytes): TMA copies the A and B chunks into shared
-// memory with the 128-byte swizzle -- the K-major layout the MMA's shared-
-// memory descriptors describe (8-row groups 1024 bytes apart) -- into one of
-// two stages, and one thread issues four tcgen05.mma (M=128, N=BN, K=16)
-// per chunk, then tcgen05.commit to the stage's barrier so that the next
-// copy into that stage waits for the MMAs reading it.  Boxes past M, N or K
-// are zero-filled by the copy engine.  The epilogue: warp w reads TMEM
-// lanes 32w..32w+31 (rows m0 + 32w + lane) 32 columns at a time with
-// tcgen05.ld, adds the bias and writes the FP32 and/or BF16 (GELU or
-// identity) outputs.  Every wait is bounded (sl_tma.cuh); a wait that runs
-// out sets *err, the CTA waits (bounded) for its MMAs, frees its TMEM and
-// returns.
-constexpr int kTcM = 128, kTcK = 64, kTcStages = 2;
-constexpr int kTcThreads = 128;
-
-template <int BN>
-struct TcSmem {
-    static constexpr int kABytes = kTcM * kTcK * 2;  // 16 KB
-    static constexpr int kBBytes = BN * kTcK * 2;
-    static constexpr int kBytes = kTcStages * (kABytes + kBBytes) + 1024 /* barriers etc. */ + 1024 /* alignment */;
-};
+// C[M][N] = A[M][K] . B[N][K]^T on the fifth-generation tensor cores
+// (gemm_nt_tc_kernel).  One CTA (8 warps) per 128 x 32 tile of C; its
+// accumulator is 32 f32 columns x 128 lanes of tensor memory (TMEM).  K is
+// taken in chunks of 64 elements (128 bytes): TMA copies the A and B chunks
+// into shared memory with the 128-byte swizzle -- the K-major layout the MMA's
+// shared-memory descriptors describe (8-row groups 1024 bytes apart) -- into
+// one of four stages, and one thread issues up to four tcgen05.mma (M=128,
+// N=32, K=16) per chunk, then tcgen05.commit to the stage's barrier so that
+// the next copy into that stage waits for the MMAs reading it.  Boxes past M,
+// N or K are zero-filled by the copy engine.  Every wait is bounded
+// (sl_tma.cuh); a wait that runs out sets *err, the CTA waits (bounded) for
+// its MMAs, frees its TMEM and returns.
+//
+// The training products are small -- a batch of 256 rows through 256-wide
+// layers is 33 MFLOP -- so what counts is how many CTAs share one (16 of 128 x
+// 32 for a layer) and that nothing needs a pass of its own: a launch holds up
+// to two products and a bias gradient (the backward's dW, db and dX of one
+// layer), and the epilogue writes the next product's operands in the layout
+// it reads, the transposed copy too (TMEM gives a warp 32 rows of one column:
+// its 2-byte stores are contiguous in the transposed copy).  The bias gradient
+// adds in row order from the transposed copy, 16 bytes a load.
+//
+// Measured (GB300, 8-256x4-4): one epoch of 45,000 rows in batches of 256, 87.1
+// -> 12.4 ms (497 -> 70 us a step: 40 launches, three copies and a wait a step
+// before, 12 launches in a graph now); loss and gradient of 1024 rows, 696 ->
+// 224 us.  Same bits.
+constexpr int kTcM = 128, kTcN = 32, kTcK = 64, kTcStages = 4;
+constexpr int kTcThreads = 256;
+constexpr int kTcABytes = kTcM * kTcK * 2, kTcBBytes = kTcN * kTcK * 2;
+constexpr int kTcSmem = kTcStages * (kTcABytes + kTcBBytes) + 1024 /* barriers etc. */ + 1024 /* alignment */;
 
 // Shared-memory matrix descriptor of a K-major tile with the 128-byte
 // swizzle: start address >> 4 (bits 0-13), leading byte offset (unused for
@@ -228,26 +236,103 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float* v)
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-template <int BN>
-__global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_constant__ CUtensorMap mapA,
-                                                                 const __grid_constant__ CUtensorMap mapB,
-                                                                 const float* __restrict__ bias, float* Cf, bf16* Cb,
-                                                                 int ldc, int M, int N, int K, int act, int* err)
+// 16 consecutive f32 columns of this thread's TMEM lane.
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v)
 {
-    using Sm = TcSmem<BN>;
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+__device__ __forceinline__ uint32_t bf16x2(float a, float b)
+{
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);  // a in the low half
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// One product and what becomes of it.  z = C + bias (if any) goes to cf; zin
+// given, z = C * GELU'(zin); bf16(act ? GELU(z) : z) goes to cb and, transposed
+// (leading dimension ldt), to cbt.  During training the step's rows of the
+// epoch's packed inputs start at (*step + step_bias) x a_row_step rows of A and
+// x b_col_step columns of B.
+struct GemmJob {
+    CUtensorMap a, b;
+    const float *bias, *zin;
+    float* cf;
+    bf16 *cb, *cbt;
+    int ldc, ldt, M, N, K, act;
+    int a_row_step, b_col_step;
+};
+
+struct GemmLaunch {
+    GemmJob job[2];
+    int njobs;
+    // bias gradient: db_out[c] = sum over r < db_rows of db_src[c][r], r ascending
+    const bf16* db_src;
+    float* db_out;
+    int db_n, db_rows;
+    const int* step;  // NULL: step 0
+    int step_bias;
+    int* bump;        // incremented once (by a launch that does not read it)
+    int* err;
+};
+
+__host__ __device__ inline int gemm_tiles(const GemmJob& j) { return ((j.M + kTcM - 1) / kTcM) * ((j.N + kTcN - 1) / kTcN); }
+
+// The sum over the batch of one output's gradient, thread = output, in row
+// order; dZ^T rows are read 8 at a time.
+__device__ void bias_grad(const GemmLaunch& L, int c)
+{
+    if (c >= L.db_n) return;
+    const uint4* src = reinterpret_cast<const uint4*>(L.db_src + (size_t)c * L.db_rows);  // rows a multiple of 32
+    float s = 0.0f;
+#pragma unroll 4
+    for (int r = 0; r < L.db_rows / 8; ++r) {
+        const uint4 q = src[r];
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            s += __uint_as_float(w[k] << 16);
+            s += __uint_as_float(w[k] & 0xffff0000u);
+        }
+    }
+    L.db_out[c] = s;
+}
+
+__global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_constant__ GemmLaunch L)
+{
     extern __shared__ unsigned char tc_raw[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    int tile = blockIdx.x;
+    if (tile == 0 && tid == 0 && L.bump) *L.bump += 1;
+    const int tiles0 = gemm_tiles(L.job[0]);
+    const bool second = tile >= tiles0;
+    if (second) tile -= tiles0;
+    if (second && (L.njobs < 2 || tile >= gemm_tiles(L.job[1]))) {
+        bias_grad(L, (tile - (L.njobs < 2 ? 0 : gemm_tiles(L.job[1]))) * kTcThreads + tid);
+        return;
+    }
+    const GemmJob& J = L.job[second];
+
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) &
                                                            ~static_cast<uintptr_t>(1023));
-    unsigned char* sa = base;                                  // [stage][128 rows][128 B]
-    unsigned char* sb = base + kTcStages * Sm::kABytes;        // [stage][BN rows][128 B]
-    uint64_t* full = reinterpret_cast<uint64_t*>(sb + kTcStages * Sm::kBBytes);
+    unsigned char* sa = base;                            // [stage][128 rows][128 B]
+    unsigned char* sb = base + kTcStages * kTcABytes;    // [stage][32 rows][128 B]
+    uint64_t* full = reinterpret_cast<uint64_t*>(sb + kTcStages * kTcBBytes);
     uint64_t* empty = full + kTcStages;
     uint64_t* done = empty + kTcStages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
     int* failed = reinterpret_cast<int*>(tmem_slot + 1);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.y * kTcM, n0 = blockIdx.x * BN;
-    const int nk = (K + kTcK - 1) / kTcK;
+    const int tiles_n = (J.N + kTcN - 1) / kTcN;
+    const int m0 = tile / tiles_n * kTcM, n0 = tile % tiles_n * kTcN;
+    const int nk = (J.K + kTcK - 1) / kTcK;
 
     if (tid == 0) {
         for (int st = 0; st < kTcStages; ++st) {
@@ -258,9 +343,9 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
         *failed = 0;
         sl::tma::fence_barrier_init();
     }
-    if (warp == 0) {  // BN f32 columns of TMEM (a power of two >= 32)
+    if (warp == 0) {  // 32 f32 columns of TMEM
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(sl::tma::smem_addr(tmem_slot)), "r"(BN)
+                     ::"r"(sl::tma::smem_addr(tmem_slot)), "r"(kTcN)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -270,13 +355,14 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
     const uint32_t tmem = *tmem_slot;
 
     if (tid == 0) {
-        constexpr uint32_t idesc = tc_idesc_bf16(kTcM, BN);
-        const uint32_t bytes = Sm::kABytes + Sm::kBBytes;
+        constexpr uint32_t idesc = tc_idesc_bf16(kTcM, kTcN);
+        const int step = L.step ? *L.step + L.step_bias : 0;
+        const int ya = m0 + step * J.a_row_step, xb = step * J.b_col_step;
         auto issue = [&](int kc) {
             const int st = kc % kTcStages;
-            sl::tma::mbar_arrive_expect_tx(&full[st], bytes);
-            sl::tma::load_2d(sa + st * Sm::kABytes, &mapA, kc * kTcK, m0, &full[st]);
-            sl::tma::load_2d(sb + st * Sm::kBBytes, &mapB, kc * kTcK, n0, &full[st]);
+            sl::tma::mbar_arrive_expect_tx(&full[st], kTcABytes + kTcBBytes);
+            sl::tma::load_2d(sa + st * kTcABytes, &J.a, kc * kTcK, ya, &full[st]);
+            sl::tma::load_2d(sb + st * kTcBBytes, &J.b, xb + kc * kTcK, n0, &full[st]);
         };
         int issued = 0;
         for (; issued < nk && issued < kTcStages; ++issued) issue(issued);
@@ -287,10 +373,11 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
             const uint32_t par = (uint32_t)(kc / kTcStages) & 1u;
             if (!sl::tma::mbar_wait(&full[st], par)) { ok = false; break; }
             tc_fence_after();
-            const uint32_t a0 = sl::tma::smem_addr(sa + st * Sm::kABytes);
-            const uint32_t b0 = sl::tma::smem_addr(sb + st * Sm::kBBytes);
-#pragma unroll
-            for (int k = 0; k < kTcK / 16; ++k)
+            const uint32_t a0 = sl::tma::smem_addr(sa + st * kTcABytes);
+            const uint32_t b0 = sl::tma::smem_addr(sb + st * kTcBBytes);
+            // past K the boxes hold zeros, or another step's columns
+            const int steps = min(kTcK, J.K - kc * kTcK + 15) / 16;
+            for (int k = 0; k < steps; ++k)
                 tc_mma(tmem, tc_desc_sw128(a0 + 32 * k), tc_desc_sw128(b0 + 32 * k), idesc, (kc | k) != 0);
             tc_commit(&empty[st]);
             if (kc + kTcStages < nk) {
@@ -314,21 +401,54 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
     __syncthreads();
     // the same decision in every thread (tcgen05.ld is warp-collective)
     if (*failed) {
-        if (tid == 0) atomicExch(err, 1);
+        if (tid == 0) atomicExch(L.err, 1);
     } else {
-        const int row = m0 + warp * 32 + lane;
-#pragma unroll 1
-        for (int cg = 0; cg < BN / 32; ++cg) {
-            float v[32];
-            tc_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cg * 32), v);
-            if (row < M) {
+        // warp w: TMEM lanes 32 (w mod 4) .., columns 16 (w / 4) ..
+        const int row = m0 + (warp & 3) * 32 + lane, c0 = (warp >> 2) * 16;
+        float v[16];
+        tc_ld16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
+        const int col = n0 + c0;
+        if (row < J.M) {
+            const size_t at = (size_t)row * J.ldc + col;
+            if (J.ldc % 8 == 0 && col + 16 <= J.N) {  // whole 16-byte groups
+                if (J.bias)
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
-                    const int col = n0 + cg * 32 + i;
-                    if (col >= N) break;
-                    const float z = v[i] + (bias ? bias[col] : 0.0f);
-                    if (Cf) Cf[(size_t)row * ldc + col] = z;
-                    if (Cb) Cb[(size_t)row * ldc + col] = __float2bfloat16(act ? gelu(z) : z);
+                    for (int i = 0; i < 16; ++i) v[i] += __ldg(J.bias + col + i);
+                if (J.zin) {
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4) {
+                        const float4 z = *reinterpret_cast<const float4*>(J.zin + at + i);
+                        v[i] *= gelu_grad(z.x);
+                        v[i + 1] *= gelu_grad(z.y);
+                        v[i + 2] *= gelu_grad(z.z);
+                        v[i + 3] *= gelu_grad(z.w);
+                    }
+                }
+                if (J.cf)
+#pragma unroll
+                    for (int i = 0; i < 16; i += 4)
+                        *reinterpret_cast<float4*>(J.cf + at + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+                if (J.cb) {
+                    uint32_t h[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        h[i] = J.act ? bf16x2(gelu(v[2 * i]), gelu(v[2 * i + 1])) : bf16x2(v[2 * i], v[2 * i + 1]);
+                    uint4* dst = reinterpret_cast<uint4*>(J.cb + at);
+                    dst[0] = make_uint4(h[0], h[1], h[2], h[3]);
+                    dst[1] = make_uint4(h[4], h[5], h[6], h[7]);
+                    if (J.cbt) {
+                        uint16_t* t = reinterpret_cast<uint16_t*>(J.cbt) + (size_t)col * J.ldt + row;
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) t[(size_t)i * J.ldt] = (uint16_t)(h[i >> 1] >> (16 * (i & 1)));
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    if (col + i >= J.N) break;
+                    const float z = v[i] + (J.bias ? J.bias[col + i] : 0.0f);
+                    if (J.cf) J.cf[at + i] = z;
+                    if (J.cb) J.cb[at + i] = __float2bfloat16(J.act ? gelu(z) : z);
                 }
             }
         }
@@ -336,7 +456,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTcN) : "memory");
 }
 
 // ----------------------------------------------- the whole forward pass --
@@ -381,12 +501,6 @@ __device__ __forceinline__ bool fw_wait(uint64_t* bar, uint32_t parity, volatile
             return false;
         }
     return true;
-}
-
-__device__ __forceinline__ uint32_t bf16x2(float a, float b)
-{
-    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);  // a in the low half
-    return *reinterpret_cast<const uint32_t*>(&v);
 }
 
 // byte of row r's 16-byte group g (8 columns) of the activations
@@ -533,7 +647,7 @@ __global__ void __launch_bounds__(kFwThreads, 2) mlp_forward_kernel(const __grid
                         if (!ok) break;
                         tc_fence_after();
                         const uint32_t b0 = sl::tma::smem_addr(sw + st * kFwWBytes);
-                        const uint32_t idesc = tc_idesc_bf16(kTcM, min(kFwTileN, N - n0));
+                        const uint32_t idesc = tc_idesc_bf16(kFwRows, min(kFwTileN, N - n0));
                         for (int k = 0; k < steps; ++k)
                             tc_mma(tmem + (uint32_t)n0, tc_desc_sw128(a0 + 32 * k), tc_desc_sw128(b0 + 32 * k), idesc,
                                    (kc | k) != 0);
@@ -570,37 +684,34 @@ __global__ void __launch_bounds__(kFwThreads, 2) mlp_forward_kernel(const __grid
                      : "memory");
 }
 
-// out[c][r] = in[r][c]
-__global__ void transpose_kernel(const bf16* __restrict__ in, int rows, int cols, int ldi, bf16* out, int ldo)
+// The inputs of rows idx[0 .. rows) (NULL: rows 0 ..) as bf16 rows of ld
+// columns, zero past n_in and past row n, and transposed (leading dimension
+// rows); targets gathered alongside.  Thread = row.
+__global__ void pack_kernel(const float* __restrict__ x, const float* __restrict__ y, const int* __restrict__ idx,
+                            int rows, int n, int n_in, int n_out, int ld, bf16* xb, bf16* xt, float* yb)
 {
-    __shared__ bf16 t[32][33];
-    const int bx = blockIdx.x * 32, by = blockIdx.y * 32;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = by + y, c = bx + threadIdx.x;
-        t[y][threadIdx.x] = (r < rows && c < cols) ? in[(size_t)r * ldi + c] : __float2bfloat16(0.0f);
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= rows) return;
+    const int src = idx ? idx[r] : r;
+    for (int c = 0; c < ld; ++c) {
+        const bf16 v = __float2bfloat16(c < n_in && src < n ? x[(size_t)src * n_in + c] : 0.0f);
+        xb[(size_t)r * ld + c] = v;
+        if (xt) xt[(size_t)c * rows + r] = v;
     }
-    __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int c = bx + y, r = by + threadIdx.x;
-        if (c < cols && r < rows) out[(size_t)c * ldo + r] = t[threadIdx.x][y];
-    }
+    if (yb)
+        for (int c = 0; c < n_out; ++c) yb[(size_t)r * n_out + c] = y[(size_t)src * n_out + c];
 }
 
-// float -> bf16 rows (input features, zero padding beyond n)
-__global__ void pack_input_kernel(const float* __restrict__ x, int M, int n, int ld, bf16* out)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= M * ld) return;
-    const int r = i / ld, c = i - r * ld;
-    out[i] = __float2bfloat16(c < n ? x[(size_t)r * n + c] : 0.0f);
-}
-
-// MSE over the first n_out columns: dZ = 2 (z - y) / (M n_out), loss partials
+// MSE over the first n_out columns: dZ = 2 (z - y) / (M n_out), row-major and
+// transposed, and the loss in one partial sum per 256 entries of dZ
 __global__ void mse_grad_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ y, int M, int n_out,
-                                bf16* dz, int ld, float* loss_partial)
+                                bf16* dz, bf16* dzt, int ld, float* loss_partial, const int* step, int step_bias)
 {
     __shared__ float red[256];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int st = step ? *step + step_bias : 0;
+    y += (size_t)st * M * n_out;
+    loss_partial += (size_t)st * gridDim.x;
     float l = 0.0f;
     if (i < M * ld) {
         const int r = i / ld, c = i - r * ld;
@@ -611,6 +722,7 @@ __global__ void mse_grad_kernel(const float* __restrict__ z, int ldz, const floa
             g = 2.0f * e / (float)(M * n_out);
         }
         dz[i] = __float2bfloat16(g);
+        dzt[(size_t)c * M + r] = __float2bfloat16(g);
     }
     red[threadIdx.x] = l;
     __syncthreads();
@@ -621,31 +733,37 @@ __global__ void mse_grad_kernel(const float* __restrict__ z, int ldz, const floa
     if (threadIdx.x == 0) loss_partial[blockIdx.x] = red[0];
 }
 
-// dZ = bf16(dX * GELU'(Z)) elementwise
-__global__ void gelu_back_kernel(const float* __restrict__ dx, const float* __restrict__ z, int n, bf16* dz)
+// A layer's place in the parameter vector: W [dout][din] at w, then b
+struct LayerAt {
+    long long w;
+    int din, dout;
+};
+
+// bf16 copy of parameter i, and for a weight the copy's transposed place
+__device__ __forceinline__ void put_bf16(bf16* pb, bf16* wt, const LayerAt* at, int layers, int i, float v)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dz[i] = __float2bfloat16(dx[i] * gelu_grad(z[i]));
+    pb[i] = __float2bfloat16(v);
+    int l = 0;
+    while (l + 1 < layers && i >= at[l + 1].w) ++l;
+    const long long k = i - at[l].w;
+    if (k < (long long)at[l].din * at[l].dout) {
+        const int r = (int)(k / at[l].din), c = (int)(k - (long long)r * at[l].din);
+        wt[at[l].w + (long long)c * at[l].dout + r] = __float2bfloat16(v);
+    }
 }
 
-// db[c] = sum_r dZ[r][c]  (dZ bf16 [M][ld])
-__global__ void bias_grad_kernel(const bf16* __restrict__ dz, int M, int ld, int n, float* db)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= n) return;
-    float s = 0.0f;
-    for (int r = 0; r < M; ++r) s += __bfloat162float(dz[(size_t)r * ld + c]);
-    db[c] = s;
-}
-
-// Adam on fp32 master parameters; refreshes the bf16 copy.  mask: the
-// parameter is live (padding stays 0).
-__global__ void adam_kernel(float* p, const float* g, float* m, float* v, bf16* pb, const uint8_t* mask, int n, float lr,
-                            float b1, float b2, float eps, float c1, float c2)
+// Adam on fp32 master parameters; refreshes the bf16 copies.  mask: the
+// parameter is live (padding stays 0).  coef: the step's bias corrections
+// 1 - b1^t, 1 - b2^t.
+__global__ void adam_kernel(float* p, const float* g, float* m, float* v, bf16* pb, bf16* wt, const LayerAt* at,
+                            int layers, const uint8_t* mask, int n, float lr, float b1, float b2, float eps,
+                            const float2* coef, const int* step, int step_bias)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    if (mask && !mask[i]) return;
+    if (!mask[i]) return;
+    const float2 c = coef[*step + step_bias];
+    const float c1 = c.x, c2 = c.y;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
@@ -653,13 +771,13 @@ __global__ void adam_kernel(float* p, const float* g, float* m, float* v, bf16* 
     v[i] = vi;
     const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
     p[i] = pi;
-    if (pb) pb[i] = __float2bfloat16(pi);
+    put_bf16(pb, wt, at, layers, i, pi);
 }
 
-__global__ void to_bf16_kernel(const float* __restrict__ in, bf16* out, int n)
+__global__ void to_bf16_kernel(const float* __restrict__ in, bf16* pb, bf16* wt, const LayerAt* at, int layers, int n)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = __float2bfloat16(in[i]);
+    if (i < n) put_bf16(pb, wt, at, layers, i, in[i]);
 }
 
 int pad32(int x) { return (x + 31) / 32 * 32; }
@@ -675,12 +793,15 @@ struct sl_mlp {
     float *P = nullptr, *G = nullptr, *Mom = nullptr, *Var = nullptr;  // fp32 params, grads, Adam moments
     bf16* Pb = nullptr;                  // bf16 copy of params (weights used by the GEMMs)
     uint8_t* mask = nullptr;             // live parameters
-    bf16 *Wt = nullptr;                  // transposed weights scratch (max din x dout)
-    std::vector<bf16*> X;                // bf16 activations per layer input [max_batch][din]
-    std::vector<float*> Z;               // fp32 pre-activations per layer [max_batch][dout]
-    bf16 *dZ = nullptr, *dZt = nullptr, *Xt = nullptr;
-    float* dX = nullptr;
+    bf16* Wt = nullptr;                  // its weights transposed, [din][dout] at the same offsets
+    LayerAt* at = nullptr;               // the layers' places, for the kernels
+    std::vector<bf16*> X, Xt;            // bf16 activations per layer input, [M][din] and [din][M]
+    std::vector<float*> Z;               // fp32 pre-activations per layer [M][dout]
+    bf16 *dZ[2] = {}, *dZt[2] = {};      // gradients of Z, [M][dout] and [dout][M]; a layer reads one and writes the other
     float *xin = nullptr, *yin = nullptr, *loss_part = nullptr;
+    cudaStream_t stream = nullptr;       // training's launches
+    void* epoch = nullptr;               // training's copies of the data set (grown when a larger one comes)
+    size_t epoch_bytes = 0;
     int step = 0;
     int* d_err = nullptr;         // set by a tcgen05 GEMM whose bounded wait ran out
     bool tc_setup_failed = false; // a GEMM's tensor maps or launch attributes could not be set up
@@ -731,42 +852,24 @@ bool make_tc_map(CUtensorMap* map, const bf16* base, int rows, int k, int ld, in
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int BN>
-bool launch_tc(cudaStream_t st, const CUtensorMap& ma, const bf16* B, int ldb, const float* bias, float* Cf, bf16* Cb,
-               int ldc, int M, int N, int K, int act, int* err)
+// A job without its epilogue; false if a tensor map cannot be made.
+bool make_job(GemmJob* j, const bf16* A, int rows_a, int lda, const bf16* B, int ldb, int kb, int M, int N, int K)
+{
+    *j = GemmJob{};
+    j->M = M; j->N = N; j->K = K;
+    return make_tc_map(&j->a, A, rows_a, K, lda, kTcM) && make_tc_map(&j->b, B, N, kb, ldb, kTcN);
+}
+
+bool launch_gemm(const GemmLaunch& L, cudaStream_t st)
 {
     // set on every call: the attribute belongs to the current device's
     // context, and the call is a host-side table update
-    if (cudaFuncSetAttribute(gemm_nt_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, TcSmem<BN>::kBytes) !=
-        cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_nt_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem) != cudaSuccess)
         return false;
-    CUtensorMap mb;
-    if (!make_tc_map(&mb, B, N, K, ldb, BN)) return false;
-    dim3 grid((N + BN - 1) / BN, (M + kTcM - 1) / kTcM);
-    gemm_nt_tc_kernel<BN><<<grid, kTcThreads, TcSmem<BN>::kBytes, st>>>(ma, mb, bias, Cf, Cb, ldc, M, N, K, act, err);
+    int grid = gemm_tiles(L.job[0]) + (L.njobs > 1 ? gemm_tiles(L.job[1]) : 0);
+    if (L.db_out) grid += (L.db_n + kTcThreads - 1) / kTcThreads;
+    gemm_nt_tc_kernel<<<grid, kTcThreads, kTcSmem, st>>>(L);
     return true;
-}
-
-// The tcgen05 GEMM; false if its tensor maps or launch attributes cannot be
-// set up (the caller reports the error; nothing is launched then).
-bool gemm_tc(cudaStream_t st, const bf16* A, int lda, const bf16* B, int ldb, const float* bias, float* Cf, bf16* Cb,
-             int ldc, int M, int N, int K, int act, int* err)
-{
-    CUtensorMap ma;
-    if (!make_tc_map(&ma, A, M, K, lda, kTcM)) return false;
-    // at most 128 columns per CTA: the products are small (M of a few
-    // hundred rows), so more, narrower CTAs spread them over more SMs
-    if (N <= 32) return launch_tc<32>(st, ma, B, ldb, bias, Cf, Cb, ldc, M, N, K, act, err);
-    if (N <= 64) return launch_tc<64>(st, ma, B, ldb, bias, Cf, Cb, ldc, M, N, K, act, err);
-    return launch_tc<128>(st, ma, B, ldb, bias, Cf, Cb, ldc, M, N, K, act, err);
-}
-
-// Every product of the network runs on the tcgen05 GEMM.
-void gemm(sl_mlp* h, cudaStream_t st, const bf16* A, int lda, const bf16* B, int ldb, const float* bias, float* Cf,
-          bf16* Cb, int ldc, int M, int N, int K, int act)
-{
-    if (h->tc_setup_failed) return;
-    if (!gemm_tc(st, A, lda, B, ldb, bias, Cf, Cb, ldc, M, N, K, act, h->d_err)) h->tc_setup_failed = true;
 }
 
 // After a synchronisation: the GEMMs' setup and bounded waits.
@@ -783,23 +886,95 @@ int mlp_status(sl_mlp* h, const char* what)
     return SL_OK;
 }
 
-void transpose(cudaStream_t st, const bf16* in, int rows, int cols, int ldi, bf16* out, int ldo)
+// Where a batch's inputs are: its own buffers, or the rows of a training
+// epoch's (rows epoch_rows, the step's read from *step).
+struct BatchInput {
+    const bf16 *X0, *X0t;
+    const float* y;
+    int rows;           // of X0 and columns of X0t
+    int* step;          // NULL: the batch starts at row 0
+    float* loss_part;
+};
+
+// forward over M rows: the output pre-activation of the last layer is
+// Z[nl-1] ([M][dout_last], fp32).  train: the transposed activations too.
+void forward(sl_mlp* h, const BatchInput& in, int M, bool train, cudaStream_t st)
 {
-    dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
-    transpose_kernel<<<grid, block, 0, st>>>(in, rows, cols, ldi, out, ldo);
+    for (int l = 0; l < h->nl && !h->tc_setup_failed; ++l) {
+        const bool last = l == h->nl - 1;
+        const int K = h->din[l], N = h->dout[l];
+        GemmLaunch L{};
+        GemmJob& j = L.job[0];
+        L.njobs = 1;
+        L.err = h->d_err;
+        bool ok = make_job(&j, l ? h->X[l] : in.X0, l ? M : in.rows, K, h->Pb + h->w_off[l], K, K, M, N, K);
+        j.bias = h->P + h->b_off[l];
+        j.cf = h->Z[l];
+        j.cb = last ? nullptr : h->X[l + 1];
+        j.cbt = last || !train ? nullptr : h->Xt[l + 1];
+        j.ldc = N;
+        j.ldt = M;
+        j.act = 1;
+        if (l == 0) {
+            L.step = in.step;
+            j.a_row_step = M;
+        } else if (l == 1) {
+            L.bump = in.step;  // from here on *step is the step after this one
+        }
+        ok = ok && launch_gemm(L, st);
+        if (!ok) h->tc_setup_failed = true;
+    }
 }
 
-// forward over M rows of xin (already on device); the output pre-activation
-// of the last layer is Z[nl-1] ([M][dout_last], fp32)
-void forward(sl_mlp* h, int M, cudaStream_t st)
+// backward for the M rows of the last forward; fills G
+void backward(sl_mlp* h, const BatchInput& in, int M, cudaStream_t st)
 {
-    const int ld0 = h->din[0];
-    pack_input_kernel<<<(M * ld0 + 255) / 256, 256, 0, st>>>(h->xin, M, h->n_in, ld0, h->X[0]);
-    for (int l = 0; l < h->nl; ++l) {
-        const bool last = l == h->nl - 1;
-        gemm(h, st, h->X[l], h->din[l], h->Pb + h->w_off[l], h->din[l], h->P + h->b_off[l], h->Z[l],
-             last ? nullptr : h->X[l + 1], h->dout[l], M, h->dout[l], h->din[l], last ? 0 : 1);
+    const int nl = h->nl, ldo = h->dout[nl - 1];
+    const int nb = (M * ldo + 255) / 256;
+    int cur = 0;
+    mse_grad_kernel<<<nb, 256, 0, st>>>(h->Z[nl - 1], ldo, in.y, M, h->n_out, h->dZ[cur], h->dZt[cur], ldo,
+                                        in.loss_part, in.step, -1);
+    for (int l = nl - 1; l >= 0 && !h->tc_setup_failed; --l, cur ^= 1) {
+        const int K = h->din[l], N = h->dout[l];
+        GemmLaunch L{};
+        L.njobs = 1;
+        L.err = h->d_err;
+        // dW = dZ^T X: the products run over the batch
+        bool ok = make_job(&L.job[0], h->dZt[cur], N, M, l ? h->Xt[l] : in.X0t, l ? M : in.rows, l ? M : in.rows, N, K,
+                           M);
+        L.job[0].cf = h->G + h->w_off[l];
+        L.job[0].ldc = K;
+        if (l == 0) {
+            L.step = in.step;
+            L.step_bias = -1;
+            L.job[0].b_col_step = M;
+        }
+        L.db_src = h->dZt[cur];
+        L.db_out = h->G + h->b_off[l];
+        L.db_n = N;
+        L.db_rows = M;
+        if (l > 0) {  // dZ of the layer below = dZ W * GELU'(Z)
+            L.njobs = 2;
+            GemmJob& j = L.job[1];
+            ok = ok && make_job(&j, h->dZ[cur], M, N, h->Wt + h->w_off[l], N, N, M, K, N);
+            j.zin = h->Z[l - 1];
+            j.cb = h->dZ[cur ^ 1];
+            j.cbt = h->dZt[cur ^ 1];
+            j.ldc = K;
+            j.ldt = M;
+        }
+        ok = ok && launch_gemm(L, st);
+        if (!ok) h->tc_setup_failed = true;
     }
+}
+
+// The batch's own input buffers, packed from M rows of n features at x (and
+// their targets at y), device-reachable; rows n .. M - 1 are zero.
+BatchInput pack_batch(sl_mlp* h, const float* x, const float* y, int n, int M, cudaStream_t st)
+{
+    pack_kernel<<<(M + 127) / 128, 128, 0, st>>>(x, nullptr, nullptr, M, n, h->n_in, h->n_out, h->din[0], h->X[0],
+                                                 h->Xt[0], nullptr);
+    return BatchInput{h->X[0], h->Xt[0], y, M, nullptr, h->loss_part};
 }
 
 // The one-launch forward pass: networks of up to kFwMaxLayers linear layers of
@@ -842,28 +1017,6 @@ void* device_view(const sl_mlp* h, const void* p)
     return a.type == cudaMemoryTypeHost || a.type == cudaMemoryTypeManaged ? a.devicePointer : nullptr;
 }
 
-// backward for M rows with targets yin; fills G
-void backward(sl_mlp* h, int M, cudaStream_t st)
-{
-    const int L = h->nl;
-    const int ldo = h->dout[L - 1];
-    const int nb = (M * ldo + 255) / 256;
-    mse_grad_kernel<<<nb, 256, 0, st>>>(h->Z[L - 1], ldo, h->yin, M, h->n_out, h->dZ, ldo, h->loss_part);
-    for (int l = L - 1; l >= 0; --l) {
-        const int K = h->din[l], N = h->dout[l];
-        // dW = dZ^T X : A = dZ^T [N][M], B = X^T [K][M]
-        transpose(st, h->dZ, M, N, N, h->dZt, M);
-        transpose(st, h->X[l], M, K, K, h->Xt, M);
-        gemm(h, st, h->dZt, M, h->Xt, M, nullptr, h->G + h->w_off[l], nullptr, K, N, K, M, 0);
-        bias_grad_kernel<<<(N + 127) / 128, 128, 0, st>>>(h->dZ, M, N, N, h->G + h->b_off[l]);
-        if (l == 0) break;
-        // dX = dZ W : A = dZ [M][N], B = W^T [K][N]
-        transpose(st, h->Pb + h->w_off[l], N, K, K, h->Wt, N);
-        gemm(h, st, h->dZ, N, h->Wt, N, nullptr, h->dX, nullptr, K, M, K, N, 0);
-        gelu_back_kernel<<<(M * K + 255) / 256, 256, 0, st>>>(h->dX, h->Z[l - 1], M * K, h->dZ);
-    }
-}
-
 }  // namespace
 
 extern "C" {
@@ -894,14 +1047,14 @@ int sl_mlp_create(int n_in, int hidden, int hidden_layers, int n_out, int max_ba
     size_t bytes = 0;
     auto take = [&](size_t b) { size_t o = bytes; bytes = (bytes + b + 255) / 256 * 256; return o; };
     const size_t oP = take(off * 4), oG = take(off * 4), oM = take(off * 4), oV = take(off * 4), oPb = take(off * 2),
-                 oMask = take(off), oWt = take((size_t)maxw * maxw * 2);
-    std::vector<size_t> oX, oZ;
+                 oMask = take(off), oWt = take(off * 2), oAt = take(h->nl * sizeof(LayerAt));
+    std::vector<size_t> oX, oXt, oZ;
     for (int l = 0; l < h->nl; ++l) {
         oX.push_back(take((size_t)max_batch * h->din[l] * 2));
+        oXt.push_back(take((size_t)max_batch * h->din[l] * 2));
         oZ.push_back(take((size_t)max_batch * h->dout[l] * 4));
     }
-    const size_t odZ = take((size_t)max_batch * maxw * 2), odZt = take((size_t)max_batch * maxw * 2),
-                 oXt = take((size_t)max_batch * maxw * 2), odX = take((size_t)max_batch * maxw * 4),
+    const size_t odZ = take((size_t)max_batch * maxw * 2 * 4),
                  oxin = take((size_t)max_batch * n_in * 4), oyin = take((size_t)max_batch * n_out * 4),
                  oloss = take(((size_t)max_batch * maxw / 256 + 1) * 4), oerr = take(sizeof(int));
     if (cudaMalloc(&h->arena, bytes) != cudaSuccess) {
@@ -910,9 +1063,16 @@ int sl_mlp_create(int n_in, int hidden, int hidden_layers, int n_out, int max_ba
     }
     char* b = static_cast<char*>(h->arena);
     h->P = (float*)(b + oP); h->G = (float*)(b + oG); h->Mom = (float*)(b + oM); h->Var = (float*)(b + oV);
-    h->Pb = (bf16*)(b + oPb); h->mask = (uint8_t*)(b + oMask); h->Wt = (bf16*)(b + oWt);
-    for (int l = 0; l < h->nl; ++l) { h->X.push_back((bf16*)(b + oX[l])); h->Z.push_back((float*)(b + oZ[l])); }
-    h->dZ = (bf16*)(b + odZ); h->dZt = (bf16*)(b + odZt); h->Xt = (bf16*)(b + oXt); h->dX = (float*)(b + odX);
+    h->Pb = (bf16*)(b + oPb); h->mask = (uint8_t*)(b + oMask); h->Wt = (bf16*)(b + oWt); h->at = (LayerAt*)(b + oAt);
+    for (int l = 0; l < h->nl; ++l) {
+        h->X.push_back((bf16*)(b + oX[l]));
+        h->Xt.push_back((bf16*)(b + oXt[l]));
+        h->Z.push_back((float*)(b + oZ[l]));
+    }
+    for (int k = 0; k < 2; ++k) {
+        h->dZ[k] = (bf16*)(b + odZ) + (size_t)(2 * k) * max_batch * maxw;
+        h->dZt[k] = h->dZ[k] + (size_t)max_batch * maxw;
+    }
     h->xin = (float*)(b + oxin); h->yin = (float*)(b + oyin); h->loss_part = (float*)(b + oloss);
     h->d_err = (int*)(b + oerr);
     cudaMemset(h->arena, 0, bytes);
@@ -934,8 +1094,12 @@ int sl_mlp_create(int n_in, int hidden, int hidden_layers, int n_out, int max_ba
     }
     cudaMemcpy(h->P, p.data(), off * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(h->mask, mk.data(), off, cudaMemcpyHostToDevice);
-    to_bf16_kernel<<<(int)((off + 255) / 256), 256>>>(h->P, h->Pb, (int)off);
-    if (cudaDeviceSynchronize() != cudaSuccess) {
+    std::vector<LayerAt> at(h->nl);
+    for (int l = 0; l < h->nl; ++l) at[l] = {(long long)h->w_off[l], h->din[l], h->dout[l]};
+    cudaMemcpy(h->at, at.data(), at.size() * sizeof(LayerAt), cudaMemcpyHostToDevice);
+    to_bf16_kernel<<<(int)((off + 255) / 256), 256>>>(h->P, h->Pb, h->Wt, h->at, h->nl, (int)off);
+    if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaDeviceSynchronize() != cudaSuccess) {
         sl_mlp_destroy(h);
         return sl_record_error(SL_ERR_CUDA, "MLP initialisation failed");
     }
@@ -952,6 +1116,8 @@ int sl_mlp_destroy(sl_mlp* h)
 {
     if (!h) return SL_OK;
     if (h->arena) cudaFree(h->arena);
+    if (h->epoch) cudaFree(h->epoch);
+    if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return SL_OK;
 }
@@ -976,7 +1142,7 @@ int sl_mlp_set_params(sl_mlp* h, const float* params)
     if (!h || !params) return sl_record_error(SL_ERR_ARG, "null argument");
     if (cudaMemcpy(h->P, params, h->nparam * 4, cudaMemcpyHostToDevice) != cudaSuccess)
         return sl_record_error(SL_ERR_CUDA, "copy failed");
-    to_bf16_kernel<<<(int)((h->nparam + 255) / 256), 256>>>(h->P, h->Pb, (int)h->nparam);
+    to_bf16_kernel<<<(int)((h->nparam + 255) / 256), 256>>>(h->P, h->Pb, h->Wt, h->at, h->nl, (int)h->nparam);
     if (cudaDeviceSynchronize() != cudaSuccess) return sl_record_error(SL_ERR_CUDA, "bf16 refresh failed");
     return SL_OK;
 }
@@ -987,8 +1153,9 @@ int sl_mlp_gradients(sl_mlp* h, const float* x, const float* y, int M, float* gr
         return sl_record_error(SL_ERR_ARG, "M must be a multiple of 32 up to max_batch");
     cudaMemcpy(h->xin, x, (size_t)M * h->n_in * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(h->yin, y, (size_t)M * h->n_out * 4, cudaMemcpyHostToDevice);
-    forward(h, M, nullptr);
-    backward(h, M, nullptr);
+    const BatchInput in = pack_batch(h, h->xin, h->yin, M, M, nullptr);
+    forward(h, in, M, true, nullptr);
+    backward(h, in, M, nullptr);
     if (cudaDeviceSynchronize() != cudaSuccess) return sl_record_error(SL_ERR_CUDA, "MLP step failed");
     if (int r = mlp_status(h, "sl_mlp_gradients")) return r;
     if (grads) cudaMemcpy(grads, h->G, h->nparam * 4, cudaMemcpyDeviceToHost);
@@ -1012,39 +1179,86 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
     std::vector<int> idx(n);
     for (int i = 0; i < n; ++i) idx[i] = i;
     std::mt19937_64 rng(seed);
-    std::vector<float> xb((size_t)batch * h->n_in), yb((size_t)batch * h->n_out);
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const int ldo = h->dout[h->nl - 1];
+    const int ld0 = h->din[0], ldo = h->dout[h->nl - 1];
     const int nb = (batch * ldo + 255) / 256;
-    std::vector<float> part(nb);
-    int rc = SL_OK;
-    for (int ep = 0; ep < epochs && rc == SL_OK; ++ep) {
-        std::shuffle(idx.begin(), idx.end(), rng);
-        double ls = 0;
-        int steps = 0;
-        for (int s0 = 0; s0 + batch <= n; s0 += batch) {
-            for (int r = 0; r < batch; ++r) {
-                std::memcpy(&xb[(size_t)r * h->n_in], &x[(size_t)idx[s0 + r] * h->n_in], h->n_in * 4);
-                std::memcpy(&yb[(size_t)r * h->n_out], &y[(size_t)idx[s0 + r] * h->n_out], h->n_out * 4);
-            }
-            cudaMemcpyAsync(h->xin, xb.data(), xb.size() * 4, cudaMemcpyHostToDevice, nullptr);
-            cudaMemcpyAsync(h->yin, yb.data(), yb.size() * 4, cudaMemcpyHostToDevice, nullptr);
-            forward(h, batch, nullptr);
-            backward(h, batch, nullptr);
-            ++h->step;
-            const float c1 = 1.0f - std::pow(b1, (float)h->step), c2 = 1.0f - std::pow(b2, (float)h->step);
-            adam_kernel<<<(int)((h->nparam + 255) / 256), 256>>>(h->P, h->G, h->Mom, h->Var, h->Pb, h->mask,
-                                                                 (int)h->nparam, lr, b1, b2, eps, c1, c2);
-            cudaMemcpy(part.data(), h->loss_part, nb * 4, cudaMemcpyDeviceToHost);
-            double s = 0;
-            for (float v : part) s += v;
-            ls += s / ((double)batch * h->n_out);
-            ++steps;
+    const int steps = n / batch, rows = steps * batch;
+
+    // the data set on the device, and each epoch's rows in its order
+    size_t bytes = 0;
+    auto take = [&](size_t b) { size_t o = bytes; bytes = (bytes + b + 255) / 256 * 256; return o; };
+    const size_t ox = take((size_t)n * h->n_in * 4), oy = take((size_t)n * h->n_out * 4), oidx = take((size_t)rows * 4),
+                 oxp = take((size_t)rows * ld0 * 2), oxt = take((size_t)rows * ld0 * 2),
+                 oyp = take((size_t)rows * h->n_out * 4), ocoef = take((size_t)steps * sizeof(float2)),
+                 oloss = take((size_t)steps * nb * 4), ostep = take(sizeof(int));
+    if (bytes > h->epoch_bytes) {
+        if (h->epoch) cudaFree(h->epoch);
+        h->epoch = nullptr;
+        h->epoch_bytes = 0;
+        if (cudaMalloc(&h->epoch, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return sl_record_error(SL_ERR_ALLOC, "sl_mlp_train: cudaMalloc of the data set failed");
         }
-        if (cudaGetLastError() != cudaSuccess) rc = sl_record_error(SL_ERR_CUDA, "training kernel failed");
+        h->epoch_bytes = bytes;
+    }
+    char* e = static_cast<char*>(h->epoch);
+    float *dx = (float*)(e + ox), *dy = (float*)(e + oy), *yp = (float*)(e + oyp), *dloss = (float*)(e + oloss);
+    int *didx = (int*)(e + oidx), *dstep = (int*)(e + ostep);
+    bf16 *xp = (bf16*)(e + oxp), *xt = (bf16*)(e + oxt);
+    float2* dcoef = (float2*)(e + ocoef);
+    cudaStream_t st = h->stream;
+    cudaMemcpyAsync(dx, x, (size_t)n * h->n_in * 4, cudaMemcpyHostToDevice, st);
+    cudaMemcpyAsync(dy, y, (size_t)n * h->n_out * 4, cudaMemcpyHostToDevice, st);
+
+    // one step as a graph: it finds its rows by the step counter
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    const BatchInput in{xp, xt, yp, rows, dstep, dloss};
+    bool ok = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    if (ok) {
+        forward(h, in, batch, true, st);
+        backward(h, in, batch, st);
+        adam_kernel<<<(int)((h->nparam + 255) / 256), 256, 0, st>>>(h->P, h->G, h->Mom, h->Var, h->Pb, h->Wt, h->at,
+                                                                    h->nl, h->mask, (int)h->nparam, lr, b1, b2, eps,
+                                                                    dcoef, dstep, -1);
+        ok = cudaStreamEndCapture(st, &graph) == cudaSuccess && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+    }
+    if (graph) cudaGraphDestroy(graph);
+    int rc = ok ? SL_OK : sl_record_error(SL_ERR_CUDA, "sl_mlp_train: the step's graph could not be made");
+
+    std::vector<float> part((size_t)steps * nb);
+    std::vector<float2> coef(steps);
+    std::vector<int> next(idx);
+    std::shuffle(next.begin(), next.end(), rng);
+    for (int ep = 0; ep < epochs && rc == SL_OK; ++ep) {
+        idx.swap(next);
+        for (int k = 0; k < steps; ++k) {
+            ++h->step;
+            coef[k] = make_float2(1.0f - std::pow(b1, (float)h->step), 1.0f - std::pow(b2, (float)h->step));
+        }
+        cudaMemcpyAsync(didx, idx.data(), (size_t)rows * 4, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(dcoef, coef.data(), coef.size() * sizeof(float2), cudaMemcpyHostToDevice, st);
+        cudaMemsetAsync(dstep, 0, sizeof(int), st);
+        pack_kernel<<<(rows + 127) / 128, 128, 0, st>>>(dx, dy, didx, rows, n, h->n_in, h->n_out, ld0, xp, xt, yp);
+        for (int k = 0; k < steps; ++k) cudaGraphLaunch(exec, st);
+        if (ep + 1 < epochs) {  // the next epoch's order, under this one's steps
+            next = idx;
+            std::shuffle(next.begin(), next.end(), rng);
+        }
+        cudaMemcpyAsync(part.data(), dloss, part.size() * 4, cudaMemcpyDeviceToHost, st);
+        if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
+            rc = sl_record_error(SL_ERR_CUDA, "training kernel failed");
+            break;
+        }
+        double ls = 0;
+        for (int k = 0; k < steps; ++k) {
+            double s = 0;
+            for (int i = 0; i < nb; ++i) s += part[(size_t)k * nb + i];
+            ls += s / ((double)batch * h->n_out);
+        }
         if (loss_per_epoch) loss_per_epoch[ep] = (float)(ls / std::max(1, steps));
     }
-    if (cudaDeviceSynchronize() != cudaSuccess && rc == SL_OK) rc = sl_record_error(SL_ERR_CUDA, "training failed");
+    if (exec) cudaGraphExecDestroy(exec);
     if (rc == SL_OK) rc = mlp_status(h, "sl_mlp_train");
     return rc;
 }
@@ -1077,9 +1291,8 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
     for (int s0 = 0; s0 < n; s0 += B) {
         const int M = std::min(B, n - s0);
         const int Mp = (M + 31) / 32 * 32;
-        cudaMemset(h->xin, 0, (size_t)Mp * h->n_in * 4);
         cudaMemcpy(h->xin, x + (size_t)s0 * h->n_in, (size_t)M * h->n_in * 4, cudaMemcpyHostToDevice);
-        forward(h, Mp, nullptr);
+        forward(h, pack_batch(h, h->xin, nullptr, M, Mp, nullptr), Mp, false, nullptr);
         if (cudaMemcpy(zb.data(), h->Z[L - 1], (size_t)M * ldo * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
             return sl_record_error(SL_ERR_CUDA, "prediction failed");
         if (int r = mlp_status(h, "sl_mlp_predict")) return r;
@@ -1119,8 +1332,18 @@ extern "C" int sl_diag_gemm_bf16(int M, int N, int K, const uint16_t* A, const u
     cudaMemset(dErr, 0, sizeof(int));
     if (kernel == 0) {
         gemm_mma_sync(nullptr, dA, K, dB, K, dBias, dC, dCb, N, M, N, K, act);
-    } else if (!gemm_tc(nullptr, dA, K, dB, K, dBias, dC, dCb, N, M, N, K, act, dErr)) {
-        rc = sl_record_error(SL_ERR_CUDA, "sl_diag_gemm_bf16: tensor map or launch setup failed");
+    } else {
+        GemmLaunch L{};
+        L.njobs = 1;
+        L.err = dErr;
+        bool ok = make_job(&L.job[0], dA, M, K, dB, K, K, M, N, K);
+        L.job[0].bias = dBias;
+        L.job[0].cf = dC;
+        L.job[0].cb = dCb;
+        L.job[0].ldc = N;
+        L.job[0].act = act;
+        ok = ok && launch_gemm(L, nullptr);
+        if (!ok) rc = sl_record_error(SL_ERR_CUDA, "sl_diag_gemm_bf16: tensor map or launch setup failed");
     }
     if (rc == SL_OK) {
         cudaError_t e = cudaDeviceSynchronize();
