@@ -71,6 +71,8 @@ __global__ void __launch_bounds__(kDriftThreads) drift_kernel(const __grid_const
 // owns sphere B = 32Y + b and walks the 32 spheres A = 32X + a of the A
 // block; on the diagonal only a > b is a pair.  Tiles are independent; one
 // launch covers the tiles of block columns [c0, c1) with a static stride.
+constexpr int kStripRows = 8, kStrips = kBlock / kStripRows;
+
 // Tiles in column-major order: column Y holds tiles (Y..nb-1, Y); the first
 // tile of column c has index c*nb - c(c-1)/2.
 __device__ __forceinline__ long long col_offset(int nb, int c) { return (long long)c * nb - (long long)c * (c - 1) / 2; }
@@ -87,51 +89,80 @@ __device__ __forceinline__ void col_tile_coords(int nb, long long u, int& X, int
     X = c + (int)(u - col_offset(nb, c));
 }
 
+// A work item is a whole tile, or -- the tiles from `split` on, in the
+// column-major order -- a strip of 8 of its 32 rows (pair_split).  The items
+// of a launch are numbered from its first tile's; item q's energy goes to
+// pe_tile[q].
 template <bool WRITE>
 __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
-                                                          int phase)
+                                                          int phase, long long split)
 {
     __shared__ TileScratch scratch[4];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     TileScratch& ws = scratch[wib];
-    const long long nwarps = (long long)gridDim.x * 4;
+    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
 
-    // A first round of tiles in warp order; then whichever warp is free takes
-    // the next tile from the launch's counter (zeroed by the drift kernel),
-    // or, without a counter, the static stride.  A tile's results do not
+    // A first round of items in warp order; then whichever warp is free takes
+    // the next one from the launch's counter (zeroed by the drift kernel),
+    // or, without a counter, the static stride.  An item's results do not
     // depend on the warp that computes it.
-    const long long u0 = col_offset(s.nb, c0), u1 = col_offset(s.nb, c1);
+    const auto first_item = [split](long long u) { return u <= split ? u : split + (u - split) * kStrips; };
+    const long long q0 = first_item(col_offset(s.nb, c0)), q1 = first_item(col_offset(s.nb, c1));
     int* counter = s.tile_counter ? s.tile_counter + phase : nullptr;
-    for (long long u = u0 + (long long)blockIdx.x * 4 + wib; u < u1;) {
+    for (long long q = q0 + (long long)blockIdx.x * (blockDim.x >> 5) + wib; q < q1;) {
+        const bool whole = q < split;
+        const long long u = whole ? q : split + (q - split) / kStrips;
+        const int strip = whole ? 0 : (int)((q - split) % kStrips);
         int X, Y;
         col_tile_coords(s.nb, u, X, Y);
-        const long long t = (long long)X * (X + 1) / 2 + Y;  // this tile's PE slot
         load_a(s, ws.ab, lane, X * kBlock + lane);  // < npad always
         __syncwarp();
         const int B = Y * kBlock + lane;
+        const int a_end = min(kBlock, s.n - X * kBlock);
+        const int a0 = whole ? 0 : strip * kStripRows, a1 = whole ? a_end : min(a_end, a0 + kStripRows);
         double pe = 0;
         uint32_t rowbits, colbits;
-        tile_pairs<WRITE>(s, ws, X, Y, lane, 0, min(kBlock, s.n - X * kBlock), B, B < s.n, pe, rowbits, colbits);
+        tile_pairs<WRITE>(s, ws, X, Y, lane, a0, a1, B, B < s.n, pe, rowbits, colbits);
         // Contact bits: row A = 32X + lane gets block Y's bits, row B gets
         // block X's bits; on the diagonal both describe row 32X + lane.
-        if (X == Y) {
-            s.cmask[(size_t)(X * kBlock + lane) * s.nb + X] = rowbits | colbits;
+        uint32_t* wa = s.cmask + (size_t)(X * kBlock + lane) * s.nb + Y;
+        uint32_t* wb = s.cmask + (size_t)(Y * kBlock + lane) * s.nb + X;
+        if (whole) {
+            if (X == Y) {
+                *wa = rowbits | colbits;
+            } else {
+                *wa = rowbits;
+                *wb = colbits;
+            }
         } else {
-            s.cmask[(size_t)(X * kBlock + lane) * s.nb + Y] = rowbits;
-            s.cmask[(size_t)(Y * kBlock + lane) * s.nb + X] = colbits;
+            // strip w holds rows 8w .. 8w + 7: those rows' words, and byte w
+            // of every column's word.  On the diagonal, row i of strip w has
+            // its bytes below w from rowbits, byte w from both, and those
+            // above from the later strips' columns.
+            static_assert(kStripRows == 8, "a strip's column bits are one byte");
+            uint8_t* ba = reinterpret_cast<uint8_t*>(wa);
+            const int mine = lane / kStripRows;
+            if (X != Y) {
+                if (mine == strip) *wa = rowbits;
+                reinterpret_cast<uint8_t*>(wb)[strip] = (uint8_t)(colbits >> (8 * strip));
+            } else if (mine == strip) {
+                for (int k = 0; k <= strip; ++k) ba[k] = (uint8_t)((rowbits | colbits) >> (8 * k));
+            } else if (mine < strip) {
+                ba[strip] = (uint8_t)(colbits >> (8 * strip));
+            }
         }
         if (WRITE) {
             for (int off = 16; off > 0; off >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, off);
-            if (lane == 0) s.pe_tile[t] = pe;
+            if (lane == 0) s.pe_tile[q] = pe;
         }
         __syncwarp();
         if (counter) {
             int next = 0;
             if (lane == 0) next = atomicAdd(counter, 1);
-            u = u0 + nwarps + __shfl_sync(0xffffffffu, next, 0);
+            q = q0 + nwarps + __shfl_sync(0xffffffffu, next, 0);
         } else {
-            u += nwarps;
+            q += nwarps;
         }
     }
 }
@@ -204,13 +235,16 @@ __global__ void __launch_bounds__(kRowThreads) rowsum_kernel(const __grid_consta
 // ------------------------------------------------------ energy totals -----
 constexpr int kRedThreads = 256;
 
-// Per-sphere KE, mom, ang_mom terms (:282-285) reduced over a fixed tree:
-// block b sums spheres [b*chunk, (b+1)*chunk) into red[b][0..6].
+// Per-sphere KE, mom, ang_mom terms (:282-285) and the items' PE reduced over a
+// fixed tree: block b sums spheres [b*chunk, (b+1)*chunk) into red[b][0..6] and
+// its share of pe_tile into red[b][7].
 __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __grid_constant__ System s, int chunk)
 {
-    __shared__ double sh[7][kRedThreads];
+    __shared__ double sh[8][kRedThreads];
     const int tid = threadIdx.x;
-    double v[7] = {0, 0, 0, 0, 0, 0, 0};
+    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (long long t = (long long)blockIdx.x * kRedThreads + tid; t < s.nitems; t += (long long)gridDim.x * kRedThreads)
+        v[7] += s.pe_tile[t];
     const int beg = blockIdx.x * chunk, end = min(s.n, beg + chunk);
     for (int i = beg + tid; i < end; i += kRedThreads) {
         const double m = s.m[i], moi = s.moi[i];
@@ -223,28 +257,6 @@ __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __gri
         v[4] += m * cx + moi * wx; v[5] += m * cy + moi * wy; v[6] += m * cz + moi * wz;
     }
 #pragma unroll
-    for (int k = 0; k < 7; ++k) sh[k][tid] = v[k];
-    __syncthreads();
-    for (int off = kRedThreads / 2; off > 0; off >>= 1) {
-        if (tid < off) {
-#pragma unroll
-            for (int k = 0; k < 7; ++k) sh[k][tid] += sh[k][tid + off];
-        }
-        __syncthreads();
-    }
-    if (tid < 7) s.red[blockIdx.x * 8 + tid] = sh[tid][0];
-}
-
-// Final totals: PE over all tile partials, the rest over the block partials.
-__global__ void __launch_bounds__(kRedThreads) energy_final_kernel(const __grid_constant__ System s, int nred)
-{
-    __shared__ double sh[8][kRedThreads];
-    const int tid = threadIdx.x;
-    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (long long t = tid; t < s.nitems; t += kRedThreads) v[0] += s.pe_tile[t];
-    for (int b = tid; b < nred; b += kRedThreads)
-        for (int k = 0; k < 7; ++k) v[k + 1] += s.red[b * 8 + k];
-#pragma unroll
     for (int k = 0; k < 8; ++k) sh[k][tid] = v[k];
     __syncthreads();
     for (int off = kRedThreads / 2; off > 0; off >>= 1) {
@@ -254,7 +266,18 @@ __global__ void __launch_bounds__(kRedThreads) energy_final_kernel(const __grid_
         }
         __syncthreads();
     }
-    if (tid < 8) s.energy[tid] = sh[tid][0];
+    if (tid < 8) s.red[blockIdx.x * 8 + tid] = sh[tid][0];
+}
+
+// Final totals over the block partials, in block order.
+__global__ void __launch_bounds__(32) energy_final_kernel(const __grid_constant__ System s, int nred)
+{
+    const int k = threadIdx.x;
+    if (k >= 8) return;
+    double v = 0;
+#pragma unroll 8
+    for (int b = 0; b < nred; ++b) v += s.red[b * 8 + k];
+    s.energy[k == 7 ? 0 : k + 1] = v;
 }
 
 // Per-sphere derived constants (exact scalings and correctly rounded
@@ -386,7 +409,7 @@ void launch_energy(const System& s, cudaStream_t st)
     const int nred = kRedBlocks;
     const int chunk = (s.n + nred - 1) / nred;
     energy_partial_kernel<<<nred, kRedThreads, 0, st>>>(s, chunk);
-    energy_final_kernel<<<1, kRedThreads, 0, st>>>(s, nred);
+    energy_final_kernel<<<1, 32, 0, st>>>(s, nred);
 }
 
 static void launch_rowsum(const System& s, cudaStream_t st, const CUtensorMap* map, int b0, int b1, int first,
@@ -398,31 +421,57 @@ static void launch_rowsum(const System& s, cudaStream_t st, const CUtensorMap* m
         rowsum_kernel<<<(3 * s.n + kRowThreads - 1) / kRowThreads, kRowThreads, 0, st>>>(s, b0, b1, first, last);
 }
 
-static void launch_pair_columns(const System& s, bool write, int num_sms, cudaStream_t st, int c0, int c1, int phase)
+// The first tile (in the column-major order) that is taken in strips of 8
+// rows.  A strip costs its share of a tile and ~12% more (its own blocks, and
+// a quarter of the marked pairs in a warp of their own), and pays where the
+// warps are not all busy to the end.  Of the 16 warps per SM that are
+// resident, with T tiles (us per step, GB300, no strips against these):
+//   - T up to half of them: all tiles.  The step is a warp's latency, 32 rows of
+//     ~1500 cycles.  N=96 65.5 -> 30.9, N=300 69.8 -> 34.8, N=1000 111 -> 85,
+//     N=1400 128 -> 115.
+//   - more: as many as half the warps, the last ones, which shortens the tail:
+//     N=1733 162 -> 152, N=3000 311 -> 305, N=5000 692.6 -> 688.5.
+//   - a last round that is nearly full without them: none.  N=2200 (99% full):
+//     199, 205 with them.
+long long pair_split(long long tiles, int num_sms)
 {
-    const long long tiles = ((long long)c1 * s.nb - (long long)c1 * (c1 - 1) / 2) -
-                            ((long long)c0 * s.nb - (long long)c0 * (c0 - 1) / 2);
-    const int pb = pair_grid_blocks(tiles, num_sms);
-    if (write)
-        pair_tile_kernel<true><<<pb, 128, 0, st>>>(s, c0, c1, phase);
-    else
-        pair_tile_kernel<false><<<pb, 128, 0, st>>>(s, c0, c1, phase);
+    const long long warps = 16LL * num_sms;
+    if (2 * tiles <= warps) return 0;
+    return 10 * (tiles % warps) > 9 * warps ? tiles : tiles - warps / 2;
 }
 
-void launch_step(const System& s, bool write, int num_sms, cudaStream_t st, StepTimers* tm, const StepOverlap* ov,
+static void launch_pair_columns(const System& s, bool write, int num_sms, cudaStream_t st, int c0, int c1, int phase,
+                                long long split)
+{
+    const auto offset = [&](int c) { return (long long)c * s.nb - (long long)c * (c - 1) / 2; };
+    const long long t0 = offset(c0), t1 = offset(c1), cut = min(max(split, t0), t1);
+    const long long items = (cut - t0) + kStrips * (t1 - cut);
+    // few items: one warp per CTA, so that they spread over the SMs
+    const int warps = items <= 4LL * num_sms ? 1 : 4;
+    const int pb = (int)min((items + warps - 1) / warps, (long long)num_sms * 4);
+    if (write)
+        pair_tile_kernel<true><<<pb, 32 * warps, 0, st>>>(s, c0, c1, phase, split);
+    else
+        pair_tile_kernel<false><<<pb, 32 * warps, 0, st>>>(s, c0, c1, phase, split);
+}
+
+void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, StepTimers* tm, const StepOverlap* ov,
                  const CUtensorMap* map, bool int_adds)
 {
-    launch_drift(s, st);
-    if (tm) cudaEventRecord(tm->ev[0], st);
+    System s = sys;
     int cb[kPairPhases + 1];
     const int np = ov ? phase_bounds(s.nb, cb) : 1;
+    const long long split = pair_split(s.ntiles, num_sms);  // the same items, and energy sums, with and without phases
+    s.nitems = split + kStrips * (s.ntiles - split);
+    launch_drift(s, st);
+    if (tm) cudaEventRecord(tm->ev[0], st);
     if (np <= 1) {
-        launch_pair_columns(s, write, num_sms, st, 0, s.nb, 0);
+        launch_pair_columns(s, write, num_sms, st, 0, s.nb, 0, split);
         if (tm) cudaEventRecord(tm->ev[1], st);
         launch_rowsum(s, st, map, 0, s.nb, 1, 1, num_sms, int_adds);
     } else {
         for (int p = 0; p < np; ++p) {
-            launch_pair_columns(s, write, num_sms, st, cb[p], cb[p + 1], p);
+            launch_pair_columns(s, write, num_sms, st, cb[p], cb[p + 1], p, split);
             cudaEventRecord(ov->phase[p], st);
             cudaStreamWaitEvent(ov->side, ov->phase[p], 0);
             launch_rowsum(s, ov->side, map, cb[p], cb[p + 1], p == 0, p == np - 1, num_sms, int_adds);

@@ -49,7 +49,7 @@ def _uniform(n):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("make,n", [(_lattice, 100), (_packed, 64), (_packed, 37), (_no_cohesion, 97), (_light, 65),
-                                    (_equal_radii, 130), (_uniform, 31), (_uniform, 97), (_uniform, 400)])
+                                    (_equal_radii, 130), (_uniform, 31), (_uniform, 97), (_uniform, 400), (_packed, 250)])
 def test_tile_paths_bit_identical(make, n):
     from oracle.oracle import CpuOracle
     from spacelab_gb300 import BallGroup, GpuStep
@@ -73,3 +73,32 @@ def test_tile_paths_bit_identical(make, n):
         st = o.state()
         for k in ("pos", "vel", "w", "acc", "aacc"):
             assert np.array_equal(getattr(sim.group, k), st[k]), k
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [8, 9, 63, 1560, 1577, 2208, 2300])
+def test_strips_bit_identical(n):
+    """Tiles taken whole and in strips of 8 rows (pair_split): all of them (up
+    to N=1560 on 152 SMs), the last ones (N=1577: the first system with whole
+    tiles), none (N=2208), the last ones of a second round (N=2300); state and
+    contacts against the oracle over three steps, one of them a write step."""
+    from cases import material
+    from oracle.oracle import CpuOracle
+    from spacelab_gb300 import BallGroup, GpuStep
+    c = contact_case(n, 9)
+    o = CpuOracle(c["pos"], c["vel"], c["w"], c["R"], c["m"], c["moi"], OracleMaterial(), c["dt"], c["kin"], c["kout"])
+    g = BallGroup.from_arrays(c["pos"], c["vel"], c["w"], c["R"], c["m"], c["moi"])
+    with GpuStep(g, material(), "exact") as sim:
+        sim.set_scalars(c["dt"], c["kin"], c["kout"])
+        sim.init_conditions()
+        o.init()
+        for k in range(1, 4):
+            assert np.array_equal(sim.contacts(), o.contacts()), k
+            e, eo = sim.sim_one_step(k == 2), o.step(k == 2)
+            if e is not None:
+                assert abs(e.PE - eo[0]) <= 1e-10 * max(abs(eo[0]), abs(eo[1]))
+                assert abs(e.KE - eo[1]) <= 1e-12 * abs(eo[1])
+        sim.download()
+        st = o.state()
+        for key in ("pos", "vel", "w", "acc", "aacc"):
+            assert np.array_equal(getattr(sim.group, key), st[key]), key
