@@ -457,26 +457,17 @@ def run_ours(args, rank, world, local_rank) -> dict | None:
     nsm = torch.cuda.get_device_properties(local_rank).multi_processor_count
     sm_max = (clk.get("sm_max_mhz") or 2070.0) * 1e6
     pk = ctypes.c_double()
-    if args.mode in ("exact", "mixed"):
-        # both run on the FP64 pipe: the exact form's pair arithmetic, and
-        # the mixed form's 9 FP64 adds per pair (r, and the two spheres'
-        # FP64 sums), one FP64 lane-op each
+    if args.mode == "exact":
         peak_fn = "sl_diag_fp64_peak"
         _lib.check(lib.sl_diag_fp64_peak(ctypes.byref(pk)), peak_fn)
-        if args.mode == "exact":
-            work, unit = flops_launch, "TFLOP/s"
-            peak = pk.value / 1e3
-            peak_source = "measured live: FP64 FMA chains (sl_diag_fp64_peak), 2 flops per FMA"
-            nominal = nsm * 2 * 2 * sm_max / 1e12
-            nominal_source = f"{nsm} SMs x 2 FP64 FMA/clock x 2 flops x {sm_max / 1e6:.0f} MHz"
-            bound = "fp64"
-        else:
-            work, unit = F.MIXED64_FP64_OPS_PER_PAIR * w.pairs_per_step, "T FP64 lane-ops/s"
-            peak = pk.value / 2 / 1e3
-            peak_source = "measured live: FP64 FMA chains (sl_diag_fp64_peak), one lane-op per FMA"
-            nominal = nsm * 2 * sm_max / 1e12
-            nominal_source = f"{nsm} SMs x 2 FP64 lane-ops/clock x {sm_max / 1e6:.0f} MHz"
-            bound = "fp64 (adds)"
+        # the additions the kernel leaves on the FP64 pipe, its busiest unit;
+        # the rest of a pair's operations are rounded in integer arithmetic
+        work, unit = F.EXACT_FP64_OPS_PER_PAIR * w.pairs_per_step, "T FP64 lane-ops/s"
+        peak = pk.value / 2 / 1e3
+        peak_source = "measured live: FP64 FMA chains (sl_diag_fp64_peak), one lane-op per FMA"
+        nominal = nsm * 2 * sm_max / 1e12
+        nominal_source = f"{nsm} SMs x 2 FP64 lane-ops/clock x {sm_max / 1e6:.0f} MHz"
+        bound = "fp64 (adds), integer issue next to it"
     else:
         peak_fn = "sl_diag_fp32_peak"
         _lib.check(lib.sl_diag_fp32_peak(ctypes.byref(pk)), peak_fn)

@@ -247,12 +247,12 @@ int sl_create(int n, const sl_material* mat, int mode, sl_handle** out)
         for (int c = 0; c < 3; ++c) o_vec[v][c] = take(np * sizeof(double));
     size_t o_sc[8];
     for (int k = 0; k < 8; ++k) o_sc[k] = take(np * sizeof(double));
-    // FP32 per-sphere constants (both mixed forms) and the double-float
-    // positions (SL_MODE_MIXED_DF only)
+    // FP32 per-sphere constants and the positions in FP32 parts: two
+    // (SL_MODE_MIXED_DF), three (SL_MODE_MIXED)
     const bool mixed = mode != SL_MODE_EXACT;
     const bool mixed_df = mode == SL_MODE_MIXED_DF;
-    size_t o_f[10] = {};
-    for (int k = 0; k < 10; ++k) o_f[k] = take(mixed && (k < 4 || mixed_df) ? np * sizeof(float) : 0);
+    size_t o_f[13] = {};
+    for (int k = 0; k < 13; ++k) o_f[k] = take(mixed && (k < 10 || !mixed_df) ? np * sizeof(float) : 0);
     // the mixed forms keep per-tile partial sums instead of pair terms (FP64
     // in SL_MODE_MIXED, FP32 in SL_MODE_MIXED_DF), and torque terms in the
     // same type
@@ -286,8 +286,8 @@ int sl_create(int n, const sl_material* mat, int mode, sl_handle** out)
         s.f_inv_moi = reinterpret_cast<float*>(base + o_f[2]);
         s.f_Rlo = reinterpret_cast<float*>(base + o_f[3]);
     }
-    if (mixed_df)
-        for (int k = 0; k < 6; ++k) s.f_pos[k] = reinterpret_cast<float*>(base + o_f[4 + k]);
+    if (mixed)
+        for (int k = 0; k < (mixed_df ? 6 : 9); ++k) s.f_pos[k] = reinterpret_cast<float*>(base + o_f[4 + k]);
     if (mixed_df)
         s.f_part = reinterpret_cast<float*>(base + o_pair);
     else if (mixed)

@@ -67,8 +67,9 @@ struct System {
     float *f_R, *f_inv_m, *f_inv_moi;
     // and double-float (hi + lo) copies of the scaled radii's low parts and
     // of the scaled positions (x, y, z hi, then x, y, z lo), the latter
-    // written by the drift kernel every step
-    float *f_Rlo, *f_pos[6];
+    // written by the drift kernel every step; the FP64-accumulating mixed form
+    // has a third part, which holds the FP64 positions whole
+    float *f_Rlo, *f_pos[9];
     // the double-float mixed form's per-tile partial sums [3][nb][npad]
     // (FP32): entry (c, K, i) is component c of sphere i's acceleration terms
     // from the partners in 32-sphere block K

@@ -59,10 +59,14 @@ __global__ void __launch_bounds__(kDriftThreads) drift_kernel(const __grid_const
     s.wh.c[c][i] = whc;
     s.prev.c[c][i] = p;  // positions the pair distances of the previous step were taken at
     s.pos.c[c][i] = pn;
-    if (s.f_pos[0]) {  // mixed form: scaled position as double-float hi + lo
+    if (s.f_pos[0]) {  // mixed forms: scaled position as FP32 parts
+        const double unit = ldexp(1.0, s.len_shift);
         const float hi = d2f_bits(pn, s.len_shift);
+        const double rem = pn - f2d_bits(hi) * unit;  // exact, as is the next
+        const float lo = d2f_bits(rem, s.len_shift);
         s.f_pos[c][i] = hi;
-        s.f_pos[3 + c][i] = d2f_bits(pn - f2d_bits(hi) * ldexp(1.0, s.len_shift), s.len_shift);
+        s.f_pos[3 + c][i] = lo;
+        if (s.f_pos[6]) s.f_pos[6 + c][i] = d2f_bits(rem - f2d_bits(lo) * unit, s.len_shift);
     }
 }
 

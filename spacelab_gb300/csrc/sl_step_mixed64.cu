@@ -5,38 +5,42 @@
 //   * positions and the whole integration: drift_kernel (pass 1, shared with
 //     the exact form) and pass 3 in mixed64_finish_kernel
 //     (ColliderSingleCore.cpp:82-97, 263-267);
-//   * the pair subtraction r = pos[B] - pos[A] (:105), one FP64 add per
-//     component for every pair;
-//   * for pairs closer than far_sq (1.25 radii sums or more), |r|^2, the
-//     squared gap g = (R_A + R_B)^2 - |r|^2, |r| and the overlap
-//     R_A + R_B - |r| = g / (R_A + R_B + |r|) (:106-110), which sets the
+//   * the pair subtraction r = pos[B] - pos[A] (:105): the FP64 positions are
+//     held as three FP32 parts (72 bits, written by the drift), whose
+//     differences give r rounded once to FP32 (df::sub3);
+//   * for pairs closer than far_sq (1.25 radii sums or more), r itself,
+//     |r|^2, the squared gap g = (R_A + R_B)^2 - |r|^2, |r| and the overlap
+//     R_A + R_B - |r| = g / (R_A + R_B + |r|) (:106-110) in FP64, which set the
 //     contact test, the elastic force and the clamped vdW gap; and the
 //     previous-step distance test that chooses kin or kout (:119-126);
-//   * per-sphere force and torque accumulation: every pair's force is
-//     added into FP64 sums (two FP64 adds per component per pair, one for
-//     each sphere), contact torques are summed in FP64 (:249-250, 187-188);
+//   * per-sphere force and torque accumulation: a pair's force goes into both
+//     spheres' sums over the tile's 32 partners, which carry every rounding
+//     error on (df::Sum3, more than FP64's 53 bits) and end as one FP64
+//     partial; the partials, and contact torques, are summed in FP64
+//     (:249-250, 187-188);
 //   * the write-step energies: close pairs' potential in FP64, far pairs'
 //     vdW bracket by the cancellation-free series (vdw_bracket, FP32) added
-//     into FP64 sums, and the FP64 totals.
+//     the same way, and the FP64 totals.
 // FP32 does the force and torque arithmetic on the relative displacement
-// r (rounded from FP64 to FP32 on the integer pipe) and the FP64 overlap:
-// the vdW coefficient, elastic, gravity, sliding and rolling friction and
-// the torques, in lengths scaled by 2^-len_shift.
+// r and the FP64 overlap: the vdW coefficient, elastic, gravity, sliding and
+// rolling friction and the torques, in lengths scaled by 2^-len_shift.
 //
-// The work per pair is 9 FP64 adds (3 for r, 6 for the two spheres' sums),
-// the FP32 force of a far pair (no square root: S = |r|^2 - (R_A + R_B)^2,
-// T = |r|^2 - (R_A - R_B)^2), two FP32 <-> FP64 conversions per component
-// done with integer instructions, and the tile sweep's shuffles.  GB300's
-// FP64 pipe takes a warp instruction per ~20 cycles per SM, so the FP64
-// adds bound the kernel: ~5.6 SM-cycles per pair.
+// What bounds it: FP32 issue, some 150 instructions a pair, half of them the
+// six error-free sums.  On the FP64 pipe the subtraction and the sums were 9
+// adds a pair at 19 SM-cycles each (one narrow unit per SM), 171 cycles
+// for a warp's 32 pairs, and the pair kernel ran at 0.96 of that unit's rate;
+// the FP32 pipe is 72 times as wide.  N=20000 polydisperse, 20 steps: 74.2 ->
+// 23.8 ms; 3 and 5 CTAs per SM 25.2 and 23.9, the sweep unrolled 1 and 4
+// times 24.3 and 23.6.
 //
 // Accumulation order: one warp evaluates a 32 x 32 tile in a diagonal sweep
-// (lane b holds column sphere B's FP64 sum; row r's FP64 sum travels one
-// lane down per step to meet its next term), so each sphere's terms from a
-// partner block are added in a fixed order into one FP64 partial.
+// (lane b holds column sphere B's sum; row r's sum travels one lane down per
+// step to meet its next term), so each sphere's terms from a partner block
+// are added in a fixed order into one FP64 partial.
 // mixed64_finish_kernel adds a sphere's partials over the partner blocks in
 // ascending order.  Every order is fixed, so runs repeat bit for bit.
 #include "sl_device.cuh"
+#include "sl_df.cuh"
 #include "sl_kernels.h"
 #include "sl_pair_mixed.cuh"
 
@@ -46,22 +50,18 @@ namespace sl {
 
 namespace {
 
-// Row spheres of a tile in shared memory, kRow64 doubles each: position x,
-// y, z, then the scaled radius and c_vdw R^3 as two floats in one slot, then
-// the FP64 radius.  A 10-word stride puts each half-warp's 8-byte loads of
-// 16 different rows in 32 distinct banks.
-constexpr int kRow64 = 5;
+// Row spheres of a tile in shared memory, kRow64 floats each, so that a warp's
+// 16-byte loads of 32 different rows fall in distinct banks: scaled position
+// parts x, y, z and the scaled radius, the second parts and c_vdw R^3, the
+// third parts.
+constexpr int kRow64 = 12;
 constexpr int kM64Warps = 4;
 constexpr int kM64CtasPerSm = 4;  // resident CTAs per SM (the launch bounds' minimum)
 
-__device__ __forceinline__ double pack_f2(float lo, float hi)
+// a + b + c as FP64
+__device__ __forceinline__ double total(const df::Sum3& s)
 {
-    return __hiloint2double(__float_as_int(hi), __float_as_int(lo));
-}
-
-__device__ __forceinline__ float2 unpack_f2(double d)
-{
-    return make_float2(__int_as_float(__double2loint(d)), __int_as_float(__double2hiint(d)));
+    return f2d_bits(s.a) + (f2d_bits(s.b) + f2d_bits(s.c));
 }
 
 // One warp per lower-triangular 32 x 32 block tile (X, Y), X >= Y: column
@@ -74,10 +74,10 @@ __device__ __forceinline__ float2 unpack_f2(double d)
 template <bool WRITE>
 __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_kernel(const __grid_constant__ System s)
 {
-    __shared__ __align__(16) double rows_all[kM64Warps][kBlock * kRow64];
+    __shared__ __align__(16) float rows_all[kM64Warps][kBlock * kRow64];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    double* rows = rows_all[wib];
+    float* rows = rows_all[wib];
     const long long nwarps = (long long)gridDim.x * kM64Warps;
     const size_t plane = (size_t)s.npad * s.npad;  // torque planes
     const size_t pplane = (size_t)s.nb * s.npad;   // partial planes
@@ -96,26 +96,27 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
         tile_coords(t, X, Y);
         {
             const int i = X * kBlock + lane;  // < npad
-            double* row = rows + lane * kRow64;
+            float* row = rows + lane * kRow64;
             const float Ri = s.f_R[i];
-            row[0] = s.pos.c[0][i];
-            row[1] = s.pos.c[1][i];
-            row[2] = s.pos.c[2][i];
-            row[3] = pack_f2(Ri, c_vdw * (Ri * Ri * Ri));
-            row[4] = s.R[i];
+            *reinterpret_cast<float4*>(row) = make_float4(s.f_pos[0][i], s.f_pos[1][i], s.f_pos[2][i], Ri);
+            *reinterpret_cast<float4*>(row + 4) =
+                make_float4(s.f_pos[3][i], s.f_pos[4][i], s.f_pos[5][i], c_vdw * (Ri * Ri * Ri));
+            *reinterpret_cast<float4*>(row + 8) = make_float4(s.f_pos[6][i], s.f_pos[7][i], s.f_pos[8][i], 0.0f);
         }
         __syncwarp();
         const int B = Y * kBlock + lane;
         const bool bvalid = B < s.n;
-        const double bx = s.pos.c[0][B], by = s.pos.c[1][B], bz = s.pos.c[2][B];
+        const float bx1 = s.f_pos[0][B], by1 = s.f_pos[1][B], bz1 = s.f_pos[2][B];
+        const float bx2 = s.f_pos[3][B], by2 = s.f_pos[4][B], bz2 = s.f_pos[5][B];
+        const float bx3 = s.f_pos[6][B], by3 = s.f_pos[7][B], bz3 = s.f_pos[8][B];
         const float Rbs = s.f_R[B];
         const float Rb3 = Rbs * Rbs * Rbs;
         const int nA = s.n - X * kBlock;  // rows r < nA are spheres
         double pe = 0.0;       // close pairs' potential (FP64)
-        double pe_far = 0.0;   // far pairs' vdW brackets, times -Ha/6 at the end
+        df::Sum3 pe_far{};     // far pairs' vdW brackets, times -Ha/6 at the end
         uint32_t colbits = 0;
-        double ax = 0.0, ay = 0.0, az = 0.0;     // running sum of row (lane + k) mod 32 at step k
-        double bsx = 0.0, bsy = 0.0, bsz = 0.0;  // sphere B's sum
+        df::Sum3 ra[3] = {};  // running sum of row (lane + k) mod 32 at step k
+        df::Sum3 cb[3] = {};  // sphere B's sum
         // FULL: a tile off the diagonal whose rows and columns are all spheres
         auto sweep = [&](auto full_tag) {
             constexpr bool FULL = decltype(full_tag)::value;
@@ -123,17 +124,14 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
             for (int k = 0; k < kBlock; ++k) {
                 const int r = (lane + k) & (kBlock - 1);
                 const bool valid = FULL || (bvalid && r < nA && (X != Y || lane < r));
-                const double* q = rows + r * kRow64;
-                // FP64 pair subtraction (:105)
-                const double rx64 = bx - q[0];
-                const double ry64 = by - q[1];
-                const double rz64 = bz - q[2];
-                const float2 ra = unpack_f2(q[3]);
-                const float Ras = ra.x;
-                // the FP32 force arithmetic works on r rounded to FP32 (scaled)
-                const float rx = d2f_bits(rx64, sh);
-                const float ry = d2f_bits(ry64, sh);
-                const float rz = d2f_bits(rz64, sh);
+                const float4 q1 = *reinterpret_cast<const float4*>(rows + r * kRow64);
+                const float4 q2 = *reinterpret_cast<const float4*>(rows + r * kRow64 + 4);
+                const float4 q3 = *reinterpret_cast<const float4*>(rows + r * kRow64 + 8);
+                const float Ras = q1.w;
+                // the pair subtraction (:105), rounded to FP32
+                const float rx = df::sub3(bx1, bx2, bx3, q1.x, q2.x, q3.x);
+                const float ry = df::sub3(by1, by2, by3, q1.y, q2.y, q3.y);
+                const float rz = df::sub3(bz1, bz2, bz3, q1.z, q2.z, q3.z);
                 const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
                 const float sumR = Ras + Rbs, difR = Ras - Rbs;
                 const float sum2 = sumR * sumR;
@@ -144,14 +142,17 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
                 const float S = d2 - sum2;
                 const float T = fmaf(-difR, difR, d2);
                 const float P = S * T;
-                const float fr = (ra.y * Rb3) * rcp_approx(P * P);  // |F| / |r|
+                const float fr = (q2.w * Rb3) * rcp_approx(P * P);  // |F| / |r|
                 float fx = fr * rx, fy = fr * ry, fz = fr * rz;
                 const bool closep = d2 < s.far_sq * sum2;
                 if (valid && closep) {
                     const int A = X * kBlock + r;
-                    // FP64 |r|^2, squared gap, |r| and overlap (:106-110)
+                    // FP64 r, |r|^2, squared gap, |r| and overlap (:105-110)
+                    const double rx64 = s.pos.c[0][B] - s.pos.c[0][A];
+                    const double ry64 = s.pos.c[1][B] - s.pos.c[1][A];
+                    const double rz64 = s.pos.c[2][B] - s.pos.c[2][A];
                     const double d2_64 = fma(rx64, rx64, fma(ry64, ry64, rz64 * rz64));
-                    const double Ra64 = q[4], Rb64 = s.R[B];
+                    const double Ra64 = s.R[A], Rb64 = s.R[B];
                     const double sum64 = Ra64 + Rb64;
                     const double gap2 = fma(sum64, sum64, -d2_64);
                     const double dist64 = sqrt(d2_64);
@@ -178,16 +179,19 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
                         if (WRITE) pe += pair_pe_fp64(s.mat, Ra64, Rb64, gap2, d2_64, false, 0.0);
                     }
                 } else if (WRITE && valid) {
-                    pe_far += f2d_bits(vdw_bracket(d2, Ras, Rbs));
+                    pe_far.add(vdw_bracket(d2, Ras, Rbs));
                 }
                 if (!FULL && !valid) fx = fy = fz = 0.0f;
-                // FP64 accumulation of both spheres' sums (:249-250)
-                const double fxd = f2d_bits(fx), fyd = f2d_bits(fy), fzd = f2d_bits(fz);
-                ax += fxd; ay += fyd; az += fzd;
-                bsx += fxd; bsy += fyd; bsz += fzd;
-                ax = __shfl_sync(0xffffffffu, ax, nxt);
-                ay = __shfl_sync(0xffffffffu, ay, nxt);
-                az = __shfl_sync(0xffffffffu, az, nxt);
+                // both spheres' sums (:249-250)
+                const float f[3] = {fx, fy, fz};
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    ra[c].add(f[c]);
+                    cb[c].add(f[c]);
+                    ra[c].a = __shfl_sync(0xffffffffu, ra[c].a, nxt);
+                    ra[c].b = __shfl_sync(0xffffffffu, ra[c].b, nxt);
+                    ra[c].c = __shfl_sync(0xffffffffu, ra[c].c, nxt);
+                }
             }
         };
         if (X != Y && (X + 1) * kBlock <= s.n)
@@ -207,22 +211,24 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
         double* Pt = s.part64;
         if (X == Y) {  // sphere iA == B: partners j < i as A (row), j > i as B (column)
             const size_t o = (size_t)X * s.npad + iA;
-            Pt[o] = ax - bsx;
-            Pt[o + pplane] = ay - bsy;
-            Pt[o + 2 * pplane] = az - bsz;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) Pt[o + c * pplane] = total(ra[c]) - total(cb[c]);
             s.cmask[o] = rowbits | colbits;
             if (rowbits | colbits) s.contact_flag[iA] = 1;
         } else {
             const size_t oa = (size_t)Y * s.npad + iA, ob = (size_t)X * s.npad + B;
-            Pt[oa] = ax; Pt[oa + pplane] = ay; Pt[oa + 2 * pplane] = az;
-            Pt[ob] = -bsx; Pt[ob + pplane] = -bsy; Pt[ob + 2 * pplane] = -bsz;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                Pt[oa + c * pplane] = total(ra[c]);
+                Pt[ob + c * pplane] = -total(cb[c]);
+            }
             s.cmask[oa] = rowbits;
             s.cmask[ob] = colbits;
             if (rowbits) s.contact_flag[iA] = 1;  // every writer stores 1
             if (colbits) s.contact_flag[B] = 1;
         }
         if (WRITE) {
-            pe += -s.mat.Ha / 6 * pe_far;
+            pe += -s.mat.Ha / 6 * total(pe_far);
             for (int off = 16; off > 0; off >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, off);
             if (lane == 0) s.pe_tile[t] = pe;
         }

@@ -64,9 +64,8 @@ PAIR_TERM_BYTES_WRITE = 48
 PAIR_TERM_BYTES_READ = 48
 
 
-# The FP64 work per pair of the mixed form with FP64 geometry and
-# accumulation (SL_MODE_MIXED, sl_step_mixed64.cu), which bounds it: the
-# subtraction pos[B] - pos[A] (3 adds) and the two spheres' FP64 force sums
-# (3 + 3 adds).  Close pairs add their FP64 |r|^2, gap, sqrt and overlap,
-# O(N) of the O(N^2) pairs.
-MIXED64_FP64_OPS_PER_PAIR = 9
+# The FP64 additions per pair out of contact that the exact pair kernel does
+# on the FP64 pipe for equal radii (sl_pair_fast.cuh): r (3), |r|^2 (2), the
+# overlap (1), S (2), T (1), h + R + R (2).  Every product and quotient is
+# rounded in integer arithmetic.
+EXACT_FP64_OPS_PER_PAIR = 11

@@ -172,3 +172,35 @@ def test_mixed_polydisperse_n20000_energy_and_trajectory_track_fp64(mode):
     assert worst <= 1e-6, worst
     ge, gm = ex.download(), mx.download()
     assert np.abs(gm.pos - ge.pos).max() <= 1e-6 * float(g.R.max())
+
+
+@pytest.mark.parametrize("n", [33, 64, 257])
+@pytest.mark.parametrize("offset", [0.0, 3e-3, 1.0])
+def test_mixed_accumulation_keeps_fp64_precision(n, offset):
+    """The mixed form's displacements and sums carry at least FP64's
+    precision (three-part positions, error-free sums): moving the whole
+    system away from the origin by up to 10^4 radii, where FP64 positions
+    still resolve 1e-16 of the offset, changes the accelerations by no more
+    than that resolution and the FP32 force arithmetic explain.  A position
+    rounded at eps offset moves r by that much; a contact's force responds
+    with k times it, against k times its overlap.  The bar is 8 eps offset
+    over the smallest overlap of a contact, plus 2^-20 for FP32 terms."""
+    from spacelab_gb300 import BallGroup, GpuStep
+    c = contact_case(n, 40 + n)
+    shift = np.array([offset, -0.5 * offset, 0.25 * offset])
+    pos = c["pos"] + shift - shift  # the same positions as the shifted system has
+
+    def forces(p, mode):
+        g = BallGroup.from_arrays(p, c["vel"], c["w"], c["R"], c["m"], c["moi"])
+        with GpuStep(g, material(), mode) as s:
+            s.set_scalars(c["dt"], c["kin"], c["kout"])
+            s.init_conditions()
+            return s.download().acc.copy()
+
+    near, far, ex = forces(pos, "mixed"), forces(c["pos"] + shift, "mixed"), forces(pos, "exact")
+    d = np.linalg.norm(pos[:, None] - pos[None], axis=-1)
+    ov = (c["R"][:, None] + c["R"][None]) - d
+    ov = ov[np.triu_indices(n, 1)]
+    bar = 2.0 ** -20 + 8 * np.finfo(float).eps * max(offset, np.abs(pos).max()) / ov[ov > 0].min()
+    assert np.linalg.norm(far - near) <= bar * np.linalg.norm(ex)
+    assert np.linalg.norm(near - ex) <= (2.0 ** -17) * np.linalg.norm(ex)
