@@ -3,6 +3,7 @@
 #include <cuda.h>
 
 #include "sl_device.cuh"
+#include "sl_pdl.cuh"
 
 namespace sl {
 
@@ -65,8 +66,9 @@ void launch_step_mixed64(const System& s, bool write, int num_sms, cudaStream_t 
 // Whether the mixed pair kernel takes two column blocks per item (mixed_pair_items)
 // for nb row blocks on num_sms SMs: where each warp takes many items.
 bool mixed_pair_double(int nb, int num_sms);
-void launch_drift(const System& s, cudaStream_t st);
-void launch_energy(const System& s, cudaStream_t st);
+// pdl: as dependents of the stream's last kernel (launch_pdl)
+void launch_drift(const System& s, cudaStream_t st, bool pdl = true);
+void launch_energy(const System& s, cudaStream_t st, bool pdl = true);
 int pair_grid_blocks(long long tiles, int num_sms);
 // Block-column bounds cb[0..np] of the pipelined step's pair phases; returns np.
 int phase_bounds(int nb, int* cb);

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include "sl_pdl.cuh"
 #include "sl_tma.cuh"
 
 #include <algorithm>
@@ -311,11 +312,12 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
     extern __shared__ unsigned char tc_raw[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     int tile = blockIdx.x;
-    if (tile == 0 && tid == 0 && L.bump) *L.bump += 1;
+    sl::pdl_next();
     const int tiles0 = gemm_tiles(L.job[0]);
     const bool second = tile >= tiles0;
     if (second) tile -= tiles0;
     if (second && (L.njobs < 2 || tile >= gemm_tiles(L.job[1]))) {
+        sl::pdl_wait();
         bias_grad(L, (tile - (L.njobs < 2 ? 0 : gemm_tiles(L.job[1]))) * kTcThreads + tid);
         return;
     }
@@ -353,6 +355,8 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    sl::pdl_wait();
+    if (blockIdx.x == 0 && tid == 0 && L.bump) *L.bump += 1;
 
     if (tid == 0) {
         constexpr uint32_t idesc = tc_idesc_bf16(kTcM, kTcN);
@@ -708,6 +712,8 @@ __global__ void mse_grad_kernel(const float* __restrict__ z, int ldz, const floa
                                 bf16* dz, bf16* dzt, int ld, float* loss_partial, const int* step, int step_bias)
 {
     __shared__ float red[256];
+    sl::pdl_next();
+    sl::pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int st = step ? *step + step_bias : 0;
     y += (size_t)st * M * n_out;
@@ -759,6 +765,8 @@ __global__ void adam_kernel(float* p, const float* g, float* m, float* v, bf16* 
                             int layers, const uint8_t* mask, int n, float lr, float b1, float b2, float eps,
                             const float2* coef, const int* step, int step_bias)
 {
+    sl::pdl_next();
+    sl::pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (!mask[i]) return;
@@ -868,8 +876,7 @@ bool launch_gemm(const GemmLaunch& L, cudaStream_t st)
         return false;
     int grid = gemm_tiles(L.job[0]) + (L.njobs > 1 ? gemm_tiles(L.job[1]) : 0);
     if (L.db_out) grid += (L.db_n + kTcThreads - 1) / kTcThreads;
-    gemm_nt_tc_kernel<<<grid, kTcThreads, kTcSmem, st>>>(L);
-    return true;
+    return sl::launch_pdl(true, gemm_nt_tc_kernel, grid, kTcThreads, kTcSmem, st, L) == cudaSuccess;
 }
 
 // After a synchronisation: the GEMMs' setup and bounded waits.
@@ -932,8 +939,8 @@ void backward(sl_mlp* h, const BatchInput& in, int M, cudaStream_t st)
     const int nl = h->nl, ldo = h->dout[nl - 1];
     const int nb = (M * ldo + 255) / 256;
     int cur = 0;
-    mse_grad_kernel<<<nb, 256, 0, st>>>(h->Z[nl - 1], ldo, in.y, M, h->n_out, h->dZ[cur], h->dZt[cur], ldo,
-                                        in.loss_part, in.step, -1);
+    sl::launch_pdl(true, mse_grad_kernel, nb, 256, 0, st, h->Z[nl - 1], ldo, in.y, M, h->n_out, h->dZ[cur], h->dZt[cur],
+                   ldo, in.loss_part, in.step, -1);
     for (int l = nl - 1; l >= 0 && !h->tc_setup_failed; --l, cur ^= 1) {
         const int K = h->din[l], N = h->dout[l];
         GemmLaunch L{};
@@ -1218,9 +1225,8 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
     if (ok) {
         forward(h, in, batch, true, st);
         backward(h, in, batch, st);
-        adam_kernel<<<(int)((h->nparam + 255) / 256), 256, 0, st>>>(h->P, h->G, h->Mom, h->Var, h->Pb, h->Wt, h->at,
-                                                                    h->nl, h->mask, (int)h->nparam, lr, b1, b2, eps,
-                                                                    dcoef, dstep, -1);
+        sl::launch_pdl(true, adam_kernel, (int)((h->nparam + 255) / 256), 256, 0, st, h->P, h->G, h->Mom, h->Var, h->Pb,
+                       h->Wt, h->at, h->nl, h->mask, (int)h->nparam, lr, b1, b2, eps, dcoef, dstep, -1);
         ok = cudaStreamEndCapture(st, &graph) == cudaSuccess && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
     }
     if (graph) cudaGraphDestroy(graph);

@@ -115,6 +115,7 @@ __global__ void __launch_bounds__(32 * kRsWarps, 16 / BPS) rowsum_tma_kernel(con
     constexpr int kBps = kStageCols >= kBlock ? kStageCols / kBlock : 1;  // partner blocks per stage
     extern __shared__ unsigned char rs_raw[];
     __shared__ __align__(8) uint64_t full_all[kRsWarps][kRsStages];
+    pdl_next();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int wg = blockIdx.x * kRsWarps + warp;  // global (component, row block) index
@@ -261,6 +262,7 @@ __global__ void __launch_bounds__(32 * kRsWarps, 8) rowsum_int_kernel(const __gr
 {
     extern __shared__ unsigned char rs_raw[];
     __shared__ __align__(8) uint64_t full_all[kRsWarps][kIsStages];
+    pdl_next();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int wg = blockIdx.x * kRsWarps + warp;  // global (component, row block) index

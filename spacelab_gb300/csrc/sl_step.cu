@@ -43,6 +43,8 @@ constexpr int kDriftThreads = 64;
 
 __global__ void __launch_bounds__(kDriftThreads) drift_kernel(const __grid_constant__ System s)
 {
+    pdl_next();
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3 * s.n) return;
     if (t == 0 && s.tile_counter)  // the pair kernels' work queues
@@ -102,6 +104,8 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
                                                           int phase, long long split)
 {
     __shared__ TileScratch scratch[4];
+    pdl_next();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     TileScratch& ws = scratch[wib];
@@ -186,6 +190,8 @@ constexpr int kRowThreads = 32;
 __global__ void __launch_bounds__(kRowThreads) rowsum_kernel(const __grid_constant__ System s, int b0, int b1,
                                                              int first, int last)
 {
+    pdl_next();
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3 * s.n) return;
     const int c = t / s.n;
@@ -244,6 +250,8 @@ constexpr int kRedThreads = 256;
 // its share of pe_tile into red[b][7].
 __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __grid_constant__ System s, int chunk)
 {
+    pdl_next();
+    pdl_wait();
     __shared__ double sh[8][kRedThreads];
     const int tid = threadIdx.x;
     double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -276,6 +284,8 @@ __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __gri
 // Final totals over the block partials, in block order.
 __global__ void __launch_bounds__(32) energy_final_kernel(const __grid_constant__ System s, int nred)
 {
+    pdl_next();
+    pdl_wait();
     const int k = threadIdx.x;
     if (k >= 8) return;
     double v = 0;
@@ -403,17 +413,17 @@ void launch_stage_out(const System& s, double* const dst[6], Vec3Soa* const arr[
     stage_out_kernel<<<(3 * s.n + 255) / 256, 256, 0, st>>>(s, p, a, want, guard);
 }
 
-void launch_drift(const System& s, cudaStream_t st)
+void launch_drift(const System& s, cudaStream_t st, bool pdl)
 {
-    drift_kernel<<<(3 * s.n + kDriftThreads - 1) / kDriftThreads, kDriftThreads, 0, st>>>(s);
+    launch_pdl(pdl, drift_kernel, (3 * s.n + kDriftThreads - 1) / kDriftThreads, kDriftThreads, 0, st, s);
 }
 
-void launch_energy(const System& s, cudaStream_t st)
+void launch_energy(const System& s, cudaStream_t st, bool pdl)
 {
     const int nred = kRedBlocks;
     const int chunk = (s.n + nred - 1) / nred;
-    energy_partial_kernel<<<nred, kRedThreads, 0, st>>>(s, chunk);
-    energy_final_kernel<<<1, 32, 0, st>>>(s, nred);
+    launch_pdl(pdl, energy_partial_kernel, nred, kRedThreads, 0, st, s, chunk);
+    launch_pdl(pdl, energy_final_kernel, 1, 32, 0, st, s, nred);
 }
 
 static void launch_rowsum(const System& s, cudaStream_t st, const CUtensorMap* map, int b0, int b1, int first,
@@ -445,18 +455,20 @@ long long pair_split(long long tiles, int num_sms)
 }
 
 static void launch_pair_columns(const System& s, bool write, int num_sms, cudaStream_t st, int c0, int c1, int phase,
-                                long long split)
+                                long long split, bool pdl)
 {
     const auto offset = [&](int c) { return (long long)c * s.nb - (long long)c * (c - 1) / 2; };
     const long long t0 = offset(c0), t1 = offset(c1), cut = min(max(split, t0), t1);
     const long long items = (cut - t0) + kStrips * (t1 - cut);
-    // few items: one warp per CTA, so that they spread over the SMs
+    // few items: one warp per CTA, so that they spread over the SMs, and a
+    // dependent launch (N=96: 25.1 -> 23.4 us per step).  A larger grid placed
+    // while the drift still runs is spread unevenly (N=1000: 82 -> 84 us), and
+    // so are the row sums placed beside the pair tiles (N=1000: 82 -> 124 us,
+    // N=5000: 674 -> 836): both are launched plainly.
     const int warps = items <= 4LL * num_sms ? 1 : 4;
     const int pb = (int)min((items + warps - 1) / warps, (long long)num_sms * 4);
-    if (write)
-        pair_tile_kernel<true><<<pb, 32 * warps, 0, st>>>(s, c0, c1, phase, split);
-    else
-        pair_tile_kernel<false><<<pb, 32 * warps, 0, st>>>(s, c0, c1, phase, split);
+    launch_pdl(pdl && warps == 1, write ? pair_tile_kernel<true> : pair_tile_kernel<false>, pb, 32 * warps, 0, st, s, c0, c1, phase,
+               split);
 }
 
 void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, StepTimers* tm, const StepOverlap* ov,
@@ -467,15 +479,17 @@ void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, St
     const int np = ov ? phase_bounds(s.nb, cb) : 1;
     const long long split = pair_split(s.ntiles, num_sms);  // the same items, and energy sums, with and without phases
     s.nitems = split + kStrips * (s.ntiles - split);
-    launch_drift(s, st);
+    // phases wait on events between the kernels: plain launches there
+    const bool pdl = np <= 1;
+    launch_drift(s, st, pdl);
     if (tm) cudaEventRecord(tm->ev[0], st);
     if (np <= 1) {
-        launch_pair_columns(s, write, num_sms, st, 0, s.nb, 0, split);
+        launch_pair_columns(s, write, num_sms, st, 0, s.nb, 0, split, pdl);
         if (tm) cudaEventRecord(tm->ev[1], st);
         launch_rowsum(s, st, map, 0, s.nb, 1, 1, num_sms, int_adds);
     } else {
         for (int p = 0; p < np; ++p) {
-            launch_pair_columns(s, write, num_sms, st, cb[p], cb[p + 1], p, split);
+            launch_pair_columns(s, write, num_sms, st, cb[p], cb[p + 1], p, split, pdl);
             cudaEventRecord(ov->phase[p], st);
             cudaStreamWaitEvent(ov->side, ov->phase[p], 0);
             launch_rowsum(s, ov->side, map, cb[p], cb[p + 1], p == 0, p == np - 1, num_sms, int_adds);
@@ -485,7 +499,7 @@ void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, St
         cudaStreamWaitEvent(st, ov->join, 0);
     }
     if (tm) cudaEventRecord(tm->ev[2], st);
-    if (write) launch_energy(s, st);
+    if (write) launch_energy(s, st, pdl);
 }
 
 }  // namespace sl

@@ -81,6 +81,8 @@ template <bool WRITE>
 __global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_kernel(const __grid_constant__ System s)
 {
     __shared__ __align__(16) float rows_all[kPairWarps][kBlock * kRowStride];
+    pdl_next();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     float* rows = rows_all[wib];
@@ -316,6 +318,8 @@ template <bool WRITE>
 __global__ void __launch_bounds__(32 * kPairWarps, kPair2CtasPerSm) mixed_pair2_kernel(const __grid_constant__ System s)
 {
     __shared__ __align__(16) float rows_all[kPairWarps][kBlock * kRowStride];
+    pdl_next();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     float* rows = rows_all[wib];
@@ -597,6 +601,8 @@ constexpr int kFinSlices = 8;
 __global__ void __launch_bounds__(32 * kFinSlices) mixed_finish_kernel(const __grid_constant__ System s)
 {
     __shared__ float fs[kFinSlices][12][kBlock];  // (s, c) of force x, y, z, then of torque x, y, z
+    pdl_next();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     const int i = blockIdx.x * kBlock + lane;  // < npad
@@ -620,16 +626,17 @@ __global__ void __launch_bounds__(32 * kFinSlices) mixed_finish_kernel(const __g
         }
     };
     constexpr int U = 8;  // loads in flight per array
-    int K = K0;
-    for (; K + U <= K1; K += U) {
+    // the last batch's entries past K1 are read as zeros: one at a time they
+    // cost a round trip each, which was most of the kernel for nb < 64
+    for (int K = K0; K < K1; K += U) {
         float v[3][U];
         uint32_t m[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const size_t o = (size_t)(K + u) * s.npad;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][u] = __ldcs(p + o + c * pplane);
-            m[u] = any_contact ? __ldcs(mk + o) : 0u;
+            for (int c = 0; c < 3; ++c) v[c][u] = K + u < K1 ? __ldcs(p + o + c * pplane) : 0.0f;
+            m[u] = any_contact && K + u < K1 ? __ldcs(mk + o) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -637,12 +644,6 @@ __global__ void __launch_bounds__(32 * kFinSlices) mixed_finish_kernel(const __g
             for (int c = 0; c < 3; ++c) f[c].add(v[c][u]);
             torques(m[u], K + u);
         }
-    }
-    for (; K < K1; ++K) {
-        const size_t o = (size_t)K * s.npad;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c].add(__ldcs(p + o + c * pplane));
-        torques(any_contact ? __ldcs(mk + o) : 0u, K);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -691,19 +692,12 @@ void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st
     // one wave of persistent warps
     long long cap = (long long)num_sms * (s.pair_double ? kPair2CtasPerSm : kPairCtasPerSm);
     const int pb = (int)(want < cap ? want : cap);
-    if (s.pair_double) {
-        if (write)
-            mixed_pair2_kernel<true><<<pb, 32 * kPairWarps, 0, st>>>(s);
-        else
-            mixed_pair2_kernel<false><<<pb, 32 * kPairWarps, 0, st>>>(s);
-    } else {
-        if (write)
-            mixed_pair_kernel<true><<<pb, 32 * kPairWarps, 0, st>>>(s);
-        else
-            mixed_pair_kernel<false><<<pb, 32 * kPairWarps, 0, st>>>(s);
-    }
+    if (s.pair_double)
+        launch_pdl(pb <= num_sms, write ? mixed_pair2_kernel<true> : mixed_pair2_kernel<false>, pb, 32 * kPairWarps, 0, st, s);
+    else
+        launch_pdl(pb <= num_sms, write ? mixed_pair_kernel<true> : mixed_pair_kernel<false>, pb, 32 * kPairWarps, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[1], st);
-    mixed_finish_kernel<<<s.nb, 32 * kFinSlices, 0, st>>>(s);
+    launch_pdl(true, mixed_finish_kernel, s.nb, 32 * kFinSlices, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[2], st);
     if (write) launch_energy(s, st);
 }

@@ -75,6 +75,8 @@ template <bool WRITE>
 __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_kernel(const __grid_constant__ System s)
 {
     __shared__ __align__(16) float rows_all[kM64Warps][kBlock * kRow64];
+    pdl_next();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     float* rows = rows_all[wib];
@@ -253,6 +255,8 @@ constexpr int kFin64Slices = 8;
 __global__ void __launch_bounds__(32 * kFin64Slices) mixed64_finish_kernel(const __grid_constant__ System s)
 {
     __shared__ double fs[kFin64Slices][6][kBlock];  // (slice, force x y z, torque x y z, sphere)
+    pdl_next();
+    pdl_wait();
     const int lane = threadIdx.x & 31;
     const int w = threadIdx.x >> 5;
     const int i = blockIdx.x * kBlock + lane;  // < npad
@@ -275,16 +279,17 @@ __global__ void __launch_bounds__(32 * kFin64Slices) mixed64_finish_kernel(const
         }
     };
     constexpr int U = 8;  // loads in flight per array
-    int K = K0;
-    for (; K + U <= K1; K += U) {
+    // the last batch's entries past K1 are read as zeros: one at a time they
+    // cost a round trip each, which was most of the kernel for nb < 64
+    for (int K = K0; K < K1; K += U) {
         double v[3][U];
         uint32_t m[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const size_t o = (size_t)(K + u) * s.npad;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][u] = __ldcs(p + o + c * pplane);
-            m[u] = any_contact ? __ldcs(mk + o) : 0u;
+            for (int c = 0; c < 3; ++c) v[c][u] = K + u < K1 ? __ldcs(p + o + c * pplane) : 0.0;
+            m[u] = any_contact && K + u < K1 ? __ldcs(mk + o) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -292,12 +297,6 @@ __global__ void __launch_bounds__(32 * kFin64Slices) mixed64_finish_kernel(const
             for (int c = 0; c < 3; ++c) f[c] += v[c][u];
             torques(m[u], K + u);
         }
-    }
-    for (; K < K1; ++K) {
-        const size_t o = (size_t)K * s.npad;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) f[c] += __ldcs(p + o + c * pplane);
-        torques(any_contact ? __ldcs(mk + o) : 0u, K);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -334,12 +333,9 @@ void launch_step_mixed64(const System& s, bool write, int num_sms, cudaStream_t 
     const long long want = (s.ntiles + kM64Warps - 1) / kM64Warps;
     const long long cap = (long long)num_sms * kM64CtasPerSm;  // one wave of persistent warps
     const int pb = (int)(want < cap ? want : cap);
-    if (write)
-        mixed64_pair_kernel<true><<<pb, 32 * kM64Warps, 0, st>>>(s);
-    else
-        mixed64_pair_kernel<false><<<pb, 32 * kM64Warps, 0, st>>>(s);
+    launch_pdl(pb <= num_sms, write ? mixed64_pair_kernel<true> : mixed64_pair_kernel<false>, pb, 32 * kM64Warps, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[1], st);
-    mixed64_finish_kernel<<<s.nb, 32 * kFin64Slices, 0, st>>>(s);
+    launch_pdl(true, mixed64_finish_kernel, s.nb, 32 * kFin64Slices, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[2], st);
     if (write) launch_energy(s, st);
 }
