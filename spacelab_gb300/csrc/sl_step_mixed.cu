@@ -41,6 +41,7 @@
 #include "sl_kernels.h"
 #include "sl_df.cuh"
 #include "sl_pair_mixed.cuh"
+#include "sl_tile_mixed.cuh"
 
 #include <type_traits>
 
@@ -76,8 +77,7 @@ __device__ __forceinline__ double fp64_d2(const System& s, int A, int B)
 // the tile's partials f_part[c][Y][A] (sphere A's terms from block Y) and
 // f_part[c][X][B] (sphere B's from block X), or on the diagonal one partial
 // f_part[c][X][i] with both; contact bits to cmask[K][i]; torques of contacts
-// to the float view of torqbuf, [A][B] and [B][A].
-template <bool WRITE>
+// to the float view of torqbuf, [A][B] and [B][A].  Plain steps.
 __global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_kernel(const __grid_constant__ System s)
 {
     __shared__ __align__(16) float rows_all[kPairWarps][kBlock * kRowStride];
@@ -95,32 +95,9 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_ke
     const float hmin_s = (float)s.mat.h_min / L;
     const float c_vdw = (float)(s.mat.Ha / 6 * 64) / L;   // dyn per unit vdw_shape
     const int nxt = (lane + 1) & (kBlock - 1);
-    // write steps: close pairs out of contact whose FP64 potential is pending.
-    // Their FP64 evaluation runs with every lane busy (the FP64 pipe takes a
-    // warp instruction per ~64 cycles however few lanes are active)
-    __shared__ int2 queue_all[WRITE ? kPairWarps : 1][WRITE ? 2 * kBlock : 1];
-    int2* q = queue_all[WRITE ? wib : 0];
-    int qn = 0;
-    double pe = 0;
-    auto flush_close = [&](int cnt) {  // pairs q[0 .. cnt), cnt <= 32; the rest move down
-        if (lane < cnt) {
-            const int A = q[lane].x, B = q[lane].y;
-            const double d2_64 = fp64_d2(s, A, B), sum64 = s.R[A] + s.R[B];
-            pe += pair_pe_fp64(s.mat, s.R[A], s.R[B], fma(sum64, sum64, -d2_64), d2_64, false, 0.0);
-        }
-        const int left = qn - cnt;
-        const int2 e = lane < left ? q[cnt + lane] : make_int2(0, 0);
-        __syncwarp();
-        if (lane < left) q[lane] = e;
-        __syncwarp();
-        qn = left;
-    };
-
-    // Tiles: a first round in warp order, then, on plain steps, whichever
-    // warp is free takes the next tile from a counter that the drift kernel
-    // zeroes (the last round of a static stride leaves SMs idle); write
-    // steps keep the static stride, so that their close-pair queues, and so
-    // the potential energy's rounding, repeat run to run.
+    // A first round of tiles in warp order, then whichever warp is free takes
+    // the next one from a counter that the drift kernel zeroes (the last round
+    // of a static stride leaves SMs idle).
     long long t = (long long)blockIdx.x * kPairWarps + wib;
     for (; t < s.ntiles;) {
         int X, Y;
@@ -143,8 +120,6 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_ke
         const float Rbs = s.f_R[B], Rblo = s.f_Rlo[B], inv_mb = s.f_inv_m[B];
         const float Rb3 = Rbs * Rbs * Rbs;
         const int nA = s.n - X * kBlock;  // rows r < nA are spheres
-        pe = 0;
-        df::Sum pe_far{0.0f, 0.0f};  // far pairs' vdW brackets (write steps)
         uint32_t colbits = 0;
         float ax = 0, ay = 0, az = 0;     // running sum of row (lane + k) mod 32 at step k
         float bsx = 0, bsy = 0, bsz = 0;  // sphere B's sum
@@ -207,26 +182,10 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_ke
                         float* tb = tbuf + (size_t)B * s.npad + A;
                         ta[0] = o.tax * ima; ta[plane] = o.tay * ima; ta[2 * plane] = o.taz * ima;
                         tb[0] = o.tbx * imb; tb[plane] = o.tby * imb; tb[2 * plane] = o.tbz * imb;
-                        if (WRITE) {
-                            const double sum64 = s.R[A] + s.R[B];
-                            pe += pair_pe_fp64(s.mat, s.R[A], s.R[B], fma(sum64, sum64, -d2_64), d2_64, true, o.k);
-                        }
                     } else {
                         const float hn = fmaxf(-ovl_s, hmin_s);                 // :211-215
                         const float f = c_vdw * vdw_shape(hn, Ras, Rbs);
                         fx = f * nx; fy = f * ny; fz = f * nz;
-                    }
-                }
-                if (WRITE) {  // write steps only
-                    if (valid && !closep) pe_far.add(vdw_bracket(d2, Ras, Rbs));
-                    // close pairs out of contact: queued, evaluated 32 at a time
-                    const bool need = valid && closep && !contact;
-                    const uint32_t m = __ballot_sync(0xffffffffu, need);
-                    if (m) {
-                        if (need) q[qn + __popc(m & ((1u << lane) - 1u))] = make_int2(X * kBlock + r, B);
-                        qn += __popc(m);
-                        __syncwarp();
-                        if (qn >= kBlock) flush_close(kBlock);
                     }
                 }
                 if (!FULL && !valid) fx = fy = fz = 0.0f;
@@ -269,20 +228,159 @@ __global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_ke
             if (rowbits) s.contact_flag[iA] = 1;  // every writer stores 1
             if (colbits) s.contact_flag[B] = 1;
         }
+        __syncwarp();
+        int k = 0;
+        if (lane == 0) k = atomicAdd(s.tile_counter, 1);
+        t = nwarps + __shfl_sync(0xffffffffu, k, 0);
+    }
+}
+
+// The same tile with its close pairs listed and evaluated one per lane before
+// the sweep (sl_tile_mixed.cuh): the same forces, added in the same order.
+// Taken on write steps and by systems of few tiles (launch_step_mixed).
+struct PairSmem {
+    float rows[kBlock * mt::kRow];  // [16] the radius's lo part, [17] 1/m
+    mt::List<3> list;
+    uint32_t rowc[kBlock], colc[kBlock];  // contact bits
+};
+
+template <bool WRITE>
+__global__ void __launch_bounds__(32 * kPairWarps, kPairCtasPerSm) mixed_pair_listed_kernel(const __grid_constant__ System s)
+{
+    __shared__ __align__(16) PairSmem smem[kPairWarps];
+    pdl_next();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const int wib = threadIdx.x >> 5;
+    PairSmem& sm = smem[wib];
+    float* rows = sm.rows;
+    const long long nwarps = (long long)gridDim.x * kPairWarps;
+    const size_t plane = (size_t)s.npad * s.npad;  // torque planes
+    const size_t pplane = (size_t)s.nb * s.npad;   // partial planes
+    float* tbuf = reinterpret_cast<float*>(s.torqbuf);
+    const int sh = s.len_shift;
+    const float L = ldexpf(1.0f, sh);
+    const float hmin_s = (float)s.mat.h_min / L;
+    const float c_vdw = (float)(s.mat.Ha / 6 * 64) / L;   // dyn per unit vdw_shape
+
+    // A first round of tiles in warp order; then whichever warp is free takes
+    // the next one from a counter that the drift kernel zeroes (the last
+    // round of a static stride leaves SMs idle).  A tile's results, its
+    // energy too, do not depend on the warp that computes it.
+    long long t = (long long)blockIdx.x * kPairWarps + wib;
+    for (; t < s.ntiles;) {
+        int X, Y;
+        tile_coords(t, X, Y);
+        {
+            const int i = X * kBlock + lane;  // < npad
+            const float Ri = s.f_R[i];
+            mt::put_row(rows, lane, {s.f_pos[0][i], s.f_pos[1][i], s.f_pos[2][i], Ri, s.f_pos[3][i], s.f_pos[4][i],
+                                     s.f_pos[5][i], c_vdw * (Ri * Ri * Ri)},
+                        make_float4(s.f_Rlo[i], s.f_inv_m[i], 0.0f, 0.0f));
+            sm.rowc[lane] = sm.colc[lane] = 0;
+        }
+        __syncwarp();
+        const int B0 = Y * kBlock + lane;
+        auto load_column = [&](int B) {
+            mt::Col c;
+            c.x = s.f_pos[0][B]; c.y = s.f_pos[1][B]; c.z = s.f_pos[2][B];
+            c.xl = s.f_pos[3][B]; c.yl = s.f_pos[4][B]; c.zl = s.f_pos[5][B];
+            c.R = s.f_R[B];
+            c.R3 = c.R * c.R * c.R;
+            c.valid = B < s.n;
+            return c;
+        };
+        const mt::Col col = load_column(B0);
+        const float inv_mb = s.f_inv_m[B0];
+        const int nA = s.n - X * kBlock;  // rows r < nA are spheres
+        double pe = 0;
+        df::Sum pe_far{0.0f, 0.0f};  // far pairs' vdW brackets (write steps)
+        float av[3], bv[3];
+        // a listed pair: double-float (~48 bits, FP32 pipe) subtraction, |r|^2
+        // and squared gap g = (R_A + R_B)^2 - |r|^2, then the contact branch or
+        // the clamped vdW
+        auto close = [&](int q, int r, int cb, double& pe_, df::Sum& far_) {
+            const int A = X * kBlock + r, B = Y * kBlock + cb;
+            const mt::Col c = load_column(B);
+            const mt::Row row = mt::get_row(rows, r);
+            float* out = sm.list.v[q];
+            const float Ras = row.R;
+            const mt::Far f = mt::far_pair(row, c);
+            if (!(f.d2 < s.far_sq * f.sum2)) {
+                out[0] = f.fr * f.rx; out[1] = f.fr * f.ry; out[2] = f.fr * f.rz;
+                if (WRITE) far_.add(vdw_bracket(f.d2, Ras, c.R));
+                return;
+            }
+            const df::F2 drx = df::sub({c.x, c.xl}, {row.x, row.xl});
+            const df::F2 dry = df::sub({c.y, c.yl}, {row.y, row.yl});
+            const df::F2 drz = df::sub({c.z, c.zl}, {row.z, row.zl});
+            const df::F2 dd2 = df::add(df::add(df::sqr(drx), df::sqr(dry)), df::sqr(drz));
+            const df::F2 sum = df::add({Ras, rows[r * mt::kRow + 16]}, {c.R, s.f_Rlo[B]});
+            const df::F2 gap2 = df::sub(df::sqr(sum), dd2);
+            const float d2s = dd2.hi;
+            const float inv_dn = rsqrtf(d2s);
+            const float dist_s = d2s * inv_dn;
+            const float ovl_s = __fdividef(gap2.hi, Ras + c.R + dist_s);
+            const float nx = drx.hi * inv_dn, ny = dry.hi * inv_dn, nz = drz.hi * inv_dn;
+            if (gap2.hi > 0.0f || (gap2.hi == 0.0f && gap2.lo > 0.0f)) {
+                atomicOr(&sm.rowc[r], 1u << cb);
+                atomicOr(&sm.colc[cb], 1u << r);
+                const ContactIn in = gather_contact(s, A, B);
+                // the kin/kout test compares |r|^2 with the previous step's,
+                // both in FP64 from the FP64 positions with one formula
+                const double d2_64 = fp64_d2(s, A, B);
+                const ContactF o = contact_mixed(in, s.mat, sh, d2_64, nx, ny, nz, dist_s * L, ovl_s * L, Ras, c.R);
+                out[0] = o.fx; out[1] = o.fy; out[2] = o.fz;
+                const float ima = s.f_inv_moi[A], imb = s.f_inv_moi[B];
+                float* ta = tbuf + (size_t)A * s.npad + B;
+                float* tb = tbuf + (size_t)B * s.npad + A;
+                ta[0] = o.tax * ima; ta[plane] = o.tay * ima; ta[2 * plane] = o.taz * ima;
+                tb[0] = o.tbx * imb; tb[plane] = o.tby * imb; tb[2 * plane] = o.tbz * imb;
+                if (WRITE) {
+                    const double sum64 = s.R[A] + s.R[B];
+                    pe_ += pair_pe_fp64(s.mat, s.R[A], s.R[B], fma(sum64, sum64, -d2_64), d2_64, true, o.k);
+                }
+                return;
+            }
+            const float hn = fmaxf(-ovl_s, hmin_s);                 // :211-215
+            const float fv = c_vdw * vdw_shape(hn, Ras, c.R);
+            out[0] = fv * nx; out[1] = fv * ny; out[2] = fv * nz;
+            if (WRITE) {
+                const double d2_64 = fp64_d2(s, A, B), sum64 = s.R[A] + s.R[B];
+                pe_ += pair_pe_fp64(s.mat, s.R[A], s.R[B], fma(sum64, sum64, -d2_64), d2_64, false, 0.0);
+            }
+        };
+        mt::tile<WRITE>(rows, sm.list, col, nA, X == Y, s.far_sq, close, [](int, int) {}, av, bv, pe, pe_far);
+        const float ax = av[0], ay = av[1], az = av[2], bsx = bv[0], bsy = bv[1], bsz = bv[2];
+        const uint32_t rowbits = sm.rowc[lane], colbits = sm.colc[lane];
+        const int iA = X * kBlock + lane, B = B0;
+        const float ima = rows[lane * mt::kRow + 17];
+        float* P = s.f_part;
+        if (X == Y) {  // sphere iA == B: partners j < i as A (row), j > i as B (column)
+            const size_t o = (size_t)X * s.npad + iA;
+            P[o] = fmaf(ima, ax, -inv_mb * bsx);
+            P[o + pplane] = fmaf(ima, ay, -inv_mb * bsy);
+            P[o + 2 * pplane] = fmaf(ima, az, -inv_mb * bsz);
+            s.cmask[o] = rowbits | colbits;
+            if (rowbits | colbits) s.contact_flag[iA] = 1;
+        } else {
+            const size_t oa = (size_t)Y * s.npad + iA, ob = (size_t)X * s.npad + B;
+            P[oa] = ima * ax; P[oa + pplane] = ima * ay; P[oa + 2 * pplane] = ima * az;
+            P[ob] = -inv_mb * bsx; P[ob + pplane] = -inv_mb * bsy; P[ob + 2 * pplane] = -inv_mb * bsz;
+            s.cmask[oa] = rowbits;
+            s.cmask[ob] = colbits;
+            if (rowbits) s.contact_flag[iA] = 1;  // every writer stores 1
+            if (colbits) s.contact_flag[B] = 1;
+        }
         if (WRITE) {
-            if (qn > 0 && t + nwarps >= s.ntiles) flush_close(qn);  // the warp's last tile
             pe += -s.mat.Ha / 6 * (f2d_bits(pe_far.s) + f2d_bits(pe_far.c));
             for (int off = 16; off > 0; off >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, off);
             if (lane == 0) s.pe_tile[t] = pe;
         }
         __syncwarp();
-        if (WRITE) {
-            t += nwarps;
-        } else {
-            int k = 0;
-            if (lane == 0) k = atomicAdd(s.tile_counter, 1);
-            t = nwarps + __shfl_sync(0xffffffffu, k, 0);
-        }
+        int k = 0;
+        if (lane == 0) k = atomicAdd(s.tile_counter, 1);
+        t = nwarps + __shfl_sync(0xffffffffu, k, 0);
     }
 }
 
@@ -628,15 +726,16 @@ __global__ void __launch_bounds__(32 * kFinSlices) mixed_finish_kernel(const __g
     constexpr int U = 8;  // loads in flight per array
     // the last batch's entries past K1 are read as zeros: one at a time they
     // cost a round trip each, which was most of the kernel for nb < 64
-    for (int K = K0; K < K1; K += U) {
+    auto batch = [&](int K, auto whole_tag) {
+        constexpr bool WHOLE = decltype(whole_tag)::value;
         float v[3][U];
         uint32_t m[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const size_t o = (size_t)(K + u) * s.npad;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][u] = K + u < K1 ? __ldcs(p + o + c * pplane) : 0.0f;
-            m[u] = any_contact && K + u < K1 ? __ldcs(mk + o) : 0u;
+            for (int c = 0; c < 3; ++c) v[c][u] = WHOLE || K + u < K1 ? __ldcs(p + o + c * pplane) : 0.0f;
+            m[u] = any_contact && (WHOLE || K + u < K1) ? __ldcs(mk + o) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -644,7 +743,10 @@ __global__ void __launch_bounds__(32 * kFinSlices) mixed_finish_kernel(const __g
             for (int c = 0; c < 3; ++c) f[c].add(v[c][u]);
             torques(m[u], K + u);
         }
-    }
+    };
+    int K = K0;
+    for (; K + U <= K1; K += U) batch(K, std::true_type{});
+    if (K < K1) batch(K, std::false_type{});
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         fs[w][2 * c][lane] = f[c].s;
@@ -686,20 +788,33 @@ bool mixed_pair_double(int nb, int num_sms)
 
 void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st, StepTimers* tm)
 {
-    launch_drift(s, st);
+    // not where the pair kernel fills the SMs: N=9000 94.9 us per step without,
+    // 98.9 with
+    const bool pdl = !s.pair_double;
+    launch_drift(s, st, pdl);
     if (tm) cudaEventRecord(tm->ev[0], st);
     long long want = (s.nitems + kPairWarps - 1) / kPairWarps;
     // one wave of persistent warps
     long long cap = (long long)num_sms * (s.pair_double ? kPair2CtasPerSm : kPairCtasPerSm);
     const int pb = (int)(want < cap ? want : cap);
+    // Listing the close pairs pays while a tile's latency shows: up to 2.5 tiles
+    // per resident warp (us per step, evaluated in the sweep / listed: N=1733
+    // 22.9 / 18.5, N=3000 32.1 / 28.8, N=4000 37.3 / 37.4, N=5000 46.7 / 51.1),
+    // and on write steps, whose FP64 potentials it makes dense (N=5000 124.6 /
+    // 109.6).
+    const bool few_tiles = 2 * s.ntiles <= 5 * cap * kPairWarps;
     if (s.pair_double)
         launch_pdl(pb <= num_sms, write ? mixed_pair2_kernel<true> : mixed_pair2_kernel<false>, pb, 32 * kPairWarps, 0, st, s);
     else
-        launch_pdl(pb <= num_sms, write ? mixed_pair_kernel<true> : mixed_pair_kernel<false>, pb, 32 * kPairWarps, 0, st, s);
+        launch_pdl(pb <= num_sms,
+                   write       ? mixed_pair_listed_kernel<true>
+                   : few_tiles ? mixed_pair_listed_kernel<false>
+                               : mixed_pair_kernel,
+                   pb, 32 * kPairWarps, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[1], st);
-    launch_pdl(true, mixed_finish_kernel, s.nb, 32 * kFinSlices, 0, st, s);
+    launch_pdl(pdl, mixed_finish_kernel, s.nb, 32 * kFinSlices, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[2], st);
-    if (write) launch_energy(s, st);
+    if (write) launch_energy(s, st, pdl);
 }
 
 }  // namespace sl

@@ -281,15 +281,16 @@ __global__ void __launch_bounds__(32 * kFin64Slices) mixed64_finish_kernel(const
     constexpr int U = 8;  // loads in flight per array
     // the last batch's entries past K1 are read as zeros: one at a time they
     // cost a round trip each, which was most of the kernel for nb < 64
-    for (int K = K0; K < K1; K += U) {
+    auto batch = [&](int K, auto whole_tag) {
+        constexpr bool WHOLE = decltype(whole_tag)::value;
         double v[3][U];
         uint32_t m[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const size_t o = (size_t)(K + u) * s.npad;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) v[c][u] = K + u < K1 ? __ldcs(p + o + c * pplane) : 0.0;
-            m[u] = any_contact && K + u < K1 ? __ldcs(mk + o) : 0u;
+            for (int c = 0; c < 3; ++c) v[c][u] = WHOLE || K + u < K1 ? __ldcs(p + o + c * pplane) : 0.0;
+            m[u] = any_contact && (WHOLE || K + u < K1) ? __ldcs(mk + o) : 0u;
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -297,7 +298,10 @@ __global__ void __launch_bounds__(32 * kFin64Slices) mixed64_finish_kernel(const
             for (int c = 0; c < 3; ++c) f[c] += v[c][u];
             torques(m[u], K + u);
         }
-    }
+    };
+    int K = K0;
+    for (; K + U <= K1; K += U) batch(K, std::true_type{});
+    if (K < K1) batch(K, std::false_type{});
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         fs[w][c][lane] = f[c];
