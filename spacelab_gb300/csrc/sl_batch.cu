@@ -184,12 +184,13 @@ __global__ void __launch_bounds__(256) batch_exact_kernel(const __grid_constant_
 // reference's order, so the result stays bit-identical -- and the half-kick
 // follows.  This evaluates each pair once where the per-sphere loop does it
 // twice, at the price of the row sums' dependent FP64 adds.
-__device__ void make_view(System& v, const Batch& b, int inst, int off, int n)
+__device__ void make_view(System& v, const Batch& b, int inst, int off, int n, int npad, double* pair, double* torq,
+                          uint32_t* mask)
 {
     v = System{};
     v.n = n;
     v.nb = (n + kBlock - 1) / kBlock;
-    v.npad = b.x_np;  // the scratch's row stride
+    v.npad = npad;  // the buffers' row stride
     v.ntiles = (long long)v.nb * (v.nb + 1) / 2;
     v.nitems = v.ntiles;
     const Vec3Soa* src[8] = {&b.pos, &b.prev, &b.vel, &b.velh, &b.w, &b.wh, &b.acc, &b.aacc};
@@ -199,9 +200,9 @@ __device__ void make_view(System& v, const Batch& b, int inst, int off, int n)
     v.R = b.R + off; v.m = b.m + off; v.moi = b.moi + off;
     v.twoR = b.twoR + off; v.fourR = b.fourR + off; v.cR3 = b.cR3 + off;
     v.rm = b.rm + off; v.inv_moi = b.inv_moi + off;
-    v.pairbuf = b.xpair + (size_t)blockIdx.x * b.xpair_cta;
-    v.torqbuf = b.xtorq + (size_t)blockIdx.x * b.xpair_cta;
-    v.cmask = b.xmask + (size_t)blockIdx.x * b.xmask_cta;
+    v.pairbuf = pair;
+    v.torqbuf = torq;
+    v.cmask = mask;
     v.sc = b.isc + inst;
     v.mat = b.mat;
     v.mat.u_s = b.u_s[inst];
@@ -223,12 +224,7 @@ __device__ double exact_tile_pass(const System& s, TileScratch* scratch)
         uint32_t rowbits, colbits;
         tile_pairs<WRITE>(s, ws, X, Y, lane, 0, min(kBlock, n - X * kBlock), min(B, n - 1), B < n, pe, rowbits,
                           colbits);
-        if (X == Y) {
-            s.cmask[(size_t)(X * kBlock + lane) * s.nb + X] = rowbits | colbits;
-        } else {
-            s.cmask[(size_t)(X * kBlock + lane) * s.nb + Y] = rowbits;
-            s.cmask[(size_t)(Y * kBlock + lane) * s.nb + X] = colbits;
-        }
+        store_contacts(s, X, Y, lane, -1, rowbits, colbits);
         __syncwarp();
     }
     return pe;
@@ -283,7 +279,9 @@ __global__ void __launch_bounds__(32 * kExactTileWarps) batch_exact_tiles_kernel
         const int off = b.off[inst], n = b.cnt[inst];
         const double dt = b.dt[inst];
         double* recs = b.energy + (size_t)inst * b.nrec * 8;
-        if (threadIdx.x == 0) make_view(sv, b, inst, off, n);
+        if (threadIdx.x == 0) make_view(sv, b, inst, off, n, b.x_np, b.xpair + (size_t)blockIdx.x * b.xpair_cta,
+                                        b.xtorq + (size_t)blockIdx.x * b.xpair_cta,
+                                        b.xmask + (size_t)blockIdx.x * b.xmask_cta);
         __syncthreads();
         if (do_init) {
             drift(b, off, n, 0.0);
@@ -315,6 +313,237 @@ __global__ void __launch_bounds__(32 * kExactTileWarps) batch_exact_tiles_kernel
     }
 }
 
+// ---------------------------------------------------------------------------
+// Lockstep form of the pair-tile pass: all instances take a step together, one
+// phase over the items of all of them, then the next, with a barrier over the
+// grid between (a cooperative launch, one CTA per SM).  In the form above an
+// instance's step is one CTA's latency -- its tiles taken by a few warps, then
+// its rows' dependent adds -- and the batch waits for its largest instances;
+// here every warp has work until a phase's last items, and only the phases'
+// order is kept.  It needs pair-term buffers for every instance (48 npad^2
+// bytes each), so it is taken where they fit the budget (sl_batch_capi.cu).
+//
+//   pairs   items (tiles, or strips of 8 rows as strip_from says) from a queue
+//   rows    one warp per (component, 32-row block): the ordered sums and pass
+//           3, and on plain steps the next step's pass 1 of the same rows
+//   energy  write steps: one CTA per instance, then pass 1 of the next step
+constexpr int kGridWarps = 16;
+
+struct GridWarp {
+    TileScratch scratch;
+    System view;
+    int inst;
+};
+
+// Row i's ordered sum of the pair terms: every entry is added, the row's own
+// column and the padding too, which are never written and hold +0.0.  16
+// bytes a load, 8 loads ahead of the adds.
+__device__ __forceinline__ double ordered_row(const double* row, int n)
+{
+    constexpr int kBatch = 8;
+    const double2* p = reinterpret_cast<const double2*>(row);
+    const int nq = (n + 1) / 2;
+    double2 cur[kBatch], nxt[kBatch];
+#pragma unroll
+    for (int k = 0; k < kBatch; ++k) cur[k] = k < nq ? __ldcs(p + k) : make_double2(0.0, 0.0);
+    double sum = 0.0;
+    for (int q = 0; q < nq; q += kBatch) {
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+            nxt[k] = q + kBatch + k < nq ? __ldcs(p + q + kBatch + k) : make_double2(0.0, 0.0);
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            sum += cur[k].x;
+            sum += cur[k].y;
+            cur[k] = nxt[k];
+        }
+    }
+    return sum;
+}
+
+// Pass 1 of one component of one sphere (:84-90)
+__device__ __forceinline__ void drift_one(const System& s, int c, int i, double v, double w, double acc, double aacc,
+                                          double dt)
+{
+    const double vh = v + (.5 * acc) * dt;
+    const double whc = w + (.5 * aacc) * dt;
+    const double p = s.pos.c[c][i];
+    s.velh.c[c][i] = vh;
+    s.wh.c[c][i] = whc;
+    s.prev.c[c][i] = p;
+    s.pos.c[c][i] = p + vh * dt;
+}
+
+// Pass 1 of every sphere
+__device__ void grid_drift(const Batch& b, bool init)
+{
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * kGridWarps + (threadIdx.x >> 5), nw = gridDim.x * kGridWarps;
+    for (int item = gw; item < 3 * b.gblocks; item += nw) {
+        const int blk = item / 3, c = item - 3 * blk;
+        const int inst = b.gblk_inst[blk], i = b.gblk[blk] * kBlock + lane;
+        const System& s = b.views[inst];
+        if (i < s.n)
+            drift_one(s, c, i, s.vel.c[c][i], s.w.c[c][i], s.acc.c[c][i], s.aacc.c[c][i], init ? 0.0 : b.dt[inst]);
+    }
+}
+
+template <bool WRITE>
+__device__ void grid_pairs(const Batch& b, GridWarp& gw, int num_sms, int* queue, double* pe_out)
+{
+    const int lane = threadIdx.x & 31;
+    const long long split = strip_from(b.gtiles, num_sms);
+    const long long items = split + kStrips * (b.gtiles - split);
+    const long long nw = (long long)gridDim.x * kGridWarps;
+    for (long long q = (long long)blockIdx.x * kGridWarps + (threadIdx.x >> 5); q < items;) {
+        const bool whole = q < split;
+        const long long u = whole ? q : split + (q - split) / kStrips;
+        const int strip = whole ? -1 : (int)((q - split) % kStrips);
+        const int4 tile = __ldg(b.gtile + u);
+        const int inst = tile.x, X = tile.w >> 16, Y = tile.w & 0xffff;
+        if (inst != gw.inst) {  // the instance's view, by the whole warp
+            __syncwarp();
+            const uint32_t* src = reinterpret_cast<const uint32_t*>(b.views + inst);
+            uint32_t* dst = reinterpret_cast<uint32_t*>(&gw.view);
+            for (int w = lane; w < (int)(sizeof(System) / 4); w += 32) dst[w] = src[w];
+            if (lane == 0) gw.inst = inst;
+            __syncwarp();
+        }
+        const System& s = gw.view;
+        load_a(s, gw.scratch.ab, lane, min(X * kBlock + lane, s.n - 1));
+        __syncwarp();
+        const int B = Y * kBlock + lane;
+        const int a_end = min(kBlock, s.n - X * kBlock);
+        const int a0 = whole ? 0 : strip * kStripRows, a1 = whole ? a_end : min(a_end, a0 + kStripRows);
+        double pe = 0;
+        uint32_t rowbits, colbits;
+        tile_pairs<WRITE>(s, gw.scratch, X, Y, lane, a0, a1, min(B, s.n - 1), B < s.n, pe, rowbits, colbits);
+        store_contacts(s, X, Y, lane, strip, rowbits, colbits);
+        if (WRITE) {
+            for (int o = 16; o > 0; o >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, o);
+            if (lane == 0) pe_out[q] = pe;
+        }
+        __syncwarp();
+        int next = 0;
+        if (lane == 0) next = atomicAdd(queue, 1);
+        q = nw + __shfl_sync(0xffffffffu, next, 0);
+    }
+}
+
+// Ordered sums and pass 3; next_dt: the following step's pass 1 too
+__device__ void grid_rows(const Batch& b, bool init, bool drift_next)
+{
+    const int lane = threadIdx.x & 31;
+    const int gw = blockIdx.x * kGridWarps + (threadIdx.x >> 5), nw = gridDim.x * kGridWarps;
+    for (int item = gw; item < 3 * b.gblocks; item += nw) {
+        const int blk = item / 3, c = item - 3 * blk;
+        const int inst = b.gblk_inst[blk], i = b.gblk[blk] * kBlock + lane;
+        const System& s = b.views[inst];
+        if (i >= s.n) continue;  // no warp-wide operation below
+        const size_t plane = (size_t)s.npad * s.npad;
+        const double acc = ordered_row(s.pairbuf + c * plane + (size_t)i * s.npad, s.n);
+        const double* trow = s.torqbuf + c * plane + (size_t)i * s.npad;
+        const uint32_t* mrow = s.cmask + (size_t)i * s.nb;
+        double aacc = 0;
+        for (int Y = 0; Y < s.nb; ++Y) {
+            uint32_t wd = mrow[Y];
+            while (wd) {
+                const int j = Y * kBlock + __ffs(wd) - 1;
+                wd &= wd - 1;
+                aacc += trow[j];
+            }
+        }
+        s.acc.c[c][i] = acc;
+        s.aacc.c[c][i] = aacc;
+        const double dt = init ? 0.0 : b.dt[inst];
+        const double v = s.velh.c[c][i] + (.5 * acc) * dt;    // :265
+        const double wv = s.wh.c[c][i] + (.5 * aacc) * dt;    // :266
+        s.vel.c[c][i] = v;
+        s.w.c[c][i] = wv;
+        if (!isfinite(v) || !isfinite(wv) || !isfinite(s.pos.c[c][i])) atomicOr(&b.status[inst], 1u);
+        if (drift_next) drift_one(s, c, i, v, wv, acc, aacc, b.dt[inst]);
+    }
+}
+
+// The energy records of a write step, one CTA per instance
+__device__ void grid_energy(const Batch& b, int num_sms, const double* pe, int rec, double (*sh)[32])
+{
+    const long long split = strip_from(b.gtiles, num_sms);
+    const auto first_item = [split](long long u) { return u <= split ? u : split + (u - split) * kStrips; };
+    for (int k = blockIdx.x; k < b.ninst; k += gridDim.x) {
+        const int inst = b.order[k];
+        const System& s = b.views[inst];
+        double e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        for (long long q = first_item(b.gtile_off[k]) + threadIdx.x; q < first_item(b.gtile_off[k + 1]); q += blockDim.x)
+            e[0] += pe[q];
+        for (int i = threadIdx.x; i < s.n; i += blockDim.x) {
+            const double m = s.m[i], moi = s.moi[i];
+            const double vx = s.vel.c[0][i], vy = s.vel.c[1][i], vz = s.vel.c[2][i];
+            const double wx = s.w.c[0][i], wy = s.w.c[1][i], wz = s.w.c[2][i];
+            const double px = s.pos.c[0][i], py = s.pos.c[1][i], pz = s.pos.c[2][i];
+            e[1] += .5 * m * (vx * vx + vy * vy + vz * vz) + .5 * moi * (wx * wx + wy * wy + wz * wz);
+            e[2] += m * vx; e[3] += m * vy; e[4] += m * vz;
+            e[5] += m * (py * vz - pz * vy) + moi * wx;
+            e[6] += m * (pz * vx - px * vz) + moi * wy;
+            e[7] += m * (px * vy - py * vx) + moi * wz;
+        }
+        cta_sum8(e, sh);
+        if (threadIdx.x == 0)
+            for (int j = 0; j < 8; ++j) b.energy[((size_t)inst * b.nrec + rec) * 8 + j] = e[j];
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(32 * kGridWarps, 1) batch_exact_grid_kernel(const __grid_constant__ Batch b,
+                                                                              int num_sms, int first_step, int nsteps,
+                                                                              int skip, int do_init)
+{
+    extern __shared__ __align__(16) unsigned char grid_raw[];
+    GridWarp& gw = reinterpret_cast<GridWarp*>(grid_raw)[threadIdx.x >> 5];
+    __shared__ double sh[8][32];
+    if ((threadIdx.x & 31) == 0) gw.inst = -1;
+    __syncwarp();
+    const long long items = strip_from(b.gtiles, num_sms) + kStrips * (b.gtiles - strip_from(b.gtiles, num_sms));
+    unsigned long long phase = 0;
+    const int q0 = do_init ? -1 : 0;
+    if (q0 >= nsteps) return;
+    grid_drift(b, do_init != 0);
+    if (!batch::grid_sync(b.gsync, phase)) return;
+    for (int q = q0; q < nsteps; ++q) {
+        const int step = first_step + q, par = q & 1;
+        const bool init = q < 0, write = init || (skip > 0 && step % skip == 0), more = q + 1 < nsteps;
+        double* pe = b.gpe + par * items;
+        if (write)
+            grid_pairs<true>(b, gw, num_sms, b.gqueue + par, pe);
+        else
+            grid_pairs<false>(b, gw, num_sms, b.gqueue + par, pe);
+        if (!batch::grid_sync(b.gsync, phase)) return;
+        if (blockIdx.x == 0 && threadIdx.x == 0) b.gqueue[par ^ 1] = 0;  // the next step's queue
+        grid_rows(b, init, more && !write);
+        if (!more && !write) break;
+        if (!batch::grid_sync(b.gsync, phase)) return;
+        if (write) {
+            const int r = init ? 0 : min(step / skip, b.nrec - 1);
+            grid_energy(b, num_sms, pe, r, sh);
+            if (!more) break;
+            if (!batch::grid_sync(b.gsync, phase)) return;
+            grid_drift(b, false);
+            if (!batch::grid_sync(b.gsync, phase)) return;
+        }
+    }
+}
+
+__global__ void batch_views_kernel(const __grid_constant__ Batch b)
+{
+    const int inst = blockIdx.x * blockDim.x + threadIdx.x;
+    if (inst >= b.ninst) return;
+    const int n = b.cnt[inst];
+    System v;
+    make_view(v, b, inst, b.off[inst], n, (n + kBlock - 1) / kBlock * kBlock, b.xpair + b.gpair_off[inst],
+              b.xtorq + b.gpair_off[inst], b.xmask + b.gmask_off[inst]);
+    b.views[inst] = v;
+}
+
 __global__ void batch_derive_kernel(const __grid_constant__ Batch b)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -341,6 +570,35 @@ __global__ void batch_derive_kernel(const __grid_constant__ Batch b)
 void launch_batch_derive(const Batch& b, cudaStream_t st)
 {
     batch_derive_kernel<<<(b.total + 255) / 256, 256, 0, st>>>(b);
+    if (b.views) batch_views_kernel<<<(b.ninst + 63) / 64, 64, 0, st>>>(b);
+}
+
+static size_t exact_grid_smem()
+{
+    cudaFuncSetAttribute(batch_exact_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         kGridWarps * (int)sizeof(GridWarp));
+    return kGridWarps * sizeof(GridWarp);
+}
+
+cudaError_t launch_batch_exact_grid(const Batch& b, int num_sms, int first_step, int nsteps, int skip, int do_init,
+                                    cudaStream_t st)
+{
+    return launch_cooperative(batch_exact_grid_kernel, num_sms, 32 * kGridWarps, exact_grid_smem(), st, b, num_sms,
+                              first_step, nsteps, skip, do_init);
+}
+
+bool batch_grid_fits(bool mixed)
+{
+    if (mixed) return batch_mixed_grid_fits();
+    int nb = 0;
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_exact_grid_kernel, 32 * kGridWarps,
+                                                         exact_grid_smem()) == cudaSuccess && nb >= 1;
+}
+
+long long batch_grid_items(long long tiles, int num_sms, bool mixed)
+{
+    const long long split = mixed ? tiles : strip_from(tiles, num_sms);
+    return split + kStrips * (tiles - split);
 }
 
 // Dynamic shared memory of the pair-tile pass (above the 48 KB that need no

@@ -5,14 +5,17 @@
 #include "../../include/spacelab_batch.h"
 #include "../../include/spacelab_gpu.h"
 #include "sl_batch.h"
+#include "sl_kernels.h"
 #include "sl_pair_mixed.cuh"
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <vector>
 
 int sl_record_error(int code, const char* msg);
@@ -35,6 +38,9 @@ const int kThreadsTiles[3] = {128, 256, 512};  // the mixed pair-tile pass's can
 // most this, and at most a third of the free memory at creation
 constexpr size_t kExactTileScratchBytes = size_t(48) << 30;
 
+// Arrays of at least so many doubles (4 MB) are downloaded on a thread each.
+constexpr size_t kThreadedDownload = size_t(1) << 19;
+
 }  // namespace
 
 struct sl_batch {
@@ -49,12 +55,32 @@ struct sl_batch {
     double* snapshot = nullptr;  // initial state for the autotuner (device)
     bool uploaded = false;
     std::vector<int> counts, offsets;
+    void* grid_arena = nullptr;  // the lockstep form's scratch and lists
 };
 
 namespace {
 
+// Whether a shape runs in lockstep (sl_batch.cu): the pair-tile pass, where
+// every instance's buffers could be had.  The exact form always does (ms per
+// step, GB300, queue of whole instances at its best shape against lockstep: 32
+// collisions of up to 450 spheres 1.10 / 0.20, 256 of up to 300 0.55 / 0.36,
+// 1024 1.70 / 1.29, 4096 8.46 / 5.66; 256 of up to 1050 6.03 / 2.89).  The
+// mixed form's queue keeps an instance's partials in L2 and wins once the
+// instances spread over the CTAs evenly, so lockstep takes the batches whose
+// largest instance alone, at the shape's warps, would last 1.25 times an even
+// share (64 of up to 2400 spheres 0.92 / 0.20; 512 of them at 128, 256, 512
+// threads 3.30, 1.89, 1.03 / 1.14; 2048 at 128, 512: 4.68, 4.29 / 4.65).
+bool runs_in_lockstep(const sl_batch* h, int tile, int threads)
+{
+    if (tile != 0 || !h->b.grid) return false;
+    if (h->mode == SL_MODE_EXACT) return true;
+    const double largest = (double)h->b.part_nb * (h->b.part_nb + 1) / 2;
+    return largest * h->num_sms * 16.0 / (threads / 32) >= 1.25 * (double)h->b.gtiles;
+}
+
 int blocks_for(const sl_batch* h, int tile, int threads)
 {
+    if (runs_in_lockstep(h, tile, threads)) return h->num_sms;
     int per_sm = sl::batch_max_blocks_per_sm(tile, threads, h->mode == SL_MODE_MIXED_DF);
     if (per_sm < 1) per_sm = 1;
     long long blocks = (long long)per_sm * h->num_sms;
@@ -71,11 +97,22 @@ int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, i
     cudaGraph_t g;
     SLB_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(h->b.counter, 0, sizeof(int), h->stream);
-    if (h->mode == SL_MODE_MIXED_DF)
+    const bool lockstep = runs_in_lockstep(h, tile, threads);
+    cudaError_t launched = cudaSuccess;
+    if (lockstep) {
+        cudaMemsetAsync(h->b.gsync, 0, sizeof(sl::GridSync) + 2 * sizeof(int), h->stream);  // and the queues behind it
+        launched = h->mode == SL_MODE_MIXED_DF
+                       ? sl::launch_batch_mixed_grid(h->b, h->num_sms, first_step, nsteps, skip, do_init, h->stream)
+                       : sl::launch_batch_exact_grid(h->b, h->num_sms, first_step, nsteps, skip, do_init, h->stream);
+    } else if (h->mode == SL_MODE_MIXED_DF)
         sl::launch_batch_mixed(h->b, tile, threads, blocks, first_step, nsteps, skip, do_init, h->stream);
     else
         sl::launch_batch_exact(h->b, tile, threads, blocks, first_step, nsteps, skip, do_init, h->stream);
     SLB_CUDA(cudaStreamEndCapture(h->stream, &g));
+    if (launched != cudaSuccess) {
+        cudaGraphDestroy(g);
+        return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(launched));
+    }
     cudaGraphExec_t ge;
     const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
     cudaGraphDestroy(g);
@@ -85,6 +122,97 @@ int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, i
     cudaGraphExecDestroy(ge);
     if (e2 != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e2));
     if (e3 != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e3));
+    if (lockstep) {
+        sl::GridSync gs{};
+        SLB_CUDA(cudaMemcpy(&gs, h->b.gsync, sizeof gs, cudaMemcpyDeviceToHost));
+        if (gs.failed) return sl_record_error(SL_ERR_TIMEOUT, "a bounded wait between the batch's phases ran out");
+    }
+    return SL_OK;
+}
+
+// The lockstep form's lists and scratch (pair terms and torques of every
+// instance, or the mixed form's partials), where they fit the budget: per
+// instance 48 npad^2 bytes exact, 24 nb npad bytes mixed.
+int setup_lockstep(sl_batch* h, const std::vector<int>& order)
+{
+    sl::Batch& b = h->b;
+    const bool mixed = h->mode == SL_MODE_MIXED_DF;
+    if (!sl::batch_grid_fits(mixed)) return SL_OK;
+    std::vector<long long> tiles(b.ninst + 1), blocks(b.ninst + 1), pair(b.ninst), mask(b.ninst);
+    std::vector<int> blk_inst, blk;
+    std::vector<int4> tile;
+    long long np = 0, nm = 0;
+    for (int k = 0; k < b.ninst; ++k) {
+        const int inst = order[k], nb = (h->counts[inst] + sl::kBlock - 1) / sl::kBlock;
+        const long long npad = (long long)nb * sl::kBlock;
+        tiles[k + 1] = tiles[k] + (long long)nb * (nb + 1) / 2;
+        blocks[k + 1] = blocks[k] + nb;
+        for (int j = 0; j < nb; ++j) {
+            blk_inst.push_back(inst);
+            blk.push_back(j);
+            for (int y = 0; y <= j; ++y) tile.push_back(make_int4(inst, h->offsets[inst], h->counts[inst], j << 16 | y));
+        }
+        pair[inst] = np;
+        mask[inst] = nm;
+        np += mixed ? 6 * nb * npad : 3 * npad * npad;
+        nm += mixed ? npad * ((nb + 31) / 32) : npad * nb;  // mixed: torque marks
+    }
+    const long long items = sl::batch_grid_items(tiles[b.ninst], h->num_sms, mixed);
+    size_t off = 0;
+    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
+    const size_t o_pair = take((size_t)np * (mixed ? sizeof(float) : sizeof(double))),
+                 o_torq = take(mixed ? 0 : (size_t)np * sizeof(double)), o_mask = take((size_t)nm * sizeof(uint32_t));
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+    if (off > std::min(kExactTileScratchBytes, free_b / 3)) return SL_OK;
+    const size_t zeroed = off;  // the buffers' unwritten entries are read as +0.0
+    const size_t o_tiles = take(tiles.size() * sizeof(long long)), o_blocks = take(blocks.size() * sizeof(long long)),
+                 o_tile = take(tile.size() * sizeof(int4)), o_poff = take(pair.size() * sizeof(long long)), o_moff = take(mask.size() * sizeof(long long)),
+                 o_binst = take(blk.size() * sizeof(int)), o_blk = take(blk.size() * sizeof(int)),
+                 o_views = take(mixed ? 0 : (size_t)b.ninst * sizeof(sl::System)),
+                 o_pe = take(2 * (size_t)items * sizeof(double)), o_ke = take(blk.size() * 8 * sizeof(double)),
+                 o_sync = take(sizeof(sl::GridSync) + 2 * sizeof(int));
+    if (cudaMalloc(&h->grid_arena, off) != cudaSuccess) {
+        cudaGetLastError();
+        h->grid_arena = nullptr;
+        return SL_OK;  // the per-CTA form runs instead
+    }
+    char* p = static_cast<char*>(h->grid_arena);
+    SLB_CUDA(cudaMemsetAsync(p, 0, zeroed, h->stream));
+    auto put = [&](size_t o, const void* src, size_t bytes) {
+        return cudaMemcpyAsync(p + o, src, bytes, cudaMemcpyHostToDevice, h->stream);
+    };
+    SLB_CUDA(put(o_tiles, tiles.data(), tiles.size() * sizeof(long long)));
+    SLB_CUDA(put(o_blocks, blocks.data(), blocks.size() * sizeof(long long)));
+    SLB_CUDA(put(o_tile, tile.data(), tile.size() * sizeof(int4)));
+    SLB_CUDA(put(o_poff, pair.data(), pair.size() * sizeof(long long)));
+    SLB_CUDA(put(o_moff, mask.data(), mask.size() * sizeof(long long)));
+    SLB_CUDA(put(o_binst, blk_inst.data(), blk_inst.size() * sizeof(int)));
+    SLB_CUDA(put(o_blk, blk.data(), blk.size() * sizeof(int)));
+    SLB_CUDA(cudaStreamSynchronize(h->stream));
+    if (mixed) {
+        b.gpart = reinterpret_cast<float*>(p + o_pair);
+        b.xmask = reinterpret_cast<uint32_t*>(p + o_mask);
+    } else {
+        b.xpair = reinterpret_cast<double*>(p + o_pair);
+        b.xtorq = reinterpret_cast<double*>(p + o_torq);
+        b.xmask = reinterpret_cast<uint32_t*>(p + o_mask);
+        b.views = reinterpret_cast<sl::System*>(p + o_views);
+    }
+    b.gtile_off = reinterpret_cast<const long long*>(p + o_tiles);
+    b.gblk_off = reinterpret_cast<const long long*>(p + o_blocks);
+    b.gtile = reinterpret_cast<const int4*>(p + o_tile);
+    b.gpair_off = reinterpret_cast<const long long*>(p + o_poff);
+    b.gmask_off = reinterpret_cast<const long long*>(p + o_moff);
+    b.gblk_inst = reinterpret_cast<const int*>(p + o_binst);
+    b.gblk = reinterpret_cast<const int*>(p + o_blk);
+    b.gpe = reinterpret_cast<double*>(p + o_pe);
+    b.gke = reinterpret_cast<double*>(p + o_ke);
+    b.gsync = reinterpret_cast<sl::GridSync*>(p + o_sync);
+    b.gqueue = reinterpret_cast<int*>(b.gsync + 1);
+    b.gtiles = tiles[b.ninst];
+    b.gblocks = (int)blocks[b.ninst];
+    b.grid = 1;
     return SL_OK;
 }
 
@@ -193,6 +321,14 @@ int sl_batch_create(int ninst, const int* counts, const sl_material* mat, int mo
     b.total = (int)total;
     b.nrec = steps / skip + 1;
     b.mat = sl::Material{mat->G, mat->Ha, mat->u_s, mat->u_r, mat->h_min};
+    // largest instances first: the work queue then balances like LPT scheduling
+    std::vector<int> ord(ninst);
+    std::iota(ord.begin(), ord.end(), 0);
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return counts[a] > counts[c]; });
+    if (int r = setup_lockstep(h, ord)) {
+        sl_batch_destroy(h);
+        return r;
+    }
     const size_t T = (size_t)total;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
@@ -226,7 +362,7 @@ int sl_batch_create(int ninst, const int* counts, const sl_material* mat, int mo
     b.xmask_cta = (size_t)b.x_np * b.x_nb;
     size_t o_xpair = 0, o_xtorq = 0, o_xmask = 0;
     bool exact_tiles = false;
-    if (mode == SL_MODE_EXACT) {
+    if (mode == SL_MODE_EXACT && !b.grid) {
         const size_t per_cta = 2 * b.xpair_cta * sizeof(double) + b.xmask_cta * sizeof(uint32_t);
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
@@ -279,10 +415,6 @@ int sl_batch_create(int ninst, const int* counts, const sl_material* mat, int mo
     b.isc = reinterpret_cast<sl::Scalars*>(base + o_isc);
     b.status = reinterpret_cast<unsigned*>(base + o_st);
     h->snapshot = reinterpret_cast<double*>(base + o_snap);
-    // largest instances first: the work queue then balances like LPT scheduling
-    std::vector<int> ord(ninst);
-    std::iota(ord.begin(), ord.end(), 0);
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return counts[a] > counts[c]; });
     cudaError_t e = cudaMemsetAsync(h->arena, 0, off, h->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(order, ord.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
     if (e == cudaSuccess)
@@ -302,6 +434,7 @@ int sl_batch_destroy(sl_batch* h)
     if (!h) return SL_OK;
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->arena) cudaFree(h->arena);
+    if (h->grid_arena) cudaFree(h->grid_arena);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return SL_OK;
@@ -433,17 +566,59 @@ int sl_batch_run(sl_batch* h, int first_step, int nsteps, int do_init)
 int sl_batch_download(sl_batch* h, double* pos, double* vel, double* w, double* acc, double* aacc)
 {
     if (!h) return sl_record_error(SL_ERR_ARG, "null batch");
-    const size_t T = (size_t)h->b.total;
-    std::vector<double> tmp(T);
+    sl::Batch& b = h->b;
+    const size_t count = 3 * (size_t)b.total;
+    // A kernel transposes the arrays on the device (into the snapshot area, free
+    // outside the autotuner), and each array comes back through a small buffer
+    // on a host thread of its own.  A large batch's arrays are fresh memory in
+    // every call, and making their pages resident is most of the time: the GPU
+    // or the copy engine does it page by page (20-50 ms for 530,000 spheres),
+    // one host thread in 9 ms.
     double* outs[5] = {pos, vel, w, acc, aacc};
-    const sl::Vec3Soa* src[5] = {&h->b.pos, &h->b.vel, &h->b.w, &h->b.acc, &h->b.aacc};
+    sl::Vec3Soa* src[6] = {&b.pos, &b.vel, &b.w, &b.acc, &b.aacc, &b.prev};
+    double* dst[6] = {};
+    unsigned want = 0;
+    for (int k = 0; k < 5; ++k)
+        if (outs[k]) {
+            want |= 1u << k;
+            dst[k] = h->snapshot + (size_t)k * count;
+        }
+    if (!want) return SL_OK;
+    int dev = 0;
+    SLB_CUDA(cudaGetDevice(&dev));
+    sl::System s{};
+    s.n = b.total;
+    sl::launch_stage_out(s, dst, src, want, h->stream);
+    SLB_CUDA(cudaGetLastError());
+    SLB_CUDA(cudaStreamSynchronize(h->stream));
+    cudaError_t result[5] = {};
+    auto fetch = [&](int k) {
+        constexpr size_t kChunk = size_t(1) << 17;  // doubles
+        cudaError_t e = cudaSetDevice(dev);
+        std::unique_ptr<double[]> buf(new (std::nothrow) double[kChunk]);
+        if (!buf) e = cudaErrorMemoryAllocation;
+        for (size_t o = 0; o < count && e == cudaSuccess; o += kChunk) {
+            const size_t n = std::min(kChunk, count - o);
+            e = cudaMemcpy(buf.get(), dst[k] + o, n * sizeof(double), cudaMemcpyDeviceToHost);
+            if (e == cudaSuccess) std::memcpy(outs[k] + o, buf.get(), n * sizeof(double));
+        }
+        result[k] = e;
+    };
+    std::thread pool[5];
     for (int k = 0; k < 5; ++k) {
         if (!outs[k]) continue;
-        for (int c = 0; c < 3; ++c) {
-            SLB_CUDA(cudaMemcpy(tmp.data(), src[k]->c[c], T * sizeof(double), cudaMemcpyDeviceToHost));
-            for (size_t i = 0; i < T; ++i) outs[k][3 * i + c] = tmp[i];
-        }
+        bool started = false;
+        if (count >= kThreadedDownload) try {
+                pool[k] = std::thread(fetch, k);
+                started = true;
+            } catch (...) {  // no thread to be had
+            }
+        if (!started) fetch(k);
     }
+    for (std::thread& t : pool)
+        if (t.joinable()) t.join();
+    for (cudaError_t e : result)
+        if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
     return SL_OK;
 }
 

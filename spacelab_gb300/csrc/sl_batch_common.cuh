@@ -89,5 +89,39 @@ __device__ __forceinline__ void kick(const Batch& b, int inst, int off, int n, d
     }
 }
 
+// Waits until every CTA of the grid (all resident: a cooperative launch) has
+// arrived; `phase` counts the barriers.  Memory written before it by any CTA
+// is visible after it.  The wait is bounded: a CTA that gives up sets
+// `failed`, and every CTA then returns false.  Called by all threads.
+constexpr long long kGridWaitCycles = 1ll << 33;  // about 4 s
+
+__device__ __forceinline__ bool grid_sync(GridSync* g, unsigned long long& phase)
+{
+    __shared__ int s_ok;
+    ++phase;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(&g->arrived, 1ull) + 1 == phase * gridDim.x)
+            atomicExch(&g->released, phase);
+        bool ok = true;
+        const long long t0 = clock64();
+        volatile unsigned long long* released = &g->released;
+        volatile unsigned* failed = &g->failed;
+        while (*released < phase) {
+            if (*failed || clock64() - t0 > kGridWaitCycles) {
+                atomicExch(&g->failed, 1u);
+                ok = false;
+                break;
+            }
+            __nanosleep(40);
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
 }  // namespace batch
 }  // namespace sl

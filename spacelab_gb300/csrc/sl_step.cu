@@ -77,8 +77,6 @@ __global__ void __launch_bounds__(kDriftThreads) drift_kernel(const __grid_const
 // owns sphere B = 32Y + b and walks the 32 spheres A = 32X + a of the A
 // block; on the diagonal only a > b is a pair.  Tiles are independent; one
 // launch covers the tiles of block columns [c0, c1) with a static stride.
-constexpr int kStripRows = 8, kStrips = kBlock / kStripRows;
-
 // Tiles in column-major order: column Y holds tiles (Y..nb-1, Y); the first
 // tile of column c has index c*nb - c(c-1)/2.
 __device__ __forceinline__ long long col_offset(int nb, int c) { return (long long)c * nb - (long long)c * (c - 1) / 2; }
@@ -96,7 +94,7 @@ __device__ __forceinline__ void col_tile_coords(int nb, long long u, int& X, int
 }
 
 // A work item is a whole tile, or -- the tiles from `split` on, in the
-// column-major order -- a strip of 8 of its 32 rows (pair_split).  The items
+// column-major order -- a strip of 8 of its 32 rows (strip_from).  The items
 // of a launch are numbered from its first tile's; item q's energy goes to
 // pe_tile[q].
 template <bool WRITE>
@@ -132,34 +130,7 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
         double pe = 0;
         uint32_t rowbits, colbits;
         tile_pairs<WRITE>(s, ws, X, Y, lane, a0, a1, B, B < s.n, pe, rowbits, colbits);
-        // Contact bits: row A = 32X + lane gets block Y's bits, row B gets
-        // block X's bits; on the diagonal both describe row 32X + lane.
-        uint32_t* wa = s.cmask + (size_t)(X * kBlock + lane) * s.nb + Y;
-        uint32_t* wb = s.cmask + (size_t)(Y * kBlock + lane) * s.nb + X;
-        if (whole) {
-            if (X == Y) {
-                *wa = rowbits | colbits;
-            } else {
-                *wa = rowbits;
-                *wb = colbits;
-            }
-        } else {
-            // strip w holds rows 8w .. 8w + 7: those rows' words, and byte w
-            // of every column's word.  On the diagonal, row i of strip w has
-            // its bytes below w from rowbits, byte w from both, and those
-            // above from the later strips' columns.
-            static_assert(kStripRows == 8, "a strip's column bits are one byte");
-            uint8_t* ba = reinterpret_cast<uint8_t*>(wa);
-            const int mine = lane / kStripRows;
-            if (X != Y) {
-                if (mine == strip) *wa = rowbits;
-                reinterpret_cast<uint8_t*>(wb)[strip] = (uint8_t)(colbits >> (8 * strip));
-            } else if (mine == strip) {
-                for (int k = 0; k <= strip; ++k) ba[k] = (uint8_t)((rowbits | colbits) >> (8 * k));
-            } else if (mine < strip) {
-                ba[strip] = (uint8_t)(colbits >> (8 * strip));
-            }
-        }
+        store_contacts(s, X, Y, lane, whole ? -1 : strip, rowbits, colbits);
         if (WRITE) {
             for (int off = 16; off > 0; off >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, off);
             if (lane == 0) s.pe_tile[q] = pe;
@@ -435,25 +406,6 @@ static void launch_rowsum(const System& s, cudaStream_t st, const CUtensorMap* m
         rowsum_kernel<<<(3 * s.n + kRowThreads - 1) / kRowThreads, kRowThreads, 0, st>>>(s, b0, b1, first, last);
 }
 
-// The first tile (in the column-major order) that is taken in strips of 8
-// rows.  A strip costs its share of a tile and ~12% more (its own blocks, and
-// a quarter of the marked pairs in a warp of their own), and pays where the
-// warps are not all busy to the end.  Of the 16 warps per SM that are
-// resident, with T tiles (us per step, GB300, no strips against these):
-//   - T up to half of them: all tiles.  The step is a warp's latency, 32 rows of
-//     ~1500 cycles.  N=96 65.5 -> 30.9, N=300 69.8 -> 34.8, N=1000 111 -> 85,
-//     N=1400 128 -> 115.
-//   - more: as many as half the warps, the last ones, which shortens the tail:
-//     N=1733 162 -> 152, N=3000 311 -> 305, N=5000 692.6 -> 688.5.
-//   - a last round that is nearly full without them: none.  N=2200 (99% full):
-//     199, 205 with them.
-long long pair_split(long long tiles, int num_sms)
-{
-    const long long warps = 16LL * num_sms;
-    if (2 * tiles <= warps) return 0;
-    return 10 * (tiles % warps) > 9 * warps ? tiles : tiles - warps / 2;
-}
-
 static void launch_pair_columns(const System& s, bool write, int num_sms, cudaStream_t st, int c0, int c1, int phase,
                                 long long split, bool pdl)
 {
@@ -477,7 +429,7 @@ void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, St
     System s = sys;
     int cb[kPairPhases + 1];
     const int np = ov ? phase_bounds(s.nb, cb) : 1;
-    const long long split = pair_split(s.ntiles, num_sms);  // the same items, and energy sums, with and without phases
+    const long long split = strip_from(s.ntiles, num_sms);  // the same items, and energy sums, with and without phases
     s.nitems = split + kStrips * (s.ntiles - split);
     // phases wait on events between the kernels: plain launches there
     const bool pdl = np <= 1;

@@ -283,4 +283,58 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
     }
 }
 
+// A tile may be taken in strips of 8 of its 32 rows.
+constexpr int kStripRows = 8, kStrips = kBlock / kStripRows;
+
+// Contact words of an item of tile (X, Y): row A = 32X + lane gets block Y's
+// bits, row B block X's; on the diagonal both describe row 32X + lane.
+// strip < 0: the whole tile.  Strip w holds rows 8w .. 8w + 7: those rows'
+// words, and byte w of every column's word, so that the strips' stores are
+// disjoint.  On the diagonal, row i of strip w has its bytes below w from
+// rowbits, byte w from both, and those above from the later strips' columns.
+__device__ __forceinline__ void store_contacts(const System& s, int X, int Y, int lane, int strip, uint32_t rowbits,
+                                               uint32_t colbits)
+{
+    static_assert(kStripRows == 8, "a strip's column bits are one byte");
+    uint32_t* wa = s.cmask + (size_t)(X * kBlock + lane) * s.nb + Y;
+    uint32_t* wb = s.cmask + (size_t)(Y * kBlock + lane) * s.nb + X;
+    if (strip < 0) {
+        if (X == Y) {
+            *wa = rowbits | colbits;
+        } else {
+            *wa = rowbits;
+            *wb = colbits;
+        }
+        return;
+    }
+    uint8_t* ba = reinterpret_cast<uint8_t*>(wa);
+    const int mine = lane / kStripRows;
+    if (X != Y) {
+        if (mine == strip) *wa = rowbits;
+        reinterpret_cast<uint8_t*>(wb)[strip] = (uint8_t)(colbits >> (8 * strip));
+    } else if (mine == strip) {
+        for (int k = 0; k <= strip; ++k) ba[k] = (uint8_t)((rowbits | colbits) >> (8 * k));
+    } else if (mine < strip) {
+        ba[strip] = (uint8_t)(colbits >> (8 * strip));
+    }
+}
+
+// The first tile of T that is taken in strips.  A strip costs its share of a tile and ~12% more (its own blocks, and
+// a quarter of the marked pairs in a warp of their own), and pays where the
+// warps are not all busy to the end.  Of the 16 warps per SM that are
+// resident, with T tiles (us per step, GB300, no strips against these):
+//   - T up to half of them: all tiles.  The step is a warp's latency, 32 rows of
+//     ~1500 cycles.  N=96 65.5 -> 30.9, N=300 69.8 -> 34.8, N=1000 111 -> 85,
+//     N=1400 128 -> 115.
+//   - more: as many as half the warps, the last ones, which shortens the tail:
+//     N=1733 162 -> 152, N=3000 311 -> 305, N=5000 692.6 -> 688.5.
+//   - a last round that is nearly full without them: none.  N=2200 (99% full):
+//     199, 205 with them.
+__host__ __device__ inline long long strip_from(long long tiles, int num_sms)
+{
+    const long long warps = 16LL * num_sms;
+    if (2 * tiles <= warps) return 0;
+    return 10 * (tiles % warps) > 9 * warps ? tiles : tiles - warps / 2;
+}
+
 }  // namespace sl
