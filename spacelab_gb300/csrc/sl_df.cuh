@@ -11,6 +11,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "sl_f32x2.cuh"
+
 namespace sl {
 namespace df {
 
@@ -85,6 +87,26 @@ struct Sum3 {
         const F2 u = two_sum(b, t.lo);
         b = u.hi;
         c += u.lo;
+    }
+};
+
+// Two Sum3 at once, in packed arithmetic: the halves are separate sums, each
+// with the operations of Sum3.
+struct Sum3x2 {
+    f2::F32x2 a, b, c;
+    __device__ __forceinline__ void add(f2::F32x2 v)
+    {
+        using namespace f2;
+        const F32x2 m1 = pair2(-1.0f, -1.0f);  // x - y = y m1 + x, exactly rounded
+        const F32x2 s = add2(a, v);
+        const F32x2 vp = fma2(a, m1, s);
+        const F32x2 e = add2(fma2(fma2(vp, m1, s), m1, a), fma2(vp, m1, v));
+        a = s;
+        const F32x2 t = add2(b, e);
+        const F32x2 ep = fma2(b, m1, t);
+        const F32x2 r = add2(fma2(fma2(ep, m1, t), m1, b), fma2(ep, m1, e));
+        b = t;
+        c = add2(c, r);
     }
 };
 

@@ -25,13 +25,13 @@
 // r and the FP64 overlap: the vdW coefficient, elastic, gravity, sliding and
 // rolling friction and the torques, in lengths scaled by 2^-len_shift.
 //
-// What bounds it: FP32 issue, some 150 instructions a pair, half of them the
-// six error-free sums.  On the FP64 pipe the subtraction and the sums were 9
-// adds a pair at 19 SM-cycles each (one narrow unit per SM), 171 cycles
-// for a warp's 32 pairs, and the pair kernel ran at 0.96 of that unit's rate;
-// the FP32 pipe is 72 times as wide.  N=20000 polydisperse, 20 steps: 74.2 ->
-// 23.8 ms; 3 and 5 CTAs per SM 25.2 and 23.9, the sweep unrolled 1 and 4
-// times 24.3 and 23.6.
+// What bounds it (ncu, N=9000): the FP32 pipe at 72%, half of its work the six
+// error-free sums, beside issue at 68%; the two spheres' sums of a component
+// are added in packed arithmetic.  On the FP64 pipe the subtraction and the
+// sums were 9 adds a pair at 19 SM-cycles each (one narrow unit per SM), 171
+// cycles for a warp's 32 pairs, at 0.96 of that unit's rate; now it is 58.
+// N=20000 polydisperse, 20 steps: 74.2 -> 23.1 ms (sums one by one, unrolled
+// twice 23.8; 3 and 5 CTAs per SM 25.2 and 23.9).
 //
 // Accumulation order: one warp evaluates a 32 x 32 tile in a diagonal sweep
 // (lane b holds column sphere B's sum; row r's sum travels one lane down per
@@ -117,12 +117,13 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
         double pe = 0.0;       // close pairs' potential (FP64)
         df::Sum3 pe_far{};     // far pairs' vdW brackets, times -Ha/6 at the end
         uint32_t colbits = 0;
-        df::Sum3 ra[3] = {};  // running sum of row (lane + k) mod 32 at step k
-        df::Sum3 cb[3] = {};  // sphere B's sum
+        // low halves: the running sum of row (lane + k) mod 32 at step k; high
+        // halves: sphere B's sum
+        df::Sum3x2 sum[3] = {};
         // FULL: a tile off the diagonal whose rows and columns are all spheres
         auto sweep = [&](auto full_tag) {
             constexpr bool FULL = decltype(full_tag)::value;
-#pragma unroll 2
+#pragma unroll 4
             for (int k = 0; k < kBlock; ++k) {
                 const int r = (lane + k) & (kBlock - 1);
                 const bool valid = FULL || (bvalid && r < nA && (X != Y || lane < r));
@@ -188,11 +189,14 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
                 const float f[3] = {fx, fy, fz};
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
-                    ra[c].add(f[c]);
-                    cb[c].add(f[c]);
-                    ra[c].a = __shfl_sync(0xffffffffu, ra[c].a, nxt);
-                    ra[c].b = __shfl_sync(0xffffffffu, ra[c].b, nxt);
-                    ra[c].c = __shfl_sync(0xffffffffu, ra[c].c, nxt);
+                    sum[c].add(f2::pair2(f[c], f[c]));
+                    const auto pass = [nxt](f2::F32x2& v) {  // the row's part moves on
+                        const float2 h = f2::split2(v);
+                        v = f2::pair2(__shfl_sync(0xffffffffu, h.x, nxt), h.y);
+                    };
+                    pass(sum[c].a);
+                    pass(sum[c].b);
+                    pass(sum[c].c);
                 }
             }
         };
@@ -211,18 +215,25 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
         }
         const int iA = X * kBlock + lane;
         double* Pt = s.part64;
+        double rsum[3], csum[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 a = f2::split2(sum[c].a), b = f2::split2(sum[c].b), d = f2::split2(sum[c].c);
+            rsum[c] = total({a.x, b.x, d.x});
+            csum[c] = total({a.y, b.y, d.y});
+        }
         if (X == Y) {  // sphere iA == B: partners j < i as A (row), j > i as B (column)
             const size_t o = (size_t)X * s.npad + iA;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) Pt[o + c * pplane] = total(ra[c]) - total(cb[c]);
+            for (int c = 0; c < 3; ++c) Pt[o + c * pplane] = rsum[c] - csum[c];
             s.cmask[o] = rowbits | colbits;
             if (rowbits | colbits) s.contact_flag[iA] = 1;
         } else {
             const size_t oa = (size_t)Y * s.npad + iA, ob = (size_t)X * s.npad + B;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                Pt[oa + c * pplane] = total(ra[c]);
-                Pt[ob + c * pplane] = -total(cb[c]);
+                Pt[oa + c * pplane] = rsum[c];
+                Pt[ob + c * pplane] = -csum[c];
             }
             s.cmask[oa] = rowbits;
             s.cmask[ob] = colbits;

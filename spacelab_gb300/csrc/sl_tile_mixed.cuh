@@ -19,6 +19,7 @@
 #pragma once
 #include "sl_device.cuh"
 #include "sl_df.cuh"
+#include "sl_f32x2.cuh"
 #include "sl_pair_mixed.cuh"
 
 #include <type_traits>
@@ -32,40 +33,12 @@
 namespace sl {
 namespace mt {
 
-// Two FP32 numbers in a register pair, for the packed operations (one issue
-// slot for both; each half is the IEEE operation).
-typedef unsigned long long F32x2;
-
-__device__ __forceinline__ F32x2 pair2(float a, float b)
-{
-    F32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ float2 split2(F32x2 v)
-{
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ F32x2 add2(F32x2 a, F32x2 b)
-{
-    F32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ F32x2 mul2(F32x2 a, F32x2 b)
-{
-    F32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ F32x2 fma2(F32x2 a, F32x2 b, F32x2 c)
-{
-    F32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
+using f2::F32x2;
+using f2::add2;
+using f2::fma2;
+using f2::mul2;
+using f2::pair2;
+using f2::split2;
 
 // Rows in shared memory, kRow floats each (16-byte loads of 32 different rows
 // fall in distinct banks).  Two steps of the sweep are taken at once, so row r
