@@ -115,17 +115,12 @@ __device__ __forceinline__ bool general_pair(const System& s, const ABlock& ab, 
     return contact;
 }
 
-// The marked pairs of a tile (lane's bit a = pair (32X + a, 32Y + lane)),
-// packed and evaluated one per lane; rowbits/colbits get the contacts.  Out
-// of line: the sweep's registers are dead here.
-template <bool WRITE>
-__device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, int X, int Y, uint32_t marked)
+// Packs the pairs of a tile given by the lanes' masks (lane's bit a = pair
+// (32X + a, 32Y + lane)) into the list, entry a << 5 | lane; their number.
+__device__ __forceinline__ int pack_list(TileScratch& ws, uint32_t marked)
 {
     const int lane = threadIdx.x & 31;
-    double pe = 0;
     uint16_t* list = reinterpret_cast<uint16_t*>(ws.bstage);
-    ws.rowc[lane] = 0;
-    ws.colc[lane] = 0;
     const int cnt = __popc(marked);
     int at = cnt;
 #pragma unroll
@@ -138,12 +133,49 @@ __device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, i
     __syncwarp();  // the staging's last reads are done
     for (uint32_t w = marked; w; w &= w - 1) list[at++] = (uint16_t)(((__ffs(w) - 1) << 5) | lane);
     __syncwarp();
+    return total;
+}
+
+// The marked pairs of a tile, packed and evaluated one per lane; ws.rowc and
+// ws.colc get the contacts.  Out of line: the sweep's registers are dead here.
+template <bool WRITE>
+__device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, int X, int Y, uint32_t marked)
+{
+    const int lane = threadIdx.x & 31;
+    double pe = 0;
+    const uint16_t* list = reinterpret_cast<const uint16_t*>(ws.bstage);
+    ws.rowc[lane] = 0;
+    ws.colc[lane] = 0;
+    const int total = pack_list(ws, marked);
     for (int e = lane; e < total; e += 32) {
         const int a = list[e] >> 5, b = list[e] & 31;
         if (general_pair<WRITE>(s, ws.ab, X, a, Y * kBlock + b, pe)) {
             atomicOr(&ws.rowc[a], 1u << b);
             atomicOr(&ws.colc[b], 1u << a);
         }
+    }
+    __syncwarp();
+    return pe;
+}
+
+// The van der Waals potential of a write step's near pairs (settled by the
+// sweep, but too close for vdw_energy_series), packed and evaluated one per
+// lane as well: the closed form is ~3000 cycles of dependent FP64 divisions
+// and a logarithm, and a row of a dense cluster nearly always has one.
+// N=201 (112 strips of 8 rows, one warp each), pair kernel of a write step:
+// 63.5 -> 57.3 us.
+static __device__ __noinline__ double near_potentials(const System& s, TileScratch& ws, int X, int Y, uint32_t near)
+{
+    const ABlock& ab = ws.ab;
+    double pe = 0;
+    const uint16_t* list = reinterpret_cast<const uint16_t*>(ws.bstage);
+    const int total = pack_list(ws, near);
+    for (int e = threadIdx.x & 31; e < total; e += 32) {
+        const int a = list[e] >> 5, B = Y * kBlock + (list[e] & 31);
+        const double Ra = ab.R[a], Rb = s.R[B];
+        const double rx = s.pos.c[0][B] - ab.x[a], ry = s.pos.c[1][B] - ab.y[a], rz = s.pos.c[2][B] - ab.z[a];
+        const double h = fabs((Ra + Rb) - sqrt(rx * rx + ry * ry + rz * rz));
+        pe += vdw_energy(s.mat.Ha, h < s.mat.h_min ? s.mat.h_min : h, Ra, Rb, ab.twoR[a]);  // :239
     }
     __syncwarp();
     return pe;
@@ -169,7 +201,8 @@ __device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, i
 template <bool WRITE, bool UNI>
 __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                             double bx, double by, double bz, const pf::Sphere& sb,
-                                            const pf::Uniform& un, bool bvalid, double& pe, uint32_t& marked)
+                                            const pf::Uniform& un, bool bvalid, double& pe, uint32_t& marked,
+                                            uint32_t& near)
 {
     const ABlock& ab = ws.ab;
     const size_t plane = (size_t)s.npad * s.npad;
@@ -197,7 +230,11 @@ __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, in
         const bool mark = valid && (__double_as_longlong(pr.overlap) > 0 || !pr.fl.sure());
         if (mark) marked |= 1u << a;
         if (WRITE) {
-            if (valid && !mark) pe += vdw_energy_far_df(s.mat.Ha, pr.h, sa.R, sb.R, 2 * sa.R);  // :239
+            if (valid && !mark) {  // :239
+                const VdwArg v = vdw_arg(pr.h, sa.R, sb.R, 2 * sa.R);
+                if (v.far()) pe += vdw_energy_series(s.mat.Ha, v);
+                else near |= 1u << a;
+            }
         }
         if (valid) {
             double* pa = rowA + (size_t)a * s.npad;
@@ -263,17 +300,18 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
     const double R0 = ab.R[0], m0 = ab.m[0];
     const bool uni = __all_sync(0xffffffffu, (!areal || (same(sa.R, R0) && same(ab.m[lane], m0))) &&
                                                  (!bvalid || (same(Rb, R0) && same(mb, m0))));
-    uint32_t marked = 0;
+    uint32_t marked = 0, near = 0;
     if (!sane) {
         const uint32_t all = (a1 >= 32 ? ~0u : (1u << a1) - 1u) & ~((1u << a0) - 1u);
         marked = bvalid ? (X != Y ? all : all & ~((2u << lane) - 1u)) : 0u;
     } else if (uni) {
         const pf::Uniform un{R0 + R0, ab.fourR[0] * R0, pf::unpack(ab.cR3[0] * R0 * R0 * R0)};
-        sweep_pairs<WRITE, true>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked);
+        sweep_pairs<WRITE, true>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     } else {
         const pf::Uniform un{0.0, 0.0, {0, 0}};
-        sweep_pairs<WRITE, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked);
+        sweep_pairs<WRITE, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     }
+    if (WRITE && __any_sync(0xffffffffu, near != 0u)) pe += near_potentials(s, ws, X, Y, near);
     rowbits = colbits = 0;
     if (__any_sync(0xffffffffu, marked != 0u)) {
         pe += general_pairs<WRITE>(s, ws, X, Y, marked);

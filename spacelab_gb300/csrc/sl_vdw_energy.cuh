@@ -65,16 +65,23 @@ __host__ __device__ constexpr Coef coef(int j)
 
 }  // namespace vdwdf
 
-// U_vdw of a pair out of contact with gap h >= h_min (the value the
-// reference adds to PE at ColliderSingleCore.cpp:239).
-__device__ __forceinline__ double vdw_energy_far_df(double Ha, double h, double Ra, double Rb, double twoRa)
+// S and 2RaRb of a pair out of contact with gap h; far: w <= 1/4.
+struct VdwArg {
+    double S, two_RaRb;
+    __device__ bool far() const { return 3.0 * two_RaRb <= S; }
+};
+
+__device__ __forceinline__ VdwArg vdw_arg(double h, double Ra, double Rb, double twoRa)
 {
     const double sum = Ra + Rb;
-    const double S = h * (h + (sum + sum));  // z^2 - (Ra + Rb)^2
-    const double two_RaRb = twoRa * Rb;
-    if (!(3.0 * two_RaRb <= S)) return vdw_energy(Ha, h, Ra, Rb, twoRa);  // w > 1/4: the closed form
+    return {h * (h + (sum + sum)), twoRa * Rb};  // S = z^2 - (Ra + Rb)^2
+}
+
+// U_vdw of a far pair, by the series.
+__device__ __forceinline__ double vdw_energy_series(double Ha, const VdwArg& v)
+{
     using namespace vdwdf;
-    const df::F2 w = div(from_double(two_RaRb), from_double(S + two_RaRb));
+    const df::F2 w = div(from_double(v.two_RaRb), from_double(v.S + v.two_RaRb));
     const df::F2 x = df::sqr(w);
     constexpr Coef c13 = coef(13);
     df::F2 p{c13.hi, c13.lo};
@@ -85,6 +92,14 @@ __device__ __forceinline__ double vdw_energy_far_df(double Ha, double h, double 
     }
     const df::F2 bracket = mul(mul(w, x), p);  // sum_j 4j/(2j+1) w^(2j+1)
     return -Ha / 6 * (f2d_bits(bracket.hi) + f2d_bits(bracket.lo));
+}
+
+// U_vdw of a pair out of contact with gap h >= h_min (the value the
+// reference adds to PE at ColliderSingleCore.cpp:239).
+__device__ __forceinline__ double vdw_energy_far_df(double Ha, double h, double Ra, double Rb, double twoRa)
+{
+    const VdwArg v = vdw_arg(h, Ra, Rb, twoRa);
+    return v.far() ? vdw_energy_series(Ha, v) : vdw_energy(Ha, h, Ra, Rb, twoRa);
 }
 
 }  // namespace sl
