@@ -222,7 +222,7 @@ __device__ double exact_tile_pass(const System& s, TileScratch* scratch)
         __syncwarp();
         const int B = Y * kBlock + lane;
         uint32_t rowbits, colbits;
-        tile_pairs<WRITE>(s, ws, X, Y, lane, 0, min(kBlock, n - X * kBlock), min(B, n - 1), B < n, pe, rowbits,
+        tile_pairs<WRITE ? kPeInline : kNoPe>(s, ws, X, Y, lane, 0, min(kBlock, n - X * kBlock), min(B, n - 1), B < n, pe, rowbits,
                           colbits);
         store_contacts(s, X, Y, lane, -1, rowbits, colbits);
         __syncwarp();
@@ -417,7 +417,7 @@ __device__ void grid_pairs(const Batch& b, GridWarp& gw, int num_sms, int* queue
         const int a0 = whole ? 0 : strip * kStripRows, a1 = whole ? a_end : min(a_end, a0 + kStripRows);
         double pe = 0;
         uint32_t rowbits, colbits;
-        tile_pairs<WRITE>(s, gw.scratch, X, Y, lane, a0, a1, min(B, s.n - 1), B < s.n, pe, rowbits, colbits);
+        tile_pairs<WRITE ? kPeInline : kNoPe>(s, gw.scratch, X, Y, lane, a0, a1, min(B, s.n - 1), B < s.n, pe, rowbits, colbits);
         store_contacts(s, X, Y, lane, strip, rowbits, colbits);
         if (WRITE) {
             for (int o = 16; o > 0; o >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, o);

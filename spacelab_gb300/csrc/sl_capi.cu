@@ -260,8 +260,8 @@ int sl_create(int n, const sl_material* mat, int mode, sl_handle** out)
     const size_t o_pair = take(mixed ? 3 * (size_t)s.nb * np * part_elem : 3 * np * np * sizeof(double));
     const size_t o_torq = take(3 * np * np * (mixed_df ? sizeof(float) : sizeof(double)));
     const size_t o_mask = take(np * s.nb * sizeof(uint32_t));
-    // the exact form: up to four items per tile (strip_from)
-    const size_t o_pe = take((size_t)(mode == SL_MODE_EXACT ? 4 * s.ntiles : s.nitems) * sizeof(double));
+    const size_t o_pe = take((size_t)(mode == SL_MODE_EXACT ? sl::exact_pe_slots(s.ntiles, h->num_sms) : s.nitems) *
+                             sizeof(double));
     const size_t o_red = take(sl::kRedBlocks * 8 * sizeof(double));
     const size_t o_en = take(8 * sizeof(double));
     const size_t o_st = take(sizeof(unsigned int));

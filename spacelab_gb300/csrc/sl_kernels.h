@@ -9,6 +9,21 @@ namespace sl {
 
 constexpr int kRedBlocks = 64;  // energy reduction partial blocks
 
+// Work items per tile of the exact pair kernel, at most (strips of 8 rows).
+constexpr int kTileItems = 4;
+// Whether an exact write step's potentials are work items of their own: where
+// every warp nearly has an SM sub-partition to itself (at most four items per
+// SM), so that a step's time is one warp's.  Write steps (us, with the host's
+// wait, the potentials beside the forces against apart): N=33 73.9 -> 61.5,
+// N=96 77.9 -> 64.2, N=201 93.5 -> 80, N=400 96.6 -> 89, N=520 109.6 -> 108.9;
+// past that the warps share the pipes and the distances would be paid twice.
+inline bool pe_apart(long long ntiles, int num_sms) { return ntiles <= num_sms; }
+// pe_tile entries of an exact system.
+inline long long exact_pe_slots(long long ntiles, int num_sms)
+{
+    return kTileItems * ntiles * (pe_apart(ntiles, num_sms) ? 2 : 1);
+}
+
 // Optional per-kernel CUDA events recorded between the launches of a step:
 // ev[0] after the drift, ev[1] after the pair tiles, ev[2] after the row sums.
 struct StepTimers {

@@ -38,7 +38,7 @@ constexpr size_t kOffPair = kOffScal + 8 * kVec;
 constexpr size_t kOffTorq = kOffPair + up32(3ull * kNp * kNp);
 constexpr size_t kOffMask = kOffTorq + up32(3ull * kNp * kNp);
 constexpr size_t kOffPe = kOffMask + up32((size_t)kNp * kNb / 2 + 1);
-constexpr size_t kOffRed = kOffPe + up32(4 * kTiles);  // up to four items per tile
+constexpr size_t kOffRed = kOffPe + up32(2 * sl::kTileItems * kTiles);  // exact_pe_slots, any device
 constexpr size_t kOffEnergy = kOffRed + up32(sl::kRedBlocks * 8);
 constexpr size_t kOffStatus = kOffEnergy + 32;
 constexpr size_t kOffScalars = kOffStatus + 32;

@@ -35,6 +35,8 @@
 
 namespace sl {
 
+static_assert(kStrips == kTileItems, "strips per tile");
+
 // ---------------------------------------------------------------- pass 1 --
 // One thread per (component, sphere), in small blocks: the few FP64
 // operations per thread then spread over every SM sub-partition's FP64 unit
@@ -96,8 +98,10 @@ __device__ __forceinline__ void col_tile_coords(int nb, long long u, int& X, int
 // A work item is a whole tile, or -- the tiles from `split` on, in the
 // column-major order -- a strip of 8 of its 32 rows (strip_from).  The items
 // of a launch are numbered from its first tile's; item q's energy goes to
-// pe_tile[q].
-template <bool WRITE>
+// pe_tile[q].  kPeApart: one warp per CTA, and as many CTAs again, whose items
+// are the potentials of the first ones' pairs out of contact, to
+// pe_tile[nitems / 2 + q].
+template <int PE>
 __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
                                                           int phase, long long split)
 {
@@ -107,7 +111,9 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
     TileScratch& ws = scratch[wib];
-    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+    const int force_blocks = PE == kPeApart ? gridDim.x / 2 : gridDim.x;
+    const bool potentials = PE == kPeApart && (int)blockIdx.x >= force_blocks;
+    const long long nwarps = (long long)force_blocks * (blockDim.x >> 5);
 
     // A first round of items in warp order; then whichever warp is free takes
     // the next one from the launch's counter (zeroed by the drift kernel),
@@ -115,8 +121,9 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
     // depend on the warp that computes it.
     const auto first_item = [split](long long u) { return u <= split ? u : split + (u - split) * kStrips; };
     const long long q0 = first_item(col_offset(s.nb, c0)), q1 = first_item(col_offset(s.nb, c1));
-    int* counter = s.tile_counter ? s.tile_counter + phase : nullptr;
-    for (long long q = q0 + (long long)blockIdx.x * (blockDim.x >> 5) + wib; q < q1;) {
+    int* counter = s.tile_counter && PE != kPeApart ? s.tile_counter + phase : nullptr;
+    const int block = potentials ? blockIdx.x - force_blocks : blockIdx.x;
+    for (long long q = q0 + (long long)block * (blockDim.x >> 5) + wib; q < q1;) {
         const bool whole = q < split;
         const long long u = whole ? q : split + (q - split) / kStrips;
         const int strip = whole ? 0 : (int)((q - split) % kStrips);
@@ -128,12 +135,16 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
         const int a_end = min(kBlock, s.n - X * kBlock);
         const int a0 = whole ? 0 : strip * kStripRows, a1 = whole ? a_end : min(a_end, a0 + kStripRows);
         double pe = 0;
-        uint32_t rowbits, colbits;
-        tile_pairs<WRITE>(s, ws, X, Y, lane, a0, a1, B, B < s.n, pe, rowbits, colbits);
-        store_contacts(s, X, Y, lane, whole ? -1 : strip, rowbits, colbits);
-        if (WRITE) {
+        if (potentials) {
+            pe = strip_potentials(s, ws, X, Y, lane, a0, a1);
+        } else {
+            uint32_t rowbits, colbits;
+            tile_pairs<PE>(s, ws, X, Y, lane, a0, a1, B, B < s.n, pe, rowbits, colbits);
+            store_contacts(s, X, Y, lane, whole ? -1 : strip, rowbits, colbits);
+        }
+        if (PE != kNoPe) {
             for (int off = 16; off > 0; off >>= 1) pe += __shfl_xor_sync(0xffffffffu, pe, off);
-            if (lane == 0) s.pe_tile[q] = pe;
+            if (lane == 0) s.pe_tile[potentials ? s.nitems / 2 + q : q] = pe;
         }
         __syncwarp();
         if (counter) {
@@ -406,7 +417,7 @@ static void launch_rowsum(const System& s, cudaStream_t st, const CUtensorMap* m
         rowsum_kernel<<<(3 * s.n + kRowThreads - 1) / kRowThreads, kRowThreads, 0, st>>>(s, b0, b1, first, last);
 }
 
-static void launch_pair_columns(const System& s, bool write, int num_sms, cudaStream_t st, int c0, int c1, int phase,
+static void launch_pair_columns(const System& s, PeMode pe, int num_sms, cudaStream_t st, int c0, int c1, int phase,
                                 long long split, bool pdl)
 {
     const auto offset = [&](int c) { return (long long)c * s.nb - (long long)c * (c - 1) / 2; };
@@ -418,9 +429,10 @@ static void launch_pair_columns(const System& s, bool write, int num_sms, cudaSt
     // so are the row sums placed beside the pair tiles (N=1000: 82 -> 124 us,
     // N=5000: 674 -> 836): both are launched plainly.
     const int warps = items <= 4LL * num_sms ? 1 : 4;
-    const int pb = (int)min((items + warps - 1) / warps, (long long)num_sms * 4);
-    launch_pdl(pdl && warps == 1, write ? pair_tile_kernel<true> : pair_tile_kernel<false>, pb, 32 * warps, 0, st, s, c0, c1, phase,
-               split);
+    const int pb = pe == kPeApart ? (int)(2 * items) : (int)min((items + warps - 1) / warps, (long long)num_sms * 4);
+    const auto kernel = pe == kPeApart ? pair_tile_kernel<kPeApart>
+                        : pe == kPeInline ? pair_tile_kernel<kPeInline> : pair_tile_kernel<kNoPe>;
+    launch_pdl(pdl && pb * warps <= 4LL * num_sms, kernel, pb, 32 * warps, 0, st, s, c0, c1, phase, split);
 }
 
 void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, StepTimers* tm, const StepOverlap* ov,
@@ -431,17 +443,19 @@ void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, St
     const int np = ov ? phase_bounds(s.nb, cb) : 1;
     const long long split = strip_from(s.ntiles, num_sms);  // the same items, and energy sums, with and without phases
     s.nitems = split + kStrips * (s.ntiles - split);
+    const PeMode pe = !write ? kNoPe : pe_apart(s.ntiles, num_sms) ? kPeApart : kPeInline;
+    if (pe == kPeApart) s.nitems *= 2;
     // phases wait on events between the kernels: plain launches there
     const bool pdl = np <= 1;
     launch_drift(s, st, pdl);
     if (tm) cudaEventRecord(tm->ev[0], st);
     if (np <= 1) {
-        launch_pair_columns(s, write, num_sms, st, 0, s.nb, 0, split, pdl);
+        launch_pair_columns(s, pe, num_sms, st, 0, s.nb, 0, split, pdl);
         if (tm) cudaEventRecord(tm->ev[1], st);
         launch_rowsum(s, st, map, 0, s.nb, 1, 1, num_sms, int_adds);
     } else {
         for (int p = 0; p < np; ++p) {
-            launch_pair_columns(s, write, num_sms, st, cb[p], cb[p + 1], p, split, pdl);
+            launch_pair_columns(s, pe, num_sms, st, cb[p], cb[p + 1], p, split, pdl);
             cudaEventRecord(ov->phase[p], st);
             cudaStreamWaitEvent(ov->side, ov->phase[p], 0);
             launch_rowsum(s, ov->side, map, cb[p], cb[p + 1], p == 0, p == np - 1, num_sms, int_adds);

@@ -51,10 +51,15 @@ struct TileScratch {
 };
 static_assert(sizeof(double) * kBStageDoubles >= kBlock * kBlock * sizeof(uint16_t), "list fits in the staging");
 
+// Where a tile's potentials (write steps) are added up: nowhere; with the
+// forces; or the contacts' with the forces and the others' in work items of
+// their own (strip_potentials).
+enum PeMode { kNoPe = 0, kPeInline = 1, kPeApart = 2 };
+
 // One pair by the general path: rounds every quotient and root by its exact
 // remainder (sl_fp64_exact.cuh), with the hardware operations behind it, for
 // any operands; contact or not.
-template <bool WRITE>
+template <int PE>
 __device__ __forceinline__ bool general_pair(const System& s, const ABlock& ab, int X, int a, int B, double& pe)
 {
     const size_t plane = (size_t)s.npad * s.npad;
@@ -76,7 +81,7 @@ __device__ __forceinline__ bool general_pair(const System& s, const ABlock& ab, 
     double fx, fy, fz;
     if (contact) {
         const ContactIn in = gather_contact(s, A, B);
-        const ContactOut o = contact_pair_exact<WRITE>(in, s.mat, rx, ry, rz, dist, overlap, Ra, Rb, ab.twoR[a],
+        const ContactOut o = contact_pair_exact<PE != kNoPe>(in, s.mat, rx, ry, rz, dist, overlap, Ra, Rb, ab.twoR[a],
                                                        twoRb, ab.fourR[a], ab.cR3[a]);
         fx = o.fx; fy = o.fy; fz = o.fz;
         const double im_a = s.inv_moi[A], mo_a = s.moi[A];
@@ -89,7 +94,7 @@ __device__ __forceinline__ bool general_pair(const System& s, const ABlock& ab, 
         tb[0] = div_by_recip(o.tbx, mo_b, im_b);
         tb[plane] = div_by_recip(o.tby, mo_b, im_b);
         tb[2 * plane] = div_by_recip(o.tbz, mo_b, im_b);
-        if (WRITE) pe += o.pe;
+        if (PE != kNoPe) pe += o.pe;
     } else {
         long long hb = ob & 0x7fffffffffffffffll;                  // :211-215 |overlap|
         const long long h_min_bits = __double_as_longlong(s.mat.h_min);
@@ -99,7 +104,7 @@ __device__ __forceinline__ bool general_pair(const System& s, const ABlock& ab, 
         fx = coef * div_by_rsqrt(rx, dist, Yr, p);                    // :221-227
         fy = coef * div_by_rsqrt(ry, dist, Yr, p);
         fz = coef * div_by_rsqrt(rz, dist, Yr, p);
-        if (WRITE) pe += vdw_energy_far_df(s.mat.Ha, h, Ra, Rb, ab.twoR[a]);          // :239
+        if (PE == kPeInline) pe += vdw_energy_far_df(s.mat.Ha, h, Ra, Rb, ab.twoR[a]);  // :239
     }
     // :249-250 -- acc[A] += F/m[A]; acc[B] -= F/m[B] (stored negated)
     const double ma = ab.m[a];
@@ -138,7 +143,7 @@ __device__ __forceinline__ int pack_list(TileScratch& ws, uint32_t marked)
 
 // The marked pairs of a tile, packed and evaluated one per lane; ws.rowc and
 // ws.colc get the contacts.  Out of line: the sweep's registers are dead here.
-template <bool WRITE>
+template <int PE>
 __device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, int X, int Y, uint32_t marked)
 {
     const int lane = threadIdx.x & 31;
@@ -149,7 +154,7 @@ __device__ __noinline__ double general_pairs(const System& s, TileScratch& ws, i
     const int total = pack_list(ws, marked);
     for (int e = lane; e < total; e += 32) {
         const int a = list[e] >> 5, b = list[e] & 31;
-        if (general_pair<WRITE>(s, ws.ab, X, a, Y * kBlock + b, pe)) {
+        if (general_pair<PE>(s, ws.ab, X, a, Y * kBlock + b, pe)) {
             atomicOr(&ws.rowc[a], 1u << b);
             atomicOr(&ws.colc[b], 1u << a);
         }
@@ -181,6 +186,33 @@ static __device__ __noinline__ double near_potentials(const System& s, TileScrat
     return pe;
 }
 
+// The potentials of the pairs out of contact in rows a0 .. a1 - 1 of a tile,
+// ws.ab loaded (kPeApart).
+__device__ __forceinline__ double strip_potentials(const System& s, TileScratch& ws, int X, int Y, int lane, int a0,
+                                                   int a1)
+{
+    const ABlock& ab = ws.ab;
+    const int B = Y * kBlock + lane;
+    const double bx = s.pos.c[0][B], by = s.pos.c[1][B], bz = s.pos.c[2][B], Rb = s.R[B];
+    double pe = 0;
+    uint32_t near = 0;
+#pragma unroll 2
+    for (int a = a0; a < a1; ++a) {
+        const double Ra = ab.R[a];
+        const double rx = bx - ab.x[a], ry = by - ab.y[a], rz = bz - ab.z[a];
+        const double overlap = (Ra + Rb) - sqrt(rx * rx + ry * ry + rz * rz);
+        if (B < s.n && (X != Y || lane < a) && !(overlap > 0)) {
+            double h = fabs(overlap);
+            if (h < s.mat.h_min) h = s.mat.h_min;
+            const VdwArg v = vdw_arg(h, Ra, Rb, ab.twoR[a]);
+            if (v.far()) pe += vdw_energy_series(s.mat.Ha, v);
+            else near |= 1u << a;
+        }
+    }
+    if (__any_sync(0xffffffffu, near != 0u)) pe += near_potentials(s, ws, X, Y, near);
+    return pe;
+}
+
 // The tile (X, Y) for lane = sphere B = 32Y + lane, partners A = 32X + a for
 // a in [a0, a1) (a0 a multiple of 4): terms to pairbuf and torqbuf, contact
 // bits to rowbits (row A = 32X + lane) and colbits (row B), PE (write steps)
@@ -198,7 +230,7 @@ static __device__ __noinline__ double near_potentials(const System& s, TileScrat
 // The radius products are formed once, and sphere B's term is the negation
 // of sphere A's (RN(-x) = -RN(x)).  Every remaining operation is the general
 // form's, in its order.
-template <bool WRITE, bool UNI>
+template <int PE, bool UNI>
 __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                             double bx, double by, double bz, const pf::Sphere& sb,
                                             const pf::Uniform& un, bool bvalid, double& pe, uint32_t& marked,
@@ -229,7 +261,7 @@ __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, in
         // general path writes these entries after the sweep
         const bool mark = valid && (__double_as_longlong(pr.overlap) > 0 || !pr.fl.sure());
         if (mark) marked |= 1u << a;
-        if (WRITE) {
+        if (PE == kPeInline) {
             if (valid && !mark) {  // :239
                 const VdwArg v = vdw_arg(pr.h, sa.R, sb.R, 2 * sa.R);
                 if (v.far()) pe += vdw_energy_series(s.mat.Ha, v);
@@ -283,7 +315,7 @@ __device__ __forceinline__ void load_a(const System& s, ABlock& ab, int lane, in
 // Partners a0 .. a1 - 1 of the tile (X, Y), the A block loaded: the sweep, or
 // where a constant leaves the integer path's range (no cohesion: cR3 = 0;
 // masses far from 1) the general path for every pair, then the marked pairs.
-template <bool WRITE>
+template <int PE>
 __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                            int iB, bool bvalid, double& pe, uint32_t& rowbits, uint32_t& colbits)
 {
@@ -306,15 +338,15 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
         marked = bvalid ? (X != Y ? all : all & ~((2u << lane) - 1u)) : 0u;
     } else if (uni) {
         const pf::Uniform un{R0 + R0, ab.fourR[0] * R0, pf::unpack(ab.cR3[0] * R0 * R0 * R0)};
-        sweep_pairs<WRITE, true>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
+        sweep_pairs<PE, true>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     } else {
         const pf::Uniform un{0.0, 0.0, {0, 0}};
-        sweep_pairs<WRITE, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
+        sweep_pairs<PE, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     }
-    if (WRITE && __any_sync(0xffffffffu, near != 0u)) pe += near_potentials(s, ws, X, Y, near);
+    if (PE == kPeInline && __any_sync(0xffffffffu, near != 0u)) pe += near_potentials(s, ws, X, Y, near);
     rowbits = colbits = 0;
     if (__any_sync(0xffffffffu, marked != 0u)) {
-        pe += general_pairs<WRITE>(s, ws, X, Y, marked);
+        pe += general_pairs<PE>(s, ws, X, Y, marked);
         rowbits = ws.rowc[lane];
         colbits = ws.colc[lane];
         __syncwarp();

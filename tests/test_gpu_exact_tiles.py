@@ -102,3 +102,28 @@ def test_strips_bit_identical(n):
         st = o.state()
         for key in ("pos", "vel", "w", "acc", "aacc"):
             assert np.array_equal(getattr(sim.group, key), st[key]), key
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("n", [2, 33, 512, 513])
+def test_write_step_potentials_apart_and_inline(n, overlap):
+    """A write step's potentials in work items of their own (up to N=512 on
+    152 SMs) and beside the forces (N=513), spheres 2.3 radii apart, so
+    that PE is the near pairs' closed form and the far pairs' series alone.
+    The closed form's own rounding, eps / w^2 of a far pair's w^3, is below
+    1e-12 of the sum."""
+    from cases import material
+    from oracle.oracle import CpuOracle
+    from spacelab_gb300 import BallGroup, GpuStep
+    c = contact_case(n, 10, spacing=2.3)
+    o = CpuOracle(c["pos"], c["vel"], c["w"], c["R"], c["m"], c["moi"], OracleMaterial(), c["dt"], c["kin"], c["kout"])
+    g = BallGroup.from_arrays(c["pos"], c["vel"], c["w"], c["R"], c["m"], c["moi"])
+    with GpuStep(g, material(), "exact") as sim:
+        sim.set_overlap(overlap)
+        sim.set_scalars(c["dt"], c["kin"], c["kout"])
+        sim.init_conditions()
+        o.init()
+        for _ in range(2):
+            e, eo = sim.sim_one_step(True), o.step(True)
+            assert abs(e.PE - eo[0]) <= 1e-10 * abs(eo[0])
