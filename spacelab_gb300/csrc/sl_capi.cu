@@ -72,8 +72,9 @@ struct sl_handle {
     size_t arena_bytes = 0;
     double* staging = nullptr;  // pinned, 18 * npad doubles (per-sphere scalars at upload)
     double* d_stage = nullptr;  // device, 6 x 3 npad doubles: AoS copies of the vec3 arrays
-    double* h_energy = nullptr; // pinned, 8 doubles
-    unsigned int* h_status = nullptr;
+    double* h_energy = nullptr; // pinned, 8 doubles, written by the energy kernel
+    unsigned int* h_status = nullptr;  // pinned
+    bool status_clear = true;  // the device's status word is 0, and nothing enqueued since can have changed it
     bool uploaded = false;
     bool forces_ready = false;
     // the GPU reads and writes pageable host memory directly (cudaDevAttr-
@@ -113,6 +114,7 @@ void launch_mode_step(sl_handle* h, bool write, sl::StepTimers* tm)
 int enqueue_step(sl_handle* h, bool write)
 {
     sl::StepTimers* tm = nullptr;
+    h->status_clear = false;
     if (h->timing) {
         if (h->timers_used >= (int)h->timers.size()) {
             sl::StepTimers t;
@@ -127,12 +129,15 @@ int enqueue_step(sl_handle* h, bool write)
     return SL_OK;
 }
 
-int fetch_energy_and_status(sl_handle* h, sl_energy* out, bool want_energy)
+// Waits for the stream.  The energies of a write step are in h_energy, which
+// the energy kernel writes itself, and with them the status word; reported:
+// a stage_out kernel wrote it.  Otherwise it is copied.
+int fetch_energy_and_status(sl_handle* h, sl_energy* out, bool want_energy, bool reported = false)
 {
-    if (want_energy)
-        SL_CUDA(cudaMemcpyAsync(h->h_energy, h->sys.energy, 8 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    SL_CUDA(cudaMemcpyAsync(h->h_status, h->sys.status, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream));
+    if (!want_energy && !reported)
+        SL_CUDA(cudaMemcpyAsync(h->h_status, h->sys.status, sizeof(unsigned int), cudaMemcpyDeviceToHost, h->stream));
     SL_CUDA(cudaStreamSynchronize(h->stream));
+    h->status_clear = *h->h_status == 0;
     if (want_energy && out) {
         out->PE = h->h_energy[0];
         out->KE = h->h_energy[1];
@@ -263,7 +268,6 @@ int sl_create(int n, const sl_material* mat, int mode, sl_handle** out)
     const size_t o_pe = take((size_t)(mode == SL_MODE_EXACT ? sl::exact_pe_slots(s.ntiles, h->num_sms) : s.nitems) *
                              sizeof(double));
     const size_t o_red = take(sl::kRedBlocks * 8 * sizeof(double));
-    const size_t o_en = take(8 * sizeof(double));
     const size_t o_st = take(sizeof(unsigned int));
     const size_t o_tc = take(sl::kPairPhases * sizeof(int));  // the pair kernels' work queues
     const size_t o_cf = take(mixed ? np * sizeof(int) : 0);
@@ -298,7 +302,6 @@ int sl_create(int n, const sl_material* mat, int mode, sl_handle** out)
     s.cmask = reinterpret_cast<uint32_t*>(base + o_mask);
     s.pe_tile = reinterpret_cast<double*>(base + o_pe);
     s.red = reinterpret_cast<double*>(base + o_red);
-    s.energy = reinterpret_cast<double*>(base + o_en);
     s.status = reinterpret_cast<unsigned int*>(base + o_st);
     s.tile_counter = reinterpret_cast<int*>(base + o_tc);
     if (mixed) s.contact_flag = reinterpret_cast<int*>(base + o_cf);
@@ -311,6 +314,8 @@ int sl_create(int n, const sl_material* mat, int mode, sl_handle** out)
     e = cudaMallocHost(&h->staging, 18 * np * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_energy, 8 * sizeof(double));
     if (e == cudaSuccess) e = cudaMallocHost(&h->h_status, sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&s.energy, h->h_energy, 0);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&s.host_status, h->h_status, 0);
     if (e != cudaSuccess) { sl_destroy(h); return fail(SL_ERR_ALLOC, "pinned host allocation failed"); }
     e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) { sl_destroy(h); return cuda_fail(e, "cudaStreamSynchronize"); }
@@ -403,7 +408,8 @@ int enqueue_resume(sl_handle* h, const double* pos, const double* vel, const dou
     if (!device_check &&
         (!all_finite(pos, 3 * (size_t)n) || !all_finite(vel, 3 * (size_t)n) || !all_finite(w, 3 * (size_t)n)))
         return fail(SL_ERR_ARG, "non-finite position, velocity or spin in input");
-    SL_CUDA(cudaMemsetAsync(h->sys.status, 0, sizeof(unsigned int), h->stream));
+    if (!h->status_clear) SL_CUDA(cudaMemsetAsync(h->sys.status, 0, sizeof(unsigned int), h->stream));
+    if (device_check) h->status_clear = false;
     const size_t np = h->sys.npad;
     // the staging kernel reads each array where the GPU can reach it, else
     // from a copy in the device staging area; absent acc/aacc are zero, an
@@ -435,7 +441,7 @@ int enqueue_resume(sl_handle* h, const double* pos, const double* vel, const dou
 // reaches every array, so that nothing goes through a copy): nothing is
 // written once the staging kernel found a non-finite input.
 int enqueue_download(sl_handle* h, double* pos, double* vel, double* w, double* acc, double* aacc,
-                     bool guard = false)
+                     bool guard = false, bool report = false)
 {
     double* outs[5] = {pos, vel, w, acc, aacc};
     const size_t np = h->sys.npad;
@@ -455,7 +461,7 @@ int enqueue_download(sl_handle* h, double* pos, double* vel, double* w, double* 
                 staged[k] = true;
             }
         }
-    sl::launch_stage_out(h->sys, views, src, want, h->stream, guard);
+    sl::launch_stage_out(h->sys, views, src, want, h->stream, guard, report, report && !h->overlap);
     SL_CUDA(cudaGetLastError());
     for (int k = 0; k < 5; ++k)
         if (staged[k])
@@ -540,6 +546,7 @@ int sl_run(sl_handle* h, int first_step, int last_step, int skip, sl_energy* row
                 if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
                 h->interval_skip = skip;
             }
+            h->status_clear = false;
             SL_CUDA(cudaGraphLaunch(h->interval_exec, h->stream));
             step += skip;
             const int r = fetch_energy_and_status(h, written < max_rows && rows ? &rows[written] : nullptr, true);
@@ -588,8 +595,8 @@ int sl_step_host(sl_handle* h, double* pos, double* vel, double* w, double* acc,
     if (int r = enqueue_resume(h, pos, vel, w, acc, aacc, nullptr, reach)) return r;
     h->forces_ready = true;
     if (int r = enqueue_step(h, write != 0)) return r;
-    if (int r = enqueue_download(h, pos, vel, w, acc, aacc, reach)) return r;
-    const int r = fetch_energy_and_status(h, out, write != 0);
+    if (int r = enqueue_download(h, pos, vel, w, acc, aacc, reach, true)) return r;
+    const int r = fetch_energy_and_status(h, out, write != 0, true);
     if (r == SL_ERR_ARG) h->forces_ready = false;  // the device copy holds the rejected input
     return r;
 }
@@ -655,7 +662,7 @@ int sl_step_launches(const sl_handle* h, int write, int* count)
         int cb[sl::kPairPhases + 1];
         np = sl::phase_bounds(h->sys.nb, cb);
     }
-    *count = 1 + 2 * np + (write ? 2 : 0);  // drift, pair + row-sum per phase, energy
+    *count = 1 + 2 * np + (write ? sl::energy_launches(h->sys.n) : 0);  // drift, pair + row-sum per phase, energy
     return SL_OK;
 }
 

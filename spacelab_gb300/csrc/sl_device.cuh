@@ -60,6 +60,7 @@ struct System {
     double* red;          // [kRedBlocks][8] energy partials
     double* energy;       // [8] PE, KE, mom xyz, L xyz
     unsigned int* status; // error bits (see SL_ERR_* in spacelab_gpu.h)
+    unsigned int* host_status;  // where a step's last kernel copies them for the host, or NULL
     const Scalars* sc;
     Material mat;
     // mixed-precision form: per-sphere FP32 constants in lengths scaled by

@@ -48,11 +48,12 @@ void launch_derive(const System& s, cudaStream_t st);
 // the previous positions, takes the positions; the rest zero); out, for the
 // arrays whose bit is set in `want`.  check: arrays of `present` whose
 // non-finite values set kStatusInputNonFiniteBit; guard: stage_out writes
-// nothing once that bit is set.
+// nothing once that bit is set; report: stage_out copies the status word to
+// s.host_status; pdl: as a dependent of the stream's last kernel.
 void launch_stage_in(const System& s, const double* const src[6], Vec3Soa* const arr[6], unsigned present,
                      cudaStream_t st, unsigned check = 0);
 void launch_stage_out(const System& s, double* const dst[6], Vec3Soa* const arr[6], unsigned want, cudaStream_t st,
-                      bool guard = false);
+                      bool guard = false, bool report = false, bool pdl = false);
 // map: a tensor map of the pair-term buffer (make_pair_map) selects the
 // TMA-streamed row sums; NULL the plain-load form.
 void launch_step(const System& s, bool write, int num_sms, cudaStream_t st, StepTimers* tm,
@@ -81,6 +82,10 @@ void launch_step_mixed64(const System& s, bool write, int num_sms, cudaStream_t 
 // Whether the mixed pair kernel takes two column blocks per item (mixed_pair_items)
 // for nb row blocks on num_sms SMs: where each warp takes many items.
 bool mixed_pair_double(int nb, int num_sms);
+// Kernels of a write step's energy sums: one block where each of its threads
+// has a sphere at most (write steps, with the host's wait and its copies gone too:
+// N=33 61.7 -> 52.5 us, N=201 80 -> 68.3), else blocks of partial sums and their total.
+inline int energy_launches(int n) { return n <= 256 ? 1 : 2; }
 // pdl: as dependents of the stream's last kernel (launch_pdl)
 void launch_drift(const System& s, cudaStream_t st, bool pdl = true);
 void launch_energy(const System& s, cudaStream_t st, bool pdl = true);

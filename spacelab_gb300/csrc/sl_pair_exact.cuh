@@ -44,6 +44,17 @@ __device__ __forceinline__ double vdw_energy(double Ha, double h, double Ra, dou
     return -Ha / 6 * (two_RaRb / denom_sum + two_RaRb / denom_diff + log(denom_sum / denom_diff));
 }
 
+// The constants of sphere i derived from its radius, mass and moment of
+// inertia (exact scalings and correctly rounded reciprocals).
+__device__ __forceinline__ void derive_sphere(const System& s, int i, double R, double m, double moi)
+{
+    s.twoR[i] = 2 * R;
+    s.fourR[i] = 4 * R;
+    s.cR3[i] = s.mat.Ha / 6 * 64 * R * R * R;
+    s.rm[i] = recip_of(m);
+    s.inv_moi[i] = 1.0 / moi;
+}
+
 struct ContactOut {
     double fx, fy, fz;      // totalForceOnA
     double tax, tay, taz;   // torqueA

@@ -11,6 +11,7 @@
 #include "../../include/spacelab_gpu.h"
 #include "sl_device.cuh"
 #include "sl_kernels.h"
+#include "sl_pair_exact.cuh"
 
 #include <cuda.h>  // CUcontext, for the driver entry points below
 
@@ -40,7 +41,8 @@ constexpr size_t kOffMask = kOffTorq + up32(3ull * kNp * kNp);
 constexpr size_t kOffPe = kOffMask + up32((size_t)kNp * kNb / 2 + 1);
 constexpr size_t kOffRed = kOffPe + up32(2 * sl::kTileItems * kTiles);  // exact_pe_slots, any device
 constexpr size_t kOffEnergy = kOffRed + up32(sl::kRedBlocks * 8);
-constexpr size_t kOffStatus = kOffEnergy + 32;
+constexpr size_t kOffStatus = kOffEnergy + 32;  // 1 + kNb words of 4 bytes
+static_assert(1 + kNb <= 64, "status words fit");
 constexpr size_t kOffScalars = kOffStatus + 32;
 constexpr size_t kScratchDoubles = kOffScalars + 32;
 
@@ -52,9 +54,14 @@ constexpr int kMaxDevices = 64;
 // A real sphere's R, m or moi is not finite and > 0 (set by the load kernel).
 constexpr unsigned kStatusBadInputBit = 0x80000000u;
 
+// What the host keeps of the working memory on one device: its address, and a
+// tensor map of the pair-term buffer for each number of 32-sphere blocks.
 struct DeviceSlot {
     double* scratch = nullptr;
     int num_sms = 0;
+    bool host_direct = false;  // the GPU writes pageable host memory (cudaDevAttrPageableMemoryAccess)
+    CUtensorMap map[kNb];
+    bool has_map[kNb];
     unsigned long long ctx_id = 0;  // context the address belongs to (0 = none yet)
 };
 std::mutex g_mutex;
@@ -90,40 +97,6 @@ unsigned long long current_context_id()
     return id;
 }
 
-// Device address of g_static_scratch in the current device's current
-// context.  It is looked up (cudaGetSymbolAddress) once per device and
-// looked up again whenever the current context is not the one the cached
-// address came from: after cudaDeviceReset the primary context and its copy
-// of the array are rebuilt, and a driver-API context of its own holds
-// another copy.  Host code may not use the symbol itself as a pointer: on
-// the host it names a stand-in object, not device memory.
-int scratch_for_current_device(double** base, int* num_sms)
-{
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
-    if (dev < 0 || dev >= kMaxDevices) return sl_record_error(SL_ERR_UNSUPPORTED, "device index out of range");
-    std::lock_guard<std::mutex> lock(g_mutex);
-    DeviceSlot& slot = g_slots[dev];
-    const unsigned long long ctx = current_context_id();
-    if (!slot.scratch || ctx == 0 || ctx != slot.ctx_id) {
-        void* p = nullptr;
-        e = cudaGetSymbolAddress(&p, g_static_scratch);
-        if (e != cudaSuccess || !p)
-            return sl_record_error(SL_ERR_CUDA, (std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e)).c_str());
-        int sms = 0;
-        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
-        slot.scratch = static_cast<double*>(p);
-        slot.num_sms = sms;
-        // the lookup made the runtime's context current if none was
-        slot.ctx_id = ctx ? ctx : current_context_id();
-    }
-    *base = slot.scratch;
-    *num_sms = slot.num_sms;
-    return SL_OK;
-}
-
 sl::System static_system(double* base, int n, const sl_material& mat)
 {
     sl::System s{};
@@ -152,54 +125,123 @@ sl::System static_system(double* base, int n, const sl_material& mat)
     return s;
 }
 
-// Caller's vec3[n] device arrays -> the scratch's SoA rows; R/m/moi with
-// padding 1; acc/aacc cleared (the scratch keeps the previous call's
-// contents; the error word is cleared before this kernel runs); scalars
-// dt = 0 (a force pass), kin, kout.
-// A real sphere whose R, m or moi is not finite and > 0 sets
-// kStatusBadInputBit, as sl_upload rejects such values on the handle path.
-__global__ void static_load_kernel(const __grid_constant__ sl::System s, const double* pos, const double* vel,
-                                   const double* w, const double* R, const double* m, const double* moi,
-                                   double kin, double kout)
+// A DeviceSlot's contents for a system of nb blocks.
+struct DeviceView {
+    double* scratch;
+    int num_sms;
+    bool host_direct, has_map;
+    CUtensorMap map;
+};
+
+// Device address of g_static_scratch in the current device's current
+// context.  It is looked up (cudaGetSymbolAddress) once per device and
+// looked up again whenever the current context is not the one the cached
+// address came from: after cudaDeviceReset the primary context and its copy
+// of the array are rebuilt, and a driver-API context of its own holds
+// another copy.  Host code may not use the symbol itself as a pointer: on
+// the host it names a stand-in object, not device memory.
+int slot_for_current_device(int nb, DeviceView* view)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
+    if (dev < 0 || dev >= kMaxDevices) return sl_record_error(SL_ERR_UNSUPPORTED, "device index out of range");
+    std::lock_guard<std::mutex> lock(g_mutex);
+    DeviceSlot& slot = g_slots[dev];
+    const unsigned long long ctx = current_context_id();
+    if (!slot.scratch || ctx == 0 || ctx != slot.ctx_id) {
+        void* p = nullptr;
+        e = cudaGetSymbolAddress(&p, g_static_scratch);
+        if (e != cudaSuccess || !p)
+            return sl_record_error(SL_ERR_CUDA, (std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e)).c_str());
+        int sms = 0;
+        e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
+        int pageable = 0;
+        e = cudaDeviceGetAttribute(&pageable, cudaDevAttrPageableMemoryAccess, dev);
+        if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
+        slot.scratch = static_cast<double*>(p);
+        slot.num_sms = sms;
+        slot.host_direct = pageable != 0;
+        for (int k = 0; k < kNb; ++k) {
+            const sl::System s = static_system(slot.scratch, sl::kBlock * (k + 1), sl_material{});
+            slot.has_map[k] = sl::make_pair_map(s, &slot.map[k]);
+            if (!slot.has_map[k]) cudaGetLastError();  // the plain row sums are used then
+        }
+        // the lookup made the runtime's context current if none was
+        slot.ctx_id = ctx ? ctx : current_context_id();
+    }
+    view->scratch = slot.scratch;
+    view->num_sms = slot.num_sms;
+    view->host_direct = slot.host_direct;
+    view->has_map = slot.has_map[nb - 1];
+    view->map = slot.map[nb - 1];
+    return SL_OK;
+}
+
+// Caller's vec3[n] device arrays -> the scratch's SoA rows and the constants
+// derived from them; R/m/moi with padding 1; acc/aacc, the status word, and
+// the pair-term entries that no pair writes but the streamed row sums read
+// (each row's own column and its padding columns) cleared, as the scratch
+// keeps the previous call's contents in another call's layout; scalars dt = 0
+// (a force pass), kin, kout.  One warp per block of spheres, on SMs of their
+// own: the reciprocals are ~1000 dependent instructions.
+// A real sphere whose R, m or moi is not finite and > 0 sets
+// kStatusBadInputBit, as sl_upload rejects such values on the handle path, in
+// its block's own word status[1 + block].
+__global__ void __launch_bounds__(sl::kBlock) static_load_kernel(const __grid_constant__ sl::System s,
+                                                                 const double* pos, const double* vel,
+                                                                 const double* w, const double* R, const double* m,
+                                                                 const double* moi, double kin, double kout)
+{
+    sl::pdl_next();
+    const int i = blockIdx.x * sl::kBlock + threadIdx.x;
     if (i == 0) {
         sl::Scalars* sc = const_cast<sl::Scalars*>(s.sc);
         sc->dt = 0.0;
         sc->kin = kin;
         sc->kout = kout;
+        *s.status = 0;
     }
-    if (i >= s.npad) return;
     const bool real = i < s.n;
+    double r = real ? R[i] : 1.0, mi = real ? m[i] : 1.0, mo = real ? moi[i] : 1.0;
     for (int c = 0; c < 3; ++c) {
         s.pos.c[c][i] = real ? pos[3 * (size_t)i + c] : 0.0;
         s.vel.c[c][i] = real ? vel[3 * (size_t)i + c] : 0.0;
         s.w.c[c][i] = real ? w[3 * (size_t)i + c] : 0.0;
         s.acc.c[c][i] = 0.0;
         s.aacc.c[c][i] = 0.0;
+        double* row = s.pairbuf + ((size_t)c * s.npad + i) * s.npad;
+        row[i] = 0.0;
+        for (int j = s.n; j < s.npad; ++j) row[j] = 0.0;
     }
-    double r = real ? R[i] : 1.0, mi = real ? m[i] : 1.0, mo = real ? moi[i] : 1.0;
     // written so that NaN fails too; a rejected sphere is given 1.0 so that
     // the rest of the pass runs on ordinary numbers before the call fails
-    if (!(r > 0.0 && r < INFINITY) || !(mi > 0.0 && mi < INFINITY) || !(mo > 0.0 && mo < INFINITY)) {
-        atomicOr(s.status, kStatusBadInputBit);
-        r = mi = mo = 1.0;
-    }
+    const bool bad = !(r > 0.0 && r < INFINITY) || !(mi > 0.0 && mi < INFINITY) || !(mo > 0.0 && mo < INFINITY);
+    if (bad) r = mi = mo = 1.0;
     s.R[i] = r;
     s.m[i] = mi;
     s.moi[i] = mo;
+    sl::derive_sphere(s, i, r, mi, mo);
+    const bool any_bad = __any_sync(0xffffffffu, bad);
+    if (threadIdx.x == 0) s.status[1 + blockIdx.x] = any_bad ? kStatusBadInputBit : 0u;
 }
 
-__global__ void static_store_kernel(const __grid_constant__ sl::System s, double* acc, double* aacc,
-                                    double* energy)
+// acc and aacc, an element per thread, to the caller's arrays; the status
+// words, joined, to the first and to the host's.
+__global__ void static_store_kernel(const __grid_constant__ sl::System s, double* acc, double* aacc)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (energy && i < 8) energy[i] = s.energy[i];
-    if (i >= s.n) return;
-    for (int c = 0; c < 3; ++c) {
-        acc[3 * (size_t)i + c] = s.acc.c[c][i];
-        aacc[3 * (size_t)i + c] = s.aacc.c[c][i];
+    sl::pdl_wait();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t == 0) {
+        unsigned status = *s.status;
+        for (int b = 0; b < s.nb; ++b) status |= s.status[1 + b];
+        *s.status = status;
+        if (s.host_status) *s.host_status = status;
     }
+    if (t >= 3 * s.n) return;
+    acc[t] = s.acc.c[t % 3][t / 3];
+    aacc[t] = s.aacc.c[t % 3][t / 3];
 }
 
 }  // namespace
@@ -216,23 +258,21 @@ extern "C" int sl_forces_static(int n, const double* pos, const double* vel, con
         return sl_record_error(SL_ERR_ARG, "sl_forces_static: NULL input or output pointer");
     if (!(mat->h_min > 0) || !std::isfinite(kin) || !std::isfinite(kout) || kin < 0 || kout < 0)
         return sl_record_error(SL_ERR_ARG, "sl_forces_static: need h_min > 0 and finite kin, kout >= 0");
-    double* base = nullptr;
-    int num_sms = 0;
-    if (int rc = scratch_for_current_device(&base, &num_sms)) return rc;
+    DeviceView dev;
+    if (int rc = slot_for_current_device((n + sl::kBlock - 1) / sl::kBlock, &dev)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const sl::System s = static_system(base, n, *mat);
-    const int threads = 128;
-    cudaError_t e = cudaMemsetAsync(s.status, 0, sizeof(unsigned int), st);
-    if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
-    static_load_kernel<<<(s.npad + threads - 1) / threads, threads, 0, st>>>(s, pos, vel, w, R, m, moi, kin, kout);
-    sl::launch_derive(s, st);
-    sl::launch_step(s, true, num_sms, st, nullptr);
-    static_store_kernel<<<(s.npad + threads - 1) / threads, threads, 0, st>>>(s, acc, aacc, energy);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
     unsigned int status = 0;
-    e = cudaMemcpyAsync(&status, s.status, sizeof(status), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    sl::System s = static_system(dev.scratch, n, *mat);
+    if (energy) s.energy = energy;
+    static_load_kernel<<<s.nb, sl::kBlock, 0, st>>>(s, pos, vel, w, R, m, moi, kin, kout);
+    sl::launch_step(s, true, dev.num_sms, st, nullptr, nullptr, dev.has_map ? &dev.map : nullptr, false);
+    if (dev.host_direct) s.host_status = &status;
+    sl::launch_pdl(true, static_store_kernel, (3 * n + 127) / 128, 128, 0, st, s, acc, aacc);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess && !dev.host_direct)
+        e = cudaMemcpyAsync(&status, s.status, sizeof(status), cudaMemcpyDeviceToHost, st);
+    const cudaError_t done = cudaStreamSynchronize(st);  // in any case: the store kernel may hold &status
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
     if (status & kStatusBadInputBit)
         return sl_record_error(SL_ERR_ARG, "sl_forces_static: a radius, mass or moment of inertia is not finite and > 0");

@@ -230,6 +230,14 @@ constexpr int kRedThreads = 256;
 // Per-sphere KE, mom, ang_mom terms (:282-285) and the items' PE reduced over a
 // fixed tree: block b sums spheres [b*chunk, (b+1)*chunk) into red[b][0..6] and
 // its share of pe_tile into red[b][7].
+// Thread k < 8 holds total k of the reduction below; with them goes the status
+// word, final by now, so that the host needs no copy to see either.
+__device__ __forceinline__ void put_energy(const System& s, int k, double v)
+{
+    if (k < 8) s.energy[k == 7 ? 0 : k + 1] = v;
+    if (k == 8 && s.host_status) *s.host_status = *s.status;
+}
+
 __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __grid_constant__ System s, int chunk)
 {
     pdl_next();
@@ -260,20 +268,25 @@ __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __gri
         }
         __syncthreads();
     }
-    if (tid < 8) s.red[blockIdx.x * 8 + tid] = sh[tid][0];
+    if (gridDim.x == 1)
+        put_energy(s, tid, tid < 8 ? sh[tid][0] : 0);
+    else if (tid < 8)
+        s.red[blockIdx.x * 8 + tid] = sh[tid][0];
 }
 
-// Final totals over the block partials, in block order.
+// Final totals over the block partials: lane k + 8q adds every fourth one of
+// quantity k.
 __global__ void __launch_bounds__(32) energy_final_kernel(const __grid_constant__ System s, int nred)
 {
     pdl_next();
     pdl_wait();
-    const int k = threadIdx.x;
-    if (k >= 8) return;
+    const int k = threadIdx.x & 7;
     double v = 0;
 #pragma unroll 8
-    for (int b = 0; b < nred; ++b) v += s.red[b * 8 + k];
-    s.energy[k == 7 ? 0 : k + 1] = v;
+    for (int b = threadIdx.x >> 3; b < nred; b += 4) v += s.red[b * 8 + k];
+    v += __shfl_xor_sync(0xffffffffu, v, 8);
+    v += __shfl_xor_sync(0xffffffffu, v, 16);
+    put_energy(s, threadIdx.x, v);
 }
 
 // Per-sphere derived constants (exact scalings and correctly rounded
@@ -283,11 +296,7 @@ __global__ void derive_kernel(const __grid_constant__ System s)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.npad) return;
     const double R = s.R[i], m = s.m[i], moi = s.moi[i];
-    s.twoR[i] = 2 * R;
-    s.fourR[i] = 4 * R;
-    s.cR3[i] = s.mat.Ha / 6 * 64 * R * R * R;
-    s.rm[i] = recip_of(m);
-    s.inv_moi[i] = 1.0 / moi;
+    derive_sphere(s, i, R, m, moi);
     if (s.f_R) {  // mixed-precision form: FP32 constants, lengths scaled by 2^-len_shift
         const float rh = d2f_bits(R, s.len_shift);
         s.f_R[i] = rh;
@@ -315,6 +324,7 @@ struct StagePtrs {
 __global__ void stage_in_kernel(const __grid_constant__ System s, const __grid_constant__ StagePtrs src,
                                 const __grid_constant__ StageArrays arr, unsigned present, unsigned check)
 {
+    pdl_next();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= 3 * s.npad) return;
     const int i = t / 3, c = t - 3 * (t / 3);
@@ -332,9 +342,11 @@ __global__ void stage_in_kernel(const __grid_constant__ System s, const __grid_c
 }
 
 __global__ void stage_out_kernel(const __grid_constant__ System s, const __grid_constant__ StagePtrs dst,
-                                 const __grid_constant__ StageArrays arr, unsigned want, bool guard)
+                                 const __grid_constant__ StageArrays arr, unsigned want, bool guard, bool report)
 {
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (report && t == 0) *s.host_status = *s.status;
     if (t >= 3 * s.n) return;
     if (guard && (*s.status & kStatusInputNonFiniteBit)) return;  // the caller's arrays stay as they were
     const int i = t / 3, c = t - 3 * (t / 3);
@@ -384,7 +396,7 @@ void launch_stage_in(const System& s, const double* const src[6], Vec3Soa* const
 }
 
 void launch_stage_out(const System& s, double* const dst[6], Vec3Soa* const arr[6], unsigned want, cudaStream_t st,
-                      bool guard)
+                      bool guard, bool report, bool pdl)
 {
     StageArrays a;
     StagePtrs p;
@@ -392,7 +404,7 @@ void launch_stage_out(const System& s, double* const dst[6], Vec3Soa* const arr[
         a.a[k] = *arr[k];
         p.p[k] = dst[k];
     }
-    stage_out_kernel<<<(3 * s.n + 255) / 256, 256, 0, st>>>(s, p, a, want, guard);
+    launch_pdl(pdl, stage_out_kernel, (3 * s.n + 255) / 256, 256, 0, st, s, p, a, want, guard, report);
 }
 
 void launch_drift(const System& s, cudaStream_t st, bool pdl)
@@ -402,10 +414,10 @@ void launch_drift(const System& s, cudaStream_t st, bool pdl)
 
 void launch_energy(const System& s, cudaStream_t st, bool pdl)
 {
-    const int nred = kRedBlocks;
+    const int nred = energy_launches(s.n) == 1 ? 1 : kRedBlocks;
     const int chunk = (s.n + nred - 1) / nred;
     launch_pdl(pdl, energy_partial_kernel, nred, kRedThreads, 0, st, s, chunk);
-    launch_pdl(pdl, energy_final_kernel, 1, 32, 0, st, s, nred);
+    if (nred > 1) launch_pdl(pdl, energy_final_kernel, 1, 32, 0, st, s, nred);
 }
 
 static void launch_rowsum(const System& s, cudaStream_t st, const CUtensorMap* map, int b0, int b1, int first,

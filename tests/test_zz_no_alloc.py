@@ -126,3 +126,20 @@ def test_static_force_pass_rejects_sizes_beyond_capacity():
         rc = lib.sl_forces_static(n, *([None] * 6), ctypes.byref(mat), 1.0, 0.5, None, None, None, None)
         assert rc == _lib.SL_ERR_ARG
         assert b"static working memory" in lib.sl_last_error()
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 64, 201, 225, 255])
+def test_static_force_pass_after_other_layouts(n):
+    """The pair-term rows have another length at each block count, so what a
+    call finds in its rows' own and padding columns is an earlier call's
+    terms: a full one's, then non-finite ones (refused)."""
+    torch = pytest.importorskip("torch")
+    _static_call(torch, contact_case(_capacity(), 5555))
+    bad = contact_case(_capacity() - 1, 5556)
+    bad["pos"][:, 0] = float("nan")
+    _static_call(torch, bad, expect=_lib.SL_ERR_NONFINITE)
+    c = contact_case(n, 5557)
+    acc, aacc, e = _static_call(torch, c)
+    racc, raacc, re = _handle_reference(c)
+    assert np.array_equal(acc, racc) and np.array_equal(aacc, raacc)
+    _assert_energy_close(e, re, c)
