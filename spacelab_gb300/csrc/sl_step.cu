@@ -101,11 +101,11 @@ __device__ __forceinline__ void col_tile_coords(int nb, long long u, int& X, int
 // pe_tile[q].  kPeApart: one warp per CTA, and as many CTAs again, whose items
 // are the potentials of the first ones' pairs out of contact, to
 // pe_tile[nitems / 2 + q].
-template <int PE>
-__global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
+template <int PE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, WARPS == 1 ? 8 : 4) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
                                                           int phase, long long split)
 {
-    __shared__ TileScratch scratch[4];
+    __shared__ TileScratch scratch[WARPS];
     pdl_next();
     pdl_wait();
     const int lane = threadIdx.x & 31;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(128, 4) pair_tile_kernel(const __grid_constant
             pe = strip_potentials(s, ws, X, Y, lane, a0, a1);
         } else {
             uint32_t rowbits, colbits;
-            tile_pairs<PE>(s, ws, X, Y, lane, a0, a1, B, B < s.n, pe, rowbits, colbits);
+            tile_pairs<PE, WARPS == 1 ? 2 : 1>(s, ws, X, Y, lane, a0, a1, B, B < s.n, pe, rowbits, colbits);
             store_contacts(s, X, Y, lane, whole ? -1 : strip, rowbits, colbits);
         }
         if (PE != kNoPe) {
@@ -442,8 +442,15 @@ static void launch_pair_columns(const System& s, PeMode pe, int num_sms, cudaStr
     // N=5000: 674 -> 836): both are launched plainly.
     const int warps = items <= 4LL * num_sms ? 1 : 4;
     const int pb = pe == kPeApart ? (int)(2 * items) : (int)min((items + warps - 1) / warps, (long long)num_sms * 4);
-    const auto kernel = pe == kPeApart ? pair_tile_kernel<kPeApart>
-                        : pe == kPeInline ? pair_tile_kernel<kPeInline> : pair_tile_kernel<kNoPe>;
+    // One-warp CTAs may use 216 registers, and take two rows at a time (us per
+    // step, one against two: N=32 25.0 -> 23.3, N=96 32.7 -> 30.8, N=400 50.8 ->
+    // 48.9; four rows the same).  A few rows are over before the longer code
+    // is in the instruction cache: N=2 11.3, two rows 13.1, N=4 14.7, 15.1.
+    const bool two_rows = warps == 1 && s.n >= kStripRows;
+    const auto kernel = pe == kPeApart    ? pair_tile_kernel<kPeApart, 1>
+                        : pe == kPeInline ? pair_tile_kernel<kPeInline, 4>
+                        : two_rows        ? pair_tile_kernel<kNoPe, 1>
+                                          : pair_tile_kernel<kNoPe, 4>;
     launch_pdl(pdl && pb * warps <= 4LL * num_sms, kernel, pb, 32 * warps, 0, st, s, c0, c1, phase, split);
 }
 

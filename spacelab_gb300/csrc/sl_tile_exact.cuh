@@ -42,6 +42,9 @@ constexpr int kBStageRow = 5;
 constexpr int kBStagePlane = kBlock * kBStageRow;
 constexpr int kBStageDoubles = 3 * kBStagePlane;
 
+// A tile may be taken in strips of 8 of its 32 rows.
+constexpr int kStripRows = 8, kStrips = kBlock / kStripRows;
+
 // One warp's shared memory.  The list of marked pairs (at most 32 x 32
 // entries of 16 bits) takes the B staging's place after the sweep.
 struct TileScratch {
@@ -230,7 +233,11 @@ __device__ __forceinline__ double strip_potentials(const System& s, TileScratch&
 // The radius products are formed once, and sphere B's term is the negation
 // of sphere A's (RN(-x) = -RN(x)).  Every remaining operation is the general
 // form's, in its order.
-template <int PE, bool UNI>
+//
+// ROWS rows at a time (1, 2 or 4): their chains side by side, where a warp has
+// its SM sub-partition to itself.  Rows past a1 are computed from the block's
+// padding and dropped.
+template <int PE, bool UNI, int ROWS>
 __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                             double bx, double by, double bz, const pf::Sphere& sb,
                                             const pf::Uniform& un, bool bvalid, double& pe, uint32_t& marked,
@@ -244,51 +251,64 @@ __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, in
     double* my_stage = ws.bstage + lane * kBStageRow;
     double* rowA = s.pairbuf + (size_t)(X * kBlock) * s.npad + B;  // + a*npad: term for A
     double* rowB = s.pairbuf + (size_t)B * s.npad + X * kBlock;    // + a: term for B
-    for (int a = a0; a < a1; ++a) {
-        const bool valid = bvalid && (X != Y || lane < a);
-        pf::Sphere sa;
-        if (UNI) {
-            sa = sb;
-        } else {
-            sa.R = ab.R[a];
-            sa.sR = pf::unpack(sa.R);
-            sa.cR3 = ab.cR3[a];
-            sa.rm = ab.rm[a];
-            sa.em = pf::unpack(ab.m[a]).e;
-        }
-        const pf::Pair pr = pf::pair_terms<UNI>(bx - ab.x[a], by - ab.y[a], bz - ab.z[a], sa, sb, un, h_min_bits);
-        // contact (overlap > 0), or a result this path does not settle: the
-        // general path writes these entries after the sweep
-        const bool mark = valid && (__double_as_longlong(pr.overlap) > 0 || !pr.fl.sure());
-        if (mark) marked |= 1u << a;
-        if (PE == kPeInline) {
-            if (valid && !mark) {  // :239
-                const VdwArg v = vdw_arg(pr.h, sa.R, sb.R, 2 * sa.R);
-                if (v.far()) pe += vdw_energy_series(s.mat.Ha, v);
-                else near |= 1u << a;
-            }
-        }
-        if (valid) {
-            double* pa = rowA + (size_t)a * s.npad;
-            __stcs(pa, pr.ta[0]);
-            __stcs(pa + plane, pr.ta[1]);
-            __stcs(pa + 2 * plane, pr.ta[2]);
-            if (staged) {
-                double* st = my_stage + (a & 3);
-                st[0] = pr.tb[0];
-                st[kBStagePlane] = pr.tb[1];
-                st[2 * kBStagePlane] = pr.tb[2];
+    for (int r0 = a0; r0 < a1; r0 += ROWS) {
+        pf::Pair prs[ROWS];
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) {
+            const int a = r0 + k;
+            pf::Sphere sa;
+            if (UNI) {
+                sa = sb;
             } else {
-                double* pb = rowB + a;
-                __stcs(pb, pr.tb[0]);
-                __stcs(pb + plane, pr.tb[1]);
-                __stcs(pb + 2 * plane, pr.tb[2]);
+                sa.R = ab.R[a];
+                sa.sR = pf::unpack(sa.R);
+                sa.cR3 = ab.cR3[a];
+                sa.rm = ab.rm[a];
+                sa.em = pf::unpack(ab.m[a]).e;
+            }
+            prs[k] = pf::pair_terms<UNI>(bx - ab.x[a], by - ab.y[a], bz - ab.z[a], sa, sb, un, h_min_bits);
+        }
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k) {
+            const int a = r0 + k;
+            const pf::Pair& pr = prs[k];
+            const bool valid = bvalid && (X != Y || lane < a) && (ROWS == 1 || a < a1);
+            // contact (overlap > 0), or a result this path does not settle: the
+            // general path writes these entries after the sweep
+            const bool mark = valid && (__double_as_longlong(pr.overlap) > 0 || !pr.fl.sure());
+            if (mark) marked |= 1u << a;
+            if (PE == kPeInline) {
+                if (valid && !mark) {  // :239
+                    const double Ra = UNI ? sb.R : ab.R[a];
+                    const VdwArg v = vdw_arg(pr.h, Ra, sb.R, 2 * Ra);
+                    if (v.far()) pe += vdw_energy_series(s.mat.Ha, v);
+                    else near |= 1u << a;
+                }
+            }
+            if (valid) {
+                double* pa = rowA + (size_t)a * s.npad;
+                __stcs(pa, pr.ta[0]);
+                __stcs(pa + plane, pr.ta[1]);
+                __stcs(pa + 2 * plane, pr.ta[2]);
+                if (staged) {
+                    double* st = my_stage + (a & 3);
+                    st[0] = pr.tb[0];
+                    st[kBStagePlane] = pr.tb[1];
+                    st[2 * kBStagePlane] = pr.tb[2];
+                } else {
+                    double* pb = rowB + a;
+                    __stcs(pb, pr.tb[0]);
+                    __stcs(pb + plane, pr.tb[1]);
+                    __stcs(pb + 2 * plane, pr.tb[2]);
+                }
             }
         }
-        if (staged && bvalid && ((a & 3) == 3 || a == a1 - 1)) {
+        static_assert(kStripRows % ROWS == 0 && ROWS <= 4, "rows r0 .. share a sector of row B");
+        const int last = min(r0 + ROWS, a1) - 1;
+        if (staged && bvalid && ((last & 3) == 3 || last == a1 - 1)) {
             // row B, partners q0 .. q0+3: a 32-byte aligned sector (npad and
             // 32X are multiples of 4, the buffer is 256-byte aligned)
-            const int q0 = a & ~3;
+            const int q0 = last & ~3;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const double* st = my_stage + c * kBStagePlane;
@@ -315,7 +335,7 @@ __device__ __forceinline__ void load_a(const System& s, ABlock& ab, int lane, in
 // Partners a0 .. a1 - 1 of the tile (X, Y), the A block loaded: the sweep, or
 // where a constant leaves the integer path's range (no cohesion: cR3 = 0;
 // masses far from 1) the general path for every pair, then the marked pairs.
-template <int PE>
+template <int PE, int ROWS = 1>
 __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                            int iB, bool bvalid, double& pe, uint32_t& rowbits, uint32_t& colbits)
 {
@@ -338,10 +358,10 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
         marked = bvalid ? (X != Y ? all : all & ~((2u << lane) - 1u)) : 0u;
     } else if (uni) {
         const pf::Uniform un{R0 + R0, ab.fourR[0] * R0, pf::unpack(ab.cR3[0] * R0 * R0 * R0)};
-        sweep_pairs<PE, true>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
+        sweep_pairs<PE, true, ROWS>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     } else {
         const pf::Uniform un{0.0, 0.0, {0, 0}};
-        sweep_pairs<PE, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
+        sweep_pairs<PE, false, ROWS>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     }
     if (PE == kPeInline && __any_sync(0xffffffffu, near != 0u)) pe += near_potentials(s, ws, X, Y, near);
     rowbits = colbits = 0;
@@ -352,9 +372,6 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
         __syncwarp();
     }
 }
-
-// A tile may be taken in strips of 8 of its 32 rows.
-constexpr int kStripRows = 8, kStrips = kBlock / kStripRows;
 
 // Contact words of an item of tile (X, Y): row A = 32X + lane gets block Y's
 // bits, row B block X's; on the diagonal both describe row 32X + lane.
