@@ -437,7 +437,7 @@ static void launch_pair_columns(const System& s, PeMode pe, int num_sms, cudaStr
     const long long items = (cut - t0) + kStrips * (t1 - cut);
     // few items: one warp per CTA, so that they spread over the SMs, and a
     // dependent launch (N=96: 25.1 -> 23.4 us per step).  A larger grid placed
-    // while the drift still runs is spread unevenly (N=1000: 82 -> 84 us), and
+    // while the drift still runs is spread unevenly (N=500: 55.3 -> 56.5 us), and
     // so are the row sums placed beside the pair tiles (N=1000: 82 -> 124 us,
     // N=5000: 674 -> 836): both are launched plainly.
     const int warps = items <= 4LL * num_sms ? 1 : 4;
@@ -451,7 +451,7 @@ static void launch_pair_columns(const System& s, PeMode pe, int num_sms, cudaStr
                         : pe == kPeInline ? pair_tile_kernel<kPeInline, 4>
                         : two_rows        ? pair_tile_kernel<kNoPe, 1>
                                           : pair_tile_kernel<kNoPe, 4>;
-    launch_pdl(pdl && pb * warps <= 4LL * num_sms, kernel, pb, 32 * warps, 0, st, s, c0, c1, phase, split);
+    launch_pdl(pdl && pb * warps <= 2LL * num_sms, kernel, pb, 32 * warps, 0, st, s, c0, c1, phase, split);
 }
 
 void launch_step(const System& sys, bool write, int num_sms, cudaStream_t st, StepTimers* tm, const StepOverlap* ov,

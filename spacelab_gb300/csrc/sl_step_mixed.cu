@@ -788,11 +788,6 @@ bool mixed_pair_double(int nb, int num_sms)
 
 void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st, StepTimers* tm)
 {
-    // not where the pair kernel fills the SMs: N=9000 94.9 us per step without,
-    // 98.9 with
-    const bool pdl = !s.pair_double;
-    launch_drift(s, st, pdl);
-    if (tm) cudaEventRecord(tm->ev[0], st);
     long long want = (s.nitems + kPairWarps - 1) / kPairWarps;
     // one wave of persistent warps
     long long cap = (long long)num_sms * (s.pair_double ? kPair2CtasPerSm : kPairCtasPerSm);
@@ -803,6 +798,11 @@ void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st
     // and on write steps, whose FP64 potentials it makes dense (N=5000 124.6 /
     // 109.6).
     const bool few_tiles = 2 * s.ntiles <= 5 * cap * kPairWarps;
+    // a dependent drift not where the pair kernel fills the SMs: N=1733 17.9 us per
+    // step with, 18.4 without, N=4000 33.5, 32.8, N=9000 98.9, 94.9
+    const bool pdl = few_tiles && !s.pair_double;
+    launch_drift(s, st, pdl);
+    if (tm) cudaEventRecord(tm->ev[0], st);
     if (s.pair_double)
         launch_pdl(pb <= num_sms, write ? mixed_pair2_kernel<true> : mixed_pair2_kernel<false>, pb, 32 * kPairWarps, 0, st, s);
     else
@@ -812,7 +812,10 @@ void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st
                                : mixed_pair_kernel,
                    pb, 32 * kPairWarps, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[1], st);
-    launch_pdl(pdl, mixed_finish_kernel, s.nb, 32 * kFinSlices, 0, st, s);
+    // plainly: placed beside the pair kernel's last blocks, the finish blocks share
+    // SMs (us per step, dependent / plain: N=100 11.3 / 10.4, N=1000 19.0 / 15.7,
+    // N=2500 23.7 / 22.7)
+    mixed_finish_kernel<<<s.nb, 32 * kFinSlices, 0, st>>>(s);
     if (tm) cudaEventRecord(tm->ev[2], st);
     if (write) launch_energy(s, st, pdl);
 }
