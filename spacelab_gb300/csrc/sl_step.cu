@@ -101,8 +101,8 @@ __device__ __forceinline__ void col_tile_coords(int nb, long long u, int& X, int
 // pe_tile[q].  kPeApart: one warp per CTA, and as many CTAs again, whose items
 // are the potentials of the first ones' pairs out of contact, to
 // pe_tile[nitems / 2 + q].
-template <int PE, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, WARPS == 1 ? 8 : 4) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
+template <int PE, int WARPS, int CTAS = WARPS == 1 ? 8 : 4>
+__global__ void __launch_bounds__(32 * WARPS, CTAS) pair_tile_kernel(const __grid_constant__ System s, int c0, int c1,
                                                           int phase, long long split)
 {
     __shared__ TileScratch scratch[WARPS];
@@ -441,7 +441,12 @@ static void launch_pair_columns(const System& s, PeMode pe, int num_sms, cudaStr
     // so are the row sums placed beside the pair tiles (N=1000: 82 -> 124 us,
     // N=5000: 674 -> 836): both are launched plainly.
     const int warps = items <= 4LL * num_sms ? 1 : 4;
-    const int pb = pe == kPeApart ? (int)(2 * items) : (int)min((items + warps - 1) / warps, (long long)num_sms * 4);
+    // More items than four CTAs per SM have warps for: five, at 96 registers (us
+    // per step, four / five / six: N=2600 266 / 259 / 264, N=5000 690 / 666 / 677,
+    // N=10000 2508 / 2415 / 2449, N=20000 10.85 / 10.61 / 10.52 ms).
+    const bool many = warps == 4 && pe == kNoPe && items >= 16LL * num_sms;
+    const int ctas = many ? 5 : 4;
+    const int pb = pe == kPeApart ? (int)(2 * items) : (int)min((items + warps - 1) / warps, (long long)num_sms * ctas);
     // One-warp CTAs may use 216 registers, and take two rows at a time (us per
     // step, one against two: N=32 25.0 -> 23.3, N=96 32.7 -> 30.8, N=400 50.8 ->
     // 48.9; four rows the same).  A few rows are over before the longer code
@@ -450,6 +455,7 @@ static void launch_pair_columns(const System& s, PeMode pe, int num_sms, cudaStr
     const auto kernel = pe == kPeApart    ? pair_tile_kernel<kPeApart, 1>
                         : pe == kPeInline ? pair_tile_kernel<kPeInline, 4>
                         : two_rows        ? pair_tile_kernel<kNoPe, 1>
+                        : many            ? pair_tile_kernel<kNoPe, 4, 5>
                                           : pair_tile_kernel<kNoPe, 4>;
     launch_pdl(pdl && pb * warps <= 2LL * num_sms, kernel, pb, 32 * warps, 0, st, s, c0, c1, phase, split);
 }
