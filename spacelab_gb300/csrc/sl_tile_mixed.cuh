@@ -181,8 +181,9 @@ __device__ __forceinline__ void tile(const float* rows, List<VALUES>& list, cons
     }
     if (any) {
         const float u_thr = fmaf(far_sq, u_sum2, margin);
+        // (unrolled eight times: 512 collisions 26.1 ms, twice 25.8; 64 of them in lockstep 5.18, 5.07)
         const F32x2 cx = pair2(col.x, col.x), cy = pair2(col.y, col.y), cz = pair2(col.z, col.z);
-#pragma unroll 8
+#pragma unroll 2
         for (int k = 0; k < 32; k += 2) {
             const float* w = rows + ((lane + k) & 31) * kRow;
             const float4 q0 = *reinterpret_cast<const float4*>(w);
