@@ -43,7 +43,10 @@ int sl_batch_upload(sl_batch* b, const double* pos, const double* vel, const dou
  * blocks: in the mixed form over Z-ordered spheres with per-CTA partial sums
  * (also at 512 threads); in the exact form with per-CTA pair-term buffers and
  * ordered row sums, bit-identical to the other shapes (SL_ERR_UNSUPPORTED
- * where the largest instance makes those buffers too big). */
+ * where the largest instance makes those buffers too big).  The pair-tile
+ * pass may advance all instances in lockstep, from one queue of tiles, where
+ * that balances better than an instance per CTA; `threads` has no effect
+ * there, and the results are the same. */
 int sl_batch_set_shape(sl_batch* b, int tile, int threads);
 int sl_batch_shape(const sl_batch* b, int* tile, int* threads, int* blocks);
 

@@ -2,10 +2,14 @@
 // systems (projectile-target collisions of uneven sphere counts) advanced by
 // ONE persistent launch.
 //
-// Each CTA takes whole instances from an atomic work queue (largest first)
-// and runs all of an instance's steps before taking the next one; the only
-// synchronisation is __syncthreads inside the CTA, so no CTA ever waits on
-// another.  Within an instance a step is the reference's three passes
+// The pair-tile pass runs in lockstep where that balances better (in the exact
+// form always): a cooperative launch of one CTA per SM in which all instances
+// take a step together, their tiles and rows being one queue each and the
+// phases separated by a grid barrier (bounded; runs_in_lockstep in
+// sl_batch_capi.cu).  Otherwise each CTA takes whole instances from an atomic
+// work queue (largest first) and runs all of an instance's steps before taking
+// the next one; the only synchronisation is then __syncthreads inside the CTA.
+// The results are the same bit for bit.  Within an instance a step is the reference's three passes
 // (ColliderSingleCore.cpp:82-97, 100-256, 263-287):
 //   drift    one thread per sphere (strided);
 //   pairs    either the pair-tile pass (shape tile 0: every pair once into

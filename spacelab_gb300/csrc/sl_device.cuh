@@ -47,7 +47,8 @@ struct System {
     int n, npad, nb;
     long long ntiles;  // nb * (nb + 1) / 2 lower-triangular block tiles
     long long nitems;  // pair-kernel work items, one pe_tile entry each: ntiles, or
-                       // mixed_pair_items(nb) where pair_double is set
+                       // mixed_pair_items(nb) where pair_double is set; the exact form
+                       // sets it per launch (strips, potentials apart)
     int pair_double;   // mixed form: two column blocks per work item
     Vec3Soa pos, prev, vel, velh, w, wh, acc, aacc;
     double *R, *m, *moi, *twoR, *fourR, *cR3;
@@ -58,7 +59,7 @@ struct System {
     uint32_t* cmask;      // [npad][nb]
     double* pe_tile;      // [nitems]
     double* red;          // [kRedBlocks][8] energy partials
-    double* energy;       // [8] PE, KE, mom xyz, L xyz
+    double* energy;       // [8] PE, KE, mom xyz, L xyz (a handle's: pinned host memory)
     unsigned int* status; // error bits (see SL_ERR_* in spacelab_gpu.h)
     unsigned int* host_status;  // where a step's last kernel copies them for the host, or NULL
     const Scalars* sc;

@@ -1,16 +1,17 @@
 // sl_step.cu -- the FP64 step of SpaceLab's hot path on sm_103a, bit-exact
 // with the reference's sim_one_step (ColliderSingleCore.cpp:78-288).
 //
-// One step is four launches on the handle's stream (the row sums have a
-// TMA-streamed form in sl_rowsum_tma.cu, used whenever a tensor map of the
-// pair-term buffer could be made):
+// One step is three launches on the handle's stream, a write step four or
+// five (the row sums have a TMA-streamed form in sl_rowsum_tma.cu, used
+// whenever a tensor map of the pair-term buffer could be made):
 //   drift_kernel      pass 1 (ColliderSingleCore.cpp:82-97): velh, wh, drift,
 //                     and the previous positions that replace the reference's
 //                     O(N^2) `distances` array (ball_group.hpp:741).
 //   pair_tile_kernel  pass 2 (:100-256): every unordered pair (A > B) is
 //                     evaluated ONCE, in the reference's orientation, by one
-//                     lane of a warp that owns a 32x32 block tile; its terms
-//                     for both spheres go to pairbuf/torqbuf.
+//                     lane of a warp that owns a 32x32 block tile or, where
+//                     there are few, 8 rows of one; its terms for both
+//                     spheres go to pairbuf/torqbuf.
 //   rowsum_kernel     sums row s of pairbuf in ascending partner order -- the
 //                     order in which the reference adds terms to acc[s] --
 //                     then pass 3 (:263-267): vel, w.
@@ -18,13 +19,12 @@
 //                     |L| (:282-285), in a fixed reduction tree.
 // All arithmetic follows the reference's vec3 evaluation order
 // (vec3.hpp:44-128,180-184) and this file is compiled with --fmad=false, so
-// no multiply-add is contracted.  The square root and the quotients of the
-// non-contact path and of the mass divisions are formed as FP64 estimates
-// rounded exactly with integer arithmetic (sl_fp64_exact.cuh): the same
-// IEEE results with most of the work moved off the narrow FP64 pipe.  The
-// estimates themselves come from the integer pipe too: fixed-point mass
-// reciprocals made once at upload, a fixed-point 1/sqrt(d2) by Newton
-// iteration, and a fixed-point reciprocal of the vdW denominator.
+// no multiply-add is contracted.  The products, the square root and the
+// quotients of a pair out of contact are formed on unpacked significands with
+// integer arithmetic (sl_pair_fast.cuh): the same IEEE results with most of
+// the work moved off the narrow FP64 pipe.  A pair whose rounding that leaves
+// open, and one in contact, takes the general path after the sweep
+// (sl_fp64_exact.cuh; sl_tile_exact.cuh).
 #include "sl_device.cuh"
 #include "sl_kernels.h"
 #include "sl_fp64_exact.cuh"

@@ -33,7 +33,8 @@
 // Every order is fixed, so runs repeat bit for bit.  Large systems
 // (mixed_pair_double) take a row block against two column blocks at a time
 // (mixed_pair2_kernel): one shared-memory load of a row and one shuffle then
-// serve two pairs.
+// serve two pairs.  Small ones, and write steps, find a tile's close pairs
+// before its sweep (mixed_pair_listed_kernel, sl_tile_mixed.cuh).
 //
 // The physics follows ColliderSingleCore.cpp:104-253 term by term; only the
 // arithmetic and the evaluation order differ.

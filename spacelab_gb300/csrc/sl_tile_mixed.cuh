@@ -24,9 +24,9 @@
 
 #include <type_traits>
 
-//
-// What bounds it (GB300, ncu, the batch): the shared-memory pipe at 75%, beside
-// issue at 70%.  So the sweep takes two steps at a time in packed FP32
+// What bounds it (GB300, ncu): at 20 warps per SM the shared-memory pipe at 75%,
+// beside issue at 70%; with an instance per CTA (16 warps) latency, issue 46%.
+// So the sweep takes two steps at a time in packed FP32
 // arithmetic, and in tiles of one radius reads 24 bytes of a row instead of
 // 32.  512 collisions of up to 2400 spheres, whole instances at 512 threads:
 // 1.16 ms per step with the close path in the sweep, 1.03 listed.
@@ -138,7 +138,8 @@ __device__ __forceinline__ float warp_max(float f) { return unord(__reduce_max_s
 // and column blocks are one (pairs with lane < r).  close(q, row, col, pe,
 // pe_far) evaluates list entry q -- whatever its distance -- into list.v[q]:
 // the force on the row sphere, then the user's values; taken(q, row) is called
-// in the sweep's order, by the column's lane, when entry q's force is added.  a: the row sums, lane l's of row l; b: the lane's column sums.
+// in the sweep's order, by the column's lane, when entry q's force is added.  a:
+// the row sums, lane l's of row l; b: the lane's column sums.
 template <bool WRITE, int VALUES, class Close, class Taken>
 __device__ __forceinline__ void tile(const float* rows, List<VALUES>& list, const Col& col, int nA, bool diag,
                                      float far_sq, Close&& close, Taken&& taken, float (&a)[3], float (&b)[3],
