@@ -793,15 +793,16 @@ void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st
     // one wave of persistent warps
     long long cap = (long long)num_sms * (s.pair_double ? kPair2CtasPerSm : kPairCtasPerSm);
     const int pb = (int)(want < cap ? want : cap);
-    // Listing the close pairs pays while a tile's latency shows: up to 2.5 tiles
-    // per resident warp (us per step, evaluated in the sweep / listed: N=1733
-    // 22.9 / 18.5, N=3000 32.1 / 28.8, N=4000 37.3 / 37.4, N=5000 46.7 / 51.1),
-    // and on write steps, whose FP64 potentials it makes dense (N=5000 124.6 /
-    // 109.6).
-    const bool few_tiles = 2 * s.ntiles <= 5 * cap * kPairWarps;
+    // Listing the close pairs pays while a tile's latency shows, up to one tile per
+    // resident warp (us per step, evaluated in the sweep / listed: polydisperse
+    // cluster N=1400 18.5 / 17.1, N=1900 19.5 / 18.7, N=2400 22.5 / 22.5, N=3000
+    // 26.1 / 27.8; a collision in its impact, with more close pairs, N=1400 20.0 /
+    // 16.7, N=2400 28.6 / 22.3), and on write steps, whose FP64 potentials it
+    // makes dense (N=5000 124.6 / 109.6).
+    const bool few_tiles = s.ntiles <= cap * kPairWarps;
     // a dependent drift not where the pair kernel fills the SMs: N=1733 17.9 us per
     // step with, 18.4 without, N=4000 33.5, 32.8, N=9000 98.9, 94.9
-    const bool pdl = few_tiles && !s.pair_double;
+    const bool pdl = 2 * s.ntiles <= 5 * cap * kPairWarps;
     launch_drift(s, st, pdl);
     if (tm) cudaEventRecord(tm->ev[0], st);
     if (s.pair_double)

@@ -240,7 +240,10 @@ __device__ __forceinline__ void tile(const float* rows, List<VALUES>& list, cons
             } else {
                 const F32x2 R = pair2(q1.z, q1.w);
                 const F32x2 sumR = add2(R, cR), difR = add2(R, ncR);
-                S = add2(d2, mul2(mul2(sumR, minus1), sumR));
+                // the square rounded by itself, as in the other kernels: a packed product
+                // is fused into a packed sum
+                const float2 s = split2(sumR);
+                S = add2(d2, pair2(-__fmul_rn(s.x, s.x), -__fmul_rn(s.y, s.y)));
                 T = fma2(mul2(difR, minus1), difR, d2);
                 crr = mul2(pair2(q3.z, q3.w), cR3);
             }

@@ -204,3 +204,25 @@ def test_mixed_accumulation_keeps_fp64_precision(n, offset):
     bar = 2.0 ** -20 + 8 * np.finfo(float).eps * max(offset, np.abs(pos).max()) / ov[ov > 0].min()
     assert np.linalg.norm(far - near) <= bar * np.linalg.norm(ex)
     assert np.linalg.norm(near - ex) <= (2.0 ** -17) * np.linalg.norm(ex)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,r_spread,spacing", [(2600, 0.1, 1.97), (2600, 0.1, 3.0), (2600, 0.0, 2.3), (2497, 0.3, 2.6)])
+def test_mixed_df_listed_and_in_sweep_kernels_agree_bit_for_bit(n, r_spread, spacing):
+    """A write step lists the close pairs of a tile, a plain step of a system
+    with more tiles than warps evaluates them in the sweep: the same
+    operations in the same order, so the same state, for unequal radii too."""
+    from cases import contact_case, material
+    from spacelab_gb300 import BallGroup, GpuStep
+    c = contact_case(n, 31, r_spread=r_spread, spacing=spacing)
+    states = []
+    for write in (True, False):
+        g = BallGroup.from_arrays(c["pos"], c["vel"], c["w"], c["R"], c["m"], c["moi"])
+        with GpuStep(g, material(), "mixed_df") as sim:
+            sim.set_scalars(c["dt"], c["kin"], c["kout"])
+            sim.init_conditions()
+            for _ in range(3):
+                sim.sim_one_step(write)
+            sim.download()
+        states.append(np.stack([g.pos, g.vel, g.w, g.acc, g.aacc]))
+    assert np.array_equal(states[0], states[1])
