@@ -800,9 +800,10 @@ void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st
     // 16.7, N=2400 28.6 / 22.3), and on write steps, whose FP64 potentials it
     // makes dense (N=5000 124.6 / 109.6).
     const bool few_tiles = s.ntiles <= cap * kPairWarps;
-    // a dependent drift not where the pair kernel fills the SMs: N=1733 17.9 us per
-    // step with, 18.4 without, N=4000 33.5, 32.8, N=9000 98.9, 94.9
-    const bool pdl = 2 * s.ntiles <= 5 * cap * kPairWarps;
+    // a dependent drift not where the pair kernel fills the SMs (us per step with /
+    // without: N=1733 17.9 / 18.4, collision N=3100 35.0 / 38.4, N=3500 42.2 /
+    // 40.6, N=4000 33.5 / 32.8, N=9000 98.9 / 94.9)
+    const bool pdl = 4 * s.ntiles <= 7 * cap * kPairWarps;
     launch_drift(s, st, pdl);
     if (tm) cudaEventRecord(tm->ev[0], st);
     if (s.pair_double)
