@@ -267,7 +267,7 @@ SL_PF_FN Sig vdw_coef(const Sig& P, double num, double S, double T, Flags& fl)
 struct Sphere {
     double R;
     Sig sR;             // unpacked R
-    double cR3;         // A only: ((Ha/6 64) R) R R
+    double cR3;         // A only: ((Ha/6 64) R) R R; its sign is the force's
     u64 rm;
     int em;
 };
@@ -338,9 +338,11 @@ SL_PF_FN Pair pair_terms(double rx, double ry, double rz, const Sphere& A, const
         P = mul(mul(mul(unpack(A.cR3), B.sR, fl), B.sR, fl), B.sR, fl);
     }
     const Sig coef = vdw_coef(P, o.h + A.R + B.R, S, T, fl);           // :221-225
+    // the significands hold magnitudes: a negative Ha (repulsion) turns the signs
+    const uint32_t csign = (uint32_t)(bits_of(A.cR3) >> 32) & 0x80000000u;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        const uint32_t sign = (uint32_t)(bits_of(r[c]) >> 32) & 0x80000000u;
+        const uint32_t sign = ((uint32_t)(bits_of(r[c]) >> 32) & 0x80000000u) ^ csign;
         const Sig F = mul(coef, div_root(sr[c], root.rec, root.d.e, fl), fl);  // :227
         o.ta[c] = pack(div_fixed(F, A.rm, A.em, fl), sign);            // :249
         // -(F/m[B]), :250; equal masses: RN(-x) = -RN(x)
