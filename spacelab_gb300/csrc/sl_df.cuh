@@ -64,16 +64,6 @@ __device__ __forceinline__ F2 sqr(F2 a)
     return fast_two_sum(p.hi, p.lo);
 }
 
-// The float nearest (a1 + a2 + a3) - (b1 + b2 + b3) for two numbers in three
-// parts of falling magnitude (their first part's last place bounds the
-// second, and so on): the difference of the first parts with its exact error,
-// then the rest, which is below 2^-23 of them and is rounded at 2^-47.
-__device__ __forceinline__ float sub3(float a1, float a2, float a3, float b1, float b2, float b3)
-{
-    const F2 d = two_sum(a1, -b1);
-    return d.hi + (d.lo + ((a2 - b2) + (a3 - b3)));
-}
-
 // Running sum of FP32 terms in three parts, a + b + c: the rounding error of
 // each addition into a goes exactly into b, and b's into c -- some 70 bits, so
 // a sum of 32 terms is closer to the exact one than a running FP64 sum, for

@@ -28,6 +28,7 @@
 #include "sl_device.cuh"
 #include "sl_kernels.h"
 #include "sl_fp64_exact.cuh"
+#include "sl_parts.cuh"
 #include "sl_pair_exact.cuh"
 #include "sl_tile_exact.cuh"
 
@@ -67,7 +68,8 @@ __global__ void __launch_bounds__(kDriftThreads) drift_kernel(const __grid_const
         const double unit = ldexp(1.0, s.len_shift);
         const float hi = d2f_bits(pn, s.len_shift);
         const double rem = pn - f2d_bits(hi) * unit;  // exact, as is the next
-        const float lo = d2f_bits(rem, s.len_shift);
+        float lo = d2f_bits(rem, s.len_shift);
+        if (s.f_pos[6]) lo = parts::grid_part(hi, lo);
         s.f_pos[c][i] = hi;
         s.f_pos[3 + c][i] = lo;
         if (s.f_pos[6]) s.f_pos[6 + c][i] = d2f_bits(rem - f2d_bits(lo) * unit, s.len_shift);

@@ -6,8 +6,8 @@
 //     the exact form) and pass 3 in mixed64_finish_kernel
 //     (ColliderSingleCore.cpp:82-97, 263-267);
 //   * the pair subtraction r = pos[B] - pos[A] (:105): the FP64 positions are
-//     held as three FP32 parts (72 bits, written by the drift), whose
-//     differences give r rounded once to FP32 (df::sub3);
+//     held as three FP32 parts (written by the drift), whose differences
+//     give r rounded once to FP32 (parts::sub3, sl_parts.cuh);
 //   * for pairs closer than far_sq (1.25 radii sums or more), r itself,
 //     |r|^2, the squared gap g = (R_A + R_B)^2 - |r|^2, |r| and the overlap
 //     R_A + R_B - |r| = g / (R_A + R_B + |r|) (:106-110) in FP64, which set the
@@ -25,13 +25,14 @@
 // r and the FP64 overlap: the vdW coefficient, elastic, gravity, sliding and
 // rolling friction and the torques, in lengths scaled by 2^-len_shift.
 //
-// What bounds it (ncu, N=9000): the FP32 pipe at 72%, half of its work the six
-// error-free sums, beside issue at 68%; the two spheres' sums of a component
-// are added in packed arithmetic.  On the FP64 pipe the subtraction and the
-// sums were 9 adds a pair at 19 SM-cycles each (one narrow unit per SM), 171
-// cycles for a warp's 32 pairs, at 0.96 of that unit's rate; now it is 58.
-// N=20000 polydisperse, 20 steps: 74.2 -> 23.1 ms (sums one by one, unrolled
-// twice 23.8; 3 and 5 CTAs per SM 25.2 and 23.9).
+// What bounds it (ncu, N=9000): the FP32 pipe, then at 72% beside issue at 68%;
+// half of its work are the six error-free sums, and the two spheres' sums of a
+// component are added in packed arithmetic.  On the FP64 pipe the subtraction
+// and the sums were 9 adds a pair at 19 SM-cycles each (one narrow unit per SM),
+// 171 cycles for a warp's 32 pairs, at 0.96 of that unit's rate; now it is some
+// 60.  N=20000 polydisperse, 20 steps: 74.2 -> 23.1 ms with the subtraction to
+// 2^-47 of the coordinates (sums one by one, unrolled twice 23.8; 3 and 5 CTAs per
+// SM 25.2 and 23.9), 24.2 with it rounded once (x and y packed 24.5).
 //
 // Accumulation order: one warp evaluates a 32 x 32 tile in a diagonal sweep
 // (lane b holds column sphere B's sum; row r's sum travels one lane down per
@@ -43,6 +44,7 @@
 #include "sl_df.cuh"
 #include "sl_kernels.h"
 #include "sl_pair_mixed.cuh"
+#include "sl_parts.cuh"
 
 #include <type_traits>
 
@@ -132,9 +134,9 @@ __global__ void __launch_bounds__(32 * kM64Warps, kM64CtasPerSm) mixed64_pair_ke
                 const float4 q3 = *reinterpret_cast<const float4*>(rows + r * kRow64 + 8);
                 const float Ras = q1.w;
                 // the pair subtraction (:105), rounded to FP32
-                const float rx = df::sub3(bx1, bx2, bx3, q1.x, q2.x, q3.x);
-                const float ry = df::sub3(by1, by2, by3, q1.y, q2.y, q3.y);
-                const float rz = df::sub3(bz1, bz2, bz3, q1.z, q2.z, q3.z);
+                const float rx = parts::sub3(bx1, bx2, bx3, q1.x, q2.x, q3.x);
+                const float ry = parts::sub3(by1, by2, by3, q1.y, q2.y, q3.y);
+                const float rz = parts::sub3(bz1, bz2, bz3, q1.z, q2.z, q3.z);
                 const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
                 const float sumR = Ras + Rbs, difR = Ras - Rbs;
                 const float sum2 = sumR * sumR;
