@@ -373,8 +373,12 @@ int sl_upload(sl_handle* h, const double* pos, const double* vel, const double* 
     }
     int ex = 0;
     std::frexp(rmax, &ex);
-    h->sys.len_shift = ex - 1;
-    h->sys.far_sq = sl::far_threshold_sq(h->sys.mat.h_min, rmin);
+    const int len_shift = ex - 1;
+    const float far_sq = sl::far_threshold_sq(h->sys.mat.h_min, rmin);
+    // a captured interval holds the mixed forms' length scale and threshold
+    if (h->mode != SL_MODE_EXACT && (len_shift != h->sys.len_shift || far_sq != h->sys.far_sq)) drop_graph(h);
+    h->sys.len_shift = len_shift;
+    h->sys.far_sq = far_sq;
     // padded spheres get R = m = moi = 1 (they are never paired)
     const double* src[3] = {R, m, moi};
     double* dst[3] = {h->sys.R, h->sys.m, h->sys.moi};
