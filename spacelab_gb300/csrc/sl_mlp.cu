@@ -308,7 +308,7 @@ __device__ void bias_grad(const GemmLaunch& L, unsigned char* smem, int c0)
         for (int k = tid; k < outs * vecs; k += kTcThreads) {
             const int c = k / vecs, v = k - c * vecs;
             *reinterpret_cast<uint4*>(smem + c * kBiasStride + v * 16) =
-                __ldg(reinterpret_cast<const uint4*>(L.db_src + (size_t)(c0 + c) * L.db_rows + r0) + v);
+                reinterpret_cast<const uint4*>(L.db_src + (size_t)(c0 + c) * L.db_rows + r0)[v];
         }
         __syncthreads();
         if (tid < outs) {
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(kTcThreads) gemm_nt_tc_kernel(const __grid_con
             if (J.ldc % 8 == 0 && col + 16 <= J.N) {  // whole 16-byte groups
                 if (J.bias)
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] += __ldg(J.bias + col + i);
+                    for (int i = 0; i < 16; ++i) v[i] += J.bias[col + i];
                 if (J.zin) {
 #pragma unroll
                     for (int i = 0; i < 16; i += 4) {
@@ -731,8 +731,8 @@ __global__ void pack_kernel(const float* __restrict__ x, const float* __restrict
 
 // MSE over the first n_out columns: dZ = 2 (z - y) / (M n_out), row-major and
 // transposed, and the loss in one partial sum per 256 entries of dZ
-__global__ void mse_grad_kernel(const float* __restrict__ z, int ldz, const float* __restrict__ y, int M, int n_out,
-                                bf16* dz, bf16* dzt, int ld, float* loss_partial, const int* step, int step_bias)
+__global__ void mse_grad_kernel(const float* z, int ldz, const float* y, int M, int n_out, bf16* dz, bf16* dzt, int ld,
+                                float* loss_partial, const int* step, int step_bias)
 {
     __shared__ float red[256];
     sl::pdl_next();

@@ -7,6 +7,12 @@
 // reads, which returns when the kernel before has ended and its writes are
 // visible.  As every kernel of a chain waits, the order of the whole chain
 // holds.  Launched plainly, both calls do nothing.
+//
+// A kernel that waits is resident while earlier kernels still write what it
+// reads.  Its loads of global memory are therefore ordinary ones: no __ldg
+// and no __restrict__ parameter, which lets the compiler use the non-coherent
+// path -- that path requires data that nothing writes while the kernel is
+// resident, and the wait does not order it.
 #pragma once
 #include <cuda_runtime.h>
 #include <utility>
