@@ -8,6 +8,8 @@
 
 #include <stdint.h>
 
+#include "spacelab_batch.h"
+
 #ifdef __cplusplus
 extern "C" {
 #endif
@@ -52,6 +54,11 @@ int sl_diag_fp32_peak(double* gflops);
  * the reference. */
 int sl_diag_gemm_bf16(int M, int N, int K, const uint16_t* A, const uint16_t* B, const float* bias, int act,
                       int kernel, float* C, uint16_t* Cb);
+
+/* Error handling of the batch's lockstep form: its barrier number `barrier`
+ * (1, 2, ... within a run; 0: none) gives up at once from the next run on, as if
+ * its time had run out; the run then returns SL_ERR_TIMEOUT. */
+int sl_diag_batch_give_up(sl_batch* b, unsigned barrier);
 
 #ifdef __cplusplus
 }

@@ -117,6 +117,7 @@ _PROTOS = [
     ("sl_diag_fp64_add_latency", ctypes.c_int, [ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_double)]),
     ("sl_diag_exact_ops", ctypes.c_int, [ctypes.c_int] + [_c_double_p] * 3),
     ("sl_diag_int_ops", ctypes.c_int, [ctypes.c_int] + [_c_double_p] * 3),
+    ("sl_diag_batch_give_up", ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint]),
     # host setup (spacelab_host.h)
     ("slh_build_cluster", ctypes.c_int, [ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                          ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,

@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, 1) batch_exact_grid_kernel(co
     const int q0 = do_init ? -1 : 0;
     if (q0 >= nsteps) return;
     grid_drift(b, do_init != 0);
-    if (!batch::grid_sync(b.gsync, phase)) return;
+    if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
     for (int q = q0; q < nsteps; ++q) {
         const int step = first_step + q, par = q & 1;
         const bool init = q < 0, write = init || (skip > 0 && step % skip == 0), more = q + 1 < nsteps;
@@ -521,18 +521,18 @@ __global__ void __launch_bounds__(32 * kGridWarps, 1) batch_exact_grid_kernel(co
             grid_pairs<true>(b, gw, num_sms, b.gqueue + par, pe);
         else
             grid_pairs<false>(b, gw, num_sms, b.gqueue + par, pe);
-        if (!batch::grid_sync(b.gsync, phase)) return;
+        if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) b.gqueue[par ^ 1] = 0;  // the next step's queue
         grid_rows(b, init, more && !write);
         if (!more && !write) break;
-        if (!batch::grid_sync(b.gsync, phase)) return;
+        if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
         if (write) {
             const int r = init ? 0 : min(step / skip, b.nrec - 1);
             grid_energy(b, num_sms, pe, r, sh);
             if (!more) break;
-            if (!batch::grid_sync(b.gsync, phase)) return;
+            if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
             grid_drift(b, false);
-            if (!batch::grid_sync(b.gsync, phase)) return;
+            if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
         }
     }
 }

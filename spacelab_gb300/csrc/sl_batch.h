@@ -76,6 +76,7 @@ struct Batch {
     double* gke;       // [gblocks][8] mixed: a write step's other totals
     GridSync* gsync;
     int* gqueue;       // [2] item queues, alternating between the steps
+    unsigned give_up;  // diagnostics: the barrier that gives up at once, or 0
     int len_shift;
     Material mat;         // G, Ha, u_r, h_min shared; u_s per instance
     double* energy;       // [ninst][nrec][8]

@@ -3,6 +3,7 @@
 // arena, advanced by one persistent, graph-captured launch, with a
 // project-written autotuner for the j-tile size and threads per instance.
 #include "../../include/spacelab_batch.h"
+#include "../../include/spacelab_diag.h"
 #include "../../include/spacelab_gpu.h"
 #include "sl_batch.h"
 #include "sl_kernels.h"
@@ -56,6 +57,7 @@ struct sl_batch {
     bool uploaded = false;
     std::vector<int> counts, offsets;
     void* grid_arena = nullptr;  // the lockstep form's scratch and lists
+    size_t mark_bytes = 0;       // of b.xmask there
 };
 
 namespace {
@@ -125,7 +127,12 @@ int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, i
     if (lockstep) {
         sl::GridSync gs{};
         SLB_CUDA(cudaMemcpy(&gs, h->b.gsync, sizeof gs, cudaMemcpyDeviceToHost));
-        if (gs.failed) return sl_record_error(SL_ERR_TIMEOUT, "a bounded wait between the batch's phases ran out");
+        if (gs.failed) {
+            // the mixed form's torque marks are cleared by the phase that reads them: the
+            // next run must not find those of a run that ended between the two
+            SLB_CUDA(cudaMemset(h->b.xmask, 0, h->mark_bytes));
+            return sl_record_error(SL_ERR_TIMEOUT, "a bounded wait between the batch's phases ran out");
+        }
     }
     return SL_OK;
 }
@@ -210,6 +217,7 @@ int setup_lockstep(sl_batch* h, const std::vector<int>& order)
     b.gke = reinterpret_cast<double*>(p + o_ke);
     b.gsync = reinterpret_cast<sl::GridSync*>(p + o_sync);
     b.gqueue = reinterpret_cast<int*>(b.gsync + 1);
+    h->mark_bytes = (size_t)nm * sizeof(uint32_t);
     b.gtiles = tiles[b.ninst];
     b.gblocks = (int)blocks[b.ninst];
     b.grid = 1;
@@ -636,6 +644,13 @@ int sl_batch_status(sl_batch* h, unsigned* status)
 {
     if (!h || !status) return sl_record_error(SL_ERR_ARG, "null argument");
     SLB_CUDA(cudaMemcpy(status, h->b.status, h->b.ninst * sizeof(unsigned), cudaMemcpyDeviceToHost));
+    return SL_OK;
+}
+
+int sl_diag_batch_give_up(sl_batch* h, unsigned barrier)
+{
+    if (!h) return sl_record_error(SL_ERR_ARG, "null batch");
+    h->b.give_up = barrier;
     return SL_OK;
 }
 

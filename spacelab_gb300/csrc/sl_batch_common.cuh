@@ -92,10 +92,11 @@ __device__ __forceinline__ void kick(const Batch& b, int inst, int off, int n, d
 // Waits until every CTA of the grid (all resident: a cooperative launch) has
 // arrived; `phase` counts the barriers.  Memory written before it by any CTA
 // is visible after it.  The wait is bounded: a CTA that gives up sets
-// `failed`, and every CTA then returns false.  Called by all threads.
+// `failed`, and every CTA then returns false.  Called by all threads.  Barrier
+// `give_up` (0: none) is one whose time has run out at once (diagnostics).
 constexpr long long kGridWaitCycles = 1ll << 33;  // about 4 s
 
-__device__ __forceinline__ bool grid_sync(GridSync* g, unsigned long long& phase)
+__device__ __forceinline__ bool grid_sync(GridSync* g, unsigned long long& phase, unsigned give_up)
 {
     __shared__ int s_ok;
     ++phase;
@@ -109,7 +110,7 @@ __device__ __forceinline__ bool grid_sync(GridSync* g, unsigned long long& phase
         volatile unsigned long long* released = &g->released;
         volatile unsigned* failed = &g->failed;
         while (*released < phase) {
-            if (*failed || clock64() - t0 > kGridWaitCycles) {
+            if (*failed || phase == give_up || clock64() - t0 > kGridWaitCycles) {
                 atomicExch(&g->failed, 1u);
                 ok = false;
                 break;

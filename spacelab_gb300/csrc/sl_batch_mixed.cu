@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(32 * kGridWarpsM, 1) batch_mixed_grid_kernel(c
         if (p < b.cnt[inst])
             drift_sphere(b, b.off[inst] + p, b.perm[b.off[inst] + p], do_init ? 0.0 : b.dt[inst]);
     }
-    if (!batch::grid_sync(b.gsync, phase)) return;
+    if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
     int rec = -1;  // the record whose parts the last rows phase left
     for (int q = q0; q < nsteps; ++q) {
         const int step = first_step + q, par = q & 1;
@@ -734,12 +734,12 @@ __global__ void __launch_bounds__(32 * kGridWarpsM, 1) batch_mixed_grid_kernel(c
             grid_pairs_mixed<true>(b, sm, b.gqueue + par, b.gpe + par * b.gtiles);
         else
             grid_pairs_mixed<false>(b, sm, b.gqueue + par, b.gpe + par * b.gtiles);
-        if (!batch::grid_sync(b.gsync, phase)) return;
+        if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
         if (blockIdx.x == 0 && threadIdx.x == 0) b.gqueue[par ^ 1] = 0;  // the next step's queue
         grid_rows_mixed(b, init, write, more);
         rec = !write ? -1 : init ? 0 : min(step / skip, b.nrec - 1);
         if (!more && rec < 0) break;
-        if (!batch::grid_sync(b.gsync, phase)) return;
+        if (!batch::grid_sync(b.gsync, phase, b.give_up)) return;
         if (!more) grid_energy_mixed(b, b.gpe + par * b.gtiles, rec, sh);
     }
 }
