@@ -139,16 +139,60 @@ int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, i
 
 // The lockstep form's lists and scratch (pair terms and torques of every
 // instance, or the mixed form's partials), where they fit the budget: per
-// instance 48 npad^2 bytes exact, 24 nb npad bytes mixed.
+// instance 48 npad^2 bytes exact, 24 nb npad bytes mixed, and 16 bytes per tile.
+// The lists are made only for a batch that takes the form.
 int setup_lockstep(sl_batch* h, const std::vector<int>& order)
 {
     sl::Batch& b = h->b;
     const bool mixed = h->mode == SL_MODE_MIXED_DF;
     if (!sl::batch_grid_fits(mixed)) return SL_OK;
-    std::vector<long long> tiles(b.ninst + 1), blocks(b.ninst + 1), pair(b.ninst), mask(b.ninst);
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+    const size_t budget = std::min(kExactTileScratchBytes, free_b / 3);
+    long long ntiles = 0, nblocks = 0, np = 0, nm = 0;
+    for (int n : h->counts) {
+        const long long nb = (n + (long long)sl::kBlock - 1) / sl::kBlock, npad = nb * sl::kBlock;
+        ntiles += nb * (nb + 1) / 2;
+        nblocks += nb;
+        np += mixed ? 6 * nb * npad : 3 * npad * npad;
+        nm += mixed ? npad * ((nb + 31) / 32) : npad * nb;  // mixed: torque marks
+        if (np > (long long)(budget / sizeof(float))) return SL_OK;
+    }
+    const long long items = sl::batch_grid_items(ntiles, h->num_sms, mixed);
+    const size_t ni = (size_t)b.ninst;
+    size_t off = 0;
+    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
+    const size_t o_pair = take((size_t)np * (mixed ? sizeof(float) : sizeof(double))),
+                 o_torq = take(mixed ? 0 : (size_t)np * sizeof(double)), o_mask = take((size_t)nm * sizeof(uint32_t));
+    const size_t zeroed = off;  // the buffers' unwritten entries are read as +0.0
+    const size_t o_tiles = take((ni + 1) * sizeof(long long)), o_blocks = take((ni + 1) * sizeof(long long)),
+                 o_tile = take((size_t)ntiles * sizeof(int4)), o_poff = take(ni * sizeof(long long)),
+                 o_moff = take(ni * sizeof(long long)), o_binst = take((size_t)nblocks * sizeof(int)),
+                 o_blk = take((size_t)nblocks * sizeof(int)), o_views = take(mixed ? 0 : ni * sizeof(sl::System)),
+                 o_pe = take(2 * (size_t)items * sizeof(double)), o_ke = take((size_t)nblocks * 8 * sizeof(double)),
+                 o_sync = take(sizeof(sl::GridSync) + 2 * sizeof(int));
+    if (off > budget) return SL_OK;
+
+    std::vector<long long> tiles, blocks, pair, mask;
     std::vector<int> blk_inst, blk;
     std::vector<int4> tile;
-    long long np = 0, nm = 0;
+    try {
+        tiles.assign(ni + 1, 0);
+        blocks.assign(ni + 1, 0);
+        pair.resize(ni);
+        mask.resize(ni);
+        blk_inst.reserve((size_t)nblocks);
+        blk.reserve((size_t)nblocks);
+        tile.reserve((size_t)ntiles);
+    } catch (const std::bad_alloc&) {
+        return SL_OK;  // the per-CTA form runs instead
+    }
+    if (cudaMalloc(&h->grid_arena, off) != cudaSuccess) {
+        cudaGetLastError();
+        h->grid_arena = nullptr;
+        return SL_OK;
+    }
+    np = nm = 0;
     for (int k = 0; k < b.ninst; ++k) {
         const int inst = order[k], nb = (h->counts[inst] + sl::kBlock - 1) / sl::kBlock;
         const long long npad = (long long)nb * sl::kBlock;
@@ -162,27 +206,7 @@ int setup_lockstep(sl_batch* h, const std::vector<int>& order)
         pair[inst] = np;
         mask[inst] = nm;
         np += mixed ? 6 * nb * npad : 3 * npad * npad;
-        nm += mixed ? npad * ((nb + 31) / 32) : npad * nb;  // mixed: torque marks
-    }
-    const long long items = sl::batch_grid_items(tiles[b.ninst], h->num_sms, mixed);
-    size_t off = 0;
-    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-    const size_t o_pair = take((size_t)np * (mixed ? sizeof(float) : sizeof(double))),
-                 o_torq = take(mixed ? 0 : (size_t)np * sizeof(double)), o_mask = take((size_t)nm * sizeof(uint32_t));
-    size_t free_b = 0, total_b = 0;
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
-    if (off > std::min(kExactTileScratchBytes, free_b / 3)) return SL_OK;
-    const size_t zeroed = off;  // the buffers' unwritten entries are read as +0.0
-    const size_t o_tiles = take(tiles.size() * sizeof(long long)), o_blocks = take(blocks.size() * sizeof(long long)),
-                 o_tile = take(tile.size() * sizeof(int4)), o_poff = take(pair.size() * sizeof(long long)), o_moff = take(mask.size() * sizeof(long long)),
-                 o_binst = take(blk.size() * sizeof(int)), o_blk = take(blk.size() * sizeof(int)),
-                 o_views = take(mixed ? 0 : (size_t)b.ninst * sizeof(sl::System)),
-                 o_pe = take(2 * (size_t)items * sizeof(double)), o_ke = take(blk.size() * 8 * sizeof(double)),
-                 o_sync = take(sizeof(sl::GridSync) + 2 * sizeof(int));
-    if (cudaMalloc(&h->grid_arena, off) != cudaSuccess) {
-        cudaGetLastError();
-        h->grid_arena = nullptr;
-        return SL_OK;  // the per-CTA form runs instead
+        nm += mixed ? npad * ((nb + 31) / 32) : npad * nb;
     }
     char* p = static_cast<char*>(h->grid_arena);
     SLB_CUDA(cudaMemsetAsync(p, 0, zeroed, h->stream));
@@ -218,8 +242,8 @@ int setup_lockstep(sl_batch* h, const std::vector<int>& order)
     b.gsync = reinterpret_cast<sl::GridSync*>(p + o_sync);
     b.gqueue = reinterpret_cast<int*>(b.gsync + 1);
     h->mark_bytes = (size_t)nm * sizeof(uint32_t);
-    b.gtiles = tiles[b.ninst];
-    b.gblocks = (int)blocks[b.ninst];
+    b.gtiles = ntiles;
+    b.gblocks = (int)nblocks;
     b.grid = 1;
     return SL_OK;
 }
