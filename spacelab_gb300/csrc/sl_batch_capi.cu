@@ -248,6 +248,124 @@ int setup_lockstep(sl_batch* h, const std::vector<int>& order)
     return SL_OK;
 }
 
+// Gives the lockstep form's memory back; the batch runs its per-CTA form.
+void release_lockstep(sl_batch* h)
+{
+    sl::Batch& b = h->b;
+    cudaFree(h->grid_arena);
+    h->grid_arena = nullptr;
+    h->mark_bytes = 0;
+    b.grid = 0;
+    b.views = nullptr;
+    b.gpart = nullptr;
+    b.xpair = b.xtorq = nullptr;
+    b.xmask = nullptr;
+}
+
+// The batch's own memory: state, constants, records and the per-CTA scratch.
+int setup_arena(sl_batch* h, const std::vector<int>& ord)
+{
+    sl::Batch& b = h->b;
+    const bool mixed = h->mode == SL_MODE_MIXED_DF;
+    const int ninst = b.ninst;
+    const size_t T = (size_t)b.total;
+    size_t off = 0;
+    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
+    size_t o_vec[8][3], o_sc[8], o_f[10];
+    for (auto& v : o_vec)
+        for (auto& c : v) c = take(T * sizeof(double));
+    for (auto& s : o_sc) s = take(T * sizeof(double));
+    for (auto& f : o_f) f = take(mixed ? T * sizeof(float) : 0);
+    const size_t o_order = take(ninst * sizeof(int)), o_off = take(ninst * sizeof(int)),
+                 o_cnt = take(ninst * sizeof(int)), o_counter = take(sizeof(int));
+    const size_t o_par = take(4 * (size_t)ninst * sizeof(double));
+    const size_t o_en = take((size_t)ninst * b.nrec * 8 * sizeof(double));
+    const size_t o_st = take(ninst * sizeof(unsigned));
+    const size_t o_snap = take(15 * T * sizeof(double));
+    const size_t o_perm = take(mixed ? T * sizeof(int) : 0);
+    // mixed: the pair-tile pass's per-CTA partials, sized for the largest instance
+    const int max_n = *std::max_element(h->counts.begin(), h->counts.end());
+    b.part_nb = (max_n + sl::kBlock - 1) / sl::kBlock;
+    b.part_np = b.part_nb * sl::kBlock;
+    b.part_cta = 6 * (size_t)b.part_nb * b.part_np;
+    // no more CTAs than instances ever run at once
+    const long long max_ctas = std::min<long long>((long long)h->num_sms * sl::kTileCtasPerSm, ninst);
+    b.part_ctas = (int)max_ctas;
+    const size_t o_part = take(mixed ? b.part_cta * b.part_ctas * sizeof(float) : 0);
+    // exact: the pair-tile pass's per-CTA pair terms, torques and contact
+    // words at the largest instance's padded size, where that fits the
+    // budget for at least one CTA per SM
+    b.x_nb = b.part_nb;
+    b.x_np = b.part_np;
+    b.xpair_cta = 3 * (size_t)b.x_np * b.x_np;
+    b.xmask_cta = (size_t)b.x_np * b.x_nb;
+    size_t o_xpair = 0, o_xtorq = 0, o_xmask = 0;
+    bool exact_tiles = false;
+    if (!mixed && !b.grid) {
+        const size_t per_cta = 2 * b.xpair_cta * sizeof(double) + b.xmask_cta * sizeof(uint32_t);
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
+        const long long fit = (long long)(std::min(kExactTileScratchBytes, free_b / 3) / per_cta);
+        const long long ctas = std::min<long long>(max_ctas, fit);
+        if (ctas >= std::min<long long>(h->num_sms, ninst)) {
+            exact_tiles = true;
+            b.part_ctas = (int)ctas;
+            o_xpair = take(b.xpair_cta * ctas * sizeof(double));
+            o_xtorq = take(b.xpair_cta * ctas * sizeof(double));
+            o_xmask = take(b.xmask_cta * ctas * sizeof(uint32_t));
+        }
+    }
+    const size_t o_isc = take((size_t)ninst * sizeof(sl::Scalars));
+    h->arena_bytes = off;
+    if (cudaMalloc(&h->arena, off) != cudaSuccess) {
+        cudaGetLastError();
+        h->arena = nullptr;
+        return sl_record_error(SL_ERR_ALLOC, "cudaMalloc of the batch arena failed");
+    }
+    char* base = static_cast<char*>(h->arena);
+    sl::Vec3Soa* vecs[8] = {&b.pos, &b.prev, &b.vel, &b.velh, &b.w, &b.wh, &b.acc, &b.aacc};
+    for (int v = 0; v < 8; ++v)
+        for (int c = 0; c < 3; ++c) vecs[v]->c[c] = reinterpret_cast<double*>(base + o_vec[v][c]);
+    double* inv_m_slot = nullptr;  // 8 bytes per sphere, holds the mass reciprocals rm
+    double** scal[8] = {&b.R, &b.m, &b.moi, &b.twoR, &b.fourR, &b.cR3, &inv_m_slot, &b.inv_moi};
+    for (int k = 0; k < 8; ++k) *scal[k] = reinterpret_cast<double*>(base + o_sc[k]);
+    b.rm = reinterpret_cast<unsigned long long*>(inv_m_slot);
+    if (mixed) {
+        b.f_R = reinterpret_cast<float*>(base + o_f[0]);
+        b.f_inv_m = reinterpret_cast<float*>(base + o_f[1]);
+        b.f_inv_moi = reinterpret_cast<float*>(base + o_f[2]);
+        b.f_Rlo = reinterpret_cast<float*>(base + o_f[3]);
+        for (int k = 0; k < 6; ++k) b.f_pos[k] = reinterpret_cast<float*>(base + o_f[4 + k]);
+        b.perm = reinterpret_cast<const int*>(base + o_perm);
+        b.part = reinterpret_cast<float*>(base + o_part);
+    }
+    int* order = reinterpret_cast<int*>(base + o_order);
+    int* doff = reinterpret_cast<int*>(base + o_off);
+    int* dcnt = reinterpret_cast<int*>(base + o_cnt);
+    b.order = order; b.off = doff; b.cnt = dcnt;
+    b.counter = reinterpret_cast<int*>(base + o_counter);
+    double* par = reinterpret_cast<double*>(base + o_par);
+    b.dt = par; b.kin = par + ninst; b.kout = par + 2 * ninst; b.u_s = par + 3 * ninst;
+    b.energy = reinterpret_cast<double*>(base + o_en);
+    if (exact_tiles) {
+        b.xpair = reinterpret_cast<double*>(base + o_xpair);
+        b.xtorq = reinterpret_cast<double*>(base + o_xtorq);
+        b.xmask = reinterpret_cast<uint32_t*>(base + o_xmask);
+    }
+    b.isc = reinterpret_cast<sl::Scalars*>(base + o_isc);
+    b.status = reinterpret_cast<unsigned*>(base + o_st);
+    h->snapshot = reinterpret_cast<double*>(base + o_snap);
+    cudaError_t e = cudaMemsetAsync(h->arena, 0, off, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(order, ord.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(doff, h->offsets.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dcnt, h->counts.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
+    if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
+    return SL_OK;
+}
+
+
 // device-to-device copy of the 5 vec3 state arrays to/from the snapshot
 int snapshot_copy(sl_batch* h, bool save)
 {
@@ -357,105 +475,15 @@ int sl_batch_create(int ninst, const int* counts, const sl_material* mat, int mo
     std::vector<int> ord(ninst);
     std::iota(ord.begin(), ord.end(), 0);
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int c) { return counts[a] > counts[c]; });
-    if (int r = setup_lockstep(h, ord)) {
+    int r = setup_lockstep(h, ord);
+    if (r == SL_OK) r = setup_arena(h, ord);
+    if (r == SL_ERR_ALLOC && b.grid) {  // the memory that the lockstep form may do without
+        release_lockstep(h);
+        r = setup_arena(h, ord);
+    }
+    if (r) {
         sl_batch_destroy(h);
         return r;
-    }
-    const size_t T = (size_t)total;
-    size_t off = 0;
-    auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + bytes, 256); return o; };
-    size_t o_vec[8][3], o_sc[8], o_f[10];
-    for (auto& v : o_vec)
-        for (auto& c : v) c = take(T * sizeof(double));
-    for (auto& s : o_sc) s = take(T * sizeof(double));
-    for (auto& f : o_f) f = take(mode == SL_MODE_MIXED_DF ? T * sizeof(float) : 0);
-    const size_t o_order = take(ninst * sizeof(int)), o_off = take(ninst * sizeof(int)),
-                 o_cnt = take(ninst * sizeof(int)), o_counter = take(sizeof(int));
-    const size_t o_par = take(4 * (size_t)ninst * sizeof(double));
-    const size_t o_en = take((size_t)ninst * b.nrec * 8 * sizeof(double));
-    const size_t o_st = take(ninst * sizeof(unsigned));
-    const size_t o_snap = take(15 * T * sizeof(double));
-    const size_t o_perm = take(mode == SL_MODE_MIXED_DF ? T * sizeof(int) : 0);
-    // mixed: the pair-tile pass's per-CTA partials, sized for the largest instance
-    const int max_n = *std::max_element(counts, counts + ninst);
-    b.part_nb = (max_n + sl::kBlock - 1) / sl::kBlock;
-    b.part_np = b.part_nb * sl::kBlock;
-    b.part_cta = 6 * (size_t)b.part_nb * b.part_np;
-    // no more CTAs than instances ever run at once
-    const long long max_ctas = std::min<long long>((long long)h->num_sms * sl::kTileCtasPerSm, ninst);
-    b.part_ctas = (int)max_ctas;
-    const size_t o_part = take(mode == SL_MODE_MIXED_DF ? b.part_cta * b.part_ctas * sizeof(float) : 0);
-    // exact: the pair-tile pass's per-CTA pair terms, torques and contact
-    // words at the largest instance's padded size, where that fits the
-    // budget for at least one CTA per SM
-    b.x_nb = b.part_nb;
-    b.x_np = b.part_np;
-    b.xpair_cta = 3 * (size_t)b.x_np * b.x_np;
-    b.xmask_cta = (size_t)b.x_np * b.x_nb;
-    size_t o_xpair = 0, o_xtorq = 0, o_xmask = 0;
-    bool exact_tiles = false;
-    if (mode == SL_MODE_EXACT && !b.grid) {
-        const size_t per_cta = 2 * b.xpair_cta * sizeof(double) + b.xmask_cta * sizeof(uint32_t);
-        size_t free_b = 0, total_b = 0;
-        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
-        const long long fit = (long long)(std::min(kExactTileScratchBytes, free_b / 3) / per_cta);
-        const long long ctas = std::min<long long>(max_ctas, fit);
-        if (ctas >= std::min<long long>(h->num_sms, ninst)) {
-            exact_tiles = true;
-            b.part_ctas = (int)ctas;
-            o_xpair = take(b.xpair_cta * ctas * sizeof(double));
-            o_xtorq = take(b.xpair_cta * ctas * sizeof(double));
-            o_xmask = take(b.xmask_cta * ctas * sizeof(uint32_t));
-        }
-    }
-    const size_t o_isc = take((size_t)ninst * sizeof(sl::Scalars));
-    h->arena_bytes = off;
-    if (cudaMalloc(&h->arena, off) != cudaSuccess) {
-        sl_batch_destroy(h);
-        return sl_record_error(SL_ERR_ALLOC, "cudaMalloc of the batch arena failed");
-    }
-    char* base = static_cast<char*>(h->arena);
-    sl::Vec3Soa* vecs[8] = {&b.pos, &b.prev, &b.vel, &b.velh, &b.w, &b.wh, &b.acc, &b.aacc};
-    for (int v = 0; v < 8; ++v)
-        for (int c = 0; c < 3; ++c) vecs[v]->c[c] = reinterpret_cast<double*>(base + o_vec[v][c]);
-    double* inv_m_slot = nullptr;  // 8 bytes per sphere, holds the mass reciprocals rm
-    double** scal[8] = {&b.R, &b.m, &b.moi, &b.twoR, &b.fourR, &b.cR3, &inv_m_slot, &b.inv_moi};
-    for (int k = 0; k < 8; ++k) *scal[k] = reinterpret_cast<double*>(base + o_sc[k]);
-    b.rm = reinterpret_cast<unsigned long long*>(inv_m_slot);
-    if (mode == SL_MODE_MIXED_DF) {
-        b.f_R = reinterpret_cast<float*>(base + o_f[0]);
-        b.f_inv_m = reinterpret_cast<float*>(base + o_f[1]);
-        b.f_inv_moi = reinterpret_cast<float*>(base + o_f[2]);
-        b.f_Rlo = reinterpret_cast<float*>(base + o_f[3]);
-        for (int k = 0; k < 6; ++k) b.f_pos[k] = reinterpret_cast<float*>(base + o_f[4 + k]);
-        b.perm = reinterpret_cast<const int*>(base + o_perm);
-        b.part = reinterpret_cast<float*>(base + o_part);
-    }
-    int* order = reinterpret_cast<int*>(base + o_order);
-    int* doff = reinterpret_cast<int*>(base + o_off);
-    int* dcnt = reinterpret_cast<int*>(base + o_cnt);
-    b.order = order; b.off = doff; b.cnt = dcnt;
-    b.counter = reinterpret_cast<int*>(base + o_counter);
-    double* par = reinterpret_cast<double*>(base + o_par);
-    b.dt = par; b.kin = par + ninst; b.kout = par + 2 * ninst; b.u_s = par + 3 * ninst;
-    b.energy = reinterpret_cast<double*>(base + o_en);
-    if (exact_tiles) {
-        b.xpair = reinterpret_cast<double*>(base + o_xpair);
-        b.xtorq = reinterpret_cast<double*>(base + o_xtorq);
-        b.xmask = reinterpret_cast<uint32_t*>(base + o_xmask);
-    }
-    b.isc = reinterpret_cast<sl::Scalars*>(base + o_isc);
-    b.status = reinterpret_cast<unsigned*>(base + o_st);
-    h->snapshot = reinterpret_cast<double*>(base + o_snap);
-    cudaError_t e = cudaMemsetAsync(h->arena, 0, off, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(order, ord.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(doff, h->offsets.data(), ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dcnt, counts, ninst * sizeof(int), cudaMemcpyHostToDevice, h->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    if (e != cudaSuccess) {
-        sl_batch_destroy(h);
-        return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
     }
     *out = h;
     return SL_OK;

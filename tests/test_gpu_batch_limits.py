@@ -5,7 +5,12 @@ import subprocess
 import sys
 from pathlib import Path
 
+import numpy as np
 import pytest
+
+from cases import contact_case
+from spacelab_gb300 import BallGroup
+from spacelab_gb300 import batch as B
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +40,42 @@ def test_a_large_system_makes_no_tile_lists():
     out = subprocess.run([sys.executable, "-c", CREATE.format(root=str(ROOT))], stdout=subprocess.PIPE, text=True,
                          timeout=300, check=True).stdout
     assert int(out) < 64 * 1024, out  # KB
+
+
+def _collision(n, seed):
+    c = contact_case(n, seed)
+    col = B.Collision(n, 0, 0.0, 0.0, 0.6, 0.3, seed)
+    col.group = BallGroup.from_arrays(c["pos"], c["vel"], c["w"], c["R"], c["m"], c["moi"])
+    col.dt, col.kin, col.kout = c["dt"], c["kin"], c["kout"]
+    return col
+
+
+def _two_steps(cols, steps):
+    run = B.BatchRun(cols, "mixed_df", steps=steps, skip=1)
+    try:
+        run.set_shape(0, 512)
+        run.run(1, 2, do_init=True)
+        return run.shape()[2], run.state()
+    finally:
+        run.close()
+
+
+def test_the_required_memory_comes_first():
+    """One system of 30,000 spheres: 0.68 GB for lockstep, as much for a CTA's
+    partials.  4 GB are left free, and energy records are asked for that leave
+    0.4 GB of them."""
+    torch = pytest.importorskip("torch")
+    cols = [_collision(30000, 3)]
+    blocks, want = _two_steps(cols, 2)
+    assert blocks > 1  # lockstep, with room
+    left = 4 << 30
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - left, dtype=torch.uint8, device="cuda")
+    try:
+        part = 24 * 938 * 938 * 32
+        blocks, got = _two_steps(cols, (left - part - (400 << 20)) // 64)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert blocks == 1  # an instance per CTA
+    for k in want:
+        assert np.array_equal(got[k], want[k]), k
