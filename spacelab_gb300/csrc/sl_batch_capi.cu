@@ -72,12 +72,16 @@ namespace {
 // largest instance alone, at the shape's warps, would last 1.25 times an even
 // share (64 of up to 2400 spheres 0.92 / 0.20; 512 of them at 128, 256, 512
 // threads 3.30, 1.89, 1.03 / 1.14; 2048 at 128, 512: 4.68, 4.29 / 4.65).
+bool uneven(int largest_nb, long long tiles, int num_sms, int threads)
+{
+    const double largest = (double)largest_nb * (largest_nb + 1) / 2;
+    return largest * num_sms * 16.0 / (threads / 32) >= 1.25 * (double)tiles;
+}
+
 bool runs_in_lockstep(const sl_batch* h, int tile, int threads)
 {
     if (tile != 0 || !h->b.grid) return false;
-    if (h->mode == SL_MODE_EXACT) return true;
-    const double largest = (double)h->b.part_nb * (h->b.part_nb + 1) / 2;
-    return largest * h->num_sms * 16.0 / (threads / 32) >= 1.25 * (double)h->b.gtiles;
+    return h->mode == SL_MODE_EXACT || uneven(h->b.part_nb, h->b.gtiles, h->num_sms, threads);
 }
 
 int blocks_for(const sl_batch* h, int tile, int threads)
@@ -140,7 +144,9 @@ int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, i
 // The lockstep form's lists and scratch (pair terms and torques of every
 // instance, or the mixed form's partials), where they fit the budget: per
 // instance 48 npad^2 bytes exact, 24 nb npad bytes mixed, and 16 bytes per tile.
-// The lists are made only for a batch that takes the form.
+// The lists are made only for a batch that takes the form, and in the mixed form
+// the memory is taken only where some shape does: at the fewest threads (the
+// configuration's 4096 collisions held several GB that no shape used).
 int setup_lockstep(sl_batch* h, const std::vector<int>& order)
 {
     sl::Batch& b = h->b;
@@ -149,15 +155,17 @@ int setup_lockstep(sl_batch* h, const std::vector<int>& order)
     size_t free_b = 0, total_b = 0;
     if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) free_b = 0;
     const size_t budget = std::min(kExactTileScratchBytes, free_b / 3);
-    long long ntiles = 0, nblocks = 0, np = 0, nm = 0;
+    long long ntiles = 0, nblocks = 0, np = 0, nm = 0, largest = 0;
     for (int n : h->counts) {
         const long long nb = (n + (long long)sl::kBlock - 1) / sl::kBlock, npad = nb * sl::kBlock;
         ntiles += nb * (nb + 1) / 2;
         nblocks += nb;
+        largest = std::max(largest, nb);
         np += mixed ? 6 * nb * npad : 3 * npad * npad;
         nm += mixed ? npad * ((nb + 31) / 32) : npad * nb;  // mixed: torque marks
         if (np > (long long)(budget / sizeof(float))) return SL_OK;
     }
+    if (mixed && !uneven((int)largest, ntiles, h->num_sms, kThreads[0])) return SL_OK;
     const long long items = sl::batch_grid_items(ntiles, h->num_sms, mixed);
     const size_t ni = (size_t)b.ninst;
     size_t off = 0;

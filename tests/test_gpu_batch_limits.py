@@ -79,3 +79,21 @@ def test_the_required_memory_comes_first():
     assert blocks == 1  # an instance per CTA
     for k in want:
         assert np.array_equal(got[k], want[k]), k
+
+
+def test_even_mixed_batches_hold_no_lockstep_memory():
+    """4096 systems of 300 spheres: 0.56 GB of state and partials; lockstep,
+    which they never take, would be 0.31 GB more."""
+    torch = pytest.importorskip("torch")
+    cols = [_collision(300, 3)] * 4096
+    B.BatchRun(cols[:1], "mixed_df", steps=2, skip=1).close()  # the context's own memory
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    run = B.BatchRun(cols, "mixed_df", steps=2, skip=1)
+    held = free - torch.cuda.mem_get_info()[0]
+    run.set_shape(0, 64)
+    assert run.shape()[2] > 152  # an instance per CTA, at the fewest threads too
+    run.close()
+    state = 4096 * 300 * (24 * 8 + 8 * 8 + 15 * 8 + 10 * 4 + 4)
+    partials = 608 * 6 * 10 * 320 * 4
+    assert held < state + partials + (100 << 20), held
