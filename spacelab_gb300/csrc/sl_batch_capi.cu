@@ -591,7 +591,7 @@ int sl_batch_autotune(sl_batch* h, int sample_steps, int* tile, int* threads, do
     cudaEvent_t e0, e1;
     SLB_CUDA(cudaEventCreate(&e0));
     SLB_CUDA(cudaEventCreate(&e1));
-    float best = 1e30f;
+    float best = 1e30f, lockstep_ms = -1.0f;  // lockstep is one form at any threads: timed once
     int bt = h->tile, bth = h->threads, k = 0;
     for (int ti = 0; ti < 4; ++ti)
         for (int hi = 0; hi < 3; ++hi, ++k) {
@@ -600,8 +600,13 @@ int sl_batch_autotune(sl_batch* h, int sample_steps, int* tile, int* threads, do
                 if (times_ms) times_ms[k] = -1.0;
                 continue;
             }
-            if (int r = snapshot_copy(h, false)) return r;
             const int thr = kTiles[ti] == 0 && mixed ? kThreadsTiles[hi] : kThreads[hi];
+            const bool lockstep = runs_in_lockstep(h, kTiles[ti], thr);
+            if (lockstep && lockstep_ms >= 0) {
+                if (times_ms) times_ms[k] = lockstep_ms;
+                continue;
+            }
+            if (int r = snapshot_copy(h, false)) return r;
             // first launch compiles nothing but warms the caches; time the second
             if (int r = launch_run(h, kTiles[ti], thr, 1, 1, 0, 0)) return r;
             cudaEventRecord(e0, h->stream);
@@ -611,6 +616,7 @@ int sl_batch_autotune(sl_batch* h, int sample_steps, int* tile, int* threads, do
             float ms = 0;
             cudaEventElapsedTime(&ms, e0, e1);
             if (times_ms) times_ms[k] = ms;
+            if (lockstep) lockstep_ms = ms;
             if (ms < best) { best = ms; bt = kTiles[ti]; bth = thr; }
         }
     cudaEventDestroy(e0);
