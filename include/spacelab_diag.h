@@ -60,6 +60,10 @@ int sl_diag_gemm_bf16(int M, int N, int K, const uint16_t* A, const uint16_t* B,
  * its time had run out; the run then returns SL_ERR_TIMEOUT. */
 int sl_diag_batch_give_up(sl_batch* b, unsigned barrier);
 
+/* The batch's lockstep launches are refused from here on, as where the process
+ * has fewer SMs than the form takes: the next run changes to the per-CTA form. */
+int sl_diag_batch_refuse_lockstep(sl_batch* b);
+
 #ifdef __cplusplus
 }
 #endif

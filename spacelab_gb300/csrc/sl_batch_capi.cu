@@ -57,7 +57,9 @@ struct sl_batch {
     bool uploaded = false;
     std::vector<int> counts, offsets;
     void* grid_arena = nullptr;  // the lockstep form's scratch and lists
+    size_t pair_terms = 0;       // doubles of b.xpair there (exact)
     size_t mark_bytes = 0;       // of b.xmask there
+    bool refuse_lockstep = false;  // diagnostics: lockstep launches are refused
 };
 
 namespace {
@@ -95,39 +97,46 @@ int blocks_for(const sl_batch* h, int tile, int threads)
     return (int)blocks;
 }
 
+// The device has no room for all CTAs of a cooperative launch at once, or does
+// not know such launches.
+bool refuses(cudaError_t e) { return e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported; }
+
 // One persistent launch over all instances, captured as a CUDA graph
-// (queue reset + kernel) and launched.
-int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, int do_init, int skip)
+// (queue reset + kernel) and launched.  A lockstep launch that the device
+// refuses sets *refused; nothing has run then.
+int launch_form(sl_batch* h, bool lockstep, int tile, int threads, int first_step, int nsteps, int do_init, int skip,
+                bool* refused)
 {
     const int blocks = blocks_for(h, tile, threads);
-    cudaGraph_t g;
+    cudaGraph_t g = nullptr;
     SLB_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(h->b.counter, 0, sizeof(int), h->stream);
-    const bool lockstep = runs_in_lockstep(h, tile, threads);
-    cudaError_t launched = cudaSuccess;
+    cudaError_t e = cudaSuccess;
     if (lockstep) {
         cudaMemsetAsync(h->b.gsync, 0, sizeof(sl::GridSync) + 2 * sizeof(int), h->stream);  // and the queues behind it
-        launched = h->mode == SL_MODE_MIXED_DF
-                       ? sl::launch_batch_mixed_grid(h->b, h->num_sms, first_step, nsteps, skip, do_init, h->stream)
-                       : sl::launch_batch_exact_grid(h->b, h->num_sms, first_step, nsteps, skip, do_init, h->stream);
+        e = h->refuse_lockstep ? cudaErrorCooperativeLaunchTooLarge
+            : h->mode == SL_MODE_MIXED_DF
+                ? sl::launch_batch_mixed_grid(h->b, h->num_sms, first_step, nsteps, skip, do_init, h->stream)
+                : sl::launch_batch_exact_grid(h->b, h->num_sms, first_step, nsteps, skip, do_init, h->stream);
     } else if (h->mode == SL_MODE_MIXED_DF)
         sl::launch_batch_mixed(h->b, tile, threads, blocks, first_step, nsteps, skip, do_init, h->stream);
     else
         sl::launch_batch_exact(h->b, tile, threads, blocks, first_step, nsteps, skip, do_init, h->stream);
-    SLB_CUDA(cudaStreamEndCapture(h->stream, &g));
-    if (launched != cudaSuccess) {
-        cudaGraphDestroy(g);
-        return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(launched));
+    const cudaError_t captured = cudaStreamEndCapture(h->stream, &g);
+    if (e == cudaSuccess) e = captured;
+    cudaGraphExec_t ge = nullptr;
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&ge, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (e == cudaSuccess) e = cudaGraphLaunch(ge, h->stream);
+    const cudaError_t done = cudaStreamSynchronize(h->stream);
+    if (ge) cudaGraphExecDestroy(ge);
+    if (lockstep && refuses(e)) {
+        cudaGetLastError();
+        *refused = true;
+        return SL_OK;
     }
-    cudaGraphExec_t ge;
-    const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
-    cudaGraphDestroy(g);
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e));
-    const cudaError_t e2 = cudaGraphLaunch(ge, h->stream);
-    const cudaError_t e3 = cudaStreamSynchronize(h->stream);
-    cudaGraphExecDestroy(ge);
-    if (e2 != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e2));
-    if (e3 != cudaSuccess) return sl_record_error(SL_ERR_CUDA, cudaGetErrorString(e3));
     if (lockstep) {
         sl::GridSync gs{};
         SLB_CUDA(cudaMemcpy(&gs, h->b.gsync, sizeof gs, cudaMemcpyDeviceToHost));
@@ -139,6 +148,45 @@ int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, i
         }
     }
     return SL_OK;
+}
+
+// Gives the lockstep form's memory back; the batch runs its per-CTA form.
+void release_lockstep(sl_batch* h)
+{
+    sl::Batch& b = h->b;
+    cudaFree(h->grid_arena);
+    h->grid_arena = nullptr;
+    h->mark_bytes = 0;
+    b.grid = 0;
+    b.views = nullptr;
+    b.gpart = nullptr;
+    b.xpair = b.xtorq = nullptr;
+    b.xmask = nullptr;
+}
+
+// The per-CTA form from here on.  The exact form's per-CTA buffers are cut from
+// those of all instances, which hold the largest instance's at least once.
+void leave_lockstep(sl_batch* h)
+{
+    sl::Batch& b = h->b;
+    if (h->mode == SL_MODE_MIXED_DF) {
+        release_lockstep(h);
+        return;
+    }
+    b.grid = 0;
+    b.views = nullptr;
+    b.part_ctas = (int)std::min({(size_t)b.part_ctas, h->pair_terms / b.xpair_cta,
+                                 h->mark_bytes / sizeof(uint32_t) / b.xmask_cta});
+}
+
+int launch_run(sl_batch* h, int tile, int threads, int first_step, int nsteps, int do_init, int skip)
+{
+    bool refused = false;
+    const int r = launch_form(h, runs_in_lockstep(h, tile, threads), tile, threads, first_step, nsteps, do_init, skip,
+                              &refused);
+    if (!refused) return r;
+    leave_lockstep(h);
+    return launch_form(h, false, tile, threads, first_step, nsteps, do_init, skip, &refused);
 }
 
 // The lockstep form's lists and scratch (pair terms and torques of every
@@ -249,25 +297,12 @@ int setup_lockstep(sl_batch* h, const std::vector<int>& order)
     b.gke = reinterpret_cast<double*>(p + o_ke);
     b.gsync = reinterpret_cast<sl::GridSync*>(p + o_sync);
     b.gqueue = reinterpret_cast<int*>(b.gsync + 1);
+    h->pair_terms = (size_t)np;
     h->mark_bytes = (size_t)nm * sizeof(uint32_t);
     b.gtiles = ntiles;
     b.gblocks = (int)nblocks;
     b.grid = 1;
     return SL_OK;
-}
-
-// Gives the lockstep form's memory back; the batch runs its per-CTA form.
-void release_lockstep(sl_batch* h)
-{
-    sl::Batch& b = h->b;
-    cudaFree(h->grid_arena);
-    h->grid_arena = nullptr;
-    h->mark_bytes = 0;
-    b.grid = 0;
-    b.views = nullptr;
-    b.gpart = nullptr;
-    b.xpair = b.xtorq = nullptr;
-    b.xmask = nullptr;
 }
 
 // The batch's own memory: state, constants, records and the per-CTA scratch.
@@ -717,6 +752,13 @@ int sl_diag_batch_give_up(sl_batch* h, unsigned barrier)
 {
     if (!h) return sl_record_error(SL_ERR_ARG, "null batch");
     h->b.give_up = barrier;
+    return SL_OK;
+}
+
+int sl_diag_batch_refuse_lockstep(sl_batch* h)
+{
+    if (!h) return sl_record_error(SL_ERR_ARG, "null batch");
+    h->refuse_lockstep = true;
     return SL_OK;
 }
 
