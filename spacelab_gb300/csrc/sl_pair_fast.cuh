@@ -157,6 +157,9 @@ SL_PF_FN void check_range(Flags& fl, int e)
     fl.range |= (uint32_t)(e + (int)(SPAN / 2 - 1)) & ~(SPAN - 1);
 }
 
+// Whether two coordinates are equal up to their signs (zeros of both signs are)
+SL_PF_FN bool equal(double x, double y) { return ((bits_of(x) ^ bits_of(y)) << 1) == 0; }
+
 // An estimate H in [2^62, 2^64) of value H 2^(e - 63), normalised and rounded
 // to nearest at bit 11.  The exact value lies in (H - BELOW, H + ABOVE) after
 // normalisation, so only dropped bits in [1024 - ABOVE, 1024 + BELOW] leave
@@ -277,6 +280,7 @@ SL_PF_FN bool in_range(const Sphere& p)
     const int er = unpack(p.R).e;
     return er > -120 && er < 120 && p.em > -200 && p.em < 200;
 }
+SL_PF_FN bool is_zero(double x) { return (bits_of(x) << 1) == 0; }
 SL_PF_FN bool in_range_cR3(double cR3)
 {
     const int e = unpack(cR3).e;
@@ -303,21 +307,33 @@ struct Pair {
 // takes some 20 instructions of four schedulers: with all of these operations
 // on the FP64 pipe it was 95% busy, at 37% of the issue slots.
 // overlap is valid whenever `fl` is sure (contact: overlap > 0).
-template <bool UNI>
+//
+// ZEROS: a component of r may be zero (spheres in a plane or on a grid), and cR3
+// (no cohesion).  A zero's square and force are zeros, the force's with its
+// sign; a one takes its place in the operations, and says nothing.  Without it a
+// zero component raises the range flag.  It costs some thirty instructions a
+// pair, so the tiles take it only where they meet such pairs.
+template <bool UNI, bool ZEROS = false>
 SL_PF_FN Pair pair_terms(double rx, double ry, double rz, const Sphere& A, const Sphere& B, const Uniform& u,
                          long long h_min_bits)
 {
     Pair o;
     Flags fl;
     const double r[3] = {rx, ry, rz};
+    const Sig one{0x8000000000000000ull, 0};
+    const bool none = ZEROS && is_zero(A.cR3);
     Sig sr[3];
     double sq[3];
+    bool zero[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        sr[c] = unpack(r[c]);
+        zero[c] = ZEROS && is_zero(r[c]);
+        sr[c] = zero[c] ? one : unpack(r[c]);
         check_range<256>(fl, sr[c].e);
         sq[c] = pack(mul(sr[c], sr[c], fl), 0);
+        if (zero[c]) sq[c] = 0.0;
     }
+    if (ZEROS && zero[0] && zero[1] && zero[2]) fl.range = 1;
     const Root root = root_sig(sq[0] + sq[1] + sq[2], fl);             // :107
     o.overlap = (UNI ? u.sum : A.R + B.R) - pack(root.d, 0);           // :104, :110
     u64 hb = bits_of(o.overlap) & 0x7fffffffffffffffull;               // :211-215
@@ -328,14 +344,14 @@ SL_PF_FN Pair pair_terms(double rx, double ry, double rz, const Sphere& A, const
     const double h2 = pack(mul(sh, sh, fl), 0);
     const double tb = pack(mul(Sig{B.sR.m, B.sR.e + 1}, sh, fl), 0);  // (2 R[B]) h
     double S, T;
-    Sig P = u.P;
+    Sig P = none ? one : u.P;
     if (UNI) {
         S = h2 + tb + tb;
         T = S + u.c4;
     } else {
         S = h2 + pack(mul(Sig{A.sR.m, A.sR.e + 1}, sh, fl), 0) + tb;
         T = S + pack(mul(Sig{A.sR.m, A.sR.e + 2}, B.sR, fl), 0);
-        P = mul(mul(mul(unpack(A.cR3), B.sR, fl), B.sR, fl), B.sR, fl);
+        P = mul(mul(mul(none ? one : unpack(A.cR3), B.sR, fl), B.sR, fl), B.sR, fl);
     }
     const Sig coef = vdw_coef(P, o.h + A.R + B.R, S, T, fl);           // :221-225
     // the significands hold magnitudes: a negative Ha (repulsion) turns the signs
@@ -343,11 +359,15 @@ SL_PF_FN Pair pair_terms(double rx, double ry, double rz, const Sphere& A, const
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const uint32_t sign = ((uint32_t)(bits_of(r[c]) >> 32) & 0x80000000u) ^ csign;
-        const Sig F = mul(coef, div_root(sr[c], root.rec, root.d.e, fl), fl);  // :227
-        o.ta[c] = pack(div_fixed(F, A.rm, A.em, fl), sign);            // :249
+        // alone beside two zeros: RN(sqrt(RN(x x))) = |x|, a quotient of one
+        const bool unit = ZEROS && (zero[c] || (zero[(c + 1) % 3] && zero[(c + 2) % 3]));
+        const Sig n = unit ? one : div_root(sr[c], root.rec, root.d.e, fl);
+        const Sig F = mul(coef, n, fl);                                // :227
+        const bool nil = none || zero[c];
+        o.ta[c] = nil ? from_bits((u64)sign << 32) : pack(div_fixed(F, A.rm, A.em, fl), sign);  // :249
         // -(F/m[B]), :250; equal masses: RN(-x) = -RN(x)
-        o.tb[c] = UNI ? from_bits(bits_of(o.ta[c]) ^ 0x8000000000000000ull)
-                      : pack(div_fixed(F, B.rm, B.em, fl), sign ^ 0x80000000u);
+        o.tb[c] = UNI || nil ? from_bits(bits_of(o.ta[c]) ^ 0x8000000000000000ull)
+                             : pack(div_fixed(F, B.rm, B.em, fl), sign ^ 0x80000000u);
     }
     o.fl = fl;
     return o;

@@ -237,7 +237,7 @@ __device__ __forceinline__ double strip_potentials(const System& s, TileScratch&
 // ROWS rows at a time (1, 2 or 4): their chains side by side, where a warp has
 // its SM sub-partition to itself.  Rows past a1 are computed from the block's
 // padding and dropped.
-template <int PE, bool UNI, int ROWS>
+template <int PE, bool UNI, int ROWS, bool ZEROS>
 __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                             double bx, double by, double bz, const pf::Sphere& sb,
                                             const pf::Uniform& un, bool bvalid, double& pe, uint32_t& marked,
@@ -266,7 +266,7 @@ __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, in
                 sa.rm = ab.rm[a];
                 sa.em = pf::unpack(ab.m[a]).e;
             }
-            prs[k] = pf::pair_terms<UNI>(bx - ab.x[a], by - ab.y[a], bz - ab.z[a], sa, sb, un, h_min_bits);
+            prs[k] = pf::pair_terms<UNI, ZEROS>(bx - ab.x[a], by - ab.y[a], bz - ab.z[a], sa, sb, un, h_min_bits);
         }
 #pragma unroll
         for (int k = 0; k < ROWS; ++k) {
@@ -324,6 +324,40 @@ __device__ __forceinline__ void sweep_pairs(const System& s, TileScratch& ws, in
     }
 }
 
+// Sphere i as a pair's B
+__device__ __forceinline__ pf::Sphere column_sphere(const System& s, int i)
+{
+    const double R = s.R[i];
+    return {R, pf::unpack(R), s.cR3[i], s.rm[i], pf::unpack(s.m[i]).e};
+}
+
+// The constants of a tile of one radius and one mass
+__device__ __forceinline__ pf::Uniform tile_uniform(const ABlock& ab)
+{
+    const double R = ab.R[0];
+    return {R + R, ab.fourR[0] * R, pf::unpack(ab.cR3[0] * R * R * R)};
+}
+
+// The sweep in the ZEROS form, out of line, so that the plain one's code stays as
+// it is.  Systems that need it throughout (us per step, the general path for
+// every such pair / here): in a plane N=1000 228 / 118, N=5000 2832 / 987; no
+// cohesion N=1000 278 / 125, N=5000 3888 / 1039; a cubic lattice N=5000 1426 / 947.
+struct Swept {
+    double pe;
+    uint32_t marked, near;
+};
+
+template <int PE, bool UNI>
+__device__ __noinline__ Swept sweep_zeros(const System& s, TileScratch& ws, int X, int Y, int a0, int a1)
+{
+    const int lane = threadIdx.x & 31, B = Y * kBlock + lane, iB = min(B, s.n - 1);
+    const pf::Uniform un = UNI ? tile_uniform(ws.ab) : pf::Uniform{0.0, 0.0, {0, 0}};
+    Swept o{0.0, 0, 0};
+    sweep_pairs<PE, UNI, 1, true>(s, ws, X, Y, lane, a0, a1, s.pos.c[0][iB], s.pos.c[1][iB], s.pos.c[2][iB],
+                                  column_sphere(s, iB), un, B < s.n, o.pe, o.marked, o.near);
+    return o;
+}
+
 // Loads sphere i into lane's place of the A block.
 __device__ __forceinline__ void load_a(const System& s, ABlock& ab, int lane, int i)
 {
@@ -333,8 +367,8 @@ __device__ __forceinline__ void load_a(const System& s, ABlock& ab, int lane, in
 }
 
 // Partners a0 .. a1 - 1 of the tile (X, Y), the A block loaded: the sweep, or
-// where a constant leaves the integer path's range (no cohesion: cR3 = 0;
-// masses far from 1) the general path for every pair, then the marked pairs.
+// where a constant leaves the integer path's range (masses or strengths far
+// from 1) the general path for every pair, then the marked pairs.
 template <int PE, int ROWS = 1>
 __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int X, int Y, int lane, int a0, int a1,
                                            int iB, bool bvalid, double& pe, uint32_t& rowbits, uint32_t& colbits)
@@ -342,26 +376,41 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
     const ABlock& ab = ws.ab;
     const double bx = s.pos.c[0][iB], by = s.pos.c[1][iB], bz = s.pos.c[2][iB];
     const double Rb = s.R[iB], mb = s.m[iB];
-    const pf::Sphere sb{Rb, pf::unpack(Rb), s.cR3[iB], s.rm[iB], pf::unpack(mb).e};
+    const pf::Sphere sb = column_sphere(s, iB);
     const bool areal = X * kBlock + lane < s.n;  // padding takes no part in a pair
     const pf::Sphere sa{ab.R[lane], pf::unpack(ab.R[lane]), ab.cR3[lane], 0, pf::unpack(ab.m[lane]).e};
-    const bool sane = __all_sync(0xffffffffu, (!areal || (pf::in_range(sa) && pf::in_range_cR3(sa.cR3))) &&
+    const bool cohesive = !pf::is_zero(s.mat.Ha);  // cR3 = 0 otherwise
+    const bool sane = __all_sync(0xffffffffu, (!areal || (pf::in_range(sa) && (!cohesive || pf::in_range_cR3(sa.cR3)))) &&
                                                   (!bvalid || pf::in_range(sb)));
     // equality on the bit patterns (R, m > 0)
     const auto same = [](double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); };
     const double R0 = ab.R[0], m0 = ab.m[0];
     const bool uni = __all_sync(0xffffffffu, (!areal || (same(sa.R, R0) && same(ab.m[lane], m0))) &&
                                                  (!bvalid || (same(Rb, R0) && same(mb, m0))));
+    // The ZEROS form: without cohesion, or where the last row meets a zero
+    // displacement component (spheres in a plane or on a grid).  Either form is
+    // right for any row: a pair that the plain one does not settle takes the general
+    // path.  One row stands for the tile because a vote in every row cost the other
+    // systems up to 9% (N=5000, host step 705 -> 769 us; 709 here).
+    const int last = max(a1 - 1, 0);
+    const bool odd = __any_sync(0xffffffffu, !cohesive || (bvalid && (X != Y || lane < last) &&
+                                                           (pf::equal(bx, ab.x[last]) || pf::equal(by, ab.y[last]) ||
+                                                            pf::equal(bz, ab.z[last]))));
     uint32_t marked = 0, near = 0;
     if (!sane) {
         const uint32_t all = (a1 >= 32 ? ~0u : (1u << a1) - 1u) & ~((1u << a0) - 1u);
         marked = bvalid ? (X != Y ? all : all & ~((2u << lane) - 1u)) : 0u;
+    } else if (odd) {
+        const Swept o = uni ? sweep_zeros<PE, true>(s, ws, X, Y, a0, a1) : sweep_zeros<PE, false>(s, ws, X, Y, a0, a1);
+        pe += o.pe;
+        marked = o.marked;
+        near = o.near;
     } else if (uni) {
-        const pf::Uniform un{R0 + R0, ab.fourR[0] * R0, pf::unpack(ab.cR3[0] * R0 * R0 * R0)};
-        sweep_pairs<PE, true, ROWS>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
+        const pf::Uniform un = tile_uniform(ab);
+        sweep_pairs<PE, true, ROWS, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     } else {
         const pf::Uniform un{0.0, 0.0, {0, 0}};
-        sweep_pairs<PE, false, ROWS>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
+        sweep_pairs<PE, false, ROWS, false>(s, ws, X, Y, lane, a0, a1, bx, by, bz, sb, un, bvalid, pe, marked, near);
     }
     if (PE == kPeInline && __any_sync(0xffffffffu, near != 0u)) pe += near_potentials(s, ws, X, Y, near);
     rowbits = colbits = 0;

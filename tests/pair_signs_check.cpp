@@ -1,6 +1,7 @@
 // Host check of the exact pair force's integer path (sl_pair_fast.cuh) for
-// vdW coefficients of both signs: unflagged results against the reference's
-// expressions in IEEE doubles.  Prints "<case> <cases> <flagged>" and
+// vdW coefficients of both signs and, in the ZEROS form, zero coefficients and
+// displacement components: unflagged results against the reference's
+// expressions in IEEE doubles, signs of zeros too.  Prints "<case> <cases> <flagged>" and
 // "mismatches N".
 #include "sl_pair_fast.cuh"
 
@@ -78,10 +79,16 @@ static Pair plain(const double r[3], const Sphere& A, const Sphere& B, const Uni
     return pair_terms<UNI>(r[0], r[1], r[2], A, B, un, hm);
 }
 
+template <bool UNI>
+static Pair zeros(const double r[3], const Sphere& A, const Sphere& B, const Uniform& un, long long hm)
+{
+    return pair_terms<UNI, true>(r[0], r[1], r[2], A, B, un, hm);
+}
+
 int main(int argc, char** argv)
 {
     const long n = argc > 1 ? atol(argv[1]) : 100000;
-    Count repulsion;
+    Count repulsion, plane, line, no_cohesion;
     for (long i = 0; i < n; ++i) {
         const bool uni = i & 1;
         const int sc = (int)(rng() % 20) - 20;
@@ -91,8 +98,27 @@ int main(int argc, char** argv)
         for (double& x : r) x = number(sc + 1, sc + 6, rng() & 1);
         repulsion.add(uni ? check(plain<true>, r, Ra, Rb, ma, mb, number(-100, -70, true))
                           : check(plain<false>, r, Ra, Rb, ma, mb, number(-100, -70, true)));
+        const auto care = [&](const double* d, double cR3) {
+            return uni ? check(zeros<true>, d, Ra, Rb, ma, mb, cR3) : check(zeros<false>, d, Ra, Rb, ma, mb, cR3);
+        };
+        const double nil = rng() & 1 ? 0.0 : -0.0;
+        no_cohesion.add(care(r, nil));
+        const int c = (int)(rng() % 3);
+        r[c] = rng() & 1 ? 0.0 : -0.0;
+        plane.add(care(r, number(-100, -70, rng() & 1)));
+        no_cohesion.add(care(r, nil));
+        r[(c + 1) % 3] = rng() & 1 ? 0.0 : -0.0;
+        line.add(care(r, number(-100, -70, rng() & 1)));
+        r[(c + 2) % 3] = rng() & 1 ? 0.0 : -0.0;
+        if (care(r, number(-100, -70, false))) {  // two centres in one place
+            ++bad;
+            std::printf("zero distance accepted\n");
+        }
     }
     repulsion.print("repulsion");
+    plane.print("plane");
+    line.print("line");
+    no_cohesion.print("no_cohesion");
     std::printf("mismatches %llu\n", bad);
     return bad != 0;
 }

@@ -1,6 +1,8 @@
 """Materials and positions at the edges of the exact form's integer path
 (csrc/sl_pair_fast.cuh), bit for bit against the CPU oracle, through every
-entry point that runs the tiles: a negative Hamaker constant (repulsion).
+entry point that runs the tiles: a negative Hamaker constant (repulsion), none
+(no cohesion), spheres in a plane -- zeros of both signs -- and on a line, and a
+cluster in which only some rows of a tile meet a zero component.
 Block remainders, equal and unequal radii, write steps among them."""
 import ctypes
 
@@ -21,7 +23,40 @@ def _repulsion(n, equal):
     return contact_case(n, 21, r_spread=0.0 if equal else 0.1, spacing=2.05), -MATERIAL["Ha"]
 
 
-CASES = {"repulsion": _repulsion}
+def _no_cohesion(n, equal):
+    return contact_case(n, 22, r_spread=0.0 if equal else 0.1), 0.0
+
+
+def _flat(c, axes):
+    for k in axes:
+        c["pos"][:, k] = np.where(np.arange(len(c["pos"])) % 3 == 0, -0.0, 0.0)
+        c["vel"][:, k] = 0.0
+    return c
+
+
+def _plane(n, equal):
+    c = contact_case(n, 23, r_spread=0.0 if equal else 0.1)
+    side = int(np.ceil(n ** 0.5))
+    g = np.stack(np.meshgrid(np.arange(side), np.arange(side), indexing="ij"), -1).reshape(-1, 2)[:n]
+    c["pos"][:, :2] = (g + np.random.default_rng(4).normal(0.0, 0.01, (n, 2))) * 2.0 * c["R"].mean()
+    c["w"][:, :2] = 0.0
+    return _flat(c, [2]), MATERIAL["Ha"]
+
+
+def _line(n, equal):
+    c = contact_case(n, 24, r_spread=0.0 if equal else 0.1)
+    c["pos"][:, 0] = (np.arange(n) - n / 2) * 2.0 * c["R"].mean()
+    c["w"][:] = 0.0
+    return _flat(c, [1, 2]), MATERIAL["Ha"]
+
+
+def _some_rows(n, equal):
+    c = contact_case(n, 25, r_spread=0.0 if equal else 0.1)
+    c["pos"][n // 2::7, 1] = c["pos"][0, 1]
+    return c, MATERIAL["Ha"]
+
+
+CASES = {"repulsion": _repulsion, "no_cohesion": _no_cohesion, "plane": _plane, "line": _line, "some_rows": _some_rows}
 
 
 def _oracle(c, Ha):

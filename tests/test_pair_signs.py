@@ -20,7 +20,7 @@ def stats(tmp_path_factory):
     return {line.split()[0]: [int(v) for v in line.split()[1:]] for line in out.stdout.splitlines()}
 
 
-@pytest.mark.parametrize("case", ["repulsion"])
+@pytest.mark.parametrize("case", ["repulsion", "plane", "line", "no_cohesion"])
 def test_settled_results_are_ieee(stats, case):
     assert stats["mismatches"] == [0]
     cases, flagged = stats[case]
