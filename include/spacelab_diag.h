@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include "spacelab_batch.h"
+#include "spacelab_mlp.h"
 
 #ifdef __cplusplus
 extern "C" {
@@ -63,6 +64,11 @@ int sl_diag_batch_give_up(sl_batch* b, unsigned barrier);
 /* The batch's lockstep launches are refused from here on, as where the process
  * has fewer SMs than the form takes: the next run changes to the per-CTA form. */
 int sl_diag_batch_refuse_lockstep(sl_batch* b);
+
+/* Error handling of the surrogate network, made on the host:
+ *   SL_DIAG_MLP_LAUNCH     the launch of the next prediction is rejected. */
+#define SL_DIAG_MLP_LAUNCH 2
+int sl_diag_mlp_fail(sl_mlp* m, int what);
 
 #ifdef __cplusplus
 }

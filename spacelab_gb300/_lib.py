@@ -119,6 +119,7 @@ _PROTOS = [
     ("sl_diag_int_ops", ctypes.c_int, [ctypes.c_int] + [_c_double_p] * 3),
     ("sl_diag_batch_give_up", ctypes.c_int, [ctypes.c_void_p, ctypes.c_uint]),
     ("sl_diag_batch_refuse_lockstep", ctypes.c_int, [ctypes.c_void_p]),
+    ("sl_diag_mlp_fail", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int]),
     # host setup (spacelab_host.h)
     ("slh_build_cluster", ctypes.c_int, [ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                          ctypes.c_double, ctypes.c_double, ctypes.c_double, ctypes.c_double,

@@ -21,6 +21,7 @@
 // bf16 copies feed the GEMMs.  An mma.sync m16n8k16 kernel (gemm_nt_kernel)
 // is kept only as the second opinion of sl_diag_gemm_bf16.
 #include "../../include/spacelab_mlp.h"
+#include "../../include/spacelab_diag.h"
 #include "../../include/spacelab_gpu.h"
 
 #include <cuda.h>
@@ -841,6 +842,7 @@ struct sl_mlp {
     FwNet net{};
     int num_sms = 0;
     bool host_direct = false;     // the GPU reads and writes pageable host memory (cudaDevAttrPageableMemoryAccess)
+    int fail_next = 0;            // diagnostics: what sl_diag_mlp_fail asked for
     void* arena = nullptr;
 };
 
@@ -1023,14 +1025,44 @@ bool setup_forward(sl_mlp* h)
 }
 
 // y = network(x) for n rows; x and y where the GPU can reach them
-bool forward_fused(sl_mlp* h, const float* x, float* y, int n, cudaStream_t st)
+cudaError_t forward_fused(sl_mlp* h, const float* x, float* y, int n, cudaStream_t st)
 {
     // set on every call: the attribute belongs to the current device's context
-    if (cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwSmem) != cudaSuccess)
-        return false;
-    const int tiles = (n + kFwRows - 1) / kFwRows;
-    mlp_forward_kernel<<<std::min(tiles, 2 * h->num_sms), kFwThreads, kFwSmem, st>>>(h->net, x, y, n, h->err);
-    return true;
+    cudaError_t e = cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwSmem);
+    if (e != cudaSuccess) return e;
+    size_t smem = kFwSmem;
+    if (h->fail_next == SL_DIAG_MLP_LAUNCH) {  // more than an SM has
+        smem = size_t(1) << 20;
+        h->fail_next = 0;
+    }
+    const int tiles = n / kFwRows + (n % kFwRows != 0);
+    e = sl::launch_pdl(false, mlp_forward_kernel, (unsigned)std::min(tiles, 2 * h->num_sms), kFwThreads, smem, st, h->net,
+                       x, y, n, h->err);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+// All rows in one launch, read and written where the caller has them.
+cudaError_t predict_in_place(sl_mlp* h, const float* x, float* y, int n)
+{
+    const cudaError_t e = forward_fused(h, x, y, n, nullptr), done = cudaStreamSynchronize(nullptr);
+    return e != cudaSuccess ? e : done;
+}
+
+// A batch at a time through device staging.
+cudaError_t predict_staged(sl_mlp* h, const float* x, float* y, int n)
+{
+    cudaError_t e = cudaSuccess;
+    for (int s0 = 0; s0 < n && e == cudaSuccess; s0 += std::min(h->max_batch, n - s0)) {
+        const int M = std::min(h->max_batch, n - s0);
+        e = cudaMemcpyAsync(h->xin, x + (size_t)s0 * h->n_in, (size_t)M * h->n_in * 4, cudaMemcpyHostToDevice, nullptr);
+        if (e == cudaSuccess) e = forward_fused(h, h->xin, h->yin, M, nullptr);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(y + (size_t)s0 * h->n_out, h->yin, (size_t)M * h->n_out * 4, cudaMemcpyDeviceToHost,
+                                nullptr);
+    }
+    const cudaError_t done = cudaStreamSynchronize(nullptr);
+    return e != cudaSuccess ? e : done;
 }
 
 // A caller's host array as the GPU can use it in place, or NULL
@@ -1301,21 +1333,10 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
     if (h->fused) {
         float* vx = static_cast<float*>(device_view(h, x));
         float* vy = static_cast<float*>(device_view(h, y));
-        // what the GPU cannot reach goes through the batch's staging, a batch at a time
-        const int step = vx && vy ? n : B;
-        for (int s0 = 0; s0 < n; s0 += step) {
-            const int M = std::min(step, n - s0);
-            const float* px = vx ? vx + (size_t)s0 * h->n_in : h->xin;
-            float* py = vy ? vy + (size_t)s0 * h->n_out : h->yin;
-            if (!vx)
-                cudaMemcpyAsync(h->xin, x + (size_t)s0 * h->n_in, (size_t)M * h->n_in * 4, cudaMemcpyHostToDevice,
-                                nullptr);
-            if (!forward_fused(h, px, py, M, nullptr)) h->tc_setup_failed = true;
-            if (!vy)
-                cudaMemcpyAsync(y + (size_t)s0 * h->n_out, h->yin, (size_t)M * h->n_out * 4, cudaMemcpyDeviceToHost,
-                                nullptr);
-        }
-        if (cudaStreamSynchronize(nullptr) != cudaSuccess) return sl_record_error(SL_ERR_CUDA, "prediction failed");
+        // what the GPU cannot reach goes through the batch's staging
+        const cudaError_t e = vx && vy ? predict_in_place(h, vx, vy, n) : predict_staged(h, x, y, n);
+        if (e != cudaSuccess)
+            return sl_record_error(SL_ERR_CUDA, (std::string("sl_mlp_predict: ") + cudaGetErrorString(e)).c_str());
         return mlp_status(h, "sl_mlp_predict");
     }
     std::vector<float> zb((size_t)B * ldo);
@@ -1334,6 +1355,13 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
 }
 
 }  // extern "C"
+
+extern "C" int sl_diag_mlp_fail(sl_mlp* h, int what)
+{
+    if (!h || what < 0 || what > SL_DIAG_MLP_LAUNCH) return sl_record_error(SL_ERR_ARG, "sl_diag_mlp_fail: bad argument");
+    h->fail_next = what;
+    return SL_OK;
+}
 
 extern "C" int sl_diag_gemm_bf16(int M, int N, int K, const uint16_t* A, const uint16_t* B, const float* bias,
                                  int act, int kernel, float* C, uint16_t* Cb)
