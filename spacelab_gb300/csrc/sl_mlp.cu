@@ -916,6 +916,14 @@ int mlp_status(sl_mlp* h, const char* what)
     return SL_OK;
 }
 
+// At the start of a call, which finds the handle idle: what an earlier call left
+// is not this one's.
+void clear_status(sl_mlp* h)
+{
+    *h->err = 0;
+    h->tc_setup_failed = false;
+}
+
 // Where a batch's inputs are: its own buffers, or the rows of a training
 // epoch's (rows epoch_rows, the step's read from *step).
 struct BatchInput {
@@ -1042,11 +1050,20 @@ cudaError_t forward_fused(sl_mlp* h, const float* x, float* y, int n, cudaStream
     return e;
 }
 
-// All rows in one launch, read and written where the caller has them.
-cudaError_t predict_in_place(sl_mlp* h, const float* x, float* y, int n)
+// All rows in one launch, read and written where the caller has them.  *slow: a
+// wait ran out.  The epilogues' reads and writes of host memory are inside the
+// waits' bound, and a page may take longer (a cold mapped file).
+cudaError_t predict_in_place(sl_mlp* h, const float* x, float* y, int n, bool* slow)
 {
-    const cudaError_t e = forward_fused(h, x, y, n, nullptr), done = cudaStreamSynchronize(nullptr);
-    return e != cudaSuccess ? e : done;
+    cudaError_t e = forward_fused(h, x, y, n, nullptr);
+    const cudaError_t done = cudaStreamSynchronize(nullptr);
+    if (e == cudaSuccess) e = done;
+    if (h->fail_next == SL_DIAG_MLP_SLOW_PAGE) {
+        *h->err = 1;
+        h->fail_next = 0;
+    }
+    *slow = *static_cast<volatile int*>(h->err) != 0;
+    return e;
 }
 
 // A batch at a time through device staging.
@@ -1214,6 +1231,7 @@ int sl_mlp_gradients(sl_mlp* h, const float* x, const float* y, int M, float* gr
 {
     if (!h || !x || !y || M < 32 || M % 32 || M > h->max_batch)
         return sl_record_error(SL_ERR_ARG, "M must be a multiple of 32 up to max_batch");
+    clear_status(h);
     // the kernels read x and y where they are, or from the staging
     const float* vx = static_cast<const float*>(device_view(h, x));
     const float* vy = static_cast<const float*>(device_view(h, y));
@@ -1240,6 +1258,7 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
 {
     if (!h || !x || !y || n < batch || batch < 32 || batch % 32 || batch > h->max_batch || epochs < 1)
         return sl_record_error(SL_ERR_ARG, "bad training arguments");
+    clear_status(h);
     std::vector<int> idx(n);
     for (int i = 0; i < n; ++i) idx[i] = i;
     std::mt19937_64 rng(seed);
@@ -1329,12 +1348,18 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
 int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
 {
     if (!h || !x || !y || n < 1) return sl_record_error(SL_ERR_ARG, "bad arguments");
+    clear_status(h);
     const int B = h->max_batch, L = h->nl, ldo = h->dout[L - 1];
     if (h->fused) {
         float* vx = static_cast<float*>(device_view(h, x));
         float* vy = static_cast<float*>(device_view(h, y));
-        // what the GPU cannot reach goes through the batch's staging
-        const cudaError_t e = vx && vy ? predict_in_place(h, vx, vy, n) : predict_staged(h, x, y, n);
+        bool staged = !vx || !vy;  // what the GPU cannot reach
+        cudaError_t e = cudaSuccess;
+        if (!staged) {
+            e = predict_in_place(h, vx, vy, n, &staged);
+            if (e == cudaSuccess && staged) clear_status(h);
+        }
+        if (e == cudaSuccess && staged) e = predict_staged(h, x, y, n);
         if (e != cudaSuccess)
             return sl_record_error(SL_ERR_CUDA, (std::string("sl_mlp_predict: ") + cudaGetErrorString(e)).c_str());
         return mlp_status(h, "sl_mlp_predict");
@@ -1358,8 +1383,11 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
 
 extern "C" int sl_diag_mlp_fail(sl_mlp* h, int what)
 {
-    if (!h || what < 0 || what > SL_DIAG_MLP_LAUNCH) return sl_record_error(SL_ERR_ARG, "sl_diag_mlp_fail: bad argument");
-    h->fail_next = what;
+    if (!h || what < 0 || what > SL_DIAG_MLP_TIMED_OUT) return sl_record_error(SL_ERR_ARG, "sl_diag_mlp_fail: bad argument");
+    if (what == SL_DIAG_MLP_TIMED_OUT)
+        *h->err = 1;
+    else
+        h->fail_next = what;
     return SL_OK;
 }
 

@@ -1,6 +1,8 @@
-"""A surrogate call that goes wrong is reported, and the next one does not
-suffer from it: a rejected launch.  The failure is made on the host
-(sl_diag_mlp_fail); results bit for bit those of an untroubled call."""
+"""A surrogate call that goes wrong is reported or done another way, and the
+next one does not suffer from it: a prediction in place that meets a slow page
+of host memory, a rejected launch, a call whose wait ran out.  The failures are
+made on the host (sl_diag_mlp_fail); results bit for bit those of an untroubled
+call."""
 import numpy as np
 import pytest
 
@@ -10,7 +12,7 @@ from spacelab_gb300._lib import check
 
 pytestmark = pytest.mark.gpu
 
-LAUNCH = 2
+SLOW_PAGE, LAUNCH, TIMED_OUT = 1, 2, 3
 
 
 @pytest.fixture(scope="module")
@@ -26,6 +28,14 @@ def _fail(net, what):
     check(net.lib.sl_diag_mlp_fail(net.h, what), "sl_diag_mlp_fail")
 
 
+@pytest.mark.parametrize("n", [1, 128, 500])
+def test_a_slow_page(net, n):
+    want = net.predict(_x(n))
+    _fail(net, SLOW_PAGE)
+    assert np.array_equal(net.predict(_x(n)), want)
+    assert np.array_equal(net.predict(_x(n)), want)
+
+
 def test_a_rejected_launch(net):
     want = net.predict(_x(100))
     _fail(net, LAUNCH)
@@ -33,3 +43,15 @@ def test_a_rejected_launch(net):
         net.predict(_x(100))
     assert err.value.code == _lib.SL_ERR_CUDA
     assert np.array_equal(net.predict(_x(100)), want)
+
+
+def test_calls_after_one_that_timed_out(net):
+    x, y = _x(64), _x(64)[:, :4]
+    want, (loss, grads) = net.predict(x), net.gradients(x, y)
+    _fail(net, TIMED_OUT)
+    assert np.array_equal(net.predict(x), want)
+    _fail(net, TIMED_OUT)
+    l2, g2 = net.gradients(x, y)
+    assert l2 == loss and np.array_equal(g2, grads)
+    _fail(net, TIMED_OUT)
+    assert np.isfinite(net.train(x, y, epochs=1, batch=32)).all()
