@@ -1353,7 +1353,11 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
     if (h->fused) {
         float* vx = static_cast<float*>(device_view(h, x));
         float* vy = static_cast<float*>(device_view(h, y));
-        bool staged = !vx || !vy;  // what the GPU cannot reach
+        // staged: what the GPU cannot reach, and results over the inputs, of which
+        // one CTA would write what another has yet to read
+        const uintptr_t xa = reinterpret_cast<uintptr_t>(x), ya = reinterpret_cast<uintptr_t>(y);
+        const bool overlap = xa < ya + (size_t)n * h->n_out * 4 && ya < xa + (size_t)n * h->n_in * 4;
+        bool staged = !vx || !vy || overlap;
         cudaError_t e = cudaSuccess;
         if (!staged) {
             e = predict_in_place(h, vx, vy, n, &staged);
