@@ -814,6 +814,10 @@ __global__ void to_bf16_kernel(const float* __restrict__ in, bf16* pb, bf16* wt,
 
 int pad32(int x) { return (x + 31) / 32 * 32; }
 
+// Device memory that training keeps for a data set and its packed epoch (45,000
+// rows of 8 features take 9 MB).
+constexpr size_t kEpochBytes = size_t(256) << 20;
+
 }  // namespace
 
 struct sl_mlp {
@@ -832,7 +836,7 @@ struct sl_mlp {
     bf16 *dZ[2] = {}, *dZt[2] = {};      // gradients of Z, [M][dout] and [dout][M]; a layer reads one and writes the other
     float *xin = nullptr, *yin = nullptr;
     cudaStream_t stream = nullptr;       // training's launches
-    void* epoch = nullptr;               // training's copies of the data set (grown when a larger one comes)
+    void* epoch = nullptr;               // training's copies of the data set (grown when a larger one comes, to kEpochBytes)
     size_t epoch_bytes = 0;
     int step = 0;
     int* err = nullptr;           // set by a tcgen05 GEMM whose bounded wait ran out; pinned host memory, with
@@ -1265,33 +1269,60 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const int ld0 = h->din[0], ldo = h->dout[h->nl - 1];
     const int nb = (batch * ldo + 255) / 256;
-    const int steps = n / batch, rows = steps * batch;
+    const int steps = n / batch;
 
-    // the data set on the device, and each epoch's rows in its order
-    size_t bytes = 0;
-    auto take = [&](size_t b) { size_t o = bytes; bytes = (bytes + b + 255) / 256 * 256; return o; };
-    const size_t ox = take((size_t)n * h->n_in * 4), oy = take((size_t)n * h->n_out * 4), oidx = take((size_t)rows * 4),
-                 oxp = take((size_t)rows * ld0 * 2), oxt = take((size_t)rows * ld0 * 2),
-                 oyp = take((size_t)rows * h->n_out * 4), ocoef = take((size_t)steps * sizeof(float2)),
-                 oloss = take((size_t)steps * nb * 4), ostep = take(sizeof(int));
+    // The epoch's rows packed on the device, `seg` steps at a time.  Whole: the data
+    // set is there too, and an epoch is packed at once in its order.  Otherwise,
+    // beyond kEpochBytes or where the device has no room, the host gathers each
+    // segment's rows.
+    int seg = steps;
+    bool whole = true;
+    size_t bytes = 0, ox = 0, oy = 0, oidx = 0, oxp = 0, oxt = 0, oyp = 0, ocoef = 0, oloss = 0, ostep = 0;
+    auto layout = [&] {
+        bytes = 0;
+        auto take = [&](size_t b) { size_t o = bytes; bytes = (bytes + b + 255) / 256 * 256; return o; };
+        const size_t r = (size_t)seg * batch;
+        ox = take((whole ? (size_t)n : r) * h->n_in * 4);
+        oy = take(whole ? (size_t)n * h->n_out * 4 : 0);
+        oidx = take(whole ? r * 4 : 0);
+        oxp = take(r * ld0 * 2);
+        oxt = take(r * ld0 * 2);
+        oyp = take(r * h->n_out * 4);
+        ocoef = take((size_t)seg * sizeof(float2));
+        oloss = take((size_t)seg * nb * 4);
+        ostep = take(sizeof(int));
+    };
+    layout();
+    if (bytes > kEpochBytes) {
+        whole = false;
+        for (layout(); bytes > kEpochBytes && seg > 1; layout()) seg = (seg + 1) / 2;
+    }
     if (bytes > h->epoch_bytes) {
         if (h->epoch) cudaFree(h->epoch);
         h->epoch = nullptr;
         h->epoch_bytes = 0;
-        if (cudaMalloc(&h->epoch, bytes) != cudaSuccess) {
+        while (cudaMalloc(&h->epoch, bytes) != cudaSuccess) {
             cudaGetLastError();
-            return sl_record_error(SL_ERR_ALLOC, "sl_mlp_train: cudaMalloc of the data set failed");
+            h->epoch = nullptr;
+            if (!whole && seg == 1) return sl_record_error(SL_ERR_ALLOC, "sl_mlp_train: cudaMalloc of a batch failed");
+            if (!whole) seg = (seg + 1) / 2;
+            whole = false;
+            layout();
         }
         h->epoch_bytes = bytes;
     }
+    const int rows = seg * batch;
     char* e = static_cast<char*>(h->epoch);
     float *dx = (float*)(e + ox), *dy = (float*)(e + oy), *yp = (float*)(e + oyp), *dloss = (float*)(e + oloss);
     int *didx = (int*)(e + oidx), *dstep = (int*)(e + ostep);
     bf16 *xp = (bf16*)(e + oxp), *xt = (bf16*)(e + oxt);
     float2* dcoef = (float2*)(e + ocoef);
     cudaStream_t st = h->stream;
-    cudaMemcpyAsync(dx, x, (size_t)n * h->n_in * 4, cudaMemcpyHostToDevice, st);
-    cudaMemcpyAsync(dy, y, (size_t)n * h->n_out * 4, cudaMemcpyHostToDevice, st);
+    std::vector<float> gx(whole ? 0 : (size_t)rows * h->n_in), gy(whole ? 0 : (size_t)rows * h->n_out);
+    if (whole) {
+        cudaMemcpyAsync(dx, x, (size_t)n * h->n_in * 4, cudaMemcpyHostToDevice, st);
+        cudaMemcpyAsync(dy, y, (size_t)n * h->n_out * 4, cudaMemcpyHostToDevice, st);
+    }
 
     // one step as a graph: it finds its rows by the step counter
     cudaGraph_t graph = nullptr;
@@ -1308,37 +1339,51 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
     if (graph) cudaGraphDestroy(graph);
     int rc = ok ? SL_OK : sl_record_error(SL_ERR_CUDA, "sl_mlp_train: the step's graph could not be made");
 
-    std::vector<float> part((size_t)steps * nb);
-    std::vector<float2> coef(steps);
+    std::vector<float> part((size_t)seg * nb);
+    std::vector<float2> coef(seg);
     std::vector<int> next(idx);
     std::shuffle(next.begin(), next.end(), rng);
     for (int ep = 0; ep < epochs && rc == SL_OK; ++ep) {
         idx.swap(next);
-        for (int k = 0; k < steps; ++k) {
-            ++h->step;
-            coef[k] = make_float2(1.0f - std::pow(b1, (float)h->step), 1.0f - std::pow(b2, (float)h->step));
-        }
-        cudaMemcpyAsync(didx, idx.data(), (size_t)rows * 4, cudaMemcpyHostToDevice, st);
-        cudaMemcpyAsync(dcoef, coef.data(), coef.size() * sizeof(float2), cudaMemcpyHostToDevice, st);
-        cudaMemsetAsync(dstep, 0, sizeof(int), st);
-        pack_kernel<<<(rows + 127) / 128, 128, 0, st>>>(dx, dy, didx, rows, n, h->n_in, h->n_out, ld0, xp, xt, yp);
-        for (int k = 0; k < steps; ++k) cudaGraphLaunch(exec, st);
-        if (ep + 1 < epochs) {  // the next epoch's order, under this one's steps
-            next = idx;
-            std::shuffle(next.begin(), next.end(), rng);
-        }
-        cudaMemcpyAsync(part.data(), dloss, part.size() * 4, cudaMemcpyDeviceToHost, st);
-        if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess) {
-            rc = sl_record_error(SL_ERR_CUDA, "training kernel failed");
-            break;
-        }
         double ls = 0;
-        for (int k = 0; k < steps; ++k) {
-            double s = 0;
-            for (int i = 0; i < nb; ++i) s += part[(size_t)k * nb + i];
-            ls += s / ((double)batch * h->n_out);
+        for (int s0 = 0; s0 < steps && rc == SL_OK; s0 += seg) {
+            const int ns = std::min(seg, steps - s0), nr = ns * batch;
+            const int* order = idx.data() + (size_t)s0 * batch;
+            for (int k = 0; k < ns; ++k) {
+                ++h->step;
+                coef[k] = make_float2(1.0f - std::pow(b1, (float)h->step), 1.0f - std::pow(b2, (float)h->step));
+            }
+            cudaMemcpyAsync(dcoef, coef.data(), (size_t)ns * sizeof(float2), cudaMemcpyHostToDevice, st);
+            cudaMemsetAsync(dstep, 0, sizeof(int), st);
+            if (whole) {
+                cudaMemcpyAsync(didx, order, (size_t)nr * 4, cudaMemcpyHostToDevice, st);
+                pack_kernel<<<(rows + 127) / 128, 128, 0, st>>>(dx, dy, didx, rows, n, h->n_in, h->n_out, ld0, xp, xt,
+                                                                yp);
+            } else {
+                for (int r = 0; r < nr; ++r) {
+                    std::memcpy(&gx[(size_t)r * h->n_in], &x[(size_t)order[r] * h->n_in], h->n_in * 4);
+                    std::memcpy(&gy[(size_t)r * h->n_out], &y[(size_t)order[r] * h->n_out], h->n_out * 4);
+                }
+                cudaMemcpyAsync(dx, gx.data(), (size_t)nr * h->n_in * 4, cudaMemcpyHostToDevice, st);
+                cudaMemcpyAsync(yp, gy.data(), (size_t)nr * h->n_out * 4, cudaMemcpyHostToDevice, st);
+                pack_kernel<<<(rows + 127) / 128, 128, 0, st>>>(dx, nullptr, nullptr, rows, nr, h->n_in, h->n_out, ld0,
+                                                                xp, xt, nullptr);
+            }
+            for (int k = 0; k < ns; ++k) cudaGraphLaunch(exec, st);
+            if (s0 + ns == steps && ep + 1 < epochs) {  // the next epoch's order, under this one's last steps
+                next = idx;
+                std::shuffle(next.begin(), next.end(), rng);
+            }
+            cudaMemcpyAsync(part.data(), dloss, (size_t)ns * nb * 4, cudaMemcpyDeviceToHost, st);
+            if (cudaStreamSynchronize(st) != cudaSuccess || cudaGetLastError() != cudaSuccess)
+                rc = sl_record_error(SL_ERR_CUDA, "training kernel failed");
+            for (int k = 0; k < ns; ++k) {
+                double s = 0;
+                for (int i = 0; i < nb; ++i) s += part[(size_t)k * nb + i];
+                ls += s / ((double)batch * h->n_out);
+            }
         }
-        if (loss_per_epoch) loss_per_epoch[ep] = (float)(ls / std::max(1, steps));
+        if (loss_per_epoch && rc == SL_OK) loss_per_epoch[ep] = (float)(ls / std::max(1, steps));
     }
     if (exec) cudaGraphExecDestroy(exec);
     if (rc == SL_OK) rc = mlp_status(h, "sl_mlp_train");
