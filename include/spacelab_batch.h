@@ -46,7 +46,8 @@ int sl_batch_upload(sl_batch* b, const double* pos, const double* vel, const dou
  * where the largest instance makes those buffers too big).  The pair-tile
  * pass may advance all instances in lockstep, from one queue of tiles, where
  * that balances better than an instance per CTA; `threads` has no effect
- * there, and the results are the same. */
+ * there.  The state is the same bit for bit; the energy records are summed in
+ * another order (within 1e-10 of the largest total). */
 int sl_batch_set_shape(sl_batch* b, int tile, int threads);
 int sl_batch_shape(const sl_batch* b, int* tile, int* threads, int* blocks);
 

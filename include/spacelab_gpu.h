@@ -53,8 +53,9 @@ extern "C" {
                                displacements; FP64 positions, pair subtraction
                                r_i - r_j, overlaps of close pairs, per-sphere
                                force/torque accumulation and energy sums (the
-                               per-tile sums in FP32 parts that hold more than
-                               FP64's 53 bits); deterministic, not bit-exact */
+                               subtraction and the per-tile sums in FP32 parts:
+                               r rounded to FP32 once, sums of more than FP64's
+                               53 bits); deterministic, not bit-exact */
 #define SL_MODE_MIXED_DF 2  /* no FP64 pipe work for pairs out of contact:
                                double-float (FP32 hi + lo, ~48 bits) pair
                                subtraction and overlap of close pairs, FP32

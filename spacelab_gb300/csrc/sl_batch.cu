@@ -9,7 +9,11 @@
 // sl_batch_capi.cu).  Otherwise each CTA takes whole instances from an atomic
 // work queue (largest first) and runs all of an instance's steps before taking
 // the next one; the only synchronisation is then __syncthreads inside the CTA.
-// The results are the same bit for bit.  Within an instance a step is the reference's three passes
+// The state is the same bit for bit.  The energy records hold the same terms
+// summed in another order, which in lockstep depends on where the batch's strips
+// begin, and so on the other instances (1e-10 of the largest total).
+//
+// Within an instance a step is the reference's three passes
 // (ColliderSingleCore.cpp:82-97, 100-256, 263-287):
 //   drift    one thread per sphere (strided);
 //   pairs    either the pair-tile pass (shape tile 0: every pair once into
@@ -434,7 +438,7 @@ __device__ void grid_pairs(const Batch& b, GridWarp& gw, int num_sms, int* queue
     }
 }
 
-// Ordered sums and pass 3; next_dt: the following step's pass 1 too
+// Ordered sums and pass 3; drift_next: the following step's pass 1 too
 __device__ void grid_rows(const Batch& b, bool init, bool drift_next)
 {
     const int lane = threadIdx.x & 31;

@@ -309,140 +309,140 @@ __device__ __forceinline__ void tile_mixed(const Batch& b, int off, int n, const
     const float L = mc.L, hmin_s = mc.hmin_s, c_vdw = mc.c_vdw;
     float* rows = sm.rows;
     float* rowtq = sm.rowtq;
-        {
-            const int sA = off + min(X * kBlock + lane, n - 1);  // slot (padding rows repeat the last)
-            const float Ri = b.f_R[sA];
-            mt::put_row(rows, lane, {b.f_pos[0][sA], b.f_pos[1][sA], b.f_pos[2][sA], Ri, b.f_pos[3][sA],
-                                     b.f_pos[4][sA], b.f_pos[5][sA], c_vdw * (Ri * Ri * Ri)},
-                        make_float4(b.f_Rlo[sA], b.f_inv_m[sA], b.f_inv_moi[sA], __int_as_float(b.perm[sA] - off)));
-            rowtq[lane] = 0.0f; rowtq[kBlock + lane] = 0.0f; rowtq[2 * kBlock + lane] = 0.0f;
+    {
+        const int sA = off + min(X * kBlock + lane, n - 1);  // slot (padding rows repeat the last)
+        const float Ri = b.f_R[sA];
+        mt::put_row(rows, lane, {b.f_pos[0][sA], b.f_pos[1][sA], b.f_pos[2][sA], Ri, b.f_pos[3][sA],
+                                 b.f_pos[4][sA], b.f_pos[5][sA], c_vdw * (Ri * Ri * Ri)},
+                    make_float4(b.f_Rlo[sA], b.f_inv_m[sA], b.f_inv_moi[sA], __int_as_float(b.perm[sA] - off)));
+        rowtq[lane] = 0.0f; rowtq[kBlock + lane] = 0.0f; rowtq[2 * kBlock + lane] = 0.0f;
+    }
+    __syncwarp();
+    const int sB = Y * kBlock + lane;  // slot in the instance
+    auto load_column = [&](int slot) {
+        const int g = off + min(slot, n - 1);
+        mt::Col c;
+        c.x = b.f_pos[0][g]; c.y = b.f_pos[1][g]; c.z = b.f_pos[2][g];
+        c.xl = b.f_pos[3][g]; c.yl = b.f_pos[4][g]; c.zl = b.f_pos[5][g];
+        c.R = b.f_R[g];
+        c.R3 = c.R * c.R * c.R;
+        c.valid = slot < n;
+        return c;
+    };
+    const mt::Col col = load_column(sB);
+    const float inv_mb = b.f_inv_m[off + min(sB, n - 1)], inv_moib = b.f_inv_moi[off + min(sB, n - 1)];
+    const int nA = n - X * kBlock;
+    float ctx = 0, cty = 0, ctz = 0;     // the column sphere's torque sum
+    // listed pair (row r, column slot 32Y + cb): double-float geometry, then
+    // the contact branch in the reference's orientation (A = the larger
+    // index in the instance) or the clamped vdW; the force on the row
+    // sphere, and in contact both spheres' torques
+    auto close = [&](int q, int r, int cb, double& pe_, df::Sum& far_) {
+        const mt::Col c = load_column(Y * kBlock + cb);
+        const int gs = off + min(Y * kBlock + cb, n - 1);
+        const mt::Row row = mt::get_row(rows, r);
+        float* out = sm.list.v[q];
+        const float Ras = row.R, Rbs = c.R;
+        const mt::Far f = mt::far_pair(row, c);
+        if (!(f.d2 < b.far_sq * f.sum2)) {
+            out[0] = f.fr * f.rx; out[1] = f.fr * f.ry; out[2] = f.fr * f.rz;
+            if (WRITE) far_.add(vdw_bracket(f.d2, Ras, Rbs));
+            return;
         }
-        __syncwarp();
-        const int sB = Y * kBlock + lane;  // slot in the instance
-        auto load_column = [&](int slot) {
-            const int g = off + min(slot, n - 1);
-            mt::Col c;
-            c.x = b.f_pos[0][g]; c.y = b.f_pos[1][g]; c.z = b.f_pos[2][g];
-            c.xl = b.f_pos[3][g]; c.yl = b.f_pos[4][g]; c.zl = b.f_pos[5][g];
-            c.R = b.f_R[g];
-            c.R3 = c.R * c.R * c.R;
-            c.valid = slot < n;
-            return c;
-        };
-        const mt::Col col = load_column(sB);
-        const float inv_mb = b.f_inv_m[off + min(sB, n - 1)], inv_moib = b.f_inv_moi[off + min(sB, n - 1)];
-        const int nA = n - X * kBlock;
-        float ctx = 0, cty = 0, ctz = 0;     // the column sphere's torque sum
-        // listed pair (row r, column slot 32Y + cb): double-float geometry, then
-        // the contact branch in the reference's orientation (A = the larger
-        // index in the instance) or the clamped vdW; the force on the row
-        // sphere, and in contact both spheres' torques
-        auto close = [&](int q, int r, int cb, double& pe_, df::Sum& far_) {
-            const mt::Col c = load_column(Y * kBlock + cb);
-            const int gs = off + min(Y * kBlock + cb, n - 1);
-            const mt::Row row = mt::get_row(rows, r);
-            float* out = sm.list.v[q];
-            const float Ras = row.R, Rbs = c.R;
-            const mt::Far f = mt::far_pair(row, c);
-            if (!(f.d2 < b.far_sq * f.sum2)) {
-                out[0] = f.fr * f.rx; out[1] = f.fr * f.ry; out[2] = f.fr * f.rz;
-                if (WRITE) far_.add(vdw_bracket(f.d2, Ras, Rbs));
-                return;
+        const int iA = __float_as_int(rows[r * mt::kRow + 19]), iB = b.perm[gs] - off;
+        const df::F2 drx = df::sub({c.x, c.xl}, {row.x, row.xl});
+        const df::F2 dry = df::sub({c.y, c.yl}, {row.y, row.yl});
+        const df::F2 drz = df::sub({c.z, c.zl}, {row.z, row.zl});
+        const df::F2 dd2 = df::add(df::add(df::sqr(drx), df::sqr(dry)), df::sqr(drz));
+        const df::F2 sum = df::add({Ras, rows[r * mt::kRow + 16]}, {Rbs, b.f_Rlo[gs]});
+        const df::F2 gap2 = df::sub(df::sqr(sum), dd2);
+        const float d2s = dd2.hi;
+        const float inv_dn = rsqrtf(d2s);
+        const float dist_s = d2s * inv_dn;
+        const float ovl_s = __fdividef(gap2.hi, Ras + Rbs + dist_s);
+        const float nx = drx.hi * inv_dn, ny = dry.hi * inv_dn, nz = drz.hi * inv_dn;  // row -> column
+        const bool rowA = iA > iB;
+        const int gA = off + (rowA ? iA : iB), gB = off + (rowA ? iB : iA);
+        if (gap2.hi > 0.0f || (gap2.hi == 0.0f && gap2.lo > 0.0f)) {
+            ContactIn in;
+            for (int k = 0; k < 3; ++k) {
+                in.prevA[k] = b.prev.c[k][gA]; in.prevB[k] = b.prev.c[k][gB];
+                in.wA[k] = b.w.c[k][gA]; in.wB[k] = b.w.c[k][gB];
+                in.vA[k] = b.vel.c[k][gA]; in.vB[k] = b.vel.c[k][gB];
             }
-            const int iA = __float_as_int(rows[r * mt::kRow + 19]), iB = b.perm[gs] - off;
-            const df::F2 drx = df::sub({c.x, c.xl}, {row.x, row.xl});
-            const df::F2 dry = df::sub({c.y, c.yl}, {row.y, row.yl});
-            const df::F2 drz = df::sub({c.z, c.zl}, {row.z, row.zl});
-            const df::F2 dd2 = df::add(df::add(df::sqr(drx), df::sqr(dry)), df::sqr(drz));
-            const df::F2 sum = df::add({Ras, rows[r * mt::kRow + 16]}, {Rbs, b.f_Rlo[gs]});
-            const df::F2 gap2 = df::sub(df::sqr(sum), dd2);
-            const float d2s = dd2.hi;
-            const float inv_dn = rsqrtf(d2s);
-            const float dist_s = d2s * inv_dn;
-            const float ovl_s = __fdividef(gap2.hi, Ras + Rbs + dist_s);
-            const float nx = drx.hi * inv_dn, ny = dry.hi * inv_dn, nz = drz.hi * inv_dn;  // row -> column
-            const bool rowA = iA > iB;
-            const int gA = off + (rowA ? iA : iB), gB = off + (rowA ? iB : iA);
-            if (gap2.hi > 0.0f || (gap2.hi == 0.0f && gap2.lo > 0.0f)) {
-                ContactIn in;
-                for (int k = 0; k < 3; ++k) {
-                    in.prevA[k] = b.prev.c[k][gA]; in.prevB[k] = b.prev.c[k][gB];
-                    in.wA[k] = b.w.c[k][gA]; in.wB[k] = b.w.c[k][gB];
-                    in.vA[k] = b.vel.c[k][gA]; in.vB[k] = b.vel.c[k][gB];
-                }
-                in.mA = b.m[gA]; in.mB = b.m[gB]; in.kin = kin; in.kout = kout;
-                // kin/kout: |r|^2 against the previous step's, both FP64 by one formula
-                const double d2_64 = fp64_d2(b, gA, gB);
-                const float sg = rowA ? 1.0f : -1.0f;  // unit vector A -> B
-                const ContactF o = contact_mixed(in, M, sh, d2_64, sg * nx, sg * ny, sg * nz, dist_s * L, ovl_s * L,
-                                                 rowA ? Ras : Rbs, rowA ? Rbs : Ras);
-                out[0] = sg * o.fx; out[1] = sg * o.fy; out[2] = sg * o.fz;  // o.f acts on A; B takes -o.f
-                const float imoia = rows[r * mt::kRow + 18];
-                out[3] = (rowA ? o.tax : o.tbx) * imoia;
-                out[4] = (rowA ? o.tay : o.tby) * imoia;
-                out[5] = (rowA ? o.taz : o.tbz) * imoia;
-                out[6] = rowA ? o.tbx : o.tax;
-                out[7] = rowA ? o.tby : o.tay;
-                out[8] = rowA ? o.tbz : o.taz;
-                sm.list.pair[q] |= kTouching;
-                if (WRITE) {
-                    const double sum64 = b.R[gA] + b.R[gB];
-                    pe_ += pair_pe_fp64(M, b.R[gA], b.R[gB], fma(sum64, sum64, -d2_64), d2_64, true, o.k);
-                }
-                return;
-            }
-            const float hn = fmaxf(-ovl_s, hmin_s);
-            const float fv = c_vdw * vdw_shape(hn, Ras, Rbs);
-            out[0] = fv * nx; out[1] = fv * ny; out[2] = fv * nz;
+            in.mA = b.m[gA]; in.mB = b.m[gB]; in.kin = kin; in.kout = kout;
+            // kin/kout: |r|^2 against the previous step's, both FP64 by one formula
+            const double d2_64 = fp64_d2(b, gA, gB);
+            const float sg = rowA ? 1.0f : -1.0f;  // unit vector A -> B
+            const ContactF o = contact_mixed(in, M, sh, d2_64, sg * nx, sg * ny, sg * nz, dist_s * L, ovl_s * L,
+                                             rowA ? Ras : Rbs, rowA ? Rbs : Ras);
+            out[0] = sg * o.fx; out[1] = sg * o.fy; out[2] = sg * o.fz;  // o.f acts on A; B takes -o.f
+            const float imoia = rows[r * mt::kRow + 18];
+            out[3] = (rowA ? o.tax : o.tbx) * imoia;
+            out[4] = (rowA ? o.tay : o.tby) * imoia;
+            out[5] = (rowA ? o.taz : o.tbz) * imoia;
+            out[6] = rowA ? o.tbx : o.tax;
+            out[7] = rowA ? o.tby : o.tay;
+            out[8] = rowA ? o.tbz : o.taz;
+            sm.list.pair[q] |= kTouching;
             if (WRITE) {
-                const double d2_64 = fp64_d2(b, gA, gB), sum64 = b.R[gA] + b.R[gB];
-                pe_ += pair_pe_fp64(M, b.R[gA], b.R[gB], fma(sum64, sum64, -d2_64), d2_64, false, 0.0);
+                const double sum64 = b.R[gA] + b.R[gB];
+                pe_ += pair_pe_fp64(M, b.R[gA], b.R[gB], fma(sum64, sum64, -d2_64), d2_64, true, o.k);
             }
-        };
-        // a contact's torques, in the sweep's order: one lane per row in a step
-        auto taken = [&](int q, int r) {
-            if (!(sm.list.pair[q] & kTouching)) return;
-            const float* v = sm.list.v[q];
-            atomicAdd(&rowtq[r], v[3]);
-            atomicAdd(&rowtq[kBlock + r], v[4]);
-            atomicAdd(&rowtq[2 * kBlock + r], v[5]);
-            ctx = fmaf(v[6], inv_moib, ctx);
-            cty = fmaf(v[7], inv_moib, cty);
-            ctz = fmaf(v[8], inv_moib, ctz);
-        };
-        float av[3], bv[3];
-        mt::tile<WRITE>(rows, sm.list, col, nA, X == Y, b.far_sq, close, taken, av, bv, pe, pe_far);
-        const float ax = av[0], ay = av[1], az = av[2], bsx = bv[0], bsy = bv[1], bsz = bv[2];
-        __syncwarp();  // the row torques' shared-memory adds
-        // lane l holds row l's force sum (rows and columns beyond n hold 0)
-        const int sAl = X * kBlock + lane;
-        const float ima = rows[lane * mt::kRow + 17];
-        const float rtx = rowtq[lane], rty = rowtq[kBlock + lane], rtz = rowtq[2 * kBlock + lane];
-        // sphere at slot p: torques from block K
-        auto put_torque = [&](int K, int p, float tx, float ty, float tz) {
-            if (tmask) {
-                if (tx == 0.0f && ty == 0.0f && tz == 0.0f) return;
-                if (p < n) atomicOr(tmask + (size_t)(K >> 5) * part_np + p, 1u << (K & 31));
-            }
-            float* o = part + (size_t)K * part_np + p + 3 * pplane;
-            __stcs(o, tx); __stcs(o + pplane, ty); __stcs(o + 2 * pplane, tz);
-        };
-        if (X == Y) {  // the same sphere: partners before it in slot order (row), after it (column)
-            const size_t o = (size_t)X * part_np + sAl;
-            __stcs(part + o, fmaf(ima, ax, -inv_mb * bsx));
-            __stcs(part + o + pplane, fmaf(ima, ay, -inv_mb * bsy));
-            __stcs(part + o + 2 * pplane, fmaf(ima, az, -inv_mb * bsz));
-            put_torque(X, sAl, rtx + ctx, rty + cty, rtz + ctz);
-        } else {
-            const size_t oa = (size_t)Y * part_np + sAl, ob = (size_t)X * part_np + sB;
-            __stcs(part + oa, ima * ax); __stcs(part + oa + pplane, ima * ay); __stcs(part + oa + 2 * pplane, ima * az);
-            __stcs(part + ob, -inv_mb * bsx);
-            __stcs(part + ob + pplane, -inv_mb * bsy);
-            __stcs(part + ob + 2 * pplane, -inv_mb * bsz);
-            put_torque(Y, sAl, rtx, rty, rtz);
-            put_torque(X, sB, ctx, cty, ctz);
+            return;
         }
-        __syncwarp();
+        const float hn = fmaxf(-ovl_s, hmin_s);
+        const float fv = c_vdw * vdw_shape(hn, Ras, Rbs);
+        out[0] = fv * nx; out[1] = fv * ny; out[2] = fv * nz;
+        if (WRITE) {
+            const double d2_64 = fp64_d2(b, gA, gB), sum64 = b.R[gA] + b.R[gB];
+            pe_ += pair_pe_fp64(M, b.R[gA], b.R[gB], fma(sum64, sum64, -d2_64), d2_64, false, 0.0);
+        }
+    };
+    // a contact's torques, in the sweep's order: one lane per row in a step
+    auto taken = [&](int q, int r) {
+        if (!(sm.list.pair[q] & kTouching)) return;
+        const float* v = sm.list.v[q];
+        atomicAdd(&rowtq[r], v[3]);
+        atomicAdd(&rowtq[kBlock + r], v[4]);
+        atomicAdd(&rowtq[2 * kBlock + r], v[5]);
+        ctx = fmaf(v[6], inv_moib, ctx);
+        cty = fmaf(v[7], inv_moib, cty);
+        ctz = fmaf(v[8], inv_moib, ctz);
+    };
+    float av[3], bv[3];
+    mt::tile<WRITE>(rows, sm.list, col, nA, X == Y, b.far_sq, close, taken, av, bv, pe, pe_far);
+    const float ax = av[0], ay = av[1], az = av[2], bsx = bv[0], bsy = bv[1], bsz = bv[2];
+    __syncwarp();  // the row torques' shared-memory adds
+    // lane l holds row l's force sum (rows and columns beyond n hold 0)
+    const int sAl = X * kBlock + lane;
+    const float ima = rows[lane * mt::kRow + 17];
+    const float rtx = rowtq[lane], rty = rowtq[kBlock + lane], rtz = rowtq[2 * kBlock + lane];
+    // sphere at slot p: torques from block K
+    auto put_torque = [&](int K, int p, float tx, float ty, float tz) {
+        if (tmask) {
+            if (tx == 0.0f && ty == 0.0f && tz == 0.0f) return;
+            if (p < n) atomicOr(tmask + (size_t)(K >> 5) * part_np + p, 1u << (K & 31));
+        }
+        float* o = part + (size_t)K * part_np + p + 3 * pplane;
+        __stcs(o, tx); __stcs(o + pplane, ty); __stcs(o + 2 * pplane, tz);
+    };
+    if (X == Y) {  // the same sphere: partners before it in slot order (row), after it (column)
+        const size_t o = (size_t)X * part_np + sAl;
+        __stcs(part + o, fmaf(ima, ax, -inv_mb * bsx));
+        __stcs(part + o + pplane, fmaf(ima, ay, -inv_mb * bsy));
+        __stcs(part + o + 2 * pplane, fmaf(ima, az, -inv_mb * bsz));
+        put_torque(X, sAl, rtx + ctx, rty + cty, rtz + ctz);
+    } else {
+        const size_t oa = (size_t)Y * part_np + sAl, ob = (size_t)X * part_np + sB;
+        __stcs(part + oa, ima * ax); __stcs(part + oa + pplane, ima * ay); __stcs(part + oa + 2 * pplane, ima * az);
+        __stcs(part + ob, -inv_mb * bsx);
+        __stcs(part + ob + pplane, -inv_mb * bsy);
+        __stcs(part + ob + 2 * pplane, -inv_mb * bsz);
+        put_torque(Y, sAl, rtx, rty, rtz);
+        put_torque(X, sB, ctx, cty, ctz);
+    }
+    __syncwarp();
 }
 
 template <bool WRITE>

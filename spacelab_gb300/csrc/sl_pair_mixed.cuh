@@ -1,6 +1,6 @@
-// sl_pair_mixed.cuh -- pair physics of the mixed-precision form: FP32
-// forces and torques on FP64 displacements and squared gaps, FP64 write-step
-// potential energy (ColliderSingleCore.cpp:104-253 term by term).  Shared by
+// sl_pair_mixed.cuh -- pair physics of the mixed-precision forms: FP32
+// forces and torques on displacements and squared gaps that the callers form in
+// FP64 or double-float, FP64 write-step potential energy (ColliderSingleCore.cpp:104-253 term by term).  Shared by
 // the all-pairs mixed kernels and the batched mixed solver.
 #pragma once
 #include "sl_device.cuh"

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kDriftThreads) drift_kernel(const __grid_const
 // One warp per lower-triangular 32x32 block tile (X, Y), X >= Y.  Lane b
 // owns sphere B = 32Y + b and walks the 32 spheres A = 32X + a of the A
 // block; on the diagonal only a > b is a pair.  Tiles are independent; one
-// launch covers the tiles of block columns [c0, c1) with a static stride.
+// launch covers the tiles of block columns [c0, c1), from a queue.
 // Tiles in column-major order: column Y holds tiles (Y..nb-1, Y); the first
 // tile of column c has index c*nb - c(c-1)/2.
 __device__ __forceinline__ long long col_offset(int nb, int c) { return (long long)c * nb - (long long)c * (c - 1) / 2; }
@@ -229,9 +229,6 @@ __global__ void __launch_bounds__(kRowThreads) rowsum_kernel(const __grid_consta
 // ------------------------------------------------------ energy totals -----
 constexpr int kRedThreads = 256;
 
-// Per-sphere KE, mom, ang_mom terms (:282-285) and the items' PE reduced over a
-// fixed tree: block b sums spheres [b*chunk, (b+1)*chunk) into red[b][0..6] and
-// its share of pe_tile into red[b][7].
 // Thread k < 8 holds total k of the reduction below; with them goes the status
 // word, final by now, so that the host needs no copy to see either.
 __device__ __forceinline__ void put_energy(const System& s, int k, double v)
@@ -240,6 +237,9 @@ __device__ __forceinline__ void put_energy(const System& s, int k, double v)
     if (k == 8 && s.host_status) *s.host_status = *s.status;
 }
 
+// Per-sphere KE, mom, ang_mom terms (:282-285) and the items' PE reduced over a
+// fixed tree: block b sums spheres [b*chunk, (b+1)*chunk) into red[b][0..6] and
+// its share of pe_tile into red[b][7].
 __global__ void __launch_bounds__(kRedThreads) energy_partial_kernel(const __grid_constant__ System s, int chunk)
 {
     pdl_next();

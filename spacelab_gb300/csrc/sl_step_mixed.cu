@@ -806,6 +806,9 @@ void launch_step_mixed(const System& s, bool write, int num_sms, cudaStream_t st
     const bool pdl = 4 * s.ntiles <= 7 * cap * kPairWarps;
     launch_drift(s, st, pdl);
     if (tm) cudaEventRecord(tm->ev[0], st);
+    // a dependent pair kernel up to one CTA per SM (us per step, dependent / plain:
+    // N=64 17.2 / 17.6, N=500 18.7 / 19.2, N=800 19.1 / 19.4, N=1000 20.4 / 19.8, N=1200
+    // 22.0 / 20.8, N=1500 24.1 / 21.2, N=2000 25.4 / 23.9; the same either way past that)
     if (s.pair_double)
         launch_pdl(pb <= num_sms, write ? mixed_pair2_kernel<true> : mixed_pair2_kernel<false>, pb, 32 * kPairWarps, 0, st, s);
     else

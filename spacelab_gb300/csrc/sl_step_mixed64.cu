@@ -350,6 +350,10 @@ void launch_step_mixed64(const System& s, bool write, int num_sms, cudaStream_t 
     const long long want = (s.ntiles + kM64Warps - 1) / kM64Warps;
     const long long cap = (long long)num_sms * kM64CtasPerSm;  // one wave of persistent warps
     const int pb = (int)(want < cap ? want : cap);
+    // a dependent launch up to one CTA per SM (us per step, dependent / plain: N=64
+    // 28.8 / 29.7, N=500 27.5 / 28.2, N=1000 30.0 / 30.2, N=1080 31.0 / 30.4, N=1200 31.2 /
+    // 32.1, N=1500 32.3 / 31.8, N=2000 35.4 / 35.2): a larger grid, placed while the
+    // drift still runs, is spread unevenly over the SMs
     launch_pdl(pb <= num_sms, write ? mixed64_pair_kernel<true> : mixed64_pair_kernel<false>, pb, 32 * kM64Warps, 0, st, s);
     if (tm) cudaEventRecord(tm->ev[1], st);
     // plainly: placed beside the pair kernel's last blocks, the finish blocks share

@@ -455,10 +455,10 @@ __device__ __forceinline__ void store_contacts(const System& s, int X, int Y, in
     }
 }
 
-// The first tile of T that is taken in strips.  A strip costs its share of a tile and ~12% more (its own blocks, and
-// a quarter of the marked pairs in a warp of their own), and pays where the
-// warps are not all busy to the end.  Of the 16 warps per SM that are
-// resident, with T tiles (us per step, GB300, no strips against these):
+// The first tile of T that is taken in strips.  A strip costs its share of a
+// tile and ~12% more (its own blocks, and a quarter of the marked pairs in a warp
+// of their own), and pays where the warps are not all busy to the end.  Of 16
+// warps per SM, with T tiles (us per step, GB300, no strips against these):
 //   - T up to half of them: all tiles.  The step is a warp's latency, 32 rows of
 //     ~1500 cycles.  N=96 65.5 -> 30.9, N=300 69.8 -> 34.8, N=1000 111 -> 85,
 //     N=1400 128 -> 115.
@@ -466,6 +466,9 @@ __device__ __forceinline__ void store_contacts(const System& s, int X, int Y, in
 //     N=1733 162 -> 152, N=3000 311 -> 305, N=5000 692.6 -> 688.5.
 //   - a last round that is nearly full without them: none.  N=2200 (99% full):
 //     199, 205 with them.
+// 16 is a tuned value: large plain steps have 20 warps per SM resident, and
+// counting those is no better (16 / 20: N=2400 269 / 272, N=3000 358 / 361, N=3500
+// 443 / 446, N=4000 551 / 547, N=5000 795 / 785, N=7000 the same).
 __host__ __device__ inline long long strip_from(long long tiles, int num_sms)
 {
     const long long warps = 16LL * num_sms;
