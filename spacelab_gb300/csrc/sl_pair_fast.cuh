@@ -270,7 +270,7 @@ SL_PF_FN Sig vdw_coef(const Sig& P, double num, double S, double T, Flags& fl)
 struct Sphere {
     double R;
     Sig sR;             // unpacked R
-    double cR3;         // A only: ((Ha/6 64) R) R R; its sign is the force's
+    double cR3;         // A only: ((Ha/6 64) R) R R
     u64 rm;
     int em;
 };
@@ -309,10 +309,11 @@ struct Pair {
 // overlap is valid whenever `fl` is sure (contact: overlap > 0).
 //
 // ZEROS: a component of r may be zero (spheres in a plane or on a grid), and cR3
-// (no cohesion).  A zero's square and force are zeros, the force's with its
-// sign; a one takes its place in the operations, and says nothing.  Without it a
-// zero component raises the range flag.  It costs some thirty instructions a
-// pair, so the tiles take it only where they meet such pairs.
+// zero (no cohesion) or negative (repulsion); it is positive otherwise.  A zero's
+// square and force are zeros, the force's with its sign; a one takes its place in
+// the operations, and says nothing.  Without it a zero component raises the range
+// flag.  It costs some thirty instructions a pair, so the tiles take it only where
+// they meet such pairs.
 template <bool UNI, bool ZEROS = false>
 SL_PF_FN Pair pair_terms(double rx, double ry, double rz, const Sphere& A, const Sphere& B, const Uniform& u,
                          long long h_min_bits)
@@ -354,8 +355,8 @@ SL_PF_FN Pair pair_terms(double rx, double ry, double rz, const Sphere& A, const
         P = mul(mul(mul(none ? one : unpack(A.cR3), B.sR, fl), B.sR, fl), B.sR, fl);
     }
     const Sig coef = vdw_coef(P, o.h + A.R + B.R, S, T, fl);           // :221-225
-    // the significands hold magnitudes: a negative Ha (repulsion) turns the signs
-    const uint32_t csign = (uint32_t)(bits_of(A.cR3) >> 32) & 0x80000000u;
+    // the significands hold magnitudes: a negative cR3 turns the signs
+    const uint32_t csign = ZEROS ? (uint32_t)(bits_of(A.cR3) >> 32) & 0x80000000u : 0u;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const uint32_t sign = ((uint32_t)(bits_of(r[c]) >> 32) & 0x80000000u) ^ csign;

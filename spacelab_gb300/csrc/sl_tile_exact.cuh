@@ -340,8 +340,8 @@ __device__ __forceinline__ pf::Uniform tile_uniform(const ABlock& ab)
 
 // The sweep in the ZEROS form, out of line, so that the plain one's code stays as
 // it is.  Systems that need it throughout (us per step, the general path for
-// every such pair / here): in a plane N=1000 228 / 118, N=5000 2832 / 987; no
-// cohesion N=1000 278 / 125, N=5000 3888 / 1039; a cubic lattice N=5000 1426 / 947.
+// every such pair / here): in a plane N=1000 228 / 118, N=5000 2832 / 984; no
+// cohesion N=1000 278 / 125, N=5000 3888 / 1036; a cubic lattice N=5000 1426 / 943.
 struct Swept {
     double pe;
     uint32_t marked, near;
@@ -379,28 +379,32 @@ __device__ __forceinline__ void tile_pairs(const System& s, TileScratch& ws, int
     const pf::Sphere sb = column_sphere(s, iB);
     const bool areal = X * kBlock + lane < s.n;  // padding takes no part in a pair
     const pf::Sphere sa{ab.R[lane], pf::unpack(ab.R[lane]), ab.cR3[lane], 0, pf::unpack(ab.m[lane]).e};
-    const bool cohesive = !pf::is_zero(s.mat.Ha);  // cR3 = 0 otherwise
-    const bool sane = __all_sync(0xffffffffu, (!areal || (pf::in_range(sa) && (!cohesive || pf::in_range_cR3(sa.cR3)))) &&
-                                                  (!bvalid || pf::in_range(sb)));
+    // fit: the constants are in the integer path's range.  special: the tile takes
+    // the ZEROS form of the sweep -- without cohesion or with repulsion, or where the
+    // last row meets a zero displacement component (spheres in a plane or on a grid).
+    // Either form is right for any row: a pair that the plain one does not settle
+    // takes the general path.  One row stands for the tile because a vote in every
+    // row cost the other systems up to 9% (N=5000, host step 705 -> 769 us), and one
+    // vote covers both questions (two, and the force's sign in the plain form: 709;
+    // this 705).
+    const bool cohesive = s.mat.Ha > 0;
+    const int last = max(a1 - 1, 0);
+    const bool fit = (!areal || (pf::in_range(sa) && (pf::is_zero(s.mat.Ha) || pf::in_range_cR3(sa.cR3)))) &&
+                     (!bvalid || pf::in_range(sb));
+    const bool special = !cohesive || (bvalid && (X != Y || lane < last) &&
+                                       (pf::equal(bx, ab.x[last]) || pf::equal(by, ab.y[last]) ||
+                                        pf::equal(bz, ab.z[last])));
+    const bool plain = __all_sync(0xffffffffu, fit && !special);
     // equality on the bit patterns (R, m > 0)
     const auto same = [](double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); };
     const double R0 = ab.R[0], m0 = ab.m[0];
     const bool uni = __all_sync(0xffffffffu, (!areal || (same(sa.R, R0) && same(ab.m[lane], m0))) &&
                                                  (!bvalid || (same(Rb, R0) && same(mb, m0))));
-    // The ZEROS form: without cohesion, or where the last row meets a zero
-    // displacement component (spheres in a plane or on a grid).  Either form is
-    // right for any row: a pair that the plain one does not settle takes the general
-    // path.  One row stands for the tile because a vote in every row cost the other
-    // systems up to 9% (N=5000, host step 705 -> 769 us; 709 here).
-    const int last = max(a1 - 1, 0);
-    const bool odd = __any_sync(0xffffffffu, !cohesive || (bvalid && (X != Y || lane < last) &&
-                                                           (pf::equal(bx, ab.x[last]) || pf::equal(by, ab.y[last]) ||
-                                                            pf::equal(bz, ab.z[last]))));
     uint32_t marked = 0, near = 0;
-    if (!sane) {
+    if (!plain && !__all_sync(0xffffffffu, fit)) {
         const uint32_t all = (a1 >= 32 ? ~0u : (1u << a1) - 1u) & ~((1u << a0) - 1u);
         marked = bvalid ? (X != Y ? all : all & ~((2u << lane) - 1u)) : 0u;
-    } else if (odd) {
+    } else if (!plain) {
         const Swept o = uni ? sweep_zeros<PE, true>(s, ws, X, Y, a0, a1) : sweep_zeros<PE, false>(s, ws, X, Y, a0, a1);
         pe += o.pe;
         marked = o.marked;

@@ -1,7 +1,7 @@
-// Host check of the exact pair force's integer path (sl_pair_fast.cuh) for
-// vdW coefficients of both signs and, in the ZEROS form, zero coefficients and
-// displacement components: unflagged results against the reference's
-// expressions in IEEE doubles, signs of zeros too.  Prints "<case> <cases> <flagged>" and
+// Host check of the exact pair force's integer path (sl_pair_fast.cuh) in its
+// ZEROS form: vdW coefficients of both signs and zero, and zero displacement
+// components.  Unflagged results against the reference's expressions in IEEE
+// doubles, signs of zeros too.  Prints "<case> <cases> <flagged>" and
 // "mismatches N".
 #include "sl_pair_fast.cuh"
 
@@ -74,12 +74,6 @@ struct Count {
 };
 
 template <bool UNI>
-static Pair plain(const double r[3], const Sphere& A, const Sphere& B, const Uniform& un, long long hm)
-{
-    return pair_terms<UNI>(r[0], r[1], r[2], A, B, un, hm);
-}
-
-template <bool UNI>
 static Pair zeros(const double r[3], const Sphere& A, const Sphere& B, const Uniform& un, long long hm)
 {
     return pair_terms<UNI, true>(r[0], r[1], r[2], A, B, un, hm);
@@ -96,11 +90,10 @@ int main(int argc, char** argv)
         const double ma = number(-40, -38, false), mb = uni ? ma : number(-40, -38, false);
         double r[3];
         for (double& x : r) x = number(sc + 1, sc + 6, rng() & 1);
-        repulsion.add(uni ? check(plain<true>, r, Ra, Rb, ma, mb, number(-100, -70, true))
-                          : check(plain<false>, r, Ra, Rb, ma, mb, number(-100, -70, true)));
         const auto care = [&](const double* d, double cR3) {
             return uni ? check(zeros<true>, d, Ra, Rb, ma, mb, cR3) : check(zeros<false>, d, Ra, Rb, ma, mb, cR3);
         };
+        repulsion.add(care(r, number(-100, -70, true)));
         const double nil = rng() & 1 ? 0.0 : -0.0;
         no_cohesion.add(care(r, nil));
         const int c = (int)(rng() % 3);
