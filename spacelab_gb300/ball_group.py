@@ -24,8 +24,8 @@ import numpy as np
 from . import _lib
 from ._lib import Energy, Material, SpaceLabError, check, dptr
 
-# "mixed": FP32 force/torque arithmetic with FP64 displacements, close-pair
-# overlaps and accumulation; "mixed_df": the double-float variant
+# "mixed": FP32 force/torque arithmetic with displacements, close-pair overlaps
+# and accumulation to FP64's precision; "mixed_df": the double-float variant
 MODES = {"exact": _lib.SL_MODE_EXACT, "mixed": _lib.SL_MODE_MIXED, "mixed_df": _lib.SL_MODE_MIXED_DF}
 
 

@@ -25,9 +25,9 @@
 // r and the FP64 overlap: the vdW coefficient, elastic, gravity, sliding and
 // rolling friction and the torques, in lengths scaled by 2^-len_shift.
 //
-// What bounds it (ncu, N=9000): the FP32 pipe, then at 72% beside issue at 68%;
-// half of its work are the six error-free sums, and the two spheres' sums of a
-// component are added in packed arithmetic.  On the FP64 pipe the subtraction
+// What bounds it (ncu, N=9000): the FP32 pipe at 75%, beside issue at 71%; nearly
+// half of its work are the six error-free sums, the two spheres' of a component
+// added in packed arithmetic.  On the FP64 pipe the subtraction
 // and the sums were 9 adds a pair at 19 SM-cycles each (one narrow unit per SM),
 // 171 cycles for a warp's 32 pairs, at 0.96 of that unit's rate; now it is some
 // 60.  N=20000 polydisperse, 20 steps: 74.2 -> 23.1 ms with the subtraction to
