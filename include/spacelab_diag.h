@@ -69,10 +69,12 @@ int sl_diag_batch_refuse_lockstep(sl_batch* b);
  *   SL_DIAG_MLP_SLOW_PAGE  the next prediction in place ends as if a page of host
  *                          memory had taken longer than the kernel waits;
  *   SL_DIAG_MLP_LAUNCH     the launch of the next prediction is rejected;
- *   SL_DIAG_MLP_TIMED_OUT  the network is left as by a call whose wait ran out. */
+ *   SL_DIAG_MLP_TIMED_OUT  the network is left as by a call whose wait ran out;
+ *   SL_DIAG_MLP_SETUP      the set-up of the next layer's product fails. */
 #define SL_DIAG_MLP_SLOW_PAGE 1
 #define SL_DIAG_MLP_LAUNCH 2
 #define SL_DIAG_MLP_TIMED_OUT 3
+#define SL_DIAG_MLP_SETUP 4
 int sl_diag_mlp_fail(sl_mlp* m, int what);
 
 #ifdef __cplusplus

@@ -963,8 +963,11 @@ void forward(sl_mlp* h, const BatchInput& in, int M, bool train, cudaStream_t st
         } else if (l == 1) {
             L.bump = in.step;  // from here on *step is the step after this one
         }
-        ok = ok && launch_gemm(L, st);
-        if (!ok) h->tc_setup_failed = true;
+        ok = ok && h->fail_next != SL_DIAG_MLP_SETUP && launch_gemm(L, st);
+        if (!ok) {
+            h->tc_setup_failed = true;
+            h->fail_next = 0;
+        }
     }
 }
 
@@ -1334,10 +1337,14 @@ int sl_mlp_train(sl_mlp* h, const float* x, const float* y, int n, int epochs, i
         backward(h, in, batch, st);
         sl::launch_pdl(true, adam_kernel, (int)((h->nparam + 255) / 256), 256, 0, st, h->P, h->G, h->Mom, h->Var, h->Pb,
                        h->Wt, h->at, h->nl, h->mask, (int)h->nparam, lr, b1, b2, eps, dcoef, dstep, -1);
-        ok = cudaStreamEndCapture(st, &graph) == cudaSuccess && cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
+        // a step without one of its products must not run: Adam would take the gradients that are there
+        ok = cudaStreamEndCapture(st, &graph) == cudaSuccess && !h->tc_setup_failed &&
+             cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess;
     }
     if (graph) cudaGraphDestroy(graph);
-    int rc = ok ? SL_OK : sl_record_error(SL_ERR_CUDA, "sl_mlp_train: the step's graph could not be made");
+    int rc = ok                   ? SL_OK
+             : h->tc_setup_failed ? mlp_status(h, "sl_mlp_train")
+                                  : sl_record_error(SL_ERR_CUDA, "sl_mlp_train: the step's graph could not be made");
 
     std::vector<float> part((size_t)seg * nb);
     std::vector<float2> coef(seg);
@@ -1432,7 +1439,7 @@ int sl_mlp_predict(sl_mlp* h, const float* x, int n, float* y)
 
 extern "C" int sl_diag_mlp_fail(sl_mlp* h, int what)
 {
-    if (!h || what < 0 || what > SL_DIAG_MLP_TIMED_OUT) return sl_record_error(SL_ERR_ARG, "sl_diag_mlp_fail: bad argument");
+    if (!h || what < 0 || what > SL_DIAG_MLP_SETUP) return sl_record_error(SL_ERR_ARG, "sl_diag_mlp_fail: bad argument");
     if (what == SL_DIAG_MLP_TIMED_OUT)
         *h->err = 1;
     else

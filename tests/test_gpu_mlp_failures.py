@@ -1,7 +1,7 @@
 """A surrogate call that goes wrong is reported or done another way, and the
 next one does not suffer from it: a prediction in place that meets a slow page
 of host memory, a rejected launch, a call whose wait ran out.  The failures are
-made on the host (sl_diag_mlp_fail); results bit for bit those of an untroubled
+made on the host (sl_diag_mlp_fail), as is a product that cannot be set up; results bit for bit those of an untroubled
 call."""
 import numpy as np
 import pytest
@@ -12,7 +12,7 @@ from spacelab_gb300._lib import check
 
 pytestmark = pytest.mark.gpu
 
-SLOW_PAGE, LAUNCH, TIMED_OUT = 1, 2, 3
+SLOW_PAGE, LAUNCH, TIMED_OUT, SETUP = 1, 2, 3, 4
 
 
 @pytest.fixture(scope="module")
@@ -55,3 +55,17 @@ def test_calls_after_one_that_timed_out(net):
     assert l2 == loss and np.array_equal(g2, grads)
     _fail(net, TIMED_OUT)
     assert np.isfinite(net.train(x, y, epochs=1, batch=32)).all()
+
+
+def test_training_without_a_product_changes_nothing():
+    x, y = _x(64), _x(64)[:, :4]
+    a, b = (S.Mlp(8, 4, 64, 2, max_batch=128, seed=5) for _ in range(2))
+    a.gradients(x, y)  # gradients that a step must not take
+    before = a.params()
+    _fail(a, SETUP)
+    with pytest.raises(_lib.SpaceLabError) as err:
+        a.train(x, y, epochs=1, batch=32)
+    assert err.value.code == _lib.SL_ERR_CUDA
+    assert np.array_equal(a.params(), before)
+    assert np.array_equal(a.train(x, y, epochs=2, batch=32), b.train(x, y, epochs=2, batch=32))
+    assert np.array_equal(a.params(), b.params())
