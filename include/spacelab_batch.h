@@ -27,7 +27,10 @@ extern "C" {
 
 typedef struct sl_batch sl_batch;
 
-/* Allocate a batch for `steps` steps with an energy record every `skip`. */
+/* Allocate a batch for `steps` steps with an energy record every `skip`.  The
+ * pair-tile pass's buffers take up to 48 GB and a third of the free device memory,
+ * less where the batch's own memory needs it; without them the pass is slower or
+ * (exact form) not offered. */
 int sl_batch_create(int ninst, const int* counts, const sl_material* mat, int mode, int steps, int skip,
                     sl_batch** out);
 int sl_batch_destroy(sl_batch* b);
