@@ -33,6 +33,7 @@
 #include "sl_tma.cuh"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -511,6 +512,11 @@ constexpr int kFwXBytes = kFwRows * kFwMaxWidth * 2, kFwWBytes = kFwTileN * kTcK
 constexpr int kFwThreads = 192, kFwEpilogue = 128;
 constexpr int kFwSmem = kFwXBytes + kFwStages * kFwWBytes + 256;  // + barriers, TMEM address, failure flag
 
+// Row tiles of n rows, for any n; a tile's last row fits an int too
+__host__ __device__ constexpr int fw_tiles(int n) { return n / kFwRows + (n % kFwRows != 0); }
+static_assert(fw_tiles(1) == 1 && fw_tiles(kFwRows) == 1 && fw_tiles(kFwRows + 1) == 2, "row tiles");
+static_assert(fw_tiles(INT_MAX) == 1 << 24, "row tiles of the largest prediction");
+
 struct FwNet {
     CUtensorMap w[kFwMaxLayers];            // weights [dout][din], boxes of 64 x 128
     const float* bias[kFwMaxLayers];
@@ -549,7 +555,7 @@ __global__ void __launch_bounds__(kFwThreads, 2) mlp_forward_kernel(const __grid
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
     volatile int* failed = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ntiles = (n + kFwRows - 1) / kFwRows;
+    const int ntiles = fw_tiles(n);
     // whole 16-byte groups of the caller's rows
     const bool vec_in = net.n_in % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     const bool vec_out = net.n_out % 4 == 0 && (reinterpret_cast<uintptr_t>(y) & 15u) == 0;
@@ -1050,7 +1056,7 @@ cudaError_t forward_fused(sl_mlp* h, const float* x, float* y, int n, cudaStream
         smem = size_t(1) << 20;
         h->fail_next = 0;
     }
-    const int tiles = n / kFwRows + (n % kFwRows != 0);
+    const int tiles = fw_tiles(n);
     e = sl::launch_pdl(false, mlp_forward_kernel, (unsigned)std::min(tiles, 2 * h->num_sms), kFwThreads, smem, st, h->net,
                        x, y, n, h->err);
     if (e != cudaSuccess) cudaGetLastError();
