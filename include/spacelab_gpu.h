@@ -203,7 +203,9 @@ int sl_step_launches(const sl_handle* h, int write, int* count);
 /* Name of the pair kernel the handle's steps launch: "pair_tile_kernel"
  * (exact mode), "mixed64_pair_kernel" (SL_MODE_MIXED), "mixed_pair_kernel"
  * or, for large systems, "mixed_pair2_kernel" (two column blocks per work
- * item; SL_MODE_MIXED_DF).  The string is static. */
+ * item; SL_MODE_MIXED_DF).  "mixed_pair_kernel" names the one-column form in
+ * both its kernels: small systems and write steps launch the one that lists
+ * the close pairs, mixed_pair_listed_kernel.  The string is static. */
 int sl_pair_kernel(const sl_handle* h, const char** name);
 
 /* Per-kernel timing: when enabled, every step records CUDA events around
